@@ -2,6 +2,7 @@
 // (design-variable, worst-case and MMA entry points live in design.cu,
 // worst.cu and mma.cu.)
 #include "rso_internal.cuh"
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -167,11 +168,12 @@ static rso_status setup(rso_handle* h, int ex, int ey, int ez, const uint8_t* em
     h->xfer_n = xf;
   }
   {
-    // one partial per CTA of the fine operator kernels: 31 x 7 nodes per
-    // z-chunk of 32 planes (FP64), 31 x 3 or 31 x 7 (packed FP32, 2 or 4 rows)
+    // one partial per CTA of the fine operator kernels: 31 x 7 nodes and at
+    // least kFineZc64Min planes (FP64), or the smallest packed FP32 tile, 31 x 3
+    // nodes (2 thread rows) and kFineZcMin planes
     const Level& f0 = h->L[0];
-    // the smallest fine-kernel tile: 2 thread rows (3 new element rows), z chunks of kFineZcMin planes
-    h->fpart_n = (long long)cdiv(f0.nx, 31) * cdiv(f0.ny, 3) * cdiv(f0.nz, kFineZcMin);
+    h->fpart_n = (long long)cdiv(f0.nx, 31) * std::max((long long)cdiv(f0.ny, 3) * cdiv(f0.nz, kFineZcMin),
+                                                       (long long)cdiv(f0.ny, 7) * cdiv(f0.nz, kFineZc64Min));
     ALLOC(h->fpart, sizeof(double) * h->fpart_n);
   }
   // per-level buffers

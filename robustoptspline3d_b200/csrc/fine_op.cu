@@ -14,6 +14,7 @@
 // handled from the node-class byte.  The point Gauss-Seidel colour sweep and
 // the first Jacobi sweep from a zero iterate use K0 directly.
 #include "rso_internal.cuh"
+#include <algorithm>
 #include <cmath>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -71,11 +72,9 @@ rso_status penalise(rso_handle* h) {
 // Structural zeros (exact for the isotropic cube; checked on the host):
 // for one-bit c the translation row/column (c >> i & 1), for two-bit c the
 // entries coupling the axis outside c with the two inside it.
-__constant__ double cBd[72];  // [c][i][j]
-__constant__ float cBf[72];
 __constant__ double cD0d[9];  // diagonal 3x3 block of local node 0
 __constant__ float cD0f[9];
-// The packed FP32 kernel uses the blocks' finer structure (the isotropic
+// The kernels use the blocks' finer structure (the isotropic
 // material and the cube's rotations; checked on the host): with
 //   A0, B0, A7, B7 the diagonal and off-diagonal entries of blocks 0 and 7
 //   (full 3 x 3, a I + b (J - I)), P, Q those of the one-bit blocks
@@ -85,14 +84,13 @@ __constant__ float cD0f[9];
 // and the node-0 diagonal block D0 = [[Da, Db, Db], [Db, Da, Db], [Db, Db, Da]],
 // cWp holds, duplicated into both lanes: A0 - B0, B0, A7 - B7, B7, P, Q, R, S, Da, Db.
 __constant__ float2 cWp[10];
+__constant__ double cWd[10];  // the same ten in FP64, for the FP64 kernel
 enum { W_A0 = 0, W_B0, W_A7, W_B7, W_P, W_Q, W_R, W_S, W_DA, W_DB };
 
 template <typename T>
-__device__ __forceinline__ T bw(int i);
+__device__ __forceinline__ T ws(int i);
 template <>
-__device__ __forceinline__ double bw<double>(int i) { return cBd[i]; }
-template <>
-__device__ __forceinline__ float bw<float>(int i) { return cBf[i]; }
+__device__ __forceinline__ double ws<double>(int i) { return cWd[i]; }
 template <typename T>
 __device__ __forceinline__ T d0(int i);
 template <>
@@ -149,11 +147,8 @@ rso_status upload_walsh(rso_handle* h) {
           return RSO_ERR_INVALID_ARG;
         }
       }
-  float Bf[72], Df[9];
-  for (int i = 0; i < 72; i++) Bf[i] = (float)B[i];
+  float Df[9];
   for (int i = 0; i < 9; i++) Df[i] = (float)D0[i];
-  RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cBd, B, sizeof(B), 0, cudaMemcpyHostToDevice, h->stream));
-  RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cBf, Bf, sizeof(Bf), 0, cudaMemcpyHostToDevice, h->stream));
   RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cD0d, D0, sizeof(D0), 0, cudaMemcpyHostToDevice, h->stream));
   RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cD0f, Df, sizeof(Df), 0, cudaMemcpyHostToDevice, h->stream));
   // the finer structure the packed kernel relies on (see cWp)
@@ -184,13 +179,14 @@ rso_status upload_walsh(rso_handle* h) {
   float2 Wp[10];
   for (int i = 0; i < 10; i++) Wp[i] = make_float2((float)Wv[i], (float)Wv[i]);
   RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cWp, Wp, sizeof(Wp), 0, cudaMemcpyHostToDevice, h->stream));
+  RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cWd, Wv, sizeof(Wv), 0, cudaMemcpyHostToDevice, h->stream));
   // the host copies are stack arrays: finish the copies before returning
   RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
   return RSO_OK;
 }
 
 // Residual / apply / damped-Jacobi kernel.  A CTA of 32 x TY threads marches
-// along z through FZC node planes.  Thread (tx, ty) owns the element column
+// along z through fzc node planes (march_zc's rule).  Thread (tx, ty) owns the element column
 // (ex, ey) = (x0 - 1 + tx, y0 - 1 + ty) and the node (ex + 1, ey + 1), so a
 // CTA computes 32 x TY element columns and writes the 31 x (TY - 1) nodes
 // whose four surrounding columns it holds.  Per element layer z (between node
@@ -205,7 +201,7 @@ rso_status upload_walsh(rso_handle* h) {
 //      corners of its 4 columns through shared memory.
 // Node planes of u (3 components, 33 x (TY+1)) and element layers of rho^p are
 // staged with cp.async WPD stages ahead in WNSLOT slots.
-constexpr int WTX = 32, FZC = 32, WPD = 2, WNSLOT = 4;
+constexpr int WTX = 32, WPD = 2, WNSLOT = 4;
 static_assert((WNSLOT & (WNSLOT - 1)) == 0, "slot indices are masks of the stage number");
 
 template <typename T, int TY>
@@ -224,7 +220,7 @@ template <typename T, int MODE, int TY, bool RR = false>
 __global__ void __launch_bounds__(WTX* TY, sizeof(T) == 8 ? 2 : 3)
     k_fine_w(const Level L, const T* __restrict__ u, const T* __restrict__ f, T* __restrict__ out,
              const T* __restrict__ rp, T omega, double* __restrict__ dotp, const T* __restrict__ uprev,
-             T c1, float* __restrict__ out32) {
+             T c1, int fzc, float* __restrict__ out32) {
   // Staged rows are 16-byte aligned windows of RX entries starting at the
   // tile's first padded x index rounded down to a multiple of 4 (ox = offset
   // of the tile inside the window), copied in 16-byte chunks.
@@ -237,8 +233,8 @@ __global__ void __launch_bounds__(WTX* TY, sizeof(T) == 8 ? 2 : 3)
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * WTX + tx;
   const int x0 = blockIdx.x * (WTX - 1), y0 = blockIdx.y * (TY - 1);
   // blockIdx.z = z chunk + (number of chunks) * system; systems share rho^p
-  const int nzc = (L.nz + FZC - 1) / FZC, bsys = blockIdx.z / nzc;
-  const int z0 = (blockIdx.z - bsys * nzc) * FZC, z1 = min(z0 + FZC, L.nz);
+  const int nzc = (L.nz + fzc - 1) / fzc, bsys = blockIdx.z / nzc;
+  const int z0 = (blockIdx.z - bsys * nzc) * fzc, z1 = min(z0 + fzc, L.nz);
   {
     const long long off = (long long)bsys * 3 * L.NP;
     u += off;
@@ -415,24 +411,35 @@ __global__ void __launch_bounds__(WTX* TY, sizeof(T) == 8 ? 2 : 3)
           F[q][c] = Fn[q][c];
         }
     }
-    // blocks of B, in place (block c maps its three entries onto themselves), times rho^p
+    // rho^p B in place, in the structure of cWp (as the packed kernel: block c
+    // maps v[c ^ (1 << j)][j] to v[c ^ (1 << i)][i]): 51 operations
     const int ri = ty * RX + tx + ox;
     const T re = sr[ri];
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      T in[3], o[3];
-#pragma unroll
-      for (int j = 0; j < 3; j++) in[j] = v[c ^ (1 << j)][j];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        T s = T(0);
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-          if (!b_zero(c, i, j)) s = fma(bw<T>(c * 9 + i * 3 + j), in[j], s);
-        o[i] = s * re;
-      }
-#pragma unroll
-      for (int i = 0; i < 3; i++) v[c ^ (1 << i)][i] = o[i];
+    {
+      auto full = [&](T& a, T& b, T& c, T ab, T bb) {  // o_i = rho ((A - B) in_i + B (in_0 + in_1 + in_2))
+        const T w = bb * (a + b + c);
+        a = re * fma(ab, a, w);
+        b = re * fma(ab, b, w);
+        c = re * fma(ab, c, w);
+      };
+      auto pair = [&](T& a, T& b) {  // rho [[P, Q], [Q, P]]
+        const T o = re * fma(ws<T>(W_Q), b, ws<T>(W_P) * a);
+        b = re * fma(ws<T>(W_Q), a, ws<T>(W_P) * b);
+        a = o;
+      };
+      auto both = [&](T& a, T& b, T& c) {  // rho R (a + b) on the two axes in c, rho S on the other
+        a = b = re * (ws<T>(W_R) * (a + b));
+        c = re * (ws<T>(W_S) * c);
+      };
+      full(v[1][0], v[2][1], v[4][2], ws<T>(W_A0), ws<T>(W_B0));
+      full(v[6][0], v[5][1], v[3][2], ws<T>(W_A7), ws<T>(W_B7));
+      pair(v[3][1], v[5][2]);
+      pair(v[3][0], v[6][2]);
+      pair(v[5][0], v[6][1]);
+      both(v[2][0], v[1][1], v[7][2]);
+      both(v[4][0], v[1][2], v[7][1]);
+      both(v[4][1], v[2][2], v[7][0]);
+      v[0][0] = v[0][1] = v[0][2] = T(0);
     }
     if (MODE == 2) {
 #pragma unroll
@@ -1180,8 +1187,32 @@ __global__ void __launch_bounds__(256) k_fine_gs(const Level L, T* __restrict__ 
 
 static inline dim3 plane_grid(const Level& l) { return dim3(cdiv(l.nx, 32), cdiv(l.ny, 8), l.nz * l.nb); }
 constexpr int WTY = 8;
+// Node planes per z chunk of the FP64 kernel.  A CTA walks its chunk plane by
+// plane, one plane's latency after the other, and pays about two more planes
+// for the layer below the chunk and the first staged copies; 2 CTAs fit an SM.
+// So a chunk length costs what is larger: the planes of all CTAs spread over
+// the resident slots, or, for grids of few waves, the waves one after another.
+// The cheapest of 2 to 32 planes is taken: short chunks where long ones leave
+// SMs idle, 32 planes once the grid fills the GPU by itself.  Against 32 planes
+// always: 64 x 32 x 32 elements K u 43 -> 12 us, Jacobi step 77 -> 15 us;
+// 120 x 101 x 93 the Jacobi step 115 -> 71 us; 256^3 keeps 32 planes (the
+// residual 541 -> 436 us there is the 51-operation form of the blocks).
+static int march_zc(const Level& l) {
+  const double slots = 2.0 * 148.0;
+  const long long cols = (long long)cdiv(l.nx, WTX - 1) * cdiv(l.ny, WTY - 1) * l.nb;
+  int best = kFineZcMax;
+  double least = 1e300;
+  for (int zc = kFineZcMax; zc >= kFineZc64Min; zc /= 2) {
+    const long long nzc = cdiv(l.nz, zc), ctas = cols * nzc;
+    const double spread = (double)cols * (double)(l.nz + 2 * nzc) / slots;
+    const double waves = (double)cdiv(ctas, (long long)slots) * (std::min(zc, l.nz) + 2);
+    const double cost = ctas <= 3 * (long long)slots ? waves : spread;
+    if (cost < least) { least = cost; best = zc; }
+  }
+  return best;
+}
 static inline dim3 march_grid(const Level& l) {
-  return dim3(cdiv(l.nx, WTX - 1), cdiv(l.ny, WTY - 1), cdiv(l.nz, FZC) * l.nb);
+  return dim3(cdiv(l.nx, WTX - 1), cdiv(l.ny, WTY - 1), cdiv(l.nz, march_zc(l)) * l.nb);
 }
 constexpr bool kPairTMA = true;  // packed kernel stages with TMA (else cp.async)
 // thread rows pty of the packed FP32 kernel (2 pty element rows; rso_autotune picks 2 or 4)
@@ -1356,11 +1387,11 @@ static rso_status launch_fine(rso_handle* h, const T* u, const T* f, T* out, con
   } else {
     if (h->prof_on) prof_begin(h, cls, (double)l.nn);
     if (MODE == 0 && out32 != nullptr)
-      k_fine_w<T, MODE, WTY, true><<<march_grid(l), dim3(WTX, WTY), smem, h->stream>>>(l, u, f, out, rp, (T)omega,
-                                                                                       dotp, uprev, (T)c1, out32);
+      k_fine_w<T, MODE, WTY, true><<<march_grid(l), dim3(WTX, WTY), smem, h->stream>>>(
+          l, u, f, out, rp, (T)omega, dotp, uprev, (T)c1, march_zc(l), out32);
     else
       k_fine_w<T, MODE, WTY><<<march_grid(l), dim3(WTX, WTY), smem, h->stream>>>(
-          l, u, f, out, rp, (T)omega, MODE == 0 ? nullptr : dotp, uprev, (T)c1, nullptr);
+          l, u, f, out, rp, (T)omega, MODE == 0 ? nullptr : dotp, uprev, (T)c1, march_zc(l), nullptr);
   }
   rso::note_launch();
   if (h->prof_on) prof_end(h, cls);

@@ -227,6 +227,8 @@ void vcycle_graphs_free(rso_handle* h);
 void solve_graphs_free(rso_handle* h);
 // node planes per z chunk of the packed FP32 fine kernel (fine_op.cu)
 constexpr int kFineZcMax = 32, kFineZcMin = 4;
+// and the shortest chunk of the FP64 one
+constexpr int kFineZc64Min = 2;
 int fine_zc(const rso_handle* h);
 // kernel variant of a coarse level: 0 per node, 1 per (node, row), 2 nine threads per node (coarse_op.cu)
 int coarse_variant_of(const rso_handle* h, int level);

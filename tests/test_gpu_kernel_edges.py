@@ -1,0 +1,26 @@
+"""Kernels and dispatch rules at the sizes where they can go wrong (edges of tiles and chunks,
+remainders, the smallest and largest of a range), against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import problems as P
+from test_gpu_00_parity import make, rel, t
+
+pytestmark = pytest.mark.gpu
+
+
+# node boxes one short of, on and one past the 31 x 7 tile, and depths that give z chunks of
+# 2, 4, 8, 16 and 32 planes with full and ragged last chunks
+@pytest.mark.parametrize("dims", [(3, 2, 1), (30, 6, 1), (31, 7, 2), (29, 5, 41), (62, 41, 70), (93, 97, 65),
+                                  (130, 118, 96)])
+def test_fine_fp64_chunks(oracle, cuda, dims):
+    """FP64 K u, residual and damped Jacobi step; 1e-12 relative, the bound of the FP64 operator pieces."""
+    g, o = make(oracle, P.cantilever(*dims), n_levels=2 if dims[0] < 40 else 0, first_factor=2 if dims[0] < 40 else 4)
+    rng = np.random.default_rng(7)
+    fix = np.tile((o.node_class() & 4) > 0, 3)
+    u, f = (np.where(fix, 0.0, rng.standard_normal(3 * o.nn)) for _ in range(2))
+    assert rel(g.applyK(t(u, cuda)).cpu().numpy(), o.apply_K(u)) < 1e-12
+    assert rel(g.update_residual(t(u, cuda), t(f, cuda)).cpu().numpy(), o.residual(u, f)) < 1e-12
+    g.update_stencil()
+    jac = g.gs_relax(0, t(u, cuda), t(f, cuda), kind=1, omega=0.3).cpu().numpy()
+    assert rel(jac, o.smooth(0, u, f, kind=1, omega=0.3, sweeps=1)) < 1e-12
