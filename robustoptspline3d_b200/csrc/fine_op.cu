@@ -1111,29 +1111,36 @@ __global__ void __launch_bounds__(256) k_fine_jacobi0_v4(const Level L, const fl
     *reinterpret_cast<float4*>(out + p0 + c * NP) = make_float4(o[c][0], o[c][1], o[c][2], o[c][3]);
 }
 
-// one colour of the 8-colour point Gauss-Seidel sweep (in place)
+// One colour of the 8-colour point Gauss-Seidel sweep (in place).  A CTA takes
+// 128 consecutive nodes of the colour, x fastest (a colour's rows are half the
+// box's, so a tile of fixed width would leave lanes idle at their ends).  The
+// launches overlap (launch_pdl): node class and rho^p load under the previous
+// colour.
+constexpr int FGS = 128;
 template <typename T>
-__global__ void __launch_bounds__(256) k_fine_gs(const Level L, T* __restrict__ u, const T* __restrict__ f,
-                                                 const T* __restrict__ rp, int cx, int cy, int cz, int rev) {
-  const int x = 2 * (blockIdx.x * 32 + threadIdx.x) + cx;
-  const int y = 2 * (blockIdx.y * 8 + threadIdx.y) + cy;
-  const int z = 2 * blockIdx.z + cz;
-  if (x >= L.nx || y >= L.ny || z >= L.nz) return;
+__global__ void __launch_bounds__(FGS) k_fine_gs(const Level L, T* u, const T* f, const T* __restrict__ rp, int cx,
+                                                 int cy, int cz, int nxc, int nyc, int ntot, int rev) {
+  const unsigned i = blockIdx.x * FGS + threadIdx.x;
+  const bool in = (int)i < ntot;
+  const unsigned q = i / (unsigned)nxc, zi = q / (unsigned)nyc;
+  const int x = 2 * (int)(i - q * nxc) + cx, y = 2 * (int)(q - zi * nyc) + cy, z = 2 * (int)zi + cz;
   const long long NP = L.NP;
   const long long px = L.px, pxy = (long long)L.px * L.py;
+  const long long qx = L.qx, qxy = (long long)L.qx * L.qy;
   const long long n = L.nidx(x, y, z);
-  const uint8_t cls = L.vclass[n];
+  const uint8_t cls = in ? L.vclass[n] : (uint8_t)0;
+  const long long e0 = L.eidx(x - 1, y - 1, z - 1);
+  T r[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) r[k] = in ? rp[e0 + (k & 1) + ((k >> 1) & 1) * qx + (k >> 2) * qxy] : T(0);
+  pdl_wait();
+  pdl_trigger();
   if (!(cls & NC_ACTIVE)) return;
   if (cls & NC_SUPPORT) {
     // S = n_e I and KeU = 0 at support nodes (grid/Grid.cu:1808-1833): u = f / n_e = 0
     u[n] = 0; u[n + NP] = 0; u[n + 2 * NP] = 0;
     return;
   }
-  const long long qx = L.qx, qxy = (long long)L.qx * L.qy;
-  const long long e0 = L.eidx(x - 1, y - 1, z - 1);
-  T r[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) r[k] = rp[e0 + (k & 1) + ((k >> 1) & 1) * qx + (k >> 2) * qxy];
   T a[8][3];
 #pragma unroll
   for (int k = 0; k < 8; k++) a[k][0] = a[k][1] = a[k][2] = 0;
@@ -1489,11 +1496,17 @@ template <typename T>
 rso_status fine_gs(rso_handle* h, T* u, const T* f, const T* rp, int colour, int reverse) {
   const Level& l = h->L[0];
   int cx = colour & 1, cy = (colour >> 1) & 1, cz = colour >> 2;
-  dim3 g(cdiv((l.nx - cx + 1) / 2, 32), cdiv((l.ny - cy + 1) / 2, 8), (l.nz - cz + 1) / 2);
-  if (g.x == 0 || g.y == 0 || g.z == 0) return RSO_OK;
+  const int nxc = (l.nx - cx + 1) / 2, nyc = (l.ny - cy + 1) / 2, nzc = (l.nz - cz + 1) / 2;
+  const long long ntot = (long long)nxc * nyc * nzc;
+  if (ntot == 0) return RSO_OK;
+  if (ntot >= (1LL << 31)) {
+    h->err = "fine level too large for 32-bit node indices";
+    return RSO_ERR_UNSUPPORTED;
+  }
   const int cls = pcls<T>(PC_FINE_GS32, PC_FINE_GS64);
   if (h->prof_on) prof_begin(h, cls, (double)l.nn / 8);
-  k_fine_gs<T><<<g, dim3(32, 8), 0, h->stream>>>(l, u, f, rp, cx, cy, cz, reverse);
+  launch_pdl(k_fine_gs<T>, dim3(cdiv(ntot, FGS)), dim3(FGS), 0, h->stream, l, u, f, rp, cx, cy, cz, nxc, nyc,
+             (int)ntot, reverse);
   rso::note_launch();
   if (h->prof_on) prof_end(h, cls);
   return launch_check(h, "fine_gs");

@@ -264,6 +264,32 @@ namespace rso {
 
 inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// Programmatic dependent launch: a kernel launched with launch_pdl may start
+// while its predecessor in the stream still runs, so that its launch, its index
+// arithmetic and its first loads hide behind it.  Such a kernel calls pdl_wait()
+// before it touches anything its predecessor writes or reads for writing; until
+// then it may only read what stays fixed during a solve (stencils, rho^p, node
+// classes).  pdl_wait returns once the predecessor has ended and its writes are
+// visible.  pdl_trigger() after it lets the successor start, so at most one
+// kernel waits ahead of the running one, and everything before the running one
+// has ended.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid;
+  lc.blockDim = block;
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);  // a failure is the next launch_check's
+}
+
 rso_status launch_check(rso_handle* h, const char* what);
 
 // reductions (reduce.cu)

@@ -24,3 +24,21 @@ def test_fine_fp64_chunks(oracle, cuda, dims):
     g.update_stencil()
     jac = g.gs_relax(0, t(u, cuda), t(f, cuda), kind=1, omega=0.3).cpu().numpy()
     assert rel(jac, o.smooth(0, u, f, kind=1, omega=0.3, sweeps=1)) < 1e-12
+
+
+# coarse levels of 2 to 17 nodes an edge: colours of one node, of fewer and of more than the 32 a CTA
+# takes, with a ragged last CTA; the ellipsoid leaves inactive nodes inside the box
+@pytest.mark.parametrize("gen", [lambda: P.cantilever(6, 4, 3), lambda: P.cantilever(30, 21, 13),
+                                 lambda: P.ellipsoid(64, 36, 28)])
+@pytest.mark.parametrize("reverse", [0, 1])
+def test_coarse_gauss_seidel(oracle, cuda, gen, reverse):
+    """FP64 coloured sweeps on every coarse level; 1e-12 relative, the bound of the FP64 operator pieces."""
+    g, o = make(oracle, gen(), n_levels=3, first_factor=2)
+    g.update_stencil()
+    o.update_stencil()
+    rng = np.random.default_rng(11)
+    for lvl in range(1, o.n_levels()):
+        mask = np.tile(o.level_masks(lvl)[1], 3)
+        u, f = (rng.standard_normal(mask.size) * mask for _ in range(2))
+        got = g.gs_relax(lvl, t(u, cuda), t(f, cuda), sweeps=2, reverse=reverse).cpu().numpy()
+        assert rel(got, o.smooth(lvl, u, f, kind=0, omega=1.0, sweeps=2, reverse=reverse)) < 1e-12, lvl
