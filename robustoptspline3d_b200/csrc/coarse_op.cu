@@ -1175,11 +1175,9 @@ __device__ void bot_residual(const Level& L, const T* st, const T* u0v, const T*
   }
 }
 
-// FC: the coarsening factor when known at compile time (its loops unrolled,
-// so a thread's loads are all in flight at once), 0 to read it from C
-template <typename T, int FC = 0>
+template <typename T>
 __device__ void bot_restrict(const Level& Fl, const Level& C, const T* rf0, T* fc0, int g0, int gs) {
-  const int F = FC > 0 ? FC : C.factor;
+  const int F = C.factor;
   for (long long ib = g0; ib < C.nn * C.nb; ib += gs) {
     const long long b = ib / C.nn, i = ib - b * C.nn;
     const T* rf = rf0 + b * 3 * Fl.NP;
@@ -1212,24 +1210,30 @@ __device__ void bot_restrict(const Level& Fl, const Level& C, const T* rf0, T* f
   }
 }
 
-// the restriction with one thread per (coarse node, component) and the
-// factor known at compile time: a thread's (2F - 1)^3 loads are independent
-// and unrolled (the same sums in the same order as bot_restrict)
+// the restriction with one thread per (coarse node, component), the fourth of
+// each quad of lanes idle, and the factor known at compile time: a thread's
+// (2F - 1)^3 loads are independent and unrolled (the same sums in the same
+// order as bot_restrict).  With `first` the coarse level's first smoothing step
+// from a zero iterate, first = om D^-1 fc, comes from the same pass: the quad
+// exchanges the three components, so the step needs no phase and barrier of
+// its own (its arithmetic is that of gb_sweep's step).
 template <typename T, int F>
-__device__ void bot_restrict3(const Level& Fl, const Level& C, const T* rf0, T* fc0, int g0, int gs) {
+__device__ void bot_restrict3(const Level& Fl, const Level& C, const T* rf0, T* fc0, const T* __restrict__ st,
+                              T* first0, T om, int g0, int gs) {
   // the levels of the persistent kernel are below 2^31 nodes (checked by its
   // launcher): 32-bit index arithmetic
-  const unsigned nn = (unsigned)C.nn, nx = (unsigned)C.nx, ny = (unsigned)C.ny;
-  for (unsigned it = g0; it < 3u * nn * (unsigned)C.nb; it += gs) {
-    const unsigned ib = it / 3u, c = it - 3u * ib;
-    const unsigned b = ib / nn, i = ib - b * nn;
-    const T* rf = rf0 + (long long)b * 3 * Fl.NP + c * Fl.NP;
-    T* fc = fc0 + (long long)b * 3 * C.NP + c * C.NP;
+  const unsigned nn = (unsigned)C.nn, nx = (unsigned)C.nx, ny = (unsigned)C.ny, all = nn * (unsigned)C.nb;
+  for (unsigned it = g0; it < ((4u * all + 31u) & ~31u); it += gs) {  // whole warps: the quads shuffle
+    const unsigned ib = it >> 2, c = it & 3u;
+    const bool in = ib < all;
+    const unsigned b = in ? ib / nn : 0u, i = in ? ib - b * nn : 0u;
     const unsigned iy = i / nx, Z = iy / ny;
     const int X = (int)(i - iy * nx), Y = (int)(iy - Z * ny);
     const long long nC = C.nidx(X, Y, Z);
+    const bool act = in && (C.vclass[nC] & NC_ACTIVE);
     T sum = 0;
-    if (C.vclass[nC] & NC_ACTIVE) {
+    if (act && c < 3) {
+      const T* rf = rf0 + (long long)b * 3 * Fl.NP + c * Fl.NP;
 #pragma unroll
       for (int dz = -F + 1; dz < F; dz++) {
         const int z = F * Z + dz;
@@ -1249,7 +1253,24 @@ __device__ void bot_restrict3(const Level& Fl, const Level& C, const T* rf0, T* 
         }
       }
     }
-    fc[nC] = sum;
+    if (in && c < 3) fc0[(long long)b * 3 * C.NP + c * C.NP + nC] = sum;
+    if (first0 == nullptr) continue;
+    const int q0 = (int)(it & 28u);  // it and the lane agree modulo 32
+    const T r0 = __shfl_sync(0xffffffffu, sum, q0), r1 = __shfl_sync(0xffffffffu, sum, q0 + 1),
+            r2 = __shfl_sync(0xffffffffu, sum, q0 + 2);
+    if (!in || c == 3) continue;
+    T o = 0;
+    if (act) {
+      T S[9];
+#pragma unroll
+      for (int k = 0; k < 9; k++) S[k] = st[st_at<T>(C.NP, 13 * 9 + k, nC)];
+      const T A = S[4] * S[8] - S[5] * S[7], B = -(S[3] * S[8] - S[5] * S[6]), D = S[3] * S[7] - S[4] * S[6];
+      const T id = om / (S[0] * A + S[1] * B + S[2] * D);
+      if (c == 0) o = id * (A * r0 - (S[1] * S[8] - S[2] * S[7]) * r1 + (S[1] * S[5] - S[2] * S[4]) * r2);
+      else if (c == 1) o = id * (B * r0 + (S[0] * S[8] - S[2] * S[6]) * r1 - (S[0] * S[5] - S[2] * S[3]) * r2);
+      else o = id * (D * r0 - (S[0] * S[7] - S[1] * S[6]) * r1 + (S[0] * S[4] - S[1] * S[3]) * r2);
+    }
+    first0[(long long)b * 3 * C.NP + c * C.NP + nC] = o;
   }
 }
 
@@ -1423,46 +1444,46 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
   return v;
 }
 
-// grid-wide barrier on bar = {arrivals, generation, gave-up flag}: one arrival
-// per CTA; the last resets the count and advances the generation.  gen (thread
-// 0's copy of the generation) moves on with it.  Returns false on every
-// thread of every CTA once some wait has given up (bar[2] set): the kernel
-// then returns, and the host reports it after the solve.
+// Grid-wide barrier on bar = {arrivals, exits, gave-up flag}: one arrival per
+// CTA (a release), the arrivals counted on through the launch, so that a waiter
+// polls the very word the arrivals change (no reset, no second word to pass on:
+// 2.4 us per barrier with both, see k_bottom_grid for what is left).  goal is
+// thread 0's count of arrivals that completes its next barrier.  The last CTA to
+// leave the kernel (gbar_exit) clears the counts for the next launch.  Returns
+// false on every thread of every CTA once some wait has given up (kGbarGone in
+// the arrivals, and bar[2] for the host): the kernel then returns, and the host
+// reports it after the solve and clears all words.
 // (target, limit: the arrivals that complete the barrier and the wait's bound
 // in clock cycles; the self-test sets them, the bottom kernel keeps the grid
 // size and kGbarCycles)
-__device__ bool gbar_sync(unsigned* bar, unsigned& gen, int tid, unsigned target = 0, long long limit = kGbarCycles) {
-  __shared__ int s_ok;
-  if (target == 0) target = gridDim.x;
+constexpr unsigned kGbarGone = 1u << 31;
+__device__ bool gbar_sync(unsigned* bar, unsigned& goal, int tid, unsigned target, long long limit = kGbarCycles) {
   __syncthreads();
+  int bad = 0;
   if (tid == 0) {
-    int ok = *reinterpret_cast<volatile unsigned*>(bar + 2) == 0u;
-    if (ok) {
-      const unsigned g = gen;
-      __threadfence();
-      if (atomicAdd(bar, 1u) == target - 1) {
-        atomicExch(bar, 0u);
-        __threadfence();
-        atomicExch(bar + 1, g + 1);
-      } else {
-        const long long t0 = clock64();
-        while (ld_acquire_gpu(bar + 1) == g) {
-          if (*reinterpret_cast<volatile unsigned*>(bar + 2) != 0u) { ok = 0; break; }
-          if (clock64() - t0 > limit) {
-            atomicExch(bar + 2, 1u);
-            ok = 0;
-            break;
-          }
-          __nanosleep(64);
-        }
+    goal += target;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    const long long t0 = clock64();
+    for (;;) {
+      const unsigned v = ld_acquire_gpu(bar);
+      if (v & kGbarGone) { bad = 1; break; }
+      if (v >= goal) break;
+      if (clock64() - t0 > limit) {
+        atomicOr(bar, kGbarGone);
+        atomicExch(bar + 2, 1u);
+        bad = 1;
+        break;
       }
-      __threadfence();
-      gen = g + 1;
     }
-    s_ok = ok;
   }
-  __syncthreads();
-  return s_ok != 0;
+  return __syncthreads_or(bad) == 0;
+}
+// every CTA of a launch that passed all its barriers calls this once
+__device__ void gbar_exit(unsigned* bar, int tid) {
+  if (tid == 0 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
+    bar[0] = 0u;
+    bar[1] = 0u;
+  }
 }
 
 // one row-split sweep (MODE 2) or residual (MODE 0) of a level, tile by tile
@@ -1643,10 +1664,9 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
   constexpr int NT = gb_threads<T>();
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int g0 = blockIdx.x * NT + tid, gs = gridDim.x * NT;
-  unsigned gen = 0;
-  if (tid == 0) gen = ld_acquire_gpu(bar + 1);
+  unsigned goal = 0;
 #define GB_SYNC() \
-  if (!gbar_sync(bar, gen, tid)) return
+  if (!gbar_sync(bar, goal, tid, gridDim.x)) return
   T* ucur[BOT_MAX_LEVELS];
   // down: pre-smoothing from a zero iterate, residual, restriction
   for (int li = A.lb; li < A.nl - 1; li++) {
@@ -1655,12 +1675,14 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
     T* u = bv_u<T>(L);
     T *cur = u, *oth = bv_t<T>(L), *prv = bv_r<T>(L);
     for (int s = 0; s < A.pre; s++) {
-      if (s == 0)
-        gb_sweep<T, 2, true>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], (const T*)nullptr, A.c1[li][s], sres);
-      else
+      // the first step, from a zero iterate, ran with the restriction that
+      // formed this level's f (on the first level it is a phase of its own)
+      if (s > 0)
         gb_sweep<T, 2, false>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], s <= 1 ? (const T*)nullptr : prv,
                               A.c1[li][s], sres);
-      GB_SYNC();
+      else if (li == A.lb)
+        gb_sweep<T, 2, true>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], (const T*)nullptr, A.c1[li][s], sres);
+      if (s > 0 || li == A.lb) GB_SYNC();
       T* w = prv; prv = cur; cur = oth; oth = w;
     }
     if (A.pre == 0) {
@@ -1670,10 +1692,14 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
     ucur[li] = cur;
     gb_sweep<T, 0, false>(L, st, cur, bv_f<T>(L), oth, T(0), (const T*)nullptr, T(0), sres);
     GB_SYNC();
-    if (A.L[li + 1].factor == 2)
-      bot_restrict3<T, 2>(L, A.L[li + 1], oth, bv_f<T>(A.L[li + 1]), g0, gs);
-    else
-      bot_restrict<T>(L, A.L[li + 1], oth, bv_f<T>(A.L[li + 1]), g0, gs);
+    {
+      const Level& C = A.L[li + 1];
+      T* first = li + 1 < A.nl - 1 && A.pre > 0 ? bv_t<T>(C) : nullptr;  // where step 0 of the next level goes
+      if (C.factor == 2)
+        bot_restrict3<T, 2>(L, C, oth, bv_f<T>(C), bv_st<T>(C), first, A.om[li + 1][0], g0, gs);
+      else
+        bot_restrict3<T, 4>(L, C, oth, bv_f<T>(C), bv_st<T>(C), first, A.om[li + 1][0], g0, gs);
+    }
     if (li + 1 == A.nl - 1) {  // the coarsest iterate is zero outside the listed nodes
       const Level& C = A.L[li + 1];
       T* uc = bv_u<T>(C);
@@ -1717,24 +1743,25 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
       T* rest[2];
       for (int q = 0; q < 3; q++)
         if (bufs[q] != cur) rest[k++] = bufs[q];
-      oth = rest[0];
-      prv = rest[1];
+      // the steps write oth, prv and cur in turn: the order in which the last
+      // one writes u, where it can
+      const int swap = A.post % 3 == 2;
+      oth = rest[swap];
+      prv = rest[1 - swap];
     }
     bot_prolong3<T>(L, A.L[li + 1], ucur[li + 1], cur, g0, gs);
     GB_SYNC();
     for (int s = 0; s < A.post; s++) {
       gb_sweep<T, 2, false>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], s == 0 ? (const T*)nullptr : prv,
                             A.c1[li][s], sres);
-      GB_SYNC();
+      if (li > A.lb || s + 1 < A.post || oth != u) GB_SYNC();  // nothing follows the kernel's last step
       T* w = prv; prv = cur; cur = oth; oth = w;
     }
     ucur[li] = cur;
-    if (li == A.lb && cur != u) {
-      bot_copy<T>(L, cur, u, g0, gs);
-      GB_SYNC();
-    }
+    if (li == A.lb && cur != u) bot_copy<T>(L, cur, u, g0, gs);
   }
 #undef GB_SYNC
+  gbar_exit(bar, tid);
 }
 
 // ---------------------------------------------------------------- host wrappers
@@ -2019,10 +2046,10 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
 // short_by; with short_by > 0 no barrier completes, so every CTA's wait gives
 // up after limit cycles, sets the flag and returns (no fault, no hang).
 __global__ void k_gbar_selftest(unsigned* bar, int rounds, unsigned short_by, long long limit) {
-  unsigned gen = 0;
-  if (threadIdx.x == 0) gen = ld_acquire_gpu(bar + 1);
+  unsigned goal = 0;
   for (int r = 0; r < rounds; r++)
-    if (!gbar_sync(bar, gen, threadIdx.x, gridDim.x + short_by, limit)) return;
+    if (!gbar_sync(bar, goal, threadIdx.x, gridDim.x + short_by, limit)) return;
+  gbar_exit(bar, threadIdx.x);
 }
 
 template rso_status bottom_vcycle<double>(rso_handle*, int, int, int);

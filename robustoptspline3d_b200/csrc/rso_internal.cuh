@@ -144,7 +144,7 @@ struct rso_handle {
   double* c_R = nullptr;              // coarsest rigid motions, 3 nc x 6 row-major, orthonormal
   // reductions
   double* red = nullptr;              // partials
-  unsigned* gbar = nullptr;           // grid barrier of the persistent bottom kernel: arrivals, generation, gave-up flag
+  unsigned* gbar = nullptr;           // grid barrier of the persistent bottom kernel: arrivals, exits, gave-up flag
   double* xfer = nullptr;             // restriction scratch: z-filtered fine columns
   size_t xfer_n = 0;                  // its capacity in doubles
   double* fpart = nullptr;            // per-CTA partial sums of the fine operator kernel
