@@ -1106,6 +1106,7 @@ struct BottomArgs {
   const int* cnodes;
   int nc;
   double* cf;          // coarsest right-hand side (N doubles)
+  int tile0[BOT_MAX_LEVELS];  // persistent FP32 kernel: the CTA holding the level's first stencil tile, -1 none
 };
 
 template <typename T>
@@ -1431,10 +1432,14 @@ __global__ void __cluster_dims__(BOT_CTAS, 1, 1) __launch_bounds__(BOT_THREADS, 
 
 // The same bottom of the V-cycle as one persistent kernel over the whole GPU:
 // a cooperative launch (every CTA resident at once) whose phases are
-// separated by a grid-wide barrier.  The sweeps and residuals run as the
-// row-split per-level kernel does (tiles of 32 x CTY nodes, three threads per
-// node, the same arithmetic: bit-identical sweeps), the transfers and the
-// coarsest solve as in k_bottom.
+// separated by a grid-wide barrier.  FP32 sweeps run on four-node groups with
+// nine threads each and, on the levels that fit, on stencils held in shared
+// memory (below); FP64 sweeps as the row-split per-level kernel does (tiles of
+// 32 x CTY nodes, three threads per node).  What bounds it is latency: a phase
+// is a barrier and one round of loads.  Per V-cycle, 2 + 2 Chebyshev steps: from
+// the 33^3 level of 256^3 down 174 -> 149 us (33^3 streamed, the rest held),
+// 93 x 71 x 85 110 -> 70 us, 64^3 96 -> 59 us, 49 x 38 x 56 68 -> 37 us (all
+// held), before: two-word barriers, every stencil streamed, two CTAs per SM.
 // a barrier wait gives up after this many SM clock cycles (about 2 s)
 constexpr long long kGbarCycles = 4000000000LL;
 
@@ -1512,176 +1517,270 @@ __device__ void gb_sweep_rows(const Level& L, const T* st, const T* u, const T* 
 // latencies long.  The nine partial sums meet in shared memory in a fixed
 // order; four of the group's threads then finish one node each as k_coarse4
 // does (residual, or damped block Jacobi / Chebyshev step; halo rows
-// unwritten).
-constexpr int G9 = 32;  // node groups per tile (9 G9 threads)
-template <int MODE, bool ZERO>
-__device__ void gb_sweep4(const Level& L, const float* __restrict__ st, const float* u0v, const float* f0v,
-                          float* out0v, float omega, const float* up0v, float c1, float (*red)[12][G9]) {
-  const int tg = threadIdx.x % G9, q = threadIdx.x / G9;  // q = 3 (dz + 1) + (dy + 1)
+// unwritten).  A team of 9 G9 threads takes a tile of G9 groups, the 128 nodes
+// of one tile of the FP32 stencil.
+constexpr int G9 = 32;
+constexpr int kTeam = 9 * G9, kTeams = 1;
+static_assert(4 * G9 == ST_TILE, "a team's tile is a tile of the stencil");
+__device__ __forceinline__ void team_sync(int team) {
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeam) : "memory");
+}
+struct GroupPos {
+  long long p0 = 0;  // the group's first padded node
+  int xp = 0;        // and its padded x
+  bool work = false, any = false, act[4] = {false, false, false, false};
+};
+__device__ __forceinline__ GroupPos group_pos(const Level& L, long long g, bool valid) {
+  GroupPos P;
+  P.p0 = 4 * g;
+  if (!valid) return P;
+  // the levels of this kernel are small (NP < 2^31): 32-bit divisions
+  const unsigned p0u = (unsigned)P.p0, pxu = (unsigned)L.px, pxyu = pxu * (unsigned)L.py;
+  const int zp = (int)(p0u / pxyu);
+  const unsigned rem = p0u - (unsigned)zp * pxyu;
+  const int yp = (int)(rem / pxu);
+  P.xp = (int)(rem - (unsigned)yp * pxu);
+  P.work = !(zp < 1 || zp > L.nz || yp < 1 || yp > L.ny);  // halo row: stays zero
+  if (!P.work) return P;
+  const uchar4 cl4 = *reinterpret_cast<const uchar4*>(L.vclass + P.p0);
+  const uint8_t cls[4] = {cl4.x, cl4.y, cl4.z, cl4.w};
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int x = P.xp + k - 1;
+    P.act[k] = x >= 0 && x < L.nx && (cls[k] & NC_ACTIVE);
+    P.any = P.any || P.act[k];
+  }
+  return P;
+}
+// one tile's step; RES: st is the tile's stencil in shared memory, else the level's
+template <int MODE, bool ZERO, bool RES>
+__device__ __forceinline__ void group_step(const Level& L, const float* __restrict__ st, const GroupPos& P,
+                                           const float* u, const float* f, float* out, float omega, const float* up,
+                                           float c1, int tg, int q, int team, float (*red)[12][G9]) {
+  const long long NP = L.NP, p0 = P.p0;
   const int pz = q / 3, py = q - 3 * pz;
-  const long long NP = L.NP, px = L.px, pxy = (long long)L.px * L.py;
-  const long long ng = NP / 4, ngt = ng * L.nb;
-  const long long ntile = (ngt + G9 - 1) / G9;
-  for (long long t = blockIdx.x; t < ntile; t += gridDim.x) {
-    const long long gg = t * G9 + tg;
-    const long long bsys = gg < ngt ? (long long)((unsigned)gg / (unsigned)ng) : 0, g = gg - bsys * ng;
-    const long long vo = bsys * 3 * NP;
-    const float* u = u0v + vo;
-    const long long p0 = 4 * g;
-    bool work = gg < ngt;
-    int xp = 0;
-    bool act[4] = {false, false, false, false};
-    if (work) {
-      // the levels of this kernel are small (NP < 2^31): 32-bit divisions
-      const unsigned p0u = (unsigned)p0, pxyu = (unsigned)pxy, pxu = (unsigned)px;
-      const int zp = (int)(p0u / pxyu);
-      const unsigned rem = p0u - (unsigned)zp * pxyu;
-      const int yp = (int)(rem / pxu);
-      xp = (int)(rem - (unsigned)yp * pxu);
-      work = !(zp < 1 || zp > L.nz || yp < 1 || yp > L.ny);  // halo row: stays zero
+  auto sat = [&](int k) { return RES ? (long long)(k * (int)ST_TILE + 4 * tg) : st_at<float>(NP, k, p0); };
+  // thread q < 4 finishes node q of the group; its operands load with the rest
+  const long long n = p0 + q;
+  const bool fin = q < 4 && P.work;
+  float fv[3] = {0.f, 0.f, 0.f}, uo[3] = {0.f, 0.f, 0.f}, pv[3] = {0.f, 0.f, 0.f};
+  if (fin) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      fv[r] = f[n + r * NP];
+      if (MODE == 2 && !ZERO) uo[r] = u[n + r * NP];
+      if (MODE == 2 && up) pv[r] = up[n + r * NP];
     }
-    bool any = false;
-    if (work) {
-      const uchar4 cl4 = *reinterpret_cast<const uchar4*>(L.vclass + p0);
-      const uint8_t cls[4] = {cl4.x, cl4.y, cl4.z, cl4.w};
+  }
+  float acc[3][4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const int x = xp + k - 1;
-        act[k] = x >= 0 && x < L.nx && (cls[k] & NC_ACTIVE);
-        any = any || act[k];
-      }
-    }
-    float acc[3][4];
+  for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int r = 0; r < 3; r++)
+    for (int k = 0; k < 4; k++) acc[r][k] = 0.f;
+  if (P.any && !ZERO) {
+    const long long nb = p0 + ((long long)(pz - 1) * L.py + (py - 1)) * L.px;
+    float w[3][6];  // u at x offsets -1 .. 4 of the group's row in this neighbour row
 #pragma unroll
-      for (int k = 0; k < 4; k++) acc[r][k] = 0.f;
-    if (any && !ZERO) {
-      const long long nb = p0 + (long long)(pz - 1) * pxy + (long long)(py - 1) * px;
-      float w[3][6];  // u at x offsets -1 .. 4 of the group's row in this neighbour row
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float* uc = u + nb + c * NP;
-        const float4 m = *reinterpret_cast<const float4*>(uc);
-        // at xp = 0 the left neighbour is outside the row (the group's first
-        // node is halo, its result discarded); likewise the right one at the end
-        w[c][0] = xp > 0 ? uc[-1] : 0.f;
-        w[c][1] = m.x; w[c][2] = m.y; w[c][3] = m.z; w[c][4] = m.w;
-        w[c][5] = xp + 4 < px ? uc[4] : 0.f;
-      }
-#pragma unroll
-      for (int dx = 0; dx < 3; dx++) {
-        const int d = q * 3 + dx;
-#pragma unroll
-        for (int r = 0; r < 3; r++)
-#pragma unroll
-          for (int c = 0; c < 3; c++) {
-            const float4 sv = *reinterpret_cast<const float4*>(st + st_at<float>(NP, d * 9 + r * 3 + c, p0));
-            acc[r][0] = fmaf(sv.x, w[c][dx + 0], acc[r][0]);
-            acc[r][1] = fmaf(sv.y, w[c][dx + 1], acc[r][1]);
-            acc[r][2] = fmaf(sv.z, w[c][dx + 2], acc[r][2]);
-            acc[r][3] = fmaf(sv.w, w[c][dx + 3], acc[r][3]);
-          }
-      }
+    for (int c = 0; c < 3; c++) {
+      const float* uc = u + nb + c * NP;
+      const float4 m = *reinterpret_cast<const float4*>(uc);
+      // at xp = 0 the left neighbour is outside the row (the group's first
+      // node is halo, its result discarded); likewise the right one at the end
+      w[c][0] = P.xp > 0 ? uc[-1] : 0.f;
+      w[c][1] = m.x; w[c][2] = m.y; w[c][3] = m.z; w[c][4] = m.w;
+      w[c][5] = P.xp + 4 < L.px ? uc[4] : 0.f;
     }
 #pragma unroll
-    for (int r = 0; r < 3; r++)
+    for (int dx = 0; dx < 3; dx++) {
+      const int d = q * 3 + dx;
 #pragma unroll
-      for (int k = 0; k < 4; k++) red[q][r * 4 + k][tg] = acc[r][k];
-    __syncthreads();
-    if (q < 4 && work) {
-      // thread q finishes node k = q of the group: its rows' nine partial
-      // sums in the order dz, dy = (-1, -1) .. (1, 1)
-      const int k = q;
-      const long long n = p0 + k;
-      float a[3];
+      for (int r = 0; r < 3; r++)
 #pragma unroll
-      for (int r = 0; r < 3; r++) {
-        float sum = red[0][r * 4 + k][tg];
-#pragma unroll
-        for (int sl = 1; sl < 9; sl++) sum += red[sl][r * 4 + k][tg];
-        a[r] = sum;
-      }
-      const float* f = f0v + vo;
-      float* out = out0v + vo;
-      float res[3];
-#pragma unroll
-      for (int r = 0; r < 3; r++) res[r] = f[n + r * NP] - (act[k] ? a[r] : 0.f);
-      if (MODE == 0) {
-#pragma unroll
-        for (int r = 0; r < 3; r++) out[n + r * NP] = res[r];
-      } else if (!act[k]) {
-#pragma unroll
-        for (int r = 0; r < 3; r++) out[n + r * NP] = 0.f;
-      } else {
-        float Sk[9];
-#pragma unroll
-        for (int i = 0; i < 9; i++) Sk[i] = st[st_at<float>(NP, 13 * 9 + i, n)];
-        float uo[3], up[3];
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-          uo[r] = ZERO ? 0.f : u[n + r * NP];
-          up[r] = up0v ? up0v[vo + n + r * NP] : 0.f;
+        for (int c = 0; c < 3; c++) {
+          const float4 sv = *reinterpret_cast<const float4*>(st + sat(d * 9 + r * 3 + c));
+          acc[r][0] = fmaf(sv.x, w[c][dx + 0], acc[r][0]);
+          acc[r][1] = fmaf(sv.y, w[c][dx + 1], acc[r][1]);
+          acc[r][2] = fmaf(sv.z, w[c][dx + 2], acc[r][2]);
+          acc[r][3] = fmaf(sv.w, w[c][dx + 3], acc[r][3]);
         }
-        const float r0 = res[0], r1 = res[1], r2 = res[2];
-        const float A = Sk[4] * Sk[8] - Sk[5] * Sk[7], B = -(Sk[3] * Sk[8] - Sk[5] * Sk[6]),
-                    C = Sk[3] * Sk[7] - Sk[4] * Sk[6];
-        const float det = Sk[0] * A + Sk[1] * B + Sk[2] * C;
-        const float id = omega / det;
-        const float i01 = -(Sk[1] * Sk[8] - Sk[2] * Sk[7]), i02 = Sk[1] * Sk[5] - Sk[2] * Sk[4];
-        const float i11 = Sk[0] * Sk[8] - Sk[2] * Sk[6], i12 = -(Sk[0] * Sk[5] - Sk[2] * Sk[3]);
-        const float i21 = -(Sk[0] * Sk[7] - Sk[1] * Sk[6]), i22 = Sk[0] * Sk[4] - Sk[1] * Sk[3];
-        out[n] = uo[0] + c1 * (uo[0] - up[0]) + id * (A * r0 + i01 * r1 + i02 * r2);
-        out[n + NP] = uo[1] + c1 * (uo[1] - up[1]) + id * (B * r0 + i11 * r1 + i12 * r2);
-        out[n + 2 * NP] = uo[2] + c1 * (uo[2] - up[2]) + id * (C * r0 + i21 * r1 + i22 * r2);
-      }
     }
-    __syncthreads();  // red is reused by the next tile
+  }
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) red[q][r * 4 + k][tg] = acc[r][k];
+  team_sync(team);
+  if (fin) {
+    // the node's nine partial sums in the order dz, dy = (-1, -1) .. (1, 1)
+    float res[3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      float sum = red[0][r * 4 + q][tg];
+#pragma unroll
+      for (int sl = 1; sl < 9; sl++) sum += red[sl][r * 4 + q][tg];
+      res[r] = fv[r] - (P.act[q & 3] ? sum : 0.f);
+    }
+    if (MODE == 0) {
+#pragma unroll
+      for (int r = 0; r < 3; r++) out[n + r * NP] = res[r];
+    } else if (!P.act[q & 3]) {
+#pragma unroll
+      for (int r = 0; r < 3; r++) out[n + r * NP] = 0.f;
+    } else {
+      float Sk[9];
+#pragma unroll
+      for (int i = 0; i < 9; i++) Sk[i] = st[sat(13 * 9 + i) + q];
+      const float r0 = res[0], r1 = res[1], r2 = res[2];
+      const float A = Sk[4] * Sk[8] - Sk[5] * Sk[7], B = -(Sk[3] * Sk[8] - Sk[5] * Sk[6]),
+                  C = Sk[3] * Sk[7] - Sk[4] * Sk[6];
+      const float det = Sk[0] * A + Sk[1] * B + Sk[2] * C;
+      const float id = omega / det;
+      const float i01 = -(Sk[1] * Sk[8] - Sk[2] * Sk[7]), i02 = Sk[1] * Sk[5] - Sk[2] * Sk[4];
+      const float i11 = Sk[0] * Sk[8] - Sk[2] * Sk[6], i12 = -(Sk[0] * Sk[5] - Sk[2] * Sk[3]);
+      const float i21 = -(Sk[0] * Sk[7] - Sk[1] * Sk[6]), i22 = Sk[0] * Sk[4] - Sk[1] * Sk[3];
+      out[n] = uo[0] + c1 * (uo[0] - pv[0]) + id * (A * r0 + i01 * r1 + i02 * r2);
+      out[n + NP] = uo[1] + c1 * (uo[1] - pv[1]) + id * (B * r0 + i11 * r1 + i12 * r2);
+      out[n + 2 * NP] = uo[2] + c1 * (uo[2] - pv[2]) + id * (C * r0 + i21 * r1 + i22 * r2);
+    }
+  }
+  team_sync(team);  // red is reused by the next tile
+}
+// A level's sweep, its tiles dealt to the teams of all CTAs, or, on a level
+// whose tiles are held in shared memory (tile0 >= 0), every tile by its CTA.
+template <int MODE, bool ZERO>
+__device__ void gb_sweep4(const Level& L, const float* __restrict__ st, const float* u, const float* f, float* out,
+                          float omega, const float* up, float c1, int tid, int tile0, const GroupPos& own,
+                          const float* sst, float (*red)[9][12][G9]) {
+  const int team = tid / kTeam, q = (tid - team * kTeam) / G9, tg = tid % G9;
+  const long long ng = L.NP / 4, VS = 3 * L.NP;
+  if (tile0 >= 0) {
+    const int t = (int)blockIdx.x - tile0;
+    if (team != 0 || t < 0 || (long long)t * G9 >= ng) return;
+    for (int b = 0; b < L.nb; b++)
+      group_step<MODE, ZERO, true>(L, sst, own, u + b * VS, f + b * VS, out + b * VS, omega, up ? up + b * VS : nullptr,
+                                   c1, tg, q, team, red[team]);
+    return;
+  }
+  const long long ngt = ng * L.nb, ntile = (ngt + G9 - 1) / G9;
+  for (long long t = (long long)blockIdx.x * kTeams + team; t < ntile; t += (long long)gridDim.x * kTeams) {
+    const long long gg = t * G9 + tg;
+    const long long b = gg < ngt ? (long long)((unsigned)gg / (unsigned)ng) : 0;
+    const GroupPos P = group_pos(L, gg - b * ng, gg < ngt);
+    group_step<MODE, ZERO, false>(L, st, P, u + b * VS, f + b * VS, out + b * VS, omega, up ? up + b * VS : nullptr, c1,
+                                  tg, q, team, red[team]);
   }
 }
 
-// threads of a CTA of the persistent kernel: nine per group of G9 four-node
-// groups (FP32), 32 x CTY x 3 for the row-split sweeps (FP64)
-template <typename T>
-constexpr int gb_threads() { return sizeof(T) == 4 ? 9 * G9 : 32 * CTY * 3; }
-// shared exchange of a sweep: [9][12][G9] floats (FP32), [3][CTY][32] T (FP64)
-template <typename T>
-constexpr int gb_smem() { return sizeof(T) == 4 ? 9 * 12 * G9 * 4 : 3 * CTY * 32 * (int)sizeof(T); }
-
-template <typename T, int MODE, bool ZERO>
-__device__ __forceinline__ void gb_sweep(const Level& L, const T* st, const T* u, const T* f, T* out, T omega,
-                                         const T* uprev, T c1, unsigned char* sm) {
-  if constexpr (sizeof(T) == 4)
-    gb_sweep4<MODE, ZERO>(L, st, u, f, out, omega, uprev, c1, reinterpret_cast<float (*)[12][G9]>(sm));
-  else
-    gb_sweep_rows<T, MODE, ZERO>(L, st, u, f, out, omega, uprev, c1, reinterpret_cast<T (*)[CTY][32]>(sm));
+// The FP32 levels' stencils in shared memory.  A tile of the stencil is 128
+// nodes, [243][128] floats in one contiguous block, so one bulk copy (TMA) per
+// CTA, started when the kernel starts, brings a tile in, and the tile's four
+// sweeps and residual of a V-cycle read it there.  The tiles of the smallest
+// levels go first, one per CTA, as long as a level fits; larger levels stream
+// their stencils from L2.  What this saves is latency: a phase of such a level
+// waits for one round of vector loads and the barrier, not for 27 stencil
+// vectors a thread as well.
+constexpr int kTileBytes = 243 * (int)ST_TILE * 4;
+constexpr int kTileTries = 1 << 22;  // polls of the copy's barrier before the kernel gives up
+__device__ __forceinline__ bool tile_landed(uint64_t* bar) {
+  const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
+  for (int i = 0; i < kTileTries; i++) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(b) : "memory");
+    if (ok) return true;
+  }
+  return false;
 }
 
+// threads of a CTA of the persistent kernel: two teams (FP32), 32 x CTY x 3
+// for the row-split sweeps (FP64)
 template <typename T>
-__global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bottom_grid(const __grid_constant__ BottomArgs<T> A,
-                                                                 unsigned* bar) {
+constexpr int gb_threads() { return sizeof(T) == 4 ? kTeams * kTeam : 32 * CTY * 3; }
+// shared exchange of the sweeps: [teams][9][12][G9] floats (FP32), [3][CTY][32] T (FP64)
+template <typename T>
+constexpr int gb_smem() { return sizeof(T) == 4 ? kTeams * 9 * 12 * G9 * 4 : 3 * CTY * 32 * (int)sizeof(T); }
+
+template <typename T>
+__global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid_constant__ BottomArgs<T> A,
+                                                                    unsigned* bar) {
   __shared__ __align__(16) unsigned char sres[gb_smem<T>()];
+  extern __shared__ __align__(128) unsigned char stile[];  // FP32: this CTA's stencil tile
+  __shared__ __align__(8) uint64_t tbar;
   constexpr int NT = gb_threads<T>();
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int g0 = blockIdx.x * NT + tid, gs = gridDim.x * NT;
+  GroupPos own;
+  int own_li = -1;
+  bool landed = true;
+  if constexpr (sizeof(T) == 4) {
+    for (int li = A.lb; li < A.nl - 1; li++)
+      if (A.tile0[li] >= 0 && (int)blockIdx.x >= A.tile0[li] &&
+          (long long)((int)blockIdx.x - A.tile0[li]) * G9 < A.L[li].NP / 4)
+        own_li = li;
+    if (own_li >= 0) {
+      const Level& L = A.L[own_li];
+      const long long t = (int)blockIdx.x - A.tile0[own_li];
+      if (tid == 0) {
+        const uint32_t b = (uint32_t)__cvta_generic_to_shared(&tbar);
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "n"(kTileBytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(stile)),
+                     "l"(L.st32 + t * 243 * ST_TILE), "n"(kTileBytes), "r"(b)
+                     : "memory");
+      }
+      const long long g = t * G9 + tid % G9;
+      own = group_pos(L, g, g < L.NP / 4);
+      __syncthreads();  // the barrier's initialisation, before anyone waits on it
+      landed = false;
+    }
+  }
+  // every CTA with a tile waits for it before the tile's first use
+  auto need_tile = [&](int li) {
+    if (li != own_li || landed) return;
+    if (!tile_landed(&tbar)) {
+      atomicOr(bar, kGbarGone);
+      atomicExch(bar + 2, 1u);
+    }
+    landed = true;
+  };
+  // leaving early: not before the tile's copy has ended
+  auto leave = [&]() {
+    if (!landed) tile_landed(&tbar);
+  };
+  auto sweep = [&](auto mode, auto zero, int li, const T* u, const T* f, T* out, T omega, const T* up, T c1) {
+    constexpr int MODE = decltype(mode)::value;
+    constexpr bool ZERO = decltype(zero)::value;
+    const Level& L = A.L[li];
+    if constexpr (sizeof(T) == 4) {
+      need_tile(li);
+      gb_sweep4<MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, tid, A.tile0[li], own,
+                            reinterpret_cast<const float*>(stile), reinterpret_cast<float (*)[9][12][G9]>(sres));
+    } else {
+      gb_sweep_rows<T, MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, reinterpret_cast<T (*)[CTY][32]>(sres));
+    }
+  };
+  using M0 = std::integral_constant<int, 0>;
+  using M2 = std::integral_constant<int, 2>;
   unsigned goal = 0;
 #define GB_SYNC() \
-  if (!gbar_sync(bar, goal, tid, gridDim.x)) return
+  if (!gbar_sync(bar, goal, tid, gridDim.x)) { leave(); return; }
   T* ucur[BOT_MAX_LEVELS];
   // down: pre-smoothing from a zero iterate, residual, restriction
   for (int li = A.lb; li < A.nl - 1; li++) {
     const Level& L = A.L[li];
-    const T* st = bv_st<T>(L);
     T* u = bv_u<T>(L);
     T *cur = u, *oth = bv_t<T>(L), *prv = bv_r<T>(L);
     for (int s = 0; s < A.pre; s++) {
       // the first step, from a zero iterate, ran with the restriction that
       // formed this level's f (on the first level it is a phase of its own)
       if (s > 0)
-        gb_sweep<T, 2, false>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], s <= 1 ? (const T*)nullptr : prv,
-                              A.c1[li][s], sres);
+        sweep(M2(), std::false_type(), li, cur, bv_f<T>(L), oth, A.om[li][s], s <= 1 ? (const T*)nullptr : prv,
+              A.c1[li][s]);
       else if (li == A.lb)
-        gb_sweep<T, 2, true>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], (const T*)nullptr, A.c1[li][s], sres);
+        sweep(M2(), std::true_type(), li, cur, bv_f<T>(L), oth, A.om[li][s], (const T*)nullptr, A.c1[li][s]);
       if (s > 0 || li == A.lb) GB_SYNC();
       T* w = prv; prv = cur; cur = oth; oth = w;
     }
@@ -1690,7 +1789,7 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
       GB_SYNC();
     }
     ucur[li] = cur;
-    gb_sweep<T, 0, false>(L, st, cur, bv_f<T>(L), oth, T(0), (const T*)nullptr, T(0), sres);
+    sweep(M0(), std::false_type(), li, cur, bv_f<T>(L), oth, T(0), (const T*)nullptr, T(0));
     GB_SYNC();
     {
       const Level& C = A.L[li + 1];
@@ -1734,7 +1833,6 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
   // up: prolongation and post-smoothing; the top level ends in its u
   for (int li = A.nl - 2; li >= A.lb; li--) {
     const Level& L = A.L[li];
-    const T* st = bv_st<T>(L);
     T* u = bv_u<T>(L);
     T *cur = ucur[li], *oth, *prv;
     T* bufs[3] = {u, bv_t<T>(L), bv_r<T>(L)};
@@ -1752,8 +1850,8 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
     bot_prolong3<T>(L, A.L[li + 1], ucur[li + 1], cur, g0, gs);
     GB_SYNC();
     for (int s = 0; s < A.post; s++) {
-      gb_sweep<T, 2, false>(L, st, cur, bv_f<T>(L), oth, A.om[li][s], s == 0 ? (const T*)nullptr : prv,
-                            A.c1[li][s], sres);
+      sweep(M2(), std::false_type(), li, cur, bv_f<T>(L), oth, A.om[li][s], s == 0 ? (const T*)nullptr : prv,
+            A.c1[li][s]);
       if (li > A.lb || s + 1 < A.post || oth != u) GB_SYNC();  // nothing follows the kernel's last step
       T* w = prv; prv = cur; cur = oth; oth = w;
     }
@@ -1761,6 +1859,7 @@ __global__ void __launch_bounds__(gb_threads<T>(), sizeof(T) == 4 ? 2 : 1) k_bot
     if (li == A.lb && cur != u) bot_copy<T>(L, cur, u, g0, gs);
   }
 #undef GB_SYNC
+  leave();
   gbar_exit(bar, tid);
 }
 
@@ -2006,29 +2105,49 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
       h->err = "the persistent bottom kernel takes levels below 2^31 padded nodes";
       return RSO_ERR_UNSUPPORTED;
     }
-  // the persistent kernel: as many CTAs as the largest level has tiles, at
-  // most as many as are resident at once (a cooperative launch refuses more)
+  // the persistent kernel: at most as many CTAs as are resident at once (a
+  // cooperative launch refuses more)
   static std::atomic<int> occ_cache[2][64];
   const int ti = sizeof(T) == 4 ? 0 : 1;
   const int dev = h->device >= 0 && h->device < 64 ? h->device : 0;
+  const int dsm = sizeof(T) == 4 ? kTileBytes : 0;
   int occ = occ_cache[ti][dev].load(std::memory_order_relaxed);
   if (occ <= 0) {
-    RSO_CHECK_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bottom_grid<T>, gb_threads<T>(), 0));
+    RSO_CHECK_CUDA(h, cudaFuncSetAttribute(k_bottom_grid<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
+    RSO_CHECK_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bottom_grid<T>, gb_threads<T>(), dsm));
     occ_cache[ti][dev].store(occ, std::memory_order_relaxed);
   }
   int sms = 0;
   RSO_CHECK_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  long long need = 1;
-  for (int li = lb; li < nl; li++) {
+  const long long most = (long long)occ * sms;
+  // FP32: the levels whose stencil tiles are held in shared memory, the
+  // smallest first, one tile per CTA; then as many CTAs as hold tiles, or as
+  // the streamed levels have pairs of tiles, or the transfers and the coarsest
+  // solve have work for
+  long long need = 1, held = 0;
+  for (int li = 0; li < nl; li++) A.tile0[li] = -1;
+  for (int li = nl - 1; li >= lb; li--) {
     const Level& l = h->L[li];
-    need = std::max(need, sizeof(T) == 4 ? (long long)cdiv(l.NP / 4 * l.nb, G9)
-                                         : (long long)cdiv(l.nx, 32) * cdiv(l.ny, CTY) * l.nz * l.nb);
+    if (sizeof(T) == 8) {
+      need = std::max(need, (long long)cdiv(l.nx, 32) * cdiv(l.ny, CTY) * l.nz * l.nb);
+      continue;
+    }
+    const long long tiles = cdiv(l.NP, ST_TILE);
+    if (li == nl - 1) {
+      need = std::max<long long>(need, cdiv(3LL * h->nc * l.nb, gb_threads<T>() / 32));
+    } else if (held + tiles <= most) {
+      A.tile0[li] = (int)held;
+      held += tiles;
+    } else {
+      need = std::max<long long>(need, cdiv(tiles * l.nb, kTeams));
+    }
+    need = std::max<long long>(need, cdiv(3 * l.nn * l.nb, gb_threads<T>()));
   }
-  const int grid = (int)std::max<long long>(1, std::min<long long>(need, (long long)occ * sms));
+  const int grid = (int)std::max<long long>(1, std::min<long long>(std::max(need, held), most));
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(grid);
   lc.blockDim = sizeof(T) == 4 ? dim3(gb_threads<T>()) : dim3(32, CTY, 3);
-  lc.dynamicSmemBytes = 0;
+  lc.dynamicSmemBytes = dsm;
   lc.stream = h->stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;

@@ -42,3 +42,30 @@ def test_coarse_gauss_seidel(oracle, cuda, gen, reverse):
         u, f = (rng.standard_normal(mask.size) * mask for _ in range(2))
         got = g.gs_relax(lvl, t(u, cuda), t(f, cuda), sweeps=2, reverse=reverse).cpu().numpy()
         assert rel(got, o.smooth(lvl, u, f, kind=0, omega=1.0, sweeps=2, reverse=reverse)) < 1e-12, lvl
+
+
+# bottoms whose levels all fit in shared memory (one tile and a ragged last one, several levels), and
+# one whose first level has more stencil tiles than the GPU has SMs and is streamed
+@pytest.mark.parametrize("dims", [(17, 9, 13), (64, 64, 64), (93, 71, 85), (128, 128, 64)])
+@pytest.mark.parametrize("pre,post", [(2, 2), (1, 3)])
+def test_bottom_kernel_levels(cuda, dims, pre, post):
+    """Mixed solves with the persistent bottom kernel against per-level launches, one system and a
+    batch: the same solution to 1e-8 and iterations within one, as for every launch shape."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(*dims)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None,
+                      Config(poisson_ratio=0.4, pre=pre, post=post, smoother=2, first_factor=2 if dims[0] < 32 else 4,
+                             n_levels=3 if dims[0] < 32 else 0))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    f = t(prob["f"], cuda)
+    F = cuda.stack([f, 0.5 * f.flip(0)])
+    assert g.n_levels() > 2
+    g.set_launch_shapes(4, 1)
+    got = [g.solve(f, tol=1e-10) for _ in range(3)]  # plain launches, the capture, a replay
+    batch, infos = g.solve_batch(F, tol=1e-10)
+    g.set_launch_shapes(4, -1)
+    want, it, _, _ = g.solve(f, tol=1e-10)
+    for u, k, _, _ in got:
+        assert rel(u.cpu().numpy(), want.cpu().numpy()) < 1e-8 and abs(k - it) <= 1
+    assert rel(batch[0].cpu().numpy(), want.cpu().numpy()) < 1e-8 and abs(infos[0][0] - it) <= 1
