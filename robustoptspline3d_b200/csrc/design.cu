@@ -9,77 +9,127 @@
 // dC/dc_ijk = sum_e g_e Nx_i(x_e) Ny_j(y_e) Nz_k(z_e) is evaluated as three
 // successive one-axis contractions (a gather per output, no atomics), instead
 // of the reference's racy per-element scatter (grid/Grid.cu:3797, 3908, 8220).
+// The forward maps go through the same three contractions in reverse.
 #include "rso_internal.cuh"
 #include <cmath>
 #include <algorithm>
 
 namespace rso {
 
-// ---------------------------------------------------------------- sensitivity
-// s_e = -p rho^(p-1) u_e^T K0 u_e (energy=0) or rho^p u_e^T K0 u_e (energy=1)
-__global__ void __launch_bounds__(256) k_sensitivity(const Level L, const double* __restrict__ u,
-                                                     const float* __restrict__ rho, const double* __restrict__ K0g,
-                                                     double p, int energy, float* __restrict__ out) {
-  __shared__ double K0[576];
-  for (int i = threadIdx.x; i < 576; i += blockDim.x) K0[i] = K0g[i];
-  __syncthreads();
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.ne) return;
-  const int x = t % L.ex, y = (t / L.ex) % L.ey, z = t / ((long long)L.ex * L.ey);
-  const long long e = L.eidx(x, y, z);
-  if (!L.emask[e]) { out[e] = 0.f; return; }
-  double ue[24];
-#pragma unroll
-  for (int a = 0; a < 8; a++) {
-    const long long n = L.nidx(x + (a & 1), y + ((a >> 1) & 1), z + (a >> 2));
-    ue[3 * a] = u[n]; ue[3 * a + 1] = u[n + L.NP]; ue[3 * a + 2] = u[n + 2 * L.NP];
-  }
-  double q = 0;
-  for (int i = 0; i < 24; i++) {
-    double s = 0;
-#pragma unroll
-    for (int j = 0; j < 24; j++) s += K0[i * 24 + j] * ue[j];
-    q += ue[i] * s;
-  }
-  const double r = (double)rho[e];
-  out[e] = energy ? (float)(pow(r, p) * q) : (float)(-p * pow(r, p - 1) * q);
+// Element fields come in two layouts, the padded one of the handle and the
+// dense one of the public interface; every kernel here reads and writes either
+// through a view, so that the public calls need no conversion passes (two or
+// three of 99 us each per call at 256^3, as long as most maps themselves).
+struct View {
+  long long off, sz;
+  int sy;
+  __device__ __forceinline__ long long at(int x, int y, int z) const { return off + x + (long long)sy * y + sz * z; }
+};
+static View view_of(const Level& l, bool dense) {
+  if (dense) return {0, (long long)l.ex * l.ey, l.ex};
+  return {1 + (long long)l.qx * (1 + l.qy), (long long)l.qx * l.qy, l.qx};
+}
+// one thread per element, 32 x 8 tiles of a plane (a launch has at most 65535 planes: the kernels step on)
+static dim3 elem_grid(const Level& l) { return dim3(cdiv(l.ex, 32), cdiv(l.ey, 8), std::min(l.ez, 65535)); }
+// FP64 powers by small whole exponents are products, as accurate as pow and a
+// tenth of its instructions
+__device__ __forceinline__ double power(double r, double p) {
+  if (p == 1.0) return r;
+  if (p == 2.0) return r * r;
+  if (p == 3.0) return r * r * r;
+  return pow(r, p);
 }
 
-rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens_pad, int energy) {
+// ---------------------------------------------------------------- sensitivity
+// s_e = -p rho^(p-1) u_e^T K0 u_e (energy=0) or rho^p u_e^T K0 u_e (energy=1).
+// In the sum/difference basis of the element's nodes, w = W u_e along each axis,
+// K0 = W^T B W with the block structure of fine_op.cu, so the quadratic form is
+// a sum over the eight blocks: about 120 operations where the 24 x 24 product
+// takes 600 (256^3, FP64: 1887 us with it, bound by the FP64 units; B.c in the
+// order of cWp: A0 - B0, B0, A7 - B7, B7, P, Q, R, S).
+struct WalshB { double c[8]; };
+__global__ void __launch_bounds__(256) k_sensitivity(const Level L, const double* __restrict__ u,
+                                                     const float* __restrict__ rho, const WalshB B, double p, int energy,
+                                                     float* __restrict__ out, const View V) {
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+  if (x >= L.ex || y >= L.ey) return;
+  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
+    const long long e = L.eidx(x, y, z), o = V.at(x, y, z);
+    if (!L.emask[e]) { out[o] = 0.f; continue; }
+    double w[8][3];  // modes (mx, my, mz) as bits, component
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double f[2][4];  // xy modes of the lower and upper face
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        const double* q = u + L.nidx(x, y, z + b) + c * L.NP;
+        const double a00 = q[0], a10 = q[1], a01 = q[L.px], a11 = q[L.px + 1];
+        const double s0 = a00 + a10, d0 = a10 - a00, s1 = a01 + a11, d1 = a11 - a01;
+        f[b][0] = s0 + s1; f[b][1] = d0 + d1; f[b][2] = s1 - s0; f[b][3] = d1 - d0;
+      }
+#pragma unroll
+      for (int m = 0; m < 4; m++) { w[m][c] = f[0][m] + f[1][m]; w[m + 4][c] = f[1][m] - f[0][m]; }
+    }
+    auto full = [&](double i, double j, double k, double ab, double bb) {
+      const double t = i + j + k;
+      return ab * (i * i + j * j + k * k) + bb * (t * t);
+    };
+    auto pair = [&](double i, double j) { return B.c[4] * (i * i + j * j) + 2.0 * B.c[5] * (i * j); };
+    auto both = [&](double i, double j, double k) { return B.c[6] * ((i + j) * (i + j)) + B.c[7] * (k * k); };
+    double q = full(w[1][0], w[2][1], w[4][2], B.c[0], B.c[1]) + full(w[6][0], w[5][1], w[3][2], B.c[2], B.c[3]);
+    q += pair(w[3][1], w[5][2]) + pair(w[3][0], w[6][2]) + pair(w[5][0], w[6][1]);
+    q += both(w[2][0], w[1][1], w[7][2]) + both(w[4][0], w[1][2], w[7][1]) + both(w[4][1], w[2][2], w[7][0]);
+    const double r = (double)rho[e];
+    out[o] = energy ? (float)(power(r, p) * q) : (float)(-p * (p == 1.0 ? 1.0 : power(r, p - 1)) * q);
+  }
+}
+
+rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens, int energy, bool dense) {
   const Level& l = h->L[0];
-  k_sensitivity<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, u_pad, h->rho, h->K0_dev, h->cfg.penal, energy, sens_pad); rso::note_launch();
+  WalshB B;
+  walsh_constants(h->K0, B.c);
+  k_sensitivity<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, u_pad, h->rho, B, h->cfg.penal, energy, sens,
+                                                             view_of(l, dense)); rso::note_launch();
   return launch_check(h, "sensitivity");
 }
 
 // ---------------------------------------------------------------- Heaviside
-__global__ void k_heaviside(const Level L, const float* __restrict__ in, double beta, double rmin,
-                            const uint8_t* __restrict__ shell, int chain, const float* __restrict__ gin,
-                            float* __restrict__ out) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= L.NQ) return;
-  if (!L.emask[e]) { out[e] = 0.f; return; }
-  const double eta = 0.5, den = tanh(beta * eta) + tanh(beta * (1 - eta));
-  const double r = (double)in[e];
-  if (chain) {
-    const double t = tanh(beta * (r - eta));
-    out[e] = (float)((double)gin[e] * beta * (1 - t * t) / den);
-  } else {
-    double v = (tanh(beta * eta) + tanh(beta * (r - eta))) / den;
-    v = fmin(fmax(v, rmin), 1.0);
-    if (shell && shell[e]) v = 1.0;
-    out[e] = (float)v;
+// in, gin and out share one layout and may be the same array; t0 = tanh(beta
+// eta), den = t0 + tanh(beta (1 - eta)), the same for every element
+__global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* in, double beta, double t0, double den,
+                                                   double rmin, const uint8_t* shell, int chain, const float* gin,
+                                                   float* out, const View V) {
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+  if (x >= L.ex || y >= L.ey) return;
+  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
+    const long long o = V.at(x, y, z);
+    if (!L.emask[L.eidx(x, y, z)]) { out[o] = 0.f; continue; }
+    const double eta = 0.5;
+    const double t = tanh(beta * ((double)in[o] - eta));
+    if (chain) {
+      out[o] = (float)((double)gin[o] * beta * (1 - t * t) / den);
+    } else {
+      double v = (t0 + t) / den;
+      v = fmin(fmax(v, rmin), 1.0);
+      if (shell && shell[x + (long long)L.ex * (y + (long long)L.ey * z)]) v = 1.0;
+      out[o] = (float)v;
+    }
   }
 }
 
-rso_status heaviside(rso_handle* h, const float* in_pad, double beta, const uint8_t* shell_pad, float* out_pad) {
+rso_status heaviside(rso_handle* h, const float* in, double beta, const uint8_t* shell, float* out, bool dense) {
   const Level& l = h->L[0];
-  k_heaviside<<<cdiv(l.NQ, 256), 256, 0, h->stream>>>(l, in_pad, beta, h->cfg.rho_min, shell_pad, 0, nullptr, out_pad); rso::note_launch();
+  const double t0 = std::tanh(beta * 0.5), den = t0 + std::tanh(beta * (1 - 0.5));
+  k_heaviside<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, in, beta, t0, den, h->cfg.rho_min, shell, 0, nullptr, out,
+                                                           view_of(l, dense)); rso::note_launch();
   return launch_check(h, "heaviside");
 }
 
-rso_status heaviside_chain(rso_handle* h, const float* rho_pad, double beta, const float* gin, float* gout) {
+rso_status heaviside_chain(rso_handle* h, const float* rho, double beta, const float* gin, float* gout, bool dense) {
   const Level& l = h->L[0];
-  k_heaviside<<<cdiv(l.NQ, 256), 256, 0, h->stream>>>(l, rho_pad, beta, 0.0, nullptr, 1, gin, gout); rso::note_launch();
+  const double t0 = std::tanh(beta * 0.5), den = t0 + std::tanh(beta * (1 - 0.5));
+  k_heaviside<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, rho, beta, t0, den, 0.0, nullptr, 1, gin, gout,
+                                                           view_of(l, dense)); rso::note_launch();
   return launch_check(h, "heaviside_chain");
 }
 
@@ -87,70 +137,279 @@ rso_status heaviside_chain(rso_handle* h, const float* rho_pad, double beta, con
 // weights w(r) = 1 - 6r^2 + 8r^3 - 3r^4, r = |d|/R, |d|^2 <= R^2, reach int(R+0.5)
 struct FOff { int dx, dy, dz; double w; };
 
+// any radius: one thread per element over the tap table
 __global__ void k_filter(const Level L, const FOff* __restrict__ off, int noff, const float* __restrict__ in,
-                         float* __restrict__ out, int mode, const float* __restrict__ wsum) {
-  // mode 0: out = sum w in / sum w;  1: out = sum w (weight sums);  2: out = sum w in/W_n (adjoint)
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.ne) return;
-  const int x = t % L.ex, y = (t / L.ex) % L.ey, z = t / ((long long)L.ex * L.ey);
-  const long long e = L.eidx(x, y, z);
-  if (!L.emask[e]) { out[e] = 0.f; return; }
-  double gs = 0, ws = 0;
-  for (int k = 0; k < noff; k++) {
-    const int xx = x + off[k].dx, yy = y + off[k].dy, zz = z + off[k].dz;
-    if (xx < 0 || yy < 0 || zz < 0 || xx >= L.ex || yy >= L.ey || zz >= L.ez) continue;
-    const long long n = L.eidx(xx, yy, zz);
-    if (!L.emask[n]) continue;
-    const double w = off[k].w;
-    ws += w;
-    if (mode == 0) gs += w * (double)in[n];
-    else if (mode == 2) gs += w * (double)in[n] / (double)wsum[n];
+                         float* __restrict__ out, int mode, const float* __restrict__ wsum, const View V) {
+  // mode 0: out = sum w in / sum w;  1: out = sum w (weight sums, padded);  2: out = sum w in/W_n (adjoint)
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+  if (x >= L.ex || y >= L.ey) return;
+  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
+    const long long e = L.eidx(x, y, z), o = mode == 1 ? e : V.at(x, y, z);
+    if (!L.emask[e]) { out[o] = 0.f; continue; }
+    double gs = 0, ws = 0;
+    for (int k = 0; k < noff; k++) {
+      const int xx = x + off[k].dx, yy = y + off[k].dy, zz = z + off[k].dz;
+      if (xx < 0 || yy < 0 || zz < 0 || xx >= L.ex || yy >= L.ey || zz >= L.ez) continue;
+      const long long n = L.eidx(xx, yy, zz);
+      if (!L.emask[n]) continue;
+      const double w = off[k].w;
+      ws += w;
+      if (mode == 0) gs += w * (double)in[V.at(xx, yy, zz)];
+      else if (mode == 2) gs += w * (double)in[V.at(xx, yy, zz)] / (double)wsum[n];
+    }
+    out[o] = (float)(mode == 0 ? gs / ws : (mode == 1 ? ws : gs));
   }
-  out[e] = (float)(mode == 0 ? gs / ws : (mode == 1 ? ws : gs));
 }
 
-rso_status filter(rso_handle* h, double R, const float* in_pad, float* out_pad, int adjoint) {
-  const Level& l = h->L[0];
-  std::vector<FOff> off;
-  const int Ri = (int)(R + 0.5);
-  const double R2 = R * R;
-  for (int dx = -Ri; dx <= Ri; dx++)
-    for (int dy = -Ri; dy <= Ri; dy++)
-      for (int dz = -Ri; dz <= Ri; dz++) {
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 > R2) continue;
-        const double r = std::sqrt(r2 / R2), rr = r * r;
-        off.push_back({dx, dy, dz, 1 - 6 * rr + 8 * rr * r - 3 * rr * rr});
+// Radii from 1 to under 5.  A CTA of 32 x 8 threads marches along z through a
+// tile of columns.  Each plane, with its halo of RZ elements, is staged once in
+// shared memory as FP64 (so a value is converted once, not once per tap), and a
+// thread adds every neighbour column's value to the 2 dz + 1 outputs it reaches
+// along z, which it keeps in registers: 13 shared loads for the 33 taps of
+// R = 2.  Weights depend on |dx|, |dy|, |dz| alone and sit in shared memory by
+// column, the columns ordered by their reach in z, so that no zero weight is
+// ever multiplied.  Where the planes around an output are full (inside the box
+// and all active, a flag per plane) the weight sum is that of all taps; else
+// the taps sum the mask as well.  256^3, R = 2: 1007 us with a thread walking
+// the table (its loads and conversions), 464 us now.
+constexpr int FTX = 32, FTY = 8, kFiltRZ = 4;
+struct FCol { int dx, dy; double w[kFiltRZ + 1]; };  // one neighbour column; w by |dz|
+struct FPlan { int start[kFiltRZ + 2]; };            // columns [start[d], start[d + 1]) reach d planes up and down
+template <int RZ, int MODE>
+__global__ void __launch_bounds__(FTX* FTY) k_filter_tile(const Level L, const FCol* __restrict__ cols, const FPlan P,
+                                                          const float* __restrict__ in, float* __restrict__ out,
+                                                          const float* __restrict__ wsum, const View V, int zc) {
+  constexpr int WX = FTX + 2 * RZ, WY = FTY + 2 * RZ, NW = WX * WY, NA = 2 * RZ + 1;
+  extern __shared__ __align__(16) unsigned char fsm[];
+  double* sv = reinterpret_cast<double*>(fsm);                       // [2][NW] values, zero where masked
+  float* sm = reinterpret_cast<float*>(sv + 2 * NW);                 // [2][NW] mask
+  double* sw = reinterpret_cast<double*>(sm + 2 * NW);               // [columns][RZ + 1] weights
+  const int ncol = P.start[RZ + 1];
+  int* so = reinterpret_cast<int*>(sw + ncol * (RZ + 1));            // [columns] window offsets
+  __shared__ double wfull[RZ + 1];                                   // all columns' weights, by |dz|
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * FTX + tx;
+  const int x0 = blockIdx.x * FTX, y0 = blockIdx.y * FTY, z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.ez);
+  for (int k = tid; k < ncol; k += FTX * FTY) {
+    const FCol c = cols[k];
+    so[k] = c.dy * WX + c.dx;
+#pragma unroll
+    for (int d = 0; d <= RZ; d++) sw[k * (RZ + 1) + d] = c.w[d];
+  }
+  __syncthreads();
+  if (tid <= RZ) {
+    double s = 0;
+    for (int k = P.start[tid]; k < ncol; k++) s += sw[k * (RZ + 1) + tid];
+    wfull[tid] = s;
+  }
+  const int x = x0 + tx, y = y0 + ty;
+  double acc[NA], wac[NA];
+#pragma unroll
+  for (int k = 0; k < NA; k++) acc[k] = wac[k] = 0;
+  // planes z0 - RZ .. z1 - 1 + RZ; after plane zp output zp - RZ is complete
+  for (int zp = z0 - RZ; zp < z1 + RZ; zp++) {
+    const int buf = (zp - z0 + RZ) & 1;
+    double* v = sv + buf * NW;
+    float* m = sm + buf * NW;
+    bool full = true;
+    for (int k = tid; k < NW; k += FTX * FTY) {
+      const int wy = k / WX, wx = k - wy * WX, xx = x0 + wx - RZ, yy = y0 + wy - RZ;
+      double a = 0;
+      float on = 0.f;
+      if (xx >= 0 && yy >= 0 && zp >= 0 && xx < L.ex && yy < L.ey && zp < L.ez) {
+        const long long e = L.eidx(xx, yy, zp);
+        if (L.emask[e]) {
+          on = 1.f;
+          if (MODE != 1) a = (double)in[V.at(xx, yy, zp)];
+          if (MODE == 2) a /= (double)wsum[e];
+        }
       }
-  // the tap table is kept on the handle and rebuilt only when the radius changes
+      v[k] = a;
+      m[k] = on;
+      full = full && on != 0.f;
+    }
+    full = __syncthreads_and(full) != 0;
+    const int c0 = (ty + RZ) * WX + tx + RZ;
+    if (MODE != 1) {
+#pragma unroll
+      for (int d = 0; d <= RZ; d++)
+        for (int k = P.start[d]; k < P.start[d + 1]; k++) {
+          const double a = v[c0 + so[k]];
+          const double* w = sw + k * (RZ + 1);
+          acc[RZ] = fma(w[0], a, acc[RZ]);
+#pragma unroll
+          for (int j = 1; j <= RZ; j++)
+            if (j <= d) {  // d is a constant of the unrolled loop
+              acc[RZ + j] = fma(w[j], a, acc[RZ + j]);
+              acc[RZ - j] = fma(w[j], a, acc[RZ - j]);
+            }
+        }
+    }
+    if (MODE != 2) {
+      if (full) {
+        wac[RZ] += wfull[0];
+#pragma unroll
+        for (int j = 1; j <= RZ; j++) { wac[RZ + j] += wfull[j]; wac[RZ - j] += wfull[j]; }
+      } else {
+#pragma unroll
+        for (int d = 0; d <= RZ; d++)
+          for (int k = P.start[d]; k < P.start[d + 1]; k++) {
+            if (m[c0 + so[k]] == 0.f) continue;
+            const double* w = sw + k * (RZ + 1);
+            wac[RZ] += w[0];
+#pragma unroll
+            for (int j = 1; j <= RZ; j++)
+              if (j <= d) { wac[RZ + j] += w[j]; wac[RZ - j] += w[j]; }
+          }
+      }
+    }
+    // acc[k] belongs to output zp + k - RZ: acc[0] is complete
+    const int z = zp - RZ;
+    if (z >= z0 && x < L.ex && y < L.ey) {
+      const long long e = L.eidx(x, y, z);
+      const float r = (float)(MODE == 0 ? acc[0] / wac[0] : (MODE == 1 ? wac[0] : acc[0]));
+      out[MODE == 1 ? e : V.at(x, y, z)] = L.emask[e] ? r : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k + 1 < NA; k++) { acc[k] = acc[k + 1]; wac[k] = wac[k + 1]; }
+    acc[NA - 1] = wac[NA - 1] = 0;
+  }
+}
+
+// columns of the tap table of radius R, ordered by their reach in z
+static FPlan filter_columns(double R, int RZ, std::vector<FCol>* cols) {
+  FPlan P = {};
+  const double R2 = R * R;
+  for (int d = 0; d <= RZ; d++) {
+    P.start[d] = (int)cols->size();
+    for (int dy = -RZ; dy <= RZ; dy++)
+      for (int dx = -RZ; dx <= RZ; dx++) {
+        const int h2 = dx * dx + dy * dy;
+        if (h2 + d * d > R2 || (d < RZ && h2 + (d + 1) * (d + 1) <= R2)) continue;  // its reach is d
+        FCol c = {dx, dy, {}};
+        for (int k = 0; k <= d; k++) {
+          const double r = std::sqrt((h2 + k * k) / R2), rr = r * r;
+          c.w[k] = 1 - 6 * rr + 8 * rr * r - 3 * rr * rr;
+        }
+        cols->push_back(c);
+      }
+  }
+  for (int d = RZ + 1; d < kFiltRZ + 2; d++) P.start[d] = (int)cols->size();
+  return P;
+}
+
+template <int RZ>
+static rso_status filter_tiles(rso_handle* h, const FPlan& P, const float* in, float* out, int adjoint, const View& V) {
+  const Level& l = h->L[0];
+  const FCol* cols = static_cast<const FCol*>(h->filt_taps);
+  // planes per chunk: each chunk stages 2 RZ planes more than it writes, so
+  // chunks are as long as the grid still has four CTAs per SM with them
+  int zc = 64;
+  while (zc > 8 && (long long)cdiv(l.ex, FTX) * cdiv(l.ey, FTY) * cdiv(l.ez, zc) < 4 * 148) zc /= 2;
+  const dim3 g(cdiv(l.ex, FTX), cdiv(l.ey, FTY), cdiv(l.ez, zc)), b(FTX, FTY);
+  const int nw = (FTX + 2 * RZ) * (FTY + 2 * RZ), nc = P.start[RZ + 1];
+  const size_t smem = nw * 2 * (sizeof(double) + sizeof(float)) + nc * ((RZ + 1) * sizeof(double) + sizeof(int));
+  if (!adjoint) {
+    k_filter_tile<RZ, 0><<<g, b, smem, h->stream>>>(l, cols, P, in, out, nullptr, V, zc); rso::note_launch();
+  } else {
+    float* W = h->e_d;
+    k_filter_tile<RZ, 1><<<g, b, smem, h->stream>>>(l, cols, P, nullptr, W, nullptr, V, zc); rso::note_launch();
+    k_filter_tile<RZ, 2><<<g, b, smem, h->stream>>>(l, cols, P, in, out, W, V, zc); rso::note_launch();
+  }
+  return launch_check(h, "filter");
+}
+
+rso_status filter(rso_handle* h, double R, const float* in, float* out, int adjoint, bool dense) {
+  const Level& l = h->L[0];
+  const View V = view_of(l, dense);
+  const int Ri = (int)(R + 0.5);
+  const int RZ = R < kFiltRZ + 1 ? (int)R : 0;  // 0: the general kernel
+  std::vector<FOff> off;
+  std::vector<FCol> cols;
+  FPlan P = {};
+  if (RZ > 0) {
+    P = filter_columns(R, RZ, &cols);
+  } else {
+    const double R2 = R * R;
+    for (int dx = -Ri; dx <= Ri; dx++)
+      for (int dy = -Ri; dy <= Ri; dy++)
+        for (int dz = -Ri; dz <= Ri; dz++) {
+          const double r2 = dx * dx + dy * dy + dz * dz;
+          if (r2 > R2) continue;
+          const double r = std::sqrt(r2 / R2), rr = r * r;
+          off.push_back({dx, dy, dz, 1 - 6 * rr + 8 * rr * r - 3 * rr * rr});
+        }
+  }
+  // the table is kept on the handle and rebuilt only when the radius changes
+  const void* table = RZ > 0 ? (const void*)cols.data() : (const void*)off.data();
+  const long long bytes = RZ > 0 ? (long long)(sizeof(FCol) * cols.size()) : (long long)(sizeof(FOff) * off.size());
   if (!h->filt_taps || h->filt_radius != R) {
-    if ((long long)off.size() > h->filt_cap) {
+    h->filt_radius = -1.0;
+    if (bytes > h->filt_cap) {
       if (h->filt_taps) RSO_CHECK_CUDA(h, cudaFree(h->filt_taps));
       h->filt_taps = nullptr;
-      RSO_CHECK_CUDA(h, cudaMalloc(&h->filt_taps, sizeof(FOff) * off.size()));
-      h->filt_cap = (long long)off.size();
+      h->filt_cap = 0;
+      RSO_CHECK_CUDA(h, cudaMalloc(&h->filt_taps, bytes));
+      h->filt_cap = bytes;
     }
-    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->filt_taps, off.data(), sizeof(FOff) * off.size(), cudaMemcpyHostToDevice,
-                                      h->stream));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->filt_taps, table, bytes, cudaMemcpyHostToDevice, h->stream));
     // the host table is a local vector: finish the copy before it goes away
     RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
     h->filt_radius = R;
   }
+  if (RZ == 1) return filter_tiles<1>(h, P, in, out, adjoint, V);
+  if (RZ == 2) return filter_tiles<2>(h, P, in, out, adjoint, V);
+  if (RZ == 3) return filter_tiles<3>(h, P, in, out, adjoint, V);
+  if (RZ == 4) return filter_tiles<4>(h, P, in, out, adjoint, V);
   const FOff* d_off = static_cast<const FOff*>(h->filt_taps);
+  const int n = (int)off.size();
   if (!adjoint) {
-    k_filter<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, d_off, (int)off.size(), in_pad, out_pad, 0, nullptr); rso::note_launch();
+    k_filter<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, d_off, n, in, out, 0, nullptr, V); rso::note_launch();
   } else {
     float* W = h->e_d;
-    k_filter<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, d_off, (int)off.size(), in_pad, W, 1, nullptr); rso::note_launch();
-    k_filter<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, d_off, (int)off.size(), in_pad, out_pad, 2, W); rso::note_launch();
+    k_filter<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, d_off, n, in, W, 1, nullptr, V); rso::note_launch();
+    k_filter<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, d_off, n, in, out, 2, W, V); rso::note_launch();
   }
   return launch_check(h, "filter");
 }
 
 // ---------------------------------------------------------------- volume
-rso_status volume(rso_handle* h, const float* rho_pad, double* vol) {
+// sum of the active elements: a warp per row of elements
+constexpr int kSumBlocks = 592;
+__device__ __forceinline__ double warp_add(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+__global__ void __launch_bounds__(256) k_sum_elems(const Level L, const float* __restrict__ a, const View V,
+                                                   double* __restrict__ part) {
+  __shared__ double ws[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double s = 0;
+  for (int r = blockIdx.x * 8 + warp; r < L.ey * L.ez; r += gridDim.x * 8) {
+    const int z = r / L.ey, y = r - z * L.ey;
+    const uint8_t* m = L.emask + L.eidx(0, y, z);
+    const float* q = a + V.at(0, y, z);
+    for (int x = lane; x < L.ex; x += 32) s += m[x] ? (double)q[x] : 0.0;
+  }
+  s = warp_add(s);
+  if (lane == 0) ws[warp] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0;
+    for (int k = 0; k < 8; k++) t += ws[k];
+    part[blockIdx.x] = t;
+  }
+}
+rso_status sum_elems(rso_handle* h, const float* a, bool dense, double* dev_out) {
   const Level& l = h->L[0];
-  RSO_TRY(sum_float(h, rho_pad, l.NQ, h->scal + 14));
+  const int blocks = std::min(kSumBlocks, cdiv((long long)l.ey * l.ez, 8));
+  k_sum_elems<<<blocks, 256, 0, h->stream>>>(l, a, view_of(l, dense), h->red); rso::note_launch();
+  RSO_TRY(launch_check(h, "sum_elems"));
+  return reduce_partials(h, h->red, blocks, dev_out);
+}
+
+rso_status volume(rso_handle* h, const float* rho, double* vol, bool dense) {
+  RSO_TRY(sum_elems(h, rho, dense, h->scal + 14));
   RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 14, h->scal + 14, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
   // Grid::volumeRatio divides by the GS-padded element count (grid/Grid.cu:5642-5650)
@@ -246,127 +505,204 @@ static SplineDev spline_dev(rso_handle* h, const float* knots_dev) {
   return d;
 }
 
-// ---------------------------------------------------------------- spline forward
-__global__ void k_coeff2density(const Level L, SplineDev S, const double* __restrict__ c, double rmin,
-                                const uint8_t* __restrict__ shell, float* __restrict__ out) {
+// ---------------------------------------------------------------- spline rows
+// The tensor-product spline at the element centres is contracted one axis at a
+// time: first z, R1[z][j][i] = sum_k c[k][j][i] B_k(z), then y,
+// R2[z][y][i] = sum_j R1[z][j][i] B_j(y), a row of nb0 values per row of
+// elements; an element then sums `order` of them along x, instead of order^3
+// coefficients (the rows are nb0 / ex of the elements: 1/8 for 32 coefficients
+// on 256).  D as well as N along z or y gives the rows of the derivatives.
+// Rows outside the knots are zero.
+__global__ void __launch_bounds__(256) k_rows_z(SplineDev S, int ez, const double* __restrict__ c,
+                                                double* __restrict__ rn, double* __restrict__ rd) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.ne) return;
-  const int x = t % L.ex, y = (t / L.ex) % L.ey, z = t / ((long long)L.ex * L.ey);
-  const long long e = L.eidx(x, y, z);
-  if (!L.emask[e]) { out[e] = 0.f; return; }
-  const int o = S.order;
-  const int i = S.i0[x], j = S.i1[y], k = S.i2[z];
-  double v;
-  if (i < 0 || j < 0 || k < 0) {
-    v = -0.2;
-  } else {
-    v = 0;
-    const double* Nx = S.N0 + x * o;
-    const double* Ny = S.N1 + y * o;
-    const double* Nz = S.N2 + z * o;
-    for (int cz = 0; cz < o; cz++)
-      for (int cy = 0; cy < o; cy++) {
-        const double wyz = Ny[cy] * Nz[cz];
-        const double* row = c + (i - o) + (long long)(j - o + cy) * S.nb0 + (long long)(k - o + cz) * S.nb0 * S.nb1;
-        for (int cx = 0; cx < o; cx++) v += row[cx] * Nx[cx] * wyz;
+  const long long pl = (long long)S.nb0 * S.nb1;
+  if (t >= pl * ez) return;
+  const int z = (int)(t / pl);
+  const long long ij = t - pl * z;
+  const int k0 = S.i2[z] - S.order;
+  double n = 0, d = 0;
+  if (k0 >= 0)
+    for (int q = 0; q < S.order; q++) {
+      const double v = c[ij + (k0 + q) * pl];
+      n += v * S.N2[z * S.order + q];
+      if (rd) d += v * S.D2[z * S.order + q];
+    }
+  rn[t] = n;
+  if (rd) rd[t] = d;
+}
+// rows NN from rn; with rd also DN (D along y) and ND (D along z), `comp` apart
+__global__ void __launch_bounds__(256) k_rows_y(SplineDev S, int ey, int ez, const double* __restrict__ rn,
+                                                const double* __restrict__ rd, double* __restrict__ out,
+                                                long long comp) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= comp) return;
+  const long long yz = t / S.nb0;
+  const int i = (int)(t - yz * S.nb0), z = (int)(yz / ey), y = (int)(yz - (long long)z * ey);
+  const int j0 = S.i1[y] - S.order;
+  double nn = 0, dn = 0, nd = 0;
+  if (j0 >= 0) {
+    const long long base = i + (long long)S.nb0 * (j0 + (long long)S.nb1 * z);
+    for (int q = 0; q < S.order; q++) {
+      const double v = rn[base + (long long)q * S.nb0], N = S.N1[y * S.order + q];
+      nn += v * N;
+      if (rd) {
+        dn += v * S.D1[y * S.order + q];
+        nd += rd[base + (long long)q * S.nb0] * N;
       }
+    }
   }
-  v = fmin(fmax(v, rmin), 1.0);
-  if (shell && shell[e]) v = 1.0;
-  out[e] = (float)v;
+  out[t] = nn;
+  if (rd) { out[t + comp] = dn; out[t + 2 * comp] = nd; }
 }
 
-rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell_pad, float* out_pad) {
+static rso_status spline_rows(rso_handle* h, const SplineDev& S, const double* c, double* R, bool derivatives) {
+  const Level& l = h->L[0];
+  const long long nz = (long long)S.nb0 * S.nb1 * l.ez, comp = (long long)S.nb0 * l.ey * l.ez;
+  double* rn = h->sp.work[1];
+  double* rd = derivatives ? rn + nz : nullptr;
+  k_rows_z<<<cdiv(nz, 256), 256, 0, h->stream>>>(S, l.ez, c, rn, rd); rso::note_launch();
+  k_rows_y<<<cdiv(comp, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, rn, rd, R, comp); rso::note_launch();
+  return launch_check(h, "spline rows");
+}
+
+// ---------------------------------------------------------------- spline forward
+__global__ void __launch_bounds__(256) k_coeff2density(const Level L, SplineDev S, const double* __restrict__ R,
+                                                       double rmin, const uint8_t* __restrict__ shell,
+                                                       float* __restrict__ out, const View V) {
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+  if (x >= L.ex || y >= L.ey) return;
+  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
+    const long long o = V.at(x, y, z);
+    if (!L.emask[L.eidx(x, y, z)]) { out[o] = 0.f; continue; }
+    const int i = S.i0[x];
+    double v;
+    if (i < 0 || S.i1[y] < 0 || S.i2[z] < 0) {
+      v = -0.2;
+    } else {
+      const double* row = R + (long long)S.nb0 * (y + (long long)L.ey * z) + (i - S.order);
+      v = 0;
+      for (int q = 0; q < S.order; q++) v += row[q] * S.N0[x * S.order + q];
+    }
+    v = fmin(fmax(v, rmin), 1.0);
+    if (shell && shell[x + (long long)L.ex * (y + (long long)L.ey * z)]) v = 1.0;
+    out[o] = (float)v;
+  }
+}
+
+rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, float* out, bool dense) {
   const Level& l = h->L[0];
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
-  k_coeff2density<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, spline_dev(h, h->sp.knots_dev), c, h->cfg.rho_min,
-                                                           shell_pad, out_pad); rso::note_launch();
+  const SplineDev S = spline_dev(h, h->sp.knots_dev);
+  RSO_TRY(spline_rows(h, S, c, h->sp.work[0], false));
+  k_coeff2density<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, S, h->sp.work[0], h->cfg.rho_min, shell, out,
+                                                               view_of(l, dense)); rso::note_launch();
   return launch_check(h, "coeff2density");
 }
 
 // ---------------------------------------------------------------- separable adjoint
-// stage 1: G1[a][y][z] = sum_x w(x,y,z) Bx(x)[a - i0(x) + o]   (a = basis index along x)
-__global__ void k_sep1(const Level L, SplineDev S, const double* __restrict__ wpad, const float* __restrict__ wpadf,
-                       int dx, const int* __restrict__ lo, const int* __restrict__ hi, double* __restrict__ G1) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long tot = (long long)S.nb0 * L.ey * L.ez;
-  if (t >= tot) return;
-  const int a = t % S.nb0;
-  const long long yz = t / S.nb0;
-  const int y = yz % L.ey, z = yz / L.ey;
+// Stage 1, x: a warp takes a row of elements, `seg` of them at a time, their
+// weights in shared memory, and sums for each basis function over its support:
+// G1[z][y][a] (+)= sum_x w(x) B_a(x).  Row reads are coalesced and every weight
+// is read from memory once (a thread per (a, y, z) read each `order` times, 202
+// us at 256^3 and 32 coefficients).
+constexpr int kSeg = 128;
+// sum over the segment [xa, xb) of w B for basis function a; lo, hi its support
+__device__ __forceinline__ double seg_sum(const SplineDev& S, const double* __restrict__ B, const double* w, int a,
+                                          int lo, int hi, int xa, int xb) {
   double s = 0;
-  if (S.i1[y] >= 0 && S.i2[z] >= 0) {
-    const int o = S.order;
-    const double* B = dx ? S.D0 : S.N0;
-    for (int x = lo[a]; x <= hi[a]; x++) {
-      const long long e = L.eidx(x, y, z);
-      const double w = wpad ? wpad[e] : (double)wpadf[e];
-      if (w == 0) continue;
-      s += w * B[x * o + a - S.i0[x] + o];
-    }
-  }
-  G1[t] = s;
+  for (int x = max(lo, xa); x <= min(hi, xb - 1); x++) s += w[x - xa] * B[x * S.order + a - S.i0[x] + S.order];
+  return s;
 }
-// stage 2: G2[a][b][z] = sum_y G1[a][y][z] By(y)[b - i1(y) + o]
-__global__ void k_sep2(const Level L, SplineDev S, const double* __restrict__ G1, int dy, const int* __restrict__ lo,
-                       const int* __restrict__ hi, double* __restrict__ G2) {
+// the basis functions a segment's elements lie in the support of: [*a0, *a1)
+__device__ __forceinline__ void seg_range(const SplineDev& S, int xa, int xb, int* a0, int* a1) {
+  const int i = S.i0[xa], j = S.i0[xb - 1];
+  *a0 = i >= 0 ? i - S.order : 0;
+  *a1 = j >= 0 ? j : S.nb0;
+}
+__global__ void __launch_bounds__(256) k_adj_x(const Level L, SplineDev S, const float* __restrict__ g,
+                                               const uint8_t* __restrict__ shell, const View V,
+                                               const int* __restrict__ lo, const int* __restrict__ hi,
+                                               double* __restrict__ G1) {
+  __shared__ double w[8][kSeg];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x * 8 + warp;
+  if (r >= L.ey * L.ez) return;
+  const int z = r / L.ey, y = r - z * L.ey;
+  double* G = G1 + (long long)S.nb0 * r;
+  for (int a = lane; a < S.nb0; a += 32) G[a] = 0;
+  if (S.i1[y] < 0 || S.i2[z] < 0) return;
+  const uint8_t* m = L.emask + L.eidx(0, y, z);
+  const float* q = g + V.at(0, y, z);
+  const uint8_t* sh = shell ? shell + (long long)L.ex * r : nullptr;
+  for (int xa = 0; xa < L.ex; xa += kSeg) {
+    const int xb = min(xa + kSeg, L.ex);
+    __syncwarp();
+    for (int x = xa + lane; x < xb; x += 32) w[warp][x - xa] = m[x] && !(sh && sh[x]) ? (double)q[x] : 0.0;
+    __syncwarp();
+    int a0, a1;
+    seg_range(S, xa, xb, &a0, &a1);
+    for (int a = a0 + lane; a < a1; a += 32) G[a] += seg_sum(S, S.N0, w[warp], a, lo[a], hi[a], xa, xb);
+  }
+}
+// Stage 2, y: G2[z][b][a] = sum_y G1[z][y][a] N_b(y) (+ Gd[z][y][a] D_b(y))
+__global__ void __launch_bounds__(256) k_adj_y(SplineDev S, int ey, int ez, const double* __restrict__ G1,
+                                               const double* __restrict__ Gd, const int* __restrict__ lo,
+                                               const int* __restrict__ hi, double* __restrict__ G2) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long tot = (long long)S.nb0 * S.nb1 * L.ez;
-  if (t >= tot) return;
-  const int a = t % S.nb0, b = (t / S.nb0) % S.nb1, z = t / ((long long)S.nb0 * S.nb1);
-  const int o = S.order;
-  const double* B = dy ? S.D1 : S.N1;
+  const long long pl = (long long)S.nb0 * S.nb1;
+  if (t >= pl * ez) return;
+  const int z = (int)(t / pl), ab = (int)(t - pl * z), b = ab / S.nb0, a = ab - b * S.nb0;
   double s = 0;
-  for (int y = lo[b]; y <= hi[b]; y++) s += G1[a + (long long)S.nb0 * (y + (long long)L.ey * z)] * B[y * o + b - S.i1[y] + o];
+#pragma unroll 4
+  for (int y = lo[b]; y <= hi[b]; y++) {
+    const long long g = a + (long long)S.nb0 * (y + (long long)ey * z);
+    const int k = y * S.order + b - S.i1[y] + S.order;
+    s += G1[g] * S.N1[k];
+    if (Gd) s += Gd[g] * S.D1[k];
+  }
   G2[t] = s;
 }
-// stage 3: dc[a][b][c] += scale * sum_z G2[a][b][z] Bz(z)[c - i2(z) + o]
-__global__ void k_sep3(const Level L, SplineDev S, const double* __restrict__ G2, int dz, const int* __restrict__ lo,
-                       const int* __restrict__ hi, double scale, int accumulate, double* __restrict__ dc) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long tot = (long long)S.nb0 * S.nb1 * S.nb2;
-  if (t >= tot) return;
-  const int ab = t % ((long long)S.nb0 * S.nb1), c = t / ((long long)S.nb0 * S.nb1);
-  const int o = S.order;
-  const double* B = dz ? S.D2 : S.N2;
+// Stage 3, z: dc[c][b][a] = scale (sum_z G2[z][b][a] N_c(z) (+ Gd[z][b][a] D_c(z))); scale from
+// *count (its reciprocal, 0 for 0) when given.  The supports are a fifth of the box or
+// more and there are few coefficients, so eight lanes share one and meet by shuffles.
+__global__ void __launch_bounds__(256) k_adj_z(SplineDev S, const double* __restrict__ G2,
+                                               const double* __restrict__ Gd, const int* __restrict__ lo,
+                                               const int* __restrict__ hi, const double* __restrict__ count,
+                                               double* __restrict__ dc) {
+  const long long pl = (long long)S.nb0 * S.nb1, tot = pl * S.nb2;
+  const long long t = blockIdx.x * 32LL + threadIdx.x;  // blockDim (32, 8)
+  __shared__ double part[8][32];
   double s = 0;
-  for (int z = lo[c]; z <= hi[c]; z++) s += G2[ab + (long long)S.nb0 * S.nb1 * z] * B[z * o + c - S.i2[z] + o];
-  dc[t] = (accumulate ? dc[t] : 0.0) + scale * s;
+  if (t < tot) {
+    const int c = (int)(t / pl);
+    const long long ab = t - pl * c;
+    for (int z = lo[c] + threadIdx.y; z <= hi[c]; z += 8) {
+      const int k = z * S.order + c - S.i2[z] + S.order;
+      s += G2[ab + pl * z] * S.N2[k];
+      if (Gd) s += Gd[ab + pl * z] * S.D2[k];
+    }
+  }
+  part[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0 || t >= tot) return;
+  for (int k = 1; k < 8; k++) s += part[k][threadIdx.x];
+  const double scale = count ? (*count == 0 ? 0.0 : 1.0 / *count) : 1.0;
+  dc[t] = scale * s;
 }
 
-
-// dc (+)= scale * sum_e w_e Bx By Bz, w given as double (wd) or float (wf) padded element field
-static rso_status separable_adjoint(rso_handle* h, const double* wd, const float* wf, int dx, int dy, int dz,
-                                    double scale, int accumulate, double* dc) {
-  const Level& l = h->L[0];
-  SplineDev S = spline_dev(h, h->sp.knots_dev);
-  double* G1 = h->sp.work[0];
-  double* G2 = h->sp.work[1];
-  const long long t1 = (long long)S.nb0 * l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
-                  t3 = (long long)S.nb0 * S.nb1 * S.nb2;
-  int* r0 = h->sp.ranges[0];
-  int* r1 = h->sp.ranges[1];
-  int* r2 = h->sp.ranges[2];
-  k_sep1<<<cdiv(t1, 256), 256, 0, h->stream>>>(l, S, wd, wf, dx, r0, r0 + S.nb0, G1); rso::note_launch();
-  k_sep2<<<cdiv(t2, 256), 256, 0, h->stream>>>(l, S, G1, dy, r1, r1 + S.nb1, G2); rso::note_launch();
-  k_sep3<<<cdiv(t3, 256), 256, 0, h->stream>>>(l, S, G2, dz, r2, r2 + S.nb2, scale, accumulate, dc); rso::note_launch();
-  return launch_check(h, "separable_adjoint");
-}
-
-// element weights for the density adjoint: g on active, non-shell elements inside the spline domain
-__global__ void k_mask_weights(const Level L, const float* __restrict__ g, const uint8_t* __restrict__ shell,
-                               double* __restrict__ w) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= L.NQ) return;
-  w[e] = (L.emask[e] && !(shell && shell[e])) ? (double)g[e] : 0.0;
-}
-
-rso_status density2coeff(rso_handle* h, const float* g_pad, const uint8_t* shell_pad, double* dc) {
+rso_status density2coeff(rso_handle* h, const float* g, const uint8_t* shell, double* dc, bool dense) {
   const Level& l = h->L[0];
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
-  double* w = h->sp.work[2];
-  k_mask_weights<<<cdiv(l.NQ, 256), 256, 0, h->stream>>>(l, g_pad, shell_pad, w); rso::note_launch();
-  return separable_adjoint(h, w, nullptr, 0, 0, 0, 1.0, 0, dc);
+  const SplineDev S = spline_dev(h, h->sp.knots_dev);
+  double *G1 = h->sp.work[0], *G2 = h->sp.work[1];
+  const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1], *r2 = h->sp.ranges[2];
+  const long long rows = (long long)l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
+                  t3 = (long long)S.nb0 * S.nb1 * S.nb2;
+  k_adj_x<<<cdiv(rows, 8), 256, 0, h->stream>>>(l, S, g, shell, view_of(l, dense), r0, r0 + S.nb0, G1); rso::note_launch();
+  k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, G1, nullptr, r1, r1 + S.nb1, G2); rso::note_launch();
+  k_adj_z<<<cdiv(t3, 32), dim3(32, 8), 0, h->stream>>>(S, G2, nullptr, r2, r2 + S.nb2, nullptr, dc); rso::note_launch();
+  return launch_check(h, "density2coeff");
 }
 
 // ---------------------------------------------------------------- self-support
@@ -381,36 +717,11 @@ struct SSPar {
   double beta, cosang, mid, sc, fpara, na, ia;
 };
 
-// pass 1: value, gradient and orientation probe per active element
-__global__ void k_ss_eval(const Level L, SplineDev S, const double* __restrict__ c, SSPar P,
-                          double* __restrict__ fv, double* __restrict__ gx, double* __restrict__ gy,
-                          double* __restrict__ gz, float* __restrict__ dir) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.ne) return;
-  const int x = t % L.ex, y = (t / L.ex) % L.ey, z = t / ((long long)L.ex * L.ey);
-  const long long e = L.eidx(x, y, z);
-  if (!L.emask[e]) { fv[e] = 0; gx[e] = gy[e] = gz[e] = 0; dir[e] = 0.f; return; }
+// Sign of the orientation probe (grid/Grid.cu:7623-7714) by evaluating it: the
+// spline 0.01 h along the gradient, through the Heaviside step
+__device__ __noinline__ float probe_sign(const SplineDev& S, const double* __restrict__ c, double beta, int x, int y,
+                                         int z, bool inside, double v, double g0, double g1, double g2) {
   const int o = S.order;
-  const int I = S.i0[x], J = S.i1[y], K = S.i2[z];
-  const bool inside = I >= 0 && J >= 0 && K >= 0;
-  double v = 0, g0 = 0, g1 = 0, g2 = 0;
-  if (inside) {
-    const double *N0 = S.N0 + x * o, *N1 = S.N1 + y * o, *N2 = S.N2 + z * o;
-    const double *D0 = S.D0 + x * o, *D1 = S.D1 + y * o, *D2 = S.D2 + z * o;
-    for (int q = 0; q < o; q++)
-      for (int b = 0; b < o; b++) {
-        const double* row = c + (I - o) + (long long)(J - o + b) * S.nb0 + (long long)(K - o + q) * S.nb0 * S.nb1;
-        for (int a = 0; a < o; a++) {
-          const double cc = row[a];
-          v += cc * N0[a] * N1[b] * N2[q];
-          g0 += cc * D0[a] * N1[b] * N2[q];
-          g1 += cc * N0[a] * D1[b] * N2[q];
-          g2 += cc * N0[a] * N1[b] * D2[q];
-        }
-      }
-  }
-  fv[e] = v; gx[e] = g0; gy[e] = g1; gz[e] = g2;
-  // orientation probe 0.01 h along the gradient (grid/Grid.cu:7623-7714)
   const double pt[3] = {x + 0.5 + 0.01 * g0, y + 0.5 + 0.01 * g1, z + 0.5 + 0.01 * g2};
   int Ii[3];
   double Nb[3][6];
@@ -427,61 +738,187 @@ __global__ void k_ss_eval(const Level L, SplineDev S, const double* __restrict__
                 Nb[0][a] * Nb[1][b] * Nb[2][q];
   }
   const double vv = inside ? v : -0.1;
-  const double s = d_H(vv, P.beta) - d_H(vd, P.beta);
-  dir[e] = s > 0 ? 1.f : -1.f;
+  return d_H(vv, beta) - d_H(vd, beta) > 0 ? 1.f : -1.f;
 }
 
-// pass 2: per-element penalty, count, and the separable gradient weights
-__global__ void k_ss_penalty(const Level L, SplineDev S, SSPar P, double flip, double direction,
-                             const double* __restrict__ fv, const double* __restrict__ gx,
-                             const double* __restrict__ gy, const double* __restrict__ gz, float* __restrict__ per,
-                             double* __restrict__ wA, double* __restrict__ wZ, double* __restrict__ wX,
-                             double* __restrict__ wY, float* __restrict__ down) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.ne) return;
-  const int x = t % L.ex, y = (t / L.ex) % L.ey, z = t / ((long long)L.ex * L.ey);
-  const long long e = L.eidx(x, y, z);
-  wA[e] = wZ[e] = wX[e] = wY[e] = 0;
-  if (!L.emask[e]) { if (per) per[e] = 0.f; down[e] = 0.f; return; }
-  const double n0 = flip * gx[e], n1 = flip * gy[e], n2 = flip * gz[e];
-  const double nn = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
-  const double inner = n2 / nn / P.cosang;
-  const bool dn = n2 < 0;
-  down[e] = dn ? 1.f : 0.f;
-  const double f = fv[e];
-  const double nd = exp(-P.na * (f - 0.5) * (f - 0.5));
-  const double dnd = -2 * P.na * (f - 0.5) * nd;
-  const double ex_ = exp(-(inner - P.mid) / P.sc);
-  const double ov = 2 / (1 + ex_), dov = 2 / (1 + ex_) / (1 + ex_) / P.sc * ex_;
-  const double in_ = inner > 1 ? P.ia * (inner - 1) + 1 : 1, din = inner > 1 ? P.ia : 1;
-  double val = 0, A = 0, B = 0;
-  const int m = P.mode;
-  const bool on = (m % 2 == 1) || dn;
-  if (on) {
-    if (m <= 1) { val = pow(inner, P.fpara); B = P.fpara * pow(inner, P.fpara - 1); }
-    else if (m <= 3) { val = inner >= 1 ? P.fpara * (inner - 1) * (inner - 1) : 0; B = inner >= 1 ? 2 * P.fpara * (inner - 1) : 0; }
-    else { val = nd * ov * in_; A = dnd * ov * in_; B = nd * dov * in_ + nd * ov * din; }
+// largest |c|; one CTA
+__global__ void __launch_bounds__(1024) k_max_abs(long long n, const double* __restrict__ c, double* __restrict__ out) {
+  __shared__ double sh[32];
+  double m = 0;
+#pragma unroll 8
+  for (long long i = threadIdx.x; i < n; i += 1024) m = fmax(m, fabs(c[i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 32; k++) m = fmax(m, sh[k]);
+    *out = m;
   }
-  if (per) per[e] = (float)val;
-  const bool inside = S.i0[x] >= 0 && S.i1[y] >= 0 && S.i2[z] >= 0;
-  if (!inside) return;
-  // dinner = al*(N N dN) + be*(dN N N) + ga*(N dN N)  (see compute_spline_bg_selfsupp_constraint_dcoeff)
-  const double den = nn * nn * P.cosang;
-  const double al = direction * (nn - n2 * n2 / nn) / den;
-  const double be = -direction * n2 * n0 / nn / den;
-  const double ga = -direction * n2 * n1 / nn / den;
-  wA[e] = A;
-  wZ[e] = B * al;
-  wX[e] = B * be;
-  wY[e] = B * ga;
 }
 
+// The constraint on every element in one pass: value and gradient from the
+// spline rows, the probe's sign, the penalty, and stage 1 (x) of the separable
+// adjoint of its three weights.  A warp takes a row of elements, kSeg at a time.
+//
+// The probe walks t = 0.01 along the gradient g, so the spline there is at
+// least v + t |g|^2 (1 - t H / 2), H a bound on its second derivatives: for
+// order >= 3, |d2/dx2| <= 4 p (p - 1) M / s^2 and |d2/dxdy| <= 4 p^2 M / (s s')
+// with M the largest coefficient, s the knot spacings and p = order - 1 (hcoef
+// holds H / M).  Where that growth times the least slope of the step between the
+// two values is far above the rounding of the two tanh, the probe's sign is
+// known, -1, without evaluating it (64 coefficients, three basis recursions and
+// six tanh: 3.4 of the 3.65 ms this stage took at 256^3); elsewhere probe_sign
+// decides, as before.
+//
+// The penalty needs the sign `flip` that the sum of all probes gives.  It is
+// taken as -1 (`direction` likewise), which the sum confirms in every design
+// whose density grows along its gradient; the caller runs the pass again when
+// it does not.
+struct SSOut { double *G1, *Gy, *Gz; float* per; double* part; };
+constexpr int kSSRows = 4;
+__global__ void __launch_bounds__(32 * kSSRows) k_ss_rows(const Level L, SplineDev S, const double* __restrict__ c,
+                                                          const double* __restrict__ R, long long comp, const SSPar P,
+                                                          double flip, double direction, const double* __restrict__ cmax,
+                                                          double hcoef, double smin, const int* __restrict__ lo,
+                                                          const int* __restrict__ hi, const SSOut O, const View V) {
+  __shared__ double w[kSSRows][4][kSeg];
+  __shared__ double red[kSSRows][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x * kSSRows + warp;
+  double sdir = 0, sper = 0, sdown = 0;
+  if (r < L.ey * L.ez) {
+    const int z = r / L.ey, y = r - z * L.ey, o = S.order;
+    const long long gb = (long long)S.nb0 * r;
+    const bool in_yz = S.i1[y] >= 0 && S.i2[z] >= 0;
+    const double tH = 0.01 * hcoef * *cmax;
+    for (int a = lane; a < S.nb0; a += 32) O.G1[gb + a] = O.Gy[gb + a] = O.Gz[gb + a] = 0;
+    for (int xa = 0; xa < L.ex; xa += kSeg) {
+      const int xb = min(xa + kSeg, L.ex);
+      __syncwarp();
+      for (int x = xa + lane; x < xb; x += 32) {
+        double wA = 0, wX = 0, wY = 0, wZ = 0;
+        float val32 = 0.f;
+        if (L.emask[L.eidx(x, y, z)]) {
+          const int I = S.i0[x];
+          const bool inside = I >= 0 && in_yz;
+          double f = 0, g0 = 0, g1 = 0, g2 = 0;
+          if (inside) {
+            const double* row = R + gb + (I - o);
+            for (int q = 0; q < o; q++) {
+              const double N = S.N0[x * o + q], t = row[q];
+              f += t * N;
+              g0 += t * S.D0[x * o + q];
+              g1 += row[q + comp] * N;
+              g2 += row[q + 2 * comp] * N;
+            }
+          }
+          const double gg = g0 * g0 + g1 * g1 + g2 * g2;
+          bool known = false;
+          if (o >= 3 && tH < 1.0 && inside) {
+            const double grow = 0.01 * gg * (1 - 0.5 * tH);
+            // sech^2(s) >= exp(-2 |s|), s up to beta (|v - 1/2| + what the probe may rise)
+            const float slope = __expf((float)(-2 * P.beta * (fabs(f - 0.5) + 0.02 * gg)));
+            known = (float)(P.beta * grow) * slope > 1e-12f && grow > 1e-11 * (1 + *cmax) && 1e-4 * gg < smin * smin;
+          }
+          sdir += known ? -1.0 : (double)probe_sign(S, c, P.beta, x, y, z, inside, f, g0, g1, g2);
+          const double n0 = flip * g0, n1 = flip * g1, n2 = flip * g2;
+          const bool dn = n2 < 0;
+          if (dn) sdown += 1.0;
+          const bool on = (P.mode % 2 == 1) || dn;
+          const double nn = sqrt(gg);
+          // off: no penalty, and zero weights unless the direction is undefined
+          if (on || !(nn > 0) || isinf(nn)) {
+            const double inner = n2 / nn / P.cosang;
+            double val = 0, A = 0, B = 0;
+            if (on) {
+              const int m = P.mode;
+              if (m <= 1) { val = pow(inner, P.fpara); B = P.fpara * pow(inner, P.fpara - 1); }
+              else if (m <= 3) { val = inner >= 1 ? P.fpara * (inner - 1) * (inner - 1) : 0; B = inner >= 1 ? 2 * P.fpara * (inner - 1) : 0; }
+              else {
+                const double nd = exp(-P.na * (f - 0.5) * (f - 0.5));
+                const double dnd = -2 * P.na * (f - 0.5) * nd;
+                const double ex_ = exp(-(inner - P.mid) / P.sc);
+                const double ov = 2 / (1 + ex_), dov = 2 / (1 + ex_) / (1 + ex_) / P.sc * ex_;
+                const double in_ = inner > 1 ? P.ia * (inner - 1) + 1 : 1, din = inner > 1 ? P.ia : 1;
+                val = nd * ov * in_; A = dnd * ov * in_; B = nd * dov * in_ + nd * ov * din;
+              }
+            }
+            val32 = (float)val;
+            if (inside) {
+              // dinner = al*(N N dN) + be*(dN N N) + ga*(N dN N)  (see compute_spline_bg_selfsupp_constraint_dcoeff)
+              const double den = nn * nn * P.cosang;
+              const double al = direction * (nn - n2 * n2 / nn) / den;
+              const double be = -direction * n2 * n0 / nn / den;
+              const double ga = -direction * n2 * n1 / nn / den;
+              wA = A; wZ = B * al; wX = B * be; wY = B * ga;
+            }
+          }
+          sper += (double)val32;
+        }
+        if (O.per) O.per[V.at(x, y, z)] = val32;
+        w[warp][0][x - xa] = wA; w[warp][1][x - xa] = wX; w[warp][2][x - xa] = wY; w[warp][3][x - xa] = wZ;
+      }
+      __syncwarp();
+      if (in_yz) {
+        int a0, a1;
+        seg_range(S, xa, xb, &a0, &a1);
+        for (int a = a0 + lane; a < a1; a += 32) {
+          double s = 0, sy = 0, sz = 0;
+          for (int x = max(lo[a], xa); x <= min(hi[a], xb - 1); x++) {
+            const int k = x * o + a - S.i0[x] + o;
+            const double N = S.N0[k];
+            s += w[warp][0][x - xa] * N + w[warp][1][x - xa] * S.D0[k];
+            sy += w[warp][2][x - xa] * N;
+            sz += w[warp][3][x - xa] * N;
+          }
+          O.G1[gb + a] += s;
+          O.Gy[gb + a] += sy;
+          O.Gz[gb + a] += sz;
+        }
+      }
+    }
+  }
+  sdir = warp_add(sdir);
+  sper = warp_add(sper);
+  sdown = warp_add(sdown);
+  if (lane == 0) { red[warp][0] = sdir; red[warp][1] = sper; red[warp][2] = sdown; }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0;
+    for (int k = 0; k < kSSRows; k++) t += red[k][threadIdx.x];
+    O.part[threadIdx.x * (long long)gridDim.x + blockIdx.x] = t;
+  }
+}
+// out[0..2] = the sums of probes, penalties and downward faces; out[3] the count the mean divides by
+__global__ void __launch_bounds__(512) k_ss_sums(const double* __restrict__ part, int n, int mode, double active,
+                                                 double* __restrict__ out) {
+  __shared__ double sh[16];
+  double tot[3];
+  for (int k = 0; k < 3; k++) {
+    double s = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += 512) s += part[(long long)k * n + i];
+    s = warp_add(s);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    tot[k] = 0;
+    for (int q = 0; q < 16; q++) tot[k] += sh[q];
+  }
+  if (threadIdx.x == 0) {
+    out[0] = tot[0];
+    out[1] = tot[1];
+    out[2] = tot[2];
+    out[3] = mode % 2 == 0 ? tot[2] : active;
+  }
+}
 
 rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, double opt_angle, double default_angle,
-                       float* per_pad, double* dc, double* value, double* count, double* dirsum) {
+                       float* per_dense, double* dc, double* value, double* count, double* dirsum) {
   const Level& l = h->L[0];
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
-  SplineDev S = spline_dev(h, h->sp.knots_dev);
+  const SplineDev S = spline_dev(h, h->sp.knots_dev);
   SSPar P;
   P.mode = mode;
   P.beta = beta;
@@ -491,46 +928,59 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
   P.fpara = mode <= 1 ? 8.0 : (mode <= 3 ? 10.0 : P.sc);  // p_norm, hfunction_c, adapt_sigmoid_c (grid/Grid.h:371-378)
   P.na = 200.0;
   P.ia = 15.0;
-  double* fv = h->sp.work[3];
-  double* gx = h->sp.work[4];
-  double* gy = h->sp.work[5];
-  double* gz = h->sp.work[6];
-  float* dir = h->e_c;
-  k_ss_eval<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, S, c, P, fv, gx, gy, gz, dir); rso::note_launch();
-  RSO_TRY(launch_check(h, "ss_eval"));
-  RSO_TRY(sum_float(h, dir, l.NQ, h->scal + 13));
-  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 13, h->scal + 13, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
-  const double ds = h->h_scal[13];
-  if (dirsum) *dirsum = ds;
-  const double flip = ds < 0 ? -1.0 : 1.0;
-  const double direction = ds > 0 ? 1.0 : -1.0;
-  double* wA = h->sp.work[2];
-  double* wZ = h->sp.work[7];
-  double* wX = h->sp.work[8];
-  double* wY = h->sp.work[9];
-  float* down = h->e_d;
-  float* per = per_pad ? per_pad : h->e_b;
-  k_ss_penalty<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, S, P, flip, direction, fv, gx, gy, gz, per, wA, wZ, wX, wY,
-                                                        down); rso::note_launch();
-  RSO_TRY(launch_check(h, "ss_penalty"));
-  RSO_TRY(sum_float(h, per, l.NQ, h->scal + 12));
-  RSO_TRY(sum_float(h, down, l.NQ, h->scal + 11));
-  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 11, h->scal + 11, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
-  const double sum = h->h_scal[12], ndown = h->h_scal[11];
-  const double cnt = (mode % 2 == 0) ? ndown : (double)l.n_active_e;
+  const long long comp = (long long)S.nb0 * l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
+                  t3 = (long long)S.nb0 * S.nb1 * S.nb2;
+  const int nblk = cdiv((long long)l.ey * l.ez, kSSRows);
+  if (!h->sp.work[2])  // the rows of value and derivatives, and the partial sums, made on first use
+    RSO_CHECK_CUDA(h, cudaMalloc(&h->sp.work[2], sizeof(double) * (3 * comp + 3LL * nblk)));
+  double* R = h->sp.work[2];
+  double* sums = h->scal + 48;
+  // H / M of the probe's bound
+  const double p = S.order - 1, st[3] = {h->sp.step[0], h->sp.step[1], h->sp.step[2]};
+  double hcoef = 0;
+  for (int i = 0; i < 3; i++) {
+    double row = 4 * p * (p - 1) / (st[i] * st[i]);
+    for (int j = 0; j < 3; j++)
+      if (j != i) row += 4 * p * p / (st[i] * st[j]);
+    hcoef = std::max(hcoef, row);
+  }
+  double smin = st[0];
+  for (int i = 0; i < 3; i++) smin = std::min(smin, std::min(st[i], -(double)h->sp.bmin[i]));
+  k_max_abs<<<1, 1024, 0, h->stream>>>(h->sp.n_coeff, c, sums + 4); rso::note_launch();
+  RSO_TRY(spline_rows(h, S, c, R, true));
+  SSOut O;
+  O.G1 = h->sp.work[0];
+  O.Gy = O.G1 + comp;
+  O.Gz = O.Gy + comp;
+  O.per = per_dense;
+  O.part = R + 3 * comp;
+  double *G2 = h->sp.work[1], *G2z = G2 + t2;
+  const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1], *r2 = h->sp.ranges[2];
+  double flip = -1.0, direction = -1.0;
+  for (int pass = 0; pass < 2; pass++) {
+    k_ss_rows<<<nblk, 32 * kSSRows, 0, h->stream>>>(l, S, c, R, comp, P, flip, direction, sums + 4, hcoef, smin, r0,
+                                                    r0 + S.nb0, O, view_of(l, true)); rso::note_launch();
+    k_ss_sums<<<1, 512, 0, h->stream>>>(O.part, nblk, mode, (double)l.n_active_e, sums); rso::note_launch();
+    if (dc) {
+      k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, O.G1, O.Gy, r1, r1 + S.nb1, G2); rso::note_launch();
+      k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, O.Gz, nullptr, r1, r1 + S.nb1, G2z); rso::note_launch();
+      k_adj_z<<<cdiv(t3, 32), dim3(32, 8), 0, h->stream>>>(S, G2, G2z, r2, r2 + S.nb2, sums + 3, dc); rso::note_launch();
+    }
+    RSO_TRY(launch_check(h, "selfsupport"));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 48, sums, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
+    const double ds = h->h_scal[48];
+    const double f = ds < 0 ? -1.0 : 1.0, d = ds > 0 ? 1.0 : -1.0;
+    if (f == flip && d == direction) break;
+    flip = f;
+    direction = d;
+  }
+  const double sum = h->h_scal[49], cnt = h->h_scal[51];
+  if (dirsum) *dirsum = h->h_scal[48];
   if (count) *count = cnt;
   double v = 0;
   if (cnt != 0) v = (mode <= 1) ? std::pow(sum / cnt, 1 / P.fpara) - 1 : sum / cnt;
   if (value) *value = v;
-  if (dc) {
-    const double scale = cnt == 0 ? 0.0 : 1.0 / cnt;
-    RSO_TRY(separable_adjoint(h, wA, nullptr, 0, 0, 0, scale, 0, dc));
-    RSO_TRY(separable_adjoint(h, wZ, nullptr, 0, 0, 1, scale, 1, dc));
-    RSO_TRY(separable_adjoint(h, wX, nullptr, 1, 0, 0, scale, 1, dc));
-    RSO_TRY(separable_adjoint(h, wY, nullptr, 0, 1, 0, scale, 1, dc));
-  }
   return RSO_OK;
 }
 
@@ -602,12 +1052,10 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
     RSO_CHECK_CUDA(h, cudaMemcpy(s.ranges[a], rg.data(), sizeof(int) * rg.size(), cudaMemcpyHostToDevice));
   }
   s.n_coeff = (long long)s.nb[0] * s.nb[1] * s.nb[2];
-  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * (size_t)s.nb[0] * l.ey * l.ez));
-  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[1], sizeof(double) * (size_t)s.nb[0] * s.nb[1] * l.ez));
-  for (int i = 2; i < 10; i++) {
-    RSO_CHECK_CUDA(h, cudaMalloc(&s.work[i], sizeof(double) * l.NQ));
-    RSO_CHECK_CUDA(h, cudaMemset(s.work[i], 0, sizeof(double) * l.NQ));
-  }
+  // work[0]: spline rows, or stage 1 of the adjoints (three weights); work[1]: the two arrays of the
+  // other stage; work[2] is the self-support constraint's, made on its first call
+  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * 3 * (size_t)s.nb[0] * l.ey * l.ez));
+  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[1], sizeof(double) * 2 * (size_t)s.nb[0] * s.nb[1] * l.ez));
   cudaFree(h->coef_a); cudaFree(h->coef_b); cudaFree(h->coef_c);
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_a, sizeof(double) * s.n_coeff));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_b, sizeof(double) * s.n_coeff));

@@ -5,12 +5,6 @@
 
 using namespace rso;
 
-__global__ void k_pad_u8e(Level L, const uint8_t* __restrict__ dense, uint8_t* __restrict__ pad) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= L.ne) return;
-  int x = i % L.ex, y = (i / L.ex) % L.ey, z = i / ((long long)L.ex * L.ey);
-  pad[L.eidx(x, y, z)] = dense[i];
-}
 __global__ void k_f2d_n(const float* __restrict__ a, double* __restrict__ b, long long n) {
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < n) b[i] = (double)a[i];
@@ -20,66 +14,57 @@ __global__ void k_d2f_n(const double* __restrict__ a, float* __restrict__ b, lon
   if (i < n) b[i] = (float)a[i];
 }
 
-// padded copy of an optional dense shell mask (NULL stays NULL), in a buffer
-// the handle keeps: the first call with a mask allocates it, later calls reuse it
-static rso_status pad_shell(rso_handle* h, const uint8_t* shell, uint8_t** out) {
-  *out = nullptr;
-  if (!shell) return RSO_OK;
-  const Level& l = h->L[0];
-  if (!h->shell_pad) RSO_CHECK_CUDA(h, cudaMalloc((void**)&h->shell_pad, l.NQ));
-  RSO_CHECK_CUDA(h, cudaMemsetAsync(h->shell_pad, 0, l.NQ, h->stream));
-  k_pad_u8e<<<cdiv(l.ne, 256), 256, 0, h->stream>>>(l, shell, h->shell_pad); rso::note_launch();
-  *out = h->shell_pad;
-  return launch_check(h, "pad_shell");
-}
-
-static rso_status finish(rso_handle* h, uint8_t* = nullptr) {
+static rso_status finish(rso_handle* h) {
   RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
   return RSO_OK;
 }
 
-extern "C" rso_status rso_sensitivity(rso_handle* h, const double* u, float* sens) {
-  if (!h || !u || !sens) return RSO_ERR_INVALID_ARG;
+// The maps read and write the caller's arrays directly.  An output may overlap
+// an input: the input (n floats) is then read from a copy in a scratch field.
+static rso_status apart(rso_handle* h, const float** in, long long n, const float* out, long long n_out, float* scratch) {
+  if (*in >= out + n_out || *in + n <= out) return RSO_OK;
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(scratch, *in, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream));
+  *in = scratch;
+  return RSO_OK;
+}
+
+static rso_status sensitivity_api(rso_handle* h, const double* u, float* out, int energy) {
+  if (!h || !u || !out) return RSO_ERR_INVALID_ARG;
   RSO_TRY(pad_nodes(h, 0, u, h->L[0].u64));
   RSO_TRY(zero_support(h, h->L[0].u64));
-  RSO_TRY(sensitivity(h, h->L[0].u64, h->e_a, 0));
-  RSO_TRY(unpad_elems_f(h, h->e_a, sens));
+  RSO_TRY(sensitivity(h, h->L[0].u64, out, energy, true));
   return finish(h);
 }
 
+extern "C" rso_status rso_sensitivity(rso_handle* h, const double* u, float* sens) {
+  return sensitivity_api(h, u, sens, 0);
+}
 extern "C" rso_status rso_element_energy(rso_handle* h, const double* u, float* en) {
-  if (!h || !u || !en) return RSO_ERR_INVALID_ARG;
-  RSO_TRY(pad_nodes(h, 0, u, h->L[0].u64));
-  RSO_TRY(zero_support(h, h->L[0].u64));
-  RSO_TRY(sensitivity(h, h->L[0].u64, h->e_a, 1));
-  RSO_TRY(unpad_elems_f(h, h->e_a, en));
-  return finish(h);
+  return sensitivity_api(h, u, en, 1);
 }
 
 extern "C" rso_status rso_heaviside(rso_handle* h, const float* in, double beta, const uint8_t* shell, float* out) {
   if (!h || !in || !out) return RSO_ERR_INVALID_ARG;
-  uint8_t* sh = nullptr;
-  RSO_TRY(pad_shell(h, shell, &sh));
-  RSO_TRY(pad_elems_f(h, in, h->e_a));
-  RSO_TRY(heaviside(h, h->e_a, beta, sh, h->e_b));
-  RSO_TRY(unpad_elems_f(h, h->e_b, out));
-  return finish(h, sh);
+  const long long ne = h->L[0].ne;
+  RSO_TRY(apart(h, &in, ne, out, ne, h->e_a));
+  RSO_TRY(heaviside(h, in, beta, shell, out, true));
+  return finish(h);
 }
 
 extern "C" rso_status rso_heaviside_chain(rso_handle* h, const float* rho, double beta, const float* gin, float* gout) {
   if (!h || !rho || !gin || !gout) return RSO_ERR_INVALID_ARG;
-  RSO_TRY(pad_elems_f(h, rho, h->e_a));
-  RSO_TRY(pad_elems_f(h, gin, h->e_b));
-  RSO_TRY(heaviside_chain(h, h->e_a, beta, h->e_b, h->e_c));
-  RSO_TRY(unpad_elems_f(h, h->e_c, gout));
+  const long long ne = h->L[0].ne;
+  RSO_TRY(apart(h, &rho, ne, gout, ne, h->e_a));
+  RSO_TRY(apart(h, &gin, ne, gout, ne, h->e_b));
+  RSO_TRY(heaviside_chain(h, rho, beta, gin, gout, true));
   return finish(h);
 }
 
 static rso_status filter_api(rso_handle* h, double R, const float* in, float* out, int adjoint) {
   if (!h || !in || !out || !(R > 0)) return RSO_ERR_INVALID_ARG;
-  RSO_TRY(pad_elems_f(h, in, h->e_a));
-  RSO_TRY(filter(h, R, h->e_a, h->e_b, adjoint));
-  RSO_TRY(unpad_elems_f(h, h->e_b, out));
+  const long long ne = h->L[0].ne;
+  RSO_TRY(apart(h, &in, ne, out, ne, h->e_a));
+  RSO_TRY(filter(h, R, in, out, adjoint, true));
   return finish(h);
 }
 
@@ -95,8 +80,7 @@ extern "C" rso_status rso_density_filter_adjoint(rso_handle* h, double R, const 
 
 extern "C" rso_status rso_volume(rso_handle* h, const float* rho, double* vol) {
   if (!h || !rho || !vol) return RSO_ERR_INVALID_ARG;
-  RSO_TRY(pad_elems_f(h, rho, h->e_a));
-  return volume(h, h->e_a, vol);
+  return volume(h, rho, vol, true);
 }
 
 extern "C" rso_status rso_spline_setup(rso_handle* h, int order, int px, int py, int pz, int* n_coeff) {
@@ -118,24 +102,18 @@ extern "C" rso_status rso_spline_axis(rso_handle* h, int axis, int* idx, double*
 extern "C" rso_status rso_coeff2density(rso_handle* h, const float* coeff, const uint8_t* shell, float* rho_hat) {
   if (!h || !coeff || !rho_hat) return RSO_ERR_INVALID_ARG;
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
-  uint8_t* sh = nullptr;
-  RSO_TRY(pad_shell(h, shell, &sh));
   k_f2d_n<<<cdiv(h->sp.n_coeff, 256), 256, 0, h->stream>>>(coeff, h->coef_a, h->sp.n_coeff); rso::note_launch();
-  RSO_TRY(coeff2density(h, h->coef_a, sh, h->e_a));
-  RSO_TRY(unpad_elems_f(h, h->e_a, rho_hat));
-  return finish(h, sh);
+  RSO_TRY(coeff2density(h, h->coef_a, shell, rho_hat, true));
+  return finish(h);
 }
 
 extern "C" rso_status rso_density2coeff_adjoint(rso_handle* h, const float* g, const uint8_t* shell, float* dc) {
   if (!h || !g || !dc) return RSO_ERR_INVALID_ARG;
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
-  uint8_t* sh = nullptr;
-  RSO_TRY(pad_shell(h, shell, &sh));
-  RSO_TRY(pad_elems_f(h, g, h->e_a));
-  RSO_TRY(density2coeff(h, h->e_a, sh, h->coef_b));
+  RSO_TRY(density2coeff(h, g, shell, h->coef_b, true));
   k_d2f_n<<<cdiv(h->sp.n_coeff, 256), 256, 0, h->stream>>>(h->coef_b, dc, h->sp.n_coeff); rso::note_launch();
   RSO_TRY(launch_check(h, "density2coeff"));
-  return finish(h, sh);
+  return finish(h);
 }
 
 extern "C" rso_status rso_selfsupport(rso_handle* h, const float* coeff, double beta, int mode, double opt_angle,
@@ -144,9 +122,8 @@ extern "C" rso_status rso_selfsupport(rso_handle* h, const float* coeff, double 
   if (!h || !coeff || mode < 0 || mode > 5) return RSO_ERR_INVALID_ARG;
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
   k_f2d_n<<<cdiv(h->sp.n_coeff, 256), 256, 0, h->stream>>>(coeff, h->coef_a, h->sp.n_coeff); rso::note_launch();
-  RSO_TRY(selfsupport(h, h->coef_a, beta, mode, opt_angle, default_angle, h->e_a, dc ? h->coef_b : nullptr, value,
-                      count, dirsum));
-  if (per) RSO_TRY(unpad_elems_f(h, h->e_a, per));
+  RSO_TRY(selfsupport(h, h->coef_a, beta, mode, opt_angle, default_angle, per, dc ? h->coef_b : nullptr, value, count,
+                      dirsum));
   if (dc) { k_d2f_n<<<cdiv(h->sp.n_coeff, 256), 256, 0, h->stream>>>(h->coef_b, dc, h->sp.n_coeff); rso::note_launch(); }
   RSO_TRY(launch_check(h, "selfsupport"));
   return finish(h);

@@ -108,15 +108,13 @@ __host__ __device__ constexpr bool b_zero(int c, int i, int j) {
   return false;
 }
 
-rso_status upload_walsh(rso_handle* h) {
-  const double* K = h->K0;
+// B = (W K0 W^T) / 64, entry (i, j) of block c at c * 9 + i * 3 + j
+static void walsh_blocks(const double* K, double B[72]) {
   // W[m][a] = prod_axis H[m_axis][a_axis]
   auto Hh = [](int m, int b) { return m == 0 ? 1.0 : (b ? 1.0 : -1.0); };
   double W[8][8];
   for (int m = 0; m < 8; m++)
     for (int a = 0; a < 8; a++) W[m][a] = Hh(m & 1, a & 1) * Hh((m >> 1) & 1, (a >> 1) & 1) * Hh(m >> 2, a >> 2);
-  double B[72], kmax = 0;
-  for (int i = 0; i < 576; i++) kmax = std::fmax(kmax, std::fabs(K[i]));
   for (int c = 0; c < 8; c++)
     for (int i = 0; i < 3; i++)
       for (int j = 0; j < 3; j++) {
@@ -124,16 +122,29 @@ rso_status upload_walsh(rso_handle* h) {
         double s = 0;
         for (int a = 0; a < 8; a++)
           for (int b = 0; b < 8; b++) s += W[mi][a] * K[(a * 3 + i) * 24 + b * 3 + j] * W[mj][b];
-        s /= 64.0;
-        if (b_zero(c, i, j)) {
-          if (std::fabs(s) > 1e-12 * kmax) {
-            h->err = "element matrix lacks the reflection symmetry of the cube";
-            return RSO_ERR_INVALID_ARG;
-          }
-          s = 0;
-        }
-        B[c * 9 + i * 3 + j] = s;
+        B[c * 9 + i * 3 + j] = s / 64.0;
       }
+}
+
+void walsh_constants(const double* K, double c[8]) {
+  double B[72];
+  walsh_blocks(K, B);
+  const double v[8] = {B[0] - B[1], B[1], B[63] - B[64], B[64], B[13], B[14], B[27], B[35]};
+  for (int i = 0; i < 8; i++) c[i] = v[i];
+}
+
+rso_status upload_walsh(rso_handle* h) {
+  const double* K = h->K0;
+  double B[72], kmax = 0;
+  for (int i = 0; i < 576; i++) kmax = std::fmax(kmax, std::fabs(K[i]));
+  walsh_blocks(K, B);
+  for (int c = 0; c < 8; c++)
+    for (int i = 0; i < 3; i++)
+      for (int j = 0; j < 3; j++)
+        if (b_zero(c, i, j) && std::fabs(B[c * 9 + i * 3 + j]) > 1e-12 * kmax) {
+          h->err = "element matrix lacks the reflection symmetry of the cube";
+          return RSO_ERR_INVALID_ARG;
+        }
   // diagonal blocks: K0[a][a](i, j) = D0(i, j) * sigma_i(a) * sigma_j(a), sigma = 1 - 2 bit
   double D0[9];
   for (int i = 0; i < 3; i++)
@@ -175,7 +186,10 @@ rso_status upload_walsh(rso_handle* h) {
     h->err = "element matrix lacks the symmetry of an isotropic cube";
     return RSO_ERR_INVALID_ARG;
   }
-  const double Wv[10] = {A0 - B0, B0, A7 - B7, B7, Pv, Qv, Rv, Sv, Da, Db};
+  double Wv[10];
+  walsh_constants(K, Wv);
+  Wv[W_DA] = Da;
+  Wv[W_DB] = Db;
   float2 Wp[10];
   for (int i = 0; i < 10; i++) Wp[i] = make_float2((float)Wv[i], (float)Wv[i]);
   RSO_CHECK_CUDA(h, cudaMemcpyToSymbolAsync(cWp, Wp, sizeof(Wp), 0, cudaMemcpyHostToDevice, h->stream));

@@ -79,7 +79,7 @@ struct Spline {
   long long n_coeff = 0;
   float* knots_dev = nullptr;                      // the three knot vectors back to back
   int* ranges[3] = {nullptr, nullptr, nullptr};    // per basis index: first/last element coordinate in its support
-  double* work[10] = {};                           // adjoint and self-support scratch
+  double* work[3] = {};                            // spline rows, adjoint stages, self-support scratch
 };
 
 }  // namespace rso
@@ -163,7 +163,6 @@ struct rso_handle {
   long long n_gs_elements = 0;
   // design-iteration scratch
   float *e_a = nullptr, *e_b = nullptr, *e_c = nullptr, *e_d = nullptr, *e_rhohat = nullptr;
-  uint8_t* shell_pad = nullptr;       // padded copy of a caller's shell mask (design_capi.cu), made on first use
   double *coef_a = nullptr, *coef_b = nullptr, *coef_c = nullptr;
   double *coef_df = nullptr, *coef_dg = nullptr;   // MMA inputs
   double *fw = nullptr, *uw = nullptr;             // worst-case force / displacement (padded)
@@ -351,6 +350,8 @@ rso_status fine_jacobi0(rso_handle* h, const T* f, T* u_out, const T* rp, double
 template <typename T>
 rso_status fine_gs(rso_handle* h, T* u, const T* f, const T* rp, int colour, int reverse);
 rso_status upload_K0(rso_handle* h);
+// the element matrix's blocks in the sum/difference basis: A0 - B0, B0, A7 - B7, B7, P, Q, R, S
+void walsh_constants(const double* K0, double c[8]);
 rso_status penalise(rso_handle* h);
 
 // coarse levels (coarse_op.cu)
@@ -402,17 +403,20 @@ rso_status axpby(rso_handle* h, long long n, double a, const double* x, double b
 rso_status fill_d(rso_handle* h, double* p, long long n, double v);
 rso_status fill_f(rso_handle* h, float* p, long long n, float v);
 
-// design (design.cu)
-rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens_pad, int energy);
-rso_status heaviside(rso_handle* h, const float* in_pad, double beta, const uint8_t* shell_pad, float* out_pad);
-rso_status heaviside_chain(rso_handle* h, const float* rho_pad, double beta, const float* gin, float* gout);
-rso_status filter(rso_handle* h, double radius, const float* in_pad, float* out_pad, int adjoint);
-rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell_pad, float* out_pad);
-rso_status density2coeff(rso_handle* h, const float* g_pad, const uint8_t* shell_pad, double* dc);
+// design (design.cu); element fields padded, or dense (ex*ey*ez) with dense set; shell masks are dense
+rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens, int energy, bool dense = false);
+rso_status heaviside(rso_handle* h, const float* in, double beta, const uint8_t* shell, float* out, bool dense = false);
+rso_status heaviside_chain(rso_handle* h, const float* rho, double beta, const float* gin, float* gout,
+                           bool dense = false);
+rso_status filter(rso_handle* h, double radius, const float* in, float* out, int adjoint, bool dense = false);
+rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, float* out, bool dense = false);
+rso_status density2coeff(rso_handle* h, const float* g, const uint8_t* shell, double* dc, bool dense = false);
 rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, double opt_angle,
-                       double default_angle, float* per_pad, double* dc, double* value, double* count,
+                       double default_angle, float* per_dense, double* dc, double* value, double* count,
                        double* dirsum);
-rso_status volume(rso_handle* h, const float* rho_pad, double* vol);
+rso_status volume(rso_handle* h, const float* rho, double* vol, bool dense = false);
+// sum over the active elements
+rso_status sum_elems(rso_handle* h, const float* a, bool dense, double* dev_out);
 rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz);
 
 // worst case (worst.cu)

@@ -69,3 +69,72 @@ def test_bottom_kernel_levels(cuda, dims, pre, post):
     for u, k, _, _ in got:
         assert rel(u.cpu().numpy(), want.cpu().numpy()) < 1e-8 and abs(k - it) <= 1
     assert rel(batch[0].cpu().numpy(), want.cpu().numpy()) < 1e-8 and abs(infos[0][0] - it) <= 1
+
+
+# boxes below, on and past the 32 x 8 tile and the 128-element row segment; radii on both sides of
+# every reach the tiled filter is built for and past the last one (the general kernel)
+@pytest.mark.parametrize("dims,radius", [((33, 9, 10), 1.0), ((33, 9, 10), 1.9), ((32, 8, 64), 2.0), ((70, 5, 3), 2.99),
+                                         ((40, 24, 24), 3.5), ((31, 17, 20), 4.99), ((31, 17, 20), 5.0), ((9, 8, 8), 0.7)])
+@pytest.mark.parametrize("gen", [P.cantilever, lambda *d: P.voids_box(*d, nvoids=1)])
+def test_filter_tiles(oracle, cuda, gen, dims, radius):
+    """FP64 sums rounded to FP32 once: 1e-6 relative (half an FP32 ulp is 6e-8); in place as well."""
+    small = min(dims) < 8
+    g, o = make(oracle, gen(*dims), n_levels=2 if small else 0, first_factor=2 if small else 4)
+    x = np.random.default_rng(3).standard_normal(o.ne).astype(np.float32)
+    want = o.filter(radius, x.astype(np.float64))
+    assert rel(g.filterSensitivity(radius, x).cpu().numpy(), want) < 1e-6
+    assert rel(g.densityFilter(radius, x, adjoint=True).cpu().numpy(),
+               o.density_filter_adjoint(radius, x.astype(np.float64))) < 1e-6
+    buf = t(x, cuda)
+    assert g.lib.rso_filter(g.h, radius, buf.data_ptr(), buf.data_ptr()) == 0
+    assert rel(buf.cpu().numpy(), want) < 1e-6
+
+
+# orders 2 to 5 (2 and 5 outside the probe bound's C1 splines and at its end), one to many knots per
+# element row segment, rows longer than a segment; amplitudes for which the probe's sign is known
+# (1), unknown for many (30) and for all elements (3000)
+@pytest.mark.parametrize("dims,order,parts", [((20, 12, 9), 2, (3, 3, 2)), ((150, 11, 7), 3, (40, 0, 3)),
+                                              ((129, 9, 13), 4, (9, 4, 5)), ((24, 18, 20), 5, (4, 3, 6)),
+                                              ((12, 10, 8), 4, (30, 1, 9))])
+@pytest.mark.parametrize("amplitude", [1.0, 30.0, 3000.0])
+def test_spline_rows_and_overhang(oracle, cuda, dims, order, parts, amplitude):
+    """Density map and adjoint 1e-6, constraint value 1e-5 and gradient 1e-4 relative, counts and
+    probe sums equal: the bounds of these maps in the parity tests."""
+    g, o = make(oracle, P.voids_box(*dims, nvoids=1), n_levels=2, first_factor=2)
+    n = o.spline_setup(order, parts)
+    assert g.set_spline_partition(*parts, order) == n
+    rng = np.random.default_rng(19)
+    c = (amplitude * rng.normal(0.5, 0.15, n)).astype(np.float32)
+    x = rng.standard_normal(o.ne).astype(np.float32)
+    assert rel(g.coeff2density(c).cpu().numpy(), o.coeff2density(c.astype(np.float64))) < 1e-6
+    assert rel(g.ddensity2dcoeff(x).cpu().numpy(), o.density2coeff_adjoint(x.astype(np.float64))) < 1e-6
+    for mode in (4, 5):
+        v, per, dc, cnt, ds = g.deal_background_points(c, 8.0, mode)
+        vo, pero, dco, cnto, dso = o.selfsupport(c.astype(np.float64), 8.0, mode)
+        assert cnt == cnto and ds == dso
+        assert abs(v - vo) <= 1e-5 * max(abs(vo), 1e-12)
+        assert rel(per.cpu().numpy(), pero) < 1e-5
+        assert rel(dc.cpu().numpy(), dco) < 1e-4
+
+
+@pytest.mark.parametrize("penal", [1.0, 2.0, 3.0, 3.5])
+@pytest.mark.parametrize("dims", [(33, 9, 5), (30, 18, 12)])
+def test_sensitivity_modes(oracle, cuda, dims, penal):
+    """u^T K0 u summed in the sum/difference basis in FP64, rounded to FP32: 1e-6 relative."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid, element_matrix
+    prob = P.voids_box(*dims)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"], Config(penal=penal, n_levels=2,
+                                                                                          first_factor=2))
+    rho = prob["rho"].astype(np.float32)
+    g.set_density(rho.ravel())
+    u = np.random.default_rng(4).standard_normal((3, dims[2] + 1, dims[1] + 1, dims[0] + 1))
+    cls = g.node_class().reshape(u.shape[1:])
+    u[:, (cls & 4 > 0) | (cls & 1 == 0)] = 0
+    ue = np.stack([u[i, k >> 2:(k >> 2) + dims[2], (k >> 1 & 1):(k >> 1 & 1) + dims[1], (k & 1):(k & 1) + dims[0]]
+                   for k in range(8) for i in range(3)]).reshape(24, -1)
+    q = np.einsum("ie,ij,je->e", ue, element_matrix(), ue)
+    r = rho.astype(np.float64).ravel() * prob["emask"].ravel()
+    on = prob["emask"].ravel() > 0
+    want = np.where(on, -penal * np.where(on, r, 1.0) ** (penal - 1) * q, 0.0)
+    assert rel(g.computeSensitivity(t(u.ravel(), cuda)).cpu().numpy(), want) < 1e-6
+    assert rel(g.elementCompliance(t(u.ravel(), cuda)).cpu().numpy(), np.where(on, r ** penal * q, 0.0)) < 1e-6
