@@ -123,7 +123,7 @@ static void free_handle(rso_handle* h) {
   for (int a = 0; a < 3; a++) {
     cudaFree(h->sp.idx[a]); cudaFree(h->sp.N[a]); cudaFree(h->sp.dN[a]); cudaFree(h->sp.ranges[a]);
   }
-  cudaFree(h->sp.knots_dev);
+  cudaFree(h->sp.knots_dev); cudaFree(h->sp.xtab);
   for (auto p : h->sp.work) cudaFree(p);
   for (auto p : h->lanczos_u) cudaFree(p);
   cudaFree(h->e_a); cudaFree(h->e_b); cudaFree(h->e_c); cudaFree(h->e_d); cudaFree(h->e_rhohat);

@@ -31,6 +31,14 @@ static View view_of(const Level& l, bool dense) {
 }
 // one thread per element, 32 x 8 tiles of a plane (a launch has at most 65535 planes: the kernels step on)
 static dim3 elem_grid(const Level& l) { return dim3(cdiv(l.ex, 32), cdiv(l.ey, 8), std::min(l.ez, 65535)); }
+// one thread per column of zc elements: long where the tiles of a plane alone
+// give the GPU eight CTAs per SM, 4 at least (a plane is shared by two elements)
+static dim3 column_grid(const Level& l, int zc) { return dim3(cdiv(l.ex, 32), cdiv(l.ey, 8), cdiv(l.ez, zc)); }
+static int column_chunk(const Level& l) {
+  int zc = 32;
+  while (zc > 4 && (long long)cdiv(l.ex, 32) * cdiv(l.ey, 8) * cdiv(l.ez, zc) < 8 * 148) zc /= 2;
+  return std::max(zc, cdiv(l.ez, 65535));
+}
 // FP64 powers by small whole exponents are products, as accurate as pow and a
 // tenth of its instructions
 __device__ __forceinline__ double power(double r, double p) {
@@ -45,42 +53,56 @@ __device__ __forceinline__ double power(double r, double p) {
 // In the sum/difference basis of the element's nodes, w = W u_e along each axis,
 // K0 = W^T B W with the block structure of fine_op.cu, so the quadratic form is
 // a sum over the eight blocks: about 120 operations where the 24 x 24 product
-// takes 600 (256^3, FP64: 1887 us with it, bound by the FP64 units; B.c in the
-// order of cWp: A0 - B0, B0, A7 - B7, B7, P, Q, R, S).
+// takes 600.  A thread marches along z, so that a node plane is loaded and
+// transformed once for the elements on both sides.  256^3: 1887 us with the
+// product (bound by the FP64 units), 303 with a thread per element.
+// B.c in the order of cWp: A0 - B0, B0, A7 - B7, B7, P, Q, R, S.
 struct WalshB { double c[8]; };
 __global__ void __launch_bounds__(256) k_sensitivity(const Level L, const double* __restrict__ u,
                                                      const float* __restrict__ rho, const WalshB B, double p, int energy,
-                                                     float* __restrict__ out, const View V) {
+                                                     float* __restrict__ out, const View V, int zc) {
   const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
   if (x >= L.ex || y >= L.ey) return;
-  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
-    const long long e = L.eidx(x, y, z), o = V.at(x, y, z);
-    if (!L.emask[e]) { out[o] = 0.f; continue; }
-    double w[8][3];  // modes (mx, my, mz) as bits, component
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.ez);
+  // xy modes of a face's four nodes; an element's upper face is the next one's lower
+  auto face = [&](int z, double (&f)[3][4]) {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      double f[2][4];  // xy modes of the lower and upper face
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        const double* q = u + L.nidx(x, y, z + b) + c * L.NP;
-        const double a00 = q[0], a10 = q[1], a01 = q[L.px], a11 = q[L.px + 1];
-        const double s0 = a00 + a10, d0 = a10 - a00, s1 = a01 + a11, d1 = a11 - a01;
-        f[b][0] = s0 + s1; f[b][1] = d0 + d1; f[b][2] = s1 - s0; f[b][3] = d1 - d0;
-      }
-#pragma unroll
-      for (int m = 0; m < 4; m++) { w[m][c] = f[0][m] + f[1][m]; w[m + 4][c] = f[1][m] - f[0][m]; }
+      const double* q = u + L.nidx(x, y, z) + c * L.NP;
+      const double a00 = q[0], a10 = q[1], a01 = q[L.px], a11 = q[L.px + 1];
+      const double s0 = a00 + a10, d0 = a10 - a00, s1 = a01 + a11, d1 = a11 - a01;
+      f[c][0] = s0 + s1; f[c][1] = d0 + d1; f[c][2] = s1 - s0; f[c][3] = d1 - d0;
     }
-    auto full = [&](double i, double j, double k, double ab, double bb) {
-      const double t = i + j + k;
-      return ab * (i * i + j * j + k * k) + bb * (t * t);
-    };
-    auto pair = [&](double i, double j) { return B.c[4] * (i * i + j * j) + 2.0 * B.c[5] * (i * j); };
-    auto both = [&](double i, double j, double k) { return B.c[6] * ((i + j) * (i + j)) + B.c[7] * (k * k); };
+  };
+  auto full = [&](double i, double j, double k, double ab, double bb) {
+    const double t = i + j + k;
+    return ab * (i * i + j * j + k * k) + bb * (t * t);
+  };
+  auto pair = [&](double i, double j) { return B.c[4] * (i * i + j * j) + 2.0 * B.c[5] * (i * j); };
+  auto both = [&](double i, double j, double k) { return B.c[6] * ((i + j) * (i + j)) + B.c[7] * (k * k); };
+  double f[3][4];
+  face(z0, f);
+  for (int z = z0; z < z1; z++) {
+    double up[3][4], w[8][3];  // modes (mx, my, mz) as bits, component
+    face(z + 1, up);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        w[m][c] = f[c][m] + up[c][m];
+        w[m + 4][c] = up[c][m] - f[c][m];
+        f[c][m] = up[c][m];
+      }
     double q = full(w[1][0], w[2][1], w[4][2], B.c[0], B.c[1]) + full(w[6][0], w[5][1], w[3][2], B.c[2], B.c[3]);
     q += pair(w[3][1], w[5][2]) + pair(w[3][0], w[6][2]) + pair(w[5][0], w[6][1]);
     q += both(w[2][0], w[1][1], w[7][2]) + both(w[4][0], w[1][2], w[7][1]) + both(w[4][1], w[2][2], w[7][0]);
-    const double r = (double)rho[e];
-    out[o] = energy ? (float)(power(r, p) * q) : (float)(-p * (p == 1.0 ? 1.0 : power(r, p - 1)) * q);
+    const long long e = L.eidx(x, y, z);
+    float o = 0.f;
+    if (L.emask[e]) {
+      const double r = (double)rho[e];
+      o = energy ? (float)(power(r, p) * q) : (float)(-p * (p == 1.0 ? 1.0 : power(r, p - 1)) * q);
+    }
+    out[V.at(x, y, z)] = o;
   }
 }
 
@@ -88,31 +110,53 @@ rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens, int ener
   const Level& l = h->L[0];
   WalshB B;
   walsh_constants(h->K0, B.c);
-  k_sensitivity<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, u_pad, h->rho, B, h->cfg.penal, energy, sens,
-                                                             view_of(l, dense)); rso::note_launch();
+  const int zc = column_chunk(l);
+  k_sensitivity<<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, u_pad, h->rho, B, h->cfg.penal, energy, sens,
+                                                                   view_of(l, dense), zc); rso::note_launch();
   return launch_check(h, "sensitivity");
 }
 
 // ---------------------------------------------------------------- Heaviside
 // in, gin and out share one layout and may be the same array; t0 = tanh(beta
-// eta), den = t0 + tanh(beta (1 - eta)), the same for every element
-__global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* in, double beta, double t0, double den,
-                                                   double rmin, const uint8_t* shell, int chain, const float* gin,
-                                                   float* out, const View V) {
+// eta), den = t0 + tanh(beta (1 - eta)), the same for every element.  One
+// exponential serves both maps: with E = exp(-2 |x|), tanh x = sign(x) (1 - E) /
+// (1 + E) and its slope is 4 E / (1 + E)^2, without the cancellation of
+// 1 - tanh^2 in the tails.  (256^3: 122 us with tanh and a thread per
+// element, bound by instructions and by each thread's two dependent loads, 70 so,
+// a thread loading four elements of its column at once.)
+template <bool CHAIN>
+__global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* in, double beta, double t0, double rden,
+                                                   double rmin, const uint8_t* shell, const float* gin, float* out,
+                                                   const View V, int zc) {
   const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
   if (x >= L.ex || y >= L.ey) return;
-  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
-    const long long o = V.at(x, y, z);
-    if (!L.emask[L.eidx(x, y, z)]) { out[o] = 0.f; continue; }
-    const double eta = 0.5;
-    const double t = tanh(beta * ((double)in[o] - eta));
-    if (chain) {
-      out[o] = (float)((double)gin[o] * beta * (1 - t * t) / den);
-    } else {
-      double v = (t0 + t) / den;
-      v = fmin(fmax(v, rmin), 1.0);
-      if (shell && shell[x + (long long)L.ex * (y + (long long)L.ey * z)]) v = 1.0;
-      out[o] = (float)v;
+  const int z0 = blockIdx.z * zc, n = min(zc, L.ez - z0);
+  const long long o0 = V.at(x, y, z0), qxy = (long long)L.qx * L.qy;
+  const uint8_t* mask = L.emask + L.eidx(x, y, z0);
+  const uint8_t* sh = shell ? shell + x + (long long)L.ex * (y + (long long)L.ey * z0) : nullptr;
+  for (int z = 0; z < n; z += 4) {  // four elements' loads before any store (the arrays may be one)
+    float a[4], g[4];
+    bool on[4], one[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const bool ok = z + j < n;
+      on[j] = ok && mask[(z + j) * qxy];
+      a[j] = ok ? in[o0 + (z + j) * V.sz] : 0.f;
+      if (CHAIN) g[j] = ok ? gin[o0 + (z + j) * V.sz] : 0.f;
+      one[j] = !CHAIN && ok && sh && sh[(long long)(z + j) * L.ex * L.ey];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (z + j >= n) break;
+      const double s = beta * ((double)a[j] - 0.5), E = exp(-2 * fabs(s)), q = __drcp_rn(1 + E);
+      double v;
+      if (CHAIN) {
+        v = (double)g[j] * beta * (4 * E * q * q) * rden;
+      } else {
+        v = (t0 + copysign((1 - E) * q, s)) * rden;
+        v = one[j] ? 1.0 : fmin(fmax(v, rmin), 1.0);
+      }
+      out[o0 + (z + j) * V.sz] = on[j] ? (float)v : 0.f;
     }
   }
 }
@@ -120,16 +164,18 @@ __global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* i
 rso_status heaviside(rso_handle* h, const float* in, double beta, const uint8_t* shell, float* out, bool dense) {
   const Level& l = h->L[0];
   const double t0 = std::tanh(beta * 0.5), den = t0 + std::tanh(beta * (1 - 0.5));
-  k_heaviside<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, in, beta, t0, den, h->cfg.rho_min, shell, 0, nullptr, out,
-                                                           view_of(l, dense)); rso::note_launch();
+  const int zc = column_chunk(l);
+  k_heaviside<false><<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, in, beta, t0, 1 / den, h->cfg.rho_min, shell,
+                                                                        nullptr, out, view_of(l, dense), zc); rso::note_launch();
   return launch_check(h, "heaviside");
 }
 
 rso_status heaviside_chain(rso_handle* h, const float* rho, double beta, const float* gin, float* gout, bool dense) {
   const Level& l = h->L[0];
   const double t0 = std::tanh(beta * 0.5), den = t0 + std::tanh(beta * (1 - 0.5));
-  k_heaviside<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, rho, beta, t0, den, 0.0, nullptr, 1, gin, gout,
-                                                           view_of(l, dense)); rso::note_launch();
+  const int zc = column_chunk(l);
+  k_heaviside<true><<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, rho, beta, t0, 1 / den, 0.0, nullptr, gin,
+                                                                       gout, view_of(l, dense), zc); rso::note_launch();
   return launch_check(h, "heaviside_chain");
 }
 
@@ -161,105 +207,119 @@ __global__ void k_filter(const Level L, const FOff* __restrict__ off, int noff, 
   }
 }
 
-// Radii from 1 to under 5.  A CTA of 32 x 8 threads marches along z through a
+// Radii from 1 to under 5.  A CTA of 32 x 16 threads marches along z through a
 // tile of columns.  Each plane, with its halo of RZ elements, is staged once in
-// shared memory as FP64 (so a value is converted once, not once per tap), and a
-// thread adds every neighbour column's value to the 2 dz + 1 outputs it reaches
-// along z, which it keeps in registers: 13 shared loads for the 33 taps of
-// R = 2.  Weights depend on |dx|, |dy|, |dz| alone and sit in shared memory by
-// column, the columns ordered by their reach in z, so that no zero weight is
-// ever multiplied.  Where the planes around an output are full (inside the box
-// and all active, a flag per plane) the weight sum is that of all taps; else
-// the taps sum the mask as well.  256^3, R = 2: 1007 us with a thread walking
-// the table (its loads and conversions), 464 us now.
-constexpr int FTX = 32, FTY = 8, kFiltRZ = 4;
-struct FCol { int dx, dy; double w[kFiltRZ + 1]; };  // one neighbour column; w by |dz|
-struct FPlan { int start[kFiltRZ + 2]; };            // columns [start[d], start[d + 1]) reach d planes up and down
+// shared memory as FP64 (so a value is converted once, not once per tap).  The
+// weight depends on the three distances alone, so the neighbour columns at the
+// same two in-plane distances (either way round) form a class: a thread adds up
+// the four or eight columns of a class, and multiplies the sum once for each
+// plane it reaches, into the 2 RZ + 1 outputs along z that it keeps in
+// registers: 13 shared loads, 13 additions and 20 multiply-adds for the 33 taps
+// of R = 2, the weights being kernel parameters.  A class or plane outside the
+// radius is skipped, not multiplied by zero.  Where a staged plane is full
+// (inside the box and all active) its part of the weight sum is known; else the
+// mask is summed as the values are.  256^3, R = 2: 1007 us with a thread walking
+// a tap table (loads and conversions), 464 with the columns' weights read from
+// shared memory, 241 now (the next plane's loads in flight during a plane's taps).
+constexpr int FTX = 32, FTY = 16, kFiltRZ = 4;
+constexpr int fclass(int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; }
+constexpr int kFClasses = fclass(kFiltRZ, kFiltRZ) + 1;
+struct FPlan {
+  double w[kFClasses][kFiltRZ + 1];  // weight by class and |dz|
+  double plane[kFiltRZ + 1];         // sum of a full plane's weights at |dz|
+  int reach[kFClasses];              // the largest |dz| inside the radius, -1 if none is
+};
+// a staged plane's columns around p, class by class, into the outputs they reach
+template <int RZ, typename T>
+__device__ __forceinline__ void filter_taps(const FPlan& P, const T* p, double (&to)[2 * RZ + 1]) {
+  constexpr int WX = FTX + 2 * RZ;
+#pragma unroll
+  for (int a = 0; a <= RZ; a++)
+#pragma unroll
+    for (int b = 0; b <= a; b++) {
+      const int reach = P.reach[fclass(a, b)];
+      if (reach < 0) continue;
+      T t = 0;  // FP32 for the mask: small whole numbers
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int sx = q & 1 ? 1 : -1, sy = q & 2 ? 1 : -1;
+        if ((a == 0 && sx > 0) || (b == 0 && sy > 0)) continue;
+        t += p[sy * b * WX + sx * a];
+        if (a != b) t += p[sx * a * WX + sy * b];
+      }
+      const double s = (double)t;
+#pragma unroll
+      for (int j = 0; j <= RZ; j++)
+        if (j <= reach) {
+          const double w = P.w[fclass(a, b)][j];
+          to[RZ + j] = fma(w, s, to[RZ + j]);
+          if (j > 0) to[RZ - j] = fma(w, s, to[RZ - j]);
+        }
+    }
+}
 template <int RZ, int MODE>
-__global__ void __launch_bounds__(FTX* FTY) k_filter_tile(const Level L, const FCol* __restrict__ cols, const FPlan P,
+__global__ void __launch_bounds__(FTX* FTY) k_filter_tile(const Level L, const __grid_constant__ FPlan P,
                                                           const float* __restrict__ in, float* __restrict__ out,
                                                           const float* __restrict__ wsum, const View V, int zc) {
   constexpr int WX = FTX + 2 * RZ, WY = FTY + 2 * RZ, NW = WX * WY, NA = 2 * RZ + 1;
-  extern __shared__ __align__(16) unsigned char fsm[];
-  double* sv = reinterpret_cast<double*>(fsm);                       // [2][NW] values, zero where masked
-  float* sm = reinterpret_cast<float*>(sv + 2 * NW);                 // [2][NW] mask
-  double* sw = reinterpret_cast<double*>(sm + 2 * NW);               // [columns][RZ + 1] weights
-  const int ncol = P.start[RZ + 1];
-  int* so = reinterpret_cast<int*>(sw + ncol * (RZ + 1));            // [columns] window offsets
-  __shared__ double wfull[RZ + 1];                                   // all columns' weights, by |dz|
+  __shared__ double sv[2][NW];  // values, zero where masked
+  __shared__ float sm[2][NW];   // mask
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * FTX + tx;
   const int x0 = blockIdx.x * FTX, y0 = blockIdx.y * FTY, z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.ez);
-  for (int k = tid; k < ncol; k += FTX * FTY) {
-    const FCol c = cols[k];
-    so[k] = c.dy * WX + c.dx;
-#pragma unroll
-    for (int d = 0; d <= RZ; d++) sw[k * (RZ + 1) + d] = c.w[d];
-  }
-  __syncthreads();
-  if (tid <= RZ) {
-    double s = 0;
-    for (int k = P.start[tid]; k < ncol; k++) s += sw[k * (RZ + 1) + tid];
-    wfull[tid] = s;
-  }
-  const int x = x0 + tx, y = y0 + ty;
+  const int x = x0 + tx, y = y0 + ty, c0 = (ty + RZ) * WX + tx + RZ;
   double acc[NA], wac[NA];
 #pragma unroll
   for (int k = 0; k < NA; k++) acc[k] = wac[k] = 0;
+  // this thread's window entries: their offsets in a plane of the fields, -1 outside the box
+  constexpr int NK = (NW + FTX * FTY - 1) / (FTX * FTY);
+  const long long qxy = (long long)L.qx * L.qy;
+  long long eo[NK], vo[NK];
+#pragma unroll
+  for (int i = 0; i < NK; i++) {
+    const int k = i * FTX * FTY + tid, wy = k / WX, wx = k - wy * WX, xx = x0 + wx - RZ, yy = y0 + wy - RZ;
+    eo[i] = vo[i] = -1;
+    if (k < NW && xx >= 0 && yy >= 0 && xx < L.ex && yy < L.ey) {
+      eo[i] = L.eidx(xx, yy, 0);
+      vo[i] = V.at(xx, yy, 0);
+    }
+  }
+  float raw[NK], wgt[NK];
+  bool on[NK];
+  auto fetch = [&](int zp) {  // plane zp into registers
+    const bool in_z = zp >= 0 && zp < L.ez;
+#pragma unroll
+    for (int i = 0; i < NK; i++) {
+      const bool ok = in_z && eo[i] >= 0;
+      on[i] = ok && L.emask[eo[i] + qxy * zp];
+      raw[i] = MODE != 1 && ok ? in[vo[i] + V.sz * zp] : 0.f;
+      wgt[i] = MODE == 2 && ok ? wsum[eo[i] + qxy * zp] : 1.f;
+    }
+  };
+  fetch(z0 - RZ);
   // planes z0 - RZ .. z1 - 1 + RZ; after plane zp output zp - RZ is complete
   for (int zp = z0 - RZ; zp < z1 + RZ; zp++) {
     const int buf = (zp - z0 + RZ) & 1;
-    double* v = sv + buf * NW;
-    float* m = sm + buf * NW;
     bool full = true;
-    for (int k = tid; k < NW; k += FTX * FTY) {
-      const int wy = k / WX, wx = k - wy * WX, xx = x0 + wx - RZ, yy = y0 + wy - RZ;
-      double a = 0;
-      float on = 0.f;
-      if (xx >= 0 && yy >= 0 && zp >= 0 && xx < L.ex && yy < L.ey && zp < L.ez) {
-        const long long e = L.eidx(xx, yy, zp);
-        if (L.emask[e]) {
-          on = 1.f;
-          if (MODE != 1) a = (double)in[V.at(xx, yy, zp)];
-          if (MODE == 2) a /= (double)wsum[e];
-        }
-      }
-      v[k] = a;
-      m[k] = on;
-      full = full && on != 0.f;
+#pragma unroll
+    for (int i = 0; i < NK; i++) {
+      const int k = i * FTX * FTY + tid;
+      if (k >= NW) break;
+      double a = (double)raw[i];
+      if (MODE == 2) a /= (double)wgt[i];
+      sv[buf][k] = on[i] ? a : 0.0;
+      sm[buf][k] = on[i] ? 1.f : 0.f;
+      full = full && on[i];
     }
     full = __syncthreads_and(full) != 0;
-    const int c0 = (ty + RZ) * WX + tx + RZ;
-    if (MODE != 1) {
-#pragma unroll
-      for (int d = 0; d <= RZ; d++)
-        for (int k = P.start[d]; k < P.start[d + 1]; k++) {
-          const double a = v[c0 + so[k]];
-          const double* w = sw + k * (RZ + 1);
-          acc[RZ] = fma(w[0], a, acc[RZ]);
-#pragma unroll
-          for (int j = 1; j <= RZ; j++)
-            if (j <= d) {  // d is a constant of the unrolled loop
-              acc[RZ + j] = fma(w[j], a, acc[RZ + j]);
-              acc[RZ - j] = fma(w[j], a, acc[RZ - j]);
-            }
-        }
-    }
+    if (zp + 1 < z1 + RZ) fetch(zp + 1);  // in flight while this plane's taps are added
+    if (MODE != 1) filter_taps<RZ>(P, sv[buf] + c0, acc);
     if (MODE != 2) {
       if (full) {
-        wac[RZ] += wfull[0];
+        wac[RZ] += P.plane[0];
 #pragma unroll
-        for (int j = 1; j <= RZ; j++) { wac[RZ + j] += wfull[j]; wac[RZ - j] += wfull[j]; }
+        for (int j = 1; j <= RZ; j++) { wac[RZ + j] += P.plane[j]; wac[RZ - j] += P.plane[j]; }
       } else {
-#pragma unroll
-        for (int d = 0; d <= RZ; d++)
-          for (int k = P.start[d]; k < P.start[d + 1]; k++) {
-            if (m[c0 + so[k]] == 0.f) continue;
-            const double* w = sw + k * (RZ + 1);
-            wac[RZ] += w[0];
-#pragma unroll
-            for (int j = 1; j <= RZ; j++)
-              if (j <= d) { wac[RZ + j] += w[j]; wac[RZ - j] += w[j]; }
-          }
+        filter_taps<RZ>(P, sm[buf] + c0, wac);
       }
     }
     // acc[k] belongs to output zp + k - RZ: acc[0] is complete
@@ -275,45 +335,38 @@ __global__ void __launch_bounds__(FTX* FTY) k_filter_tile(const Level L, const F
   }
 }
 
-// columns of the tap table of radius R, ordered by their reach in z
-static FPlan filter_columns(double R, int RZ, std::vector<FCol>* cols) {
+static FPlan filter_plan(double R, int RZ) {
   FPlan P = {};
   const double R2 = R * R;
-  for (int d = 0; d <= RZ; d++) {
-    P.start[d] = (int)cols->size();
-    for (int dy = -RZ; dy <= RZ; dy++)
-      for (int dx = -RZ; dx <= RZ; dx++) {
-        const int h2 = dx * dx + dy * dy;
-        if (h2 + d * d > R2 || (d < RZ && h2 + (d + 1) * (d + 1) <= R2)) continue;  // its reach is d
-        FCol c = {dx, dy, {}};
-        for (int k = 0; k <= d; k++) {
-          const double r = std::sqrt((h2 + k * k) / R2), rr = r * r;
-          c.w[k] = 1 - 6 * rr + 8 * rr * r - 3 * rr * rr;
-        }
-        cols->push_back(c);
+  for (int a = 0; a <= kFiltRZ; a++)
+    for (int b = 0; b <= a; b++) {
+      const int c = fclass(a, b), h2 = a * a + b * b;
+      P.reach[c] = -1;
+      for (int d = 0; d <= RZ && a <= RZ && h2 + d * d <= R2; d++) {
+        const double r = std::sqrt((h2 + d * d) / R2), rr = r * r;
+        P.reach[c] = d;
+        P.w[c][d] = 1 - 6 * rr + 8 * rr * r - 3 * rr * rr;
+        P.plane[d] += P.w[c][d] * ((a > 0 ? 2 : 1) * (b > 0 ? 2 : 1) * (a != b ? 2 : 1));
       }
-  }
-  for (int d = RZ + 1; d < kFiltRZ + 2; d++) P.start[d] = (int)cols->size();
+    }
   return P;
 }
 
 template <int RZ>
-static rso_status filter_tiles(rso_handle* h, const FPlan& P, const float* in, float* out, int adjoint, const View& V) {
+static rso_status filter_tiles(rso_handle* h, double R, const float* in, float* out, int adjoint, const View& V) {
   const Level& l = h->L[0];
-  const FCol* cols = static_cast<const FCol*>(h->filt_taps);
+  const FPlan P = filter_plan(R, RZ);
   // planes per chunk: each chunk stages 2 RZ planes more than it writes, so
-  // chunks are as long as the grid still has four CTAs per SM with them
+  // chunks are as long as the grid still has two CTAs per SM with them
   int zc = 64;
-  while (zc > 8 && (long long)cdiv(l.ex, FTX) * cdiv(l.ey, FTY) * cdiv(l.ez, zc) < 4 * 148) zc /= 2;
+  while (zc > 8 && (long long)cdiv(l.ex, FTX) * cdiv(l.ey, FTY) * cdiv(l.ez, zc) < 2 * 148) zc /= 2;
   const dim3 g(cdiv(l.ex, FTX), cdiv(l.ey, FTY), cdiv(l.ez, zc)), b(FTX, FTY);
-  const int nw = (FTX + 2 * RZ) * (FTY + 2 * RZ), nc = P.start[RZ + 1];
-  const size_t smem = nw * 2 * (sizeof(double) + sizeof(float)) + nc * ((RZ + 1) * sizeof(double) + sizeof(int));
   if (!adjoint) {
-    k_filter_tile<RZ, 0><<<g, b, smem, h->stream>>>(l, cols, P, in, out, nullptr, V, zc); rso::note_launch();
+    k_filter_tile<RZ, 0><<<g, b, 0, h->stream>>>(l, P, in, out, nullptr, V, zc); rso::note_launch();
   } else {
     float* W = h->e_d;
-    k_filter_tile<RZ, 1><<<g, b, smem, h->stream>>>(l, cols, P, nullptr, W, nullptr, V, zc); rso::note_launch();
-    k_filter_tile<RZ, 2><<<g, b, smem, h->stream>>>(l, cols, P, in, out, W, V, zc); rso::note_launch();
+    k_filter_tile<RZ, 1><<<g, b, 0, h->stream>>>(l, P, nullptr, W, nullptr, V, zc); rso::note_launch();
+    k_filter_tile<RZ, 2><<<g, b, 0, h->stream>>>(l, P, in, out, W, V, zc); rso::note_launch();
   }
   return launch_check(h, "filter");
 }
@@ -321,45 +374,37 @@ static rso_status filter_tiles(rso_handle* h, const FPlan& P, const float* in, f
 rso_status filter(rso_handle* h, double R, const float* in, float* out, int adjoint, bool dense) {
   const Level& l = h->L[0];
   const View V = view_of(l, dense);
-  const int Ri = (int)(R + 0.5);
-  const int RZ = R < kFiltRZ + 1 ? (int)R : 0;  // 0: the general kernel
+  if (R >= 1 && R < 2) return filter_tiles<1>(h, R, in, out, adjoint, V);
+  if (R >= 2 && R < 3) return filter_tiles<2>(h, R, in, out, adjoint, V);
+  if (R >= 3 && R < 4) return filter_tiles<3>(h, R, in, out, adjoint, V);
+  if (R >= 4 && R < 5) return filter_tiles<4>(h, R, in, out, adjoint, V);
   std::vector<FOff> off;
-  std::vector<FCol> cols;
-  FPlan P = {};
-  if (RZ > 0) {
-    P = filter_columns(R, RZ, &cols);
-  } else {
-    const double R2 = R * R;
-    for (int dx = -Ri; dx <= Ri; dx++)
-      for (int dy = -Ri; dy <= Ri; dy++)
-        for (int dz = -Ri; dz <= Ri; dz++) {
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          if (r2 > R2) continue;
-          const double r = std::sqrt(r2 / R2), rr = r * r;
-          off.push_back({dx, dy, dz, 1 - 6 * rr + 8 * rr * r - 3 * rr * rr});
-        }
-  }
-  // the table is kept on the handle and rebuilt only when the radius changes
-  const void* table = RZ > 0 ? (const void*)cols.data() : (const void*)off.data();
-  const long long bytes = RZ > 0 ? (long long)(sizeof(FCol) * cols.size()) : (long long)(sizeof(FOff) * off.size());
+  const int Ri = (int)(R + 0.5);
+  const double R2 = R * R;
+  for (int dx = -Ri; dx <= Ri; dx++)
+    for (int dy = -Ri; dy <= Ri; dy++)
+      for (int dz = -Ri; dz <= Ri; dz++) {
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 > R2) continue;
+        const double r = std::sqrt(r2 / R2), rr = r * r;
+        off.push_back({dx, dy, dz, 1 - 6 * rr + 8 * rr * r - 3 * rr * rr});
+      }
+  // the tap table is kept on the handle and rebuilt only when the radius changes
   if (!h->filt_taps || h->filt_radius != R) {
     h->filt_radius = -1.0;
-    if (bytes > h->filt_cap) {
+    if ((long long)off.size() > h->filt_cap) {
       if (h->filt_taps) RSO_CHECK_CUDA(h, cudaFree(h->filt_taps));
       h->filt_taps = nullptr;
       h->filt_cap = 0;
-      RSO_CHECK_CUDA(h, cudaMalloc(&h->filt_taps, bytes));
-      h->filt_cap = bytes;
+      RSO_CHECK_CUDA(h, cudaMalloc(&h->filt_taps, sizeof(FOff) * off.size()));
+      h->filt_cap = (long long)off.size();
     }
-    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->filt_taps, table, bytes, cudaMemcpyHostToDevice, h->stream));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->filt_taps, off.data(), sizeof(FOff) * off.size(), cudaMemcpyHostToDevice,
+                                      h->stream));
     // the host table is a local vector: finish the copy before it goes away
     RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
     h->filt_radius = R;
   }
-  if (RZ == 1) return filter_tiles<1>(h, P, in, out, adjoint, V);
-  if (RZ == 2) return filter_tiles<2>(h, P, in, out, adjoint, V);
-  if (RZ == 3) return filter_tiles<3>(h, P, in, out, adjoint, V);
-  if (RZ == 4) return filter_tiles<4>(h, P, in, out, adjoint, V);
   const FOff* d_off = static_cast<const FOff*>(h->filt_taps);
   const int n = (int)off.size();
   if (!adjoint) {
@@ -389,7 +434,11 @@ __global__ void __launch_bounds__(256) k_sum_elems(const Level L, const float* _
     const int z = r / L.ey, y = r - z * L.ey;
     const uint8_t* m = L.emask + L.eidx(0, y, z);
     const float* q = a + V.at(0, y, z);
-    for (int x = lane; x < L.ex; x += 32) s += m[x] ? (double)q[x] : 0.0;
+#pragma unroll 8
+    for (int x = lane; x < L.ex; x += 32) {
+      const float v = q[x];
+      s += m[x] ? (double)v : 0.0;
+    }
   }
   s = warp_add(s);
   if (lane == 0) ws[warp] = s;
@@ -490,6 +539,9 @@ struct SplineDev {
   const float *k0, *k1, *k2;
   const int *i0, *i1, *i2;
   const double *N0, *N1, *N2, *D0, *D1, *D2;
+  // x tables by function: tN, tD[q * ex + x] as N0, D0[x * order + q]; and the
+  // values over each function's support, bN, bD[k * nb0 + a] at x = lo[a] + k
+  const double *tN, *tD, *bN, *bD;
 };
 
 static SplineDev spline_dev(rso_handle* h, const float* knots_dev) {
@@ -502,6 +554,8 @@ static SplineDev spline_dev(rso_handle* h, const float* knots_dev) {
   d.i0 = s.idx[0]; d.i1 = s.idx[1]; d.i2 = s.idx[2];
   d.N0 = s.N[0]; d.N1 = s.N[1]; d.N2 = s.N[2];
   d.D0 = s.dN[0]; d.D1 = s.dN[1]; d.D2 = s.dN[2];
+  const long long no = (long long)s.order * h->L[0].ex, nb = (long long)s.nb[0] * s.sup;
+  d.tN = s.xtab; d.tD = d.tN + no; d.bN = d.tD + no; d.bD = d.bN + nb;
   return d;
 }
 
@@ -567,26 +621,34 @@ static rso_status spline_rows(rso_handle* h, const SplineDev& S, const double* c
 }
 
 // ---------------------------------------------------------------- spline forward
+// a thread keeps its x's basis values and walks along z (134 us at 256^3 with one
+// element per thread, which loaded them each time: bound by those loads; 63 now)
+template <int O>
 __global__ void __launch_bounds__(256) k_coeff2density(const Level L, SplineDev S, const double* __restrict__ R,
                                                        double rmin, const uint8_t* __restrict__ shell,
-                                                       float* __restrict__ out, const View V) {
+                                                       float* __restrict__ out, const View V, int zc) {
   const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
   if (x >= L.ex || y >= L.ey) return;
-  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
-    const long long o = V.at(x, y, z);
-    if (!L.emask[L.eidx(x, y, z)]) { out[o] = 0.f; continue; }
-    const int i = S.i0[x];
-    double v;
-    if (i < 0 || S.i1[y] < 0 || S.i2[z] < 0) {
-      v = -0.2;
-    } else {
-      const double* row = R + (long long)S.nb0 * (y + (long long)L.ey * z) + (i - S.order);
-      v = 0;
-      for (int q = 0; q < S.order; q++) v += row[q] * S.N0[x * S.order + q];
-    }
+  const int i = S.i0[x];
+  const bool in_xy = i >= 0 && S.i1[y] >= 0;
+  double N[O];
+#pragma unroll
+  for (int q = 0; q < O; q++) N[q] = S.tN[(long long)q * L.ex + x];
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.ez);
+  const long long rs = (long long)S.nb0 * L.ey, qxy = (long long)L.qx * L.qy;
+  const double* row = R + (long long)S.nb0 * (y + (long long)L.ey * z0) + (in_xy ? i - O : 0);
+  const uint8_t* mask = L.emask + L.eidx(x, y, z0);
+  const uint8_t* sh = shell ? shell + x + (long long)L.ex * (y + (long long)L.ey * z0) : nullptr;
+  out += V.at(x, y, z0);
+#pragma unroll 4
+  for (int z = 0; z < z1 - z0; z++) {
+    double v = 0;
+#pragma unroll
+    for (int q = 0; q < O; q++) v += row[z * rs + q] * N[q];  // outside the knots: any row, not used
+    if (!in_xy || S.i2[z0 + z] < 0) v = -0.2;
     v = fmin(fmax(v, rmin), 1.0);
-    if (shell && shell[x + (long long)L.ex * (y + (long long)L.ey * z)]) v = 1.0;
-    out[o] = (float)v;
+    if (sh && sh[(long long)z * L.ex * L.ey]) v = 1.0;
+    out[z * V.sz] = mask[z * qxy] ? (float)v : 0.f;
   }
 }
 
@@ -595,54 +657,69 @@ rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, f
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
   const SplineDev S = spline_dev(h, h->sp.knots_dev);
   RSO_TRY(spline_rows(h, S, c, h->sp.work[0], false));
-  k_coeff2density<<<elem_grid(l), dim3(32, 8), 0, h->stream>>>(l, S, h->sp.work[0], h->cfg.rho_min, shell, out,
-                                                               view_of(l, dense)); rso::note_launch();
+  const int zc = column_chunk(l);
+  const dim3 g = column_grid(l, zc), b(32, 8);
+  const View V = view_of(l, dense);
+  const double* R = h->sp.work[0];
+  const double rmin = h->cfg.rho_min;
+  if (S.order == 2) k_coeff2density<2><<<g, b, 0, h->stream>>>(l, S, R, rmin, shell, out, V, zc);
+  else if (S.order == 3) k_coeff2density<3><<<g, b, 0, h->stream>>>(l, S, R, rmin, shell, out, V, zc);
+  else if (S.order == 4) k_coeff2density<4><<<g, b, 0, h->stream>>>(l, S, R, rmin, shell, out, V, zc);
+  else k_coeff2density<5><<<g, b, 0, h->stream>>>(l, S, R, rmin, shell, out, V, zc);
+  rso::note_launch();
   return launch_check(h, "coeff2density");
 }
 
 // ---------------------------------------------------------------- separable adjoint
-// Stage 1, x: a warp takes a row of elements, `seg` of them at a time, their
-// weights in shared memory, and sums for each basis function over its support:
-// G1[z][y][a] (+)= sum_x w(x) B_a(x).  Row reads are coalesced and every weight
-// is read from memory once (a thread per (a, y, z) read each `order` times, 202
-// us at 256^3 and 32 coefficients).
-constexpr int kSeg = 128;
-// sum over the segment [xa, xb) of w B for basis function a; lo, hi its support
-__device__ __forceinline__ double seg_sum(const SplineDev& S, const double* __restrict__ B, const double* w, int a,
-                                          int lo, int hi, int xa, int xb) {
-  double s = 0;
-  for (int x = max(lo, xa); x <= min(hi, xb - 1); x++) s += w[x - xa] * B[x * S.order + a - S.i0[x] + S.order];
-  return s;
-}
-// the basis functions a segment's elements lie in the support of: [*a0, *a1)
-__device__ __forceinline__ void seg_range(const SplineDev& S, int xa, int xb, int* a0, int* a1) {
-  const int i = S.i0[xa], j = S.i0[xb - 1];
-  *a0 = i >= 0 ? i - S.order : 0;
-  *a1 = j >= 0 ? j : S.nb0;
-}
-__global__ void __launch_bounds__(256) k_adj_x(const Level L, SplineDev S, const float* __restrict__ g,
-                                               const uint8_t* __restrict__ shell, const View V,
-                                               const int* __restrict__ lo, const int* __restrict__ hi,
-                                               double* __restrict__ G1) {
-  __shared__ double w[8][kSeg];
+// Stage 1, x: a warp takes two rows of elements, kSeg elements at a time, their
+// weights in shared memory, and a lane sums for its basis function over its
+// support: G1[z][y][a] (+)= sum_x w(x) B_a(x).  Row reads are coalesced, every
+// weight is read from memory once, and the function's values (bN, lanes side by
+// side) serve both rows.  256^3, 32 coefficients: 202 us with a thread per
+// (a, y, z) reading the fields directly, 205 with one row per warp and the values
+// looked up through the span table, 88 now.
+constexpr int kSeg = 256, kAdjRows = 2, kAdjWarps = 4;
+__global__ void __launch_bounds__(32 * kAdjWarps) k_adj_x(const Level L, SplineDev S, const float* __restrict__ g,
+                                                          const uint8_t* __restrict__ shell, const View V,
+                                                          const int* __restrict__ lo, const int* __restrict__ hi,
+                                                          double* __restrict__ G1) {
+  __shared__ double w[kAdjWarps][kAdjRows][kSeg];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = blockIdx.x * 8 + warp;
-  if (r >= L.ey * L.ez) return;
-  const int z = r / L.ey, y = r - z * L.ey;
-  double* G = G1 + (long long)S.nb0 * r;
-  for (int a = lane; a < S.nb0; a += 32) G[a] = 0;
-  if (S.i1[y] < 0 || S.i2[z] < 0) return;
-  const uint8_t* m = L.emask + L.eidx(0, y, z);
-  const float* q = g + V.at(0, y, z);
-  const uint8_t* sh = shell ? shell + (long long)L.ex * r : nullptr;
+  const int rows = L.ey * L.ez, r0 = (blockIdx.x * kAdjWarps + warp) * kAdjRows;
+  if (r0 >= rows) return;
   for (int xa = 0; xa < L.ex; xa += kSeg) {
     const int xb = min(xa + kSeg, L.ex);
     __syncwarp();
-    for (int x = xa + lane; x < xb; x += 32) w[warp][x - xa] = m[x] && !(sh && sh[x]) ? (double)q[x] : 0.0;
+#pragma unroll
+    for (int j = 0; j < kAdjRows; j++) {
+      const int r = r0 + j, z = r / L.ey, y = r - z * L.ey;
+      const bool in = r < rows && S.i1[y] >= 0 && S.i2[z] >= 0;
+      const uint8_t* m = L.emask + (in ? L.eidx(0, y, z) : 0);
+      const float* q = g + (in ? V.at(0, y, z) : 0);
+      const uint8_t* sh = shell && in ? shell + (long long)L.ex * r : nullptr;
+#pragma unroll 4
+      for (int x = xa + lane; x < xb; x += 32) {
+        const float v = in ? q[x] : 0.f;
+        w[warp][j][x - xa] = in && m[x] && !(sh && sh[x]) ? (double)v : 0.0;
+      }
+    }
     __syncwarp();
-    int a0, a1;
-    seg_range(S, xa, xb, &a0, &a1);
-    for (int a = a0 + lane; a < a1; a += 32) G[a] += seg_sum(S, S.N0, w[warp], a, lo[a], hi[a], xa, xb);
+    for (int a = lane; a < S.nb0; a += 32) {
+      const int l0 = lo[a], ka = max(l0, xa) - l0, kb = min(hi[a], xb - 1) - l0;
+      double s[kAdjRows] = {};
+#pragma unroll 4
+      for (int k = ka; k <= kb; k++) {
+        const double B = S.bN[(long long)k * S.nb0 + a];
+#pragma unroll
+        for (int j = 0; j < kAdjRows; j++) s[j] = fma(w[warp][j][l0 + k - xa], B, s[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < kAdjRows; j++)
+        if (r0 + j < rows) {
+          double* G = G1 + (long long)S.nb0 * (r0 + j) + a;
+          *G = xa == 0 ? s[j] : *G + s[j];
+        }
+    }
   }
 }
 // Stage 2, y: G2[z][b][a] = sum_y G1[z][y][a] N_b(y) (+ Gd[z][y][a] D_b(y))
@@ -699,7 +776,8 @@ rso_status density2coeff(rso_handle* h, const float* g, const uint8_t* shell, do
   const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1], *r2 = h->sp.ranges[2];
   const long long rows = (long long)l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
                   t3 = (long long)S.nb0 * S.nb1 * S.nb2;
-  k_adj_x<<<cdiv(rows, 8), 256, 0, h->stream>>>(l, S, g, shell, view_of(l, dense), r0, r0 + S.nb0, G1); rso::note_launch();
+  k_adj_x<<<cdiv(rows, kAdjRows * kAdjWarps), 32 * kAdjWarps, 0, h->stream>>>(l, S, g, shell, view_of(l, dense), r0,
+                                                                               r0 + S.nb0, G1); rso::note_launch();
   k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, G1, nullptr, r1, r1 + S.nb1, G2); rso::note_launch();
   k_adj_z<<<cdiv(t3, 32), dim3(32, 8), 0, h->stream>>>(S, G2, nullptr, r2, r2 + S.nb2, nullptr, dc); rso::note_launch();
   return launch_check(h, "density2coeff");
@@ -759,7 +837,7 @@ __global__ void __launch_bounds__(1024) k_max_abs(long long n, const double* __r
 
 // The constraint on every element in one pass: value and gradient from the
 // spline rows, the probe's sign, the penalty, and stage 1 (x) of the separable
-// adjoint of its three weights.  A warp takes a row of elements, kSeg at a time.
+// adjoint of its three weights.  A warp takes a row of elements, kSSSeg at a time.
 //
 // The probe walks t = 0.01 along the gradient g, so the spline there is at
 // least v + t |g|^2 (1 - t H / 2), H a bound on its second derivatives: for
@@ -768,7 +846,7 @@ __global__ void __launch_bounds__(1024) k_max_abs(long long n, const double* __r
 // holds H / M).  Where that growth times the least slope of the step between the
 // two values is far above the rounding of the two tanh, the probe's sign is
 // known, -1, without evaluating it (64 coefficients, three basis recursions and
-// six tanh: 3.4 of the 3.65 ms this stage took at 256^3); elsewhere probe_sign
+// six tanh: 3.4 of the 3.65 ms this stage took at 256^3; the whole pass takes 0.66); elsewhere probe_sign
 // decides, as before.
 //
 // The penalty needs the sign `flip` that the sum of all probes gives.  It is
@@ -776,60 +854,66 @@ __global__ void __launch_bounds__(1024) k_max_abs(long long n, const double* __r
 // whose density grows along its gradient; the caller runs the pass again when
 // it does not.
 struct SSOut { double *G1, *Gy, *Gz; float* per; double* part; };
-constexpr int kSSRows = 4;
-__global__ void __launch_bounds__(32 * kSSRows) k_ss_rows(const Level L, SplineDev S, const double* __restrict__ c,
-                                                          const double* __restrict__ R, long long comp, const SSPar P,
-                                                          double flip, double direction, const double* __restrict__ cmax,
-                                                          double hcoef, double smin, const int* __restrict__ lo,
-                                                          const int* __restrict__ hi, const SSOut O, const View V) {
-  __shared__ double w[kSSRows][4][kSeg];
+constexpr int kSSRows = 4, kSSSeg = 128;
+template <int O>
+__global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, SplineDev S, const double* __restrict__ c,
+                                                             const double* __restrict__ R, long long comp, const SSPar P,
+                                                             double flip, double direction,
+                                                             const double* __restrict__ cmax, double hcoef, double smin,
+                                                             const int* __restrict__ lo, const int* __restrict__ hi,
+                                                             const SSOut Q, const View V) {
+  __shared__ double w[kSSRows][4][kSSSeg];
   __shared__ double red[kSSRows][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = blockIdx.x * kSSRows + warp;
-  double sdir = 0, sper = 0, sdown = 0;
+  double sper = 0;
+  int ndir = 0, ndown = 0;  // probes with sign +1 less those with -1; downward faces
   if (r < L.ey * L.ez) {
-    const int z = r / L.ey, y = r - z * L.ey, o = S.order;
+    const int z = r / L.ey, y = r - z * L.ey;
     const long long gb = (long long)S.nb0 * r;
     const bool in_yz = S.i1[y] >= 0 && S.i2[z] >= 0;
-    const double tH = 0.01 * hcoef * *cmax;
-    for (int a = lane; a < S.nb0; a += 32) O.G1[gb + a] = O.Gy[gb + a] = O.Gz[gb + a] = 0;
-    for (int xa = 0; xa < L.ex; xa += kSeg) {
-      const int xb = min(xa + kSeg, L.ex);
+    const double tH = 0.01 * hcoef * *cmax, least = 1e-11 * (1 + *cmax);
+    const double rcos = 1 / P.cosang, rsc = 1 / P.sc;
+    const uint8_t* mask = L.emask + L.eidx(0, y, z);
+    const double *r0 = R + gb - O, *r1 = r0 + comp, *r2 = r1 + comp;
+    float* per = Q.per ? Q.per + V.at(0, y, z) : nullptr;
+    for (int xa = 0; xa < L.ex; xa += kSSSeg) {
+      const int xb = min(xa + kSSSeg, L.ex);
       __syncwarp();
       for (int x = xa + lane; x < xb; x += 32) {
         double wA = 0, wX = 0, wY = 0, wZ = 0;
         float val32 = 0.f;
-        if (L.emask[L.eidx(x, y, z)]) {
+        if (mask[x]) {
           const int I = S.i0[x];
           const bool inside = I >= 0 && in_yz;
           double f = 0, g0 = 0, g1 = 0, g2 = 0;
           if (inside) {
-            const double* row = R + gb + (I - o);
-            for (int q = 0; q < o; q++) {
-              const double N = S.N0[x * o + q], t = row[q];
+            const double *tn = S.tN + x, *td = S.tD + x;
+#pragma unroll
+            for (int q = 0; q < O; q++) {
+              const double N = tn[q * L.ex], t = r0[I + q];
               f += t * N;
-              g0 += t * S.D0[x * o + q];
-              g1 += row[q + comp] * N;
-              g2 += row[q + 2 * comp] * N;
+              g0 += t * td[q * L.ex];
+              g1 += r1[I + q] * N;
+              g2 += r2[I + q] * N;
             }
           }
           const double gg = g0 * g0 + g1 * g1 + g2 * g2;
           bool known = false;
-          if (o >= 3 && tH < 1.0 && inside) {
+          if (O >= 3 && tH < 1.0 && inside) {
             const double grow = 0.01 * gg * (1 - 0.5 * tH);
             // sech^2(s) >= exp(-2 |s|), s up to beta (|v - 1/2| + what the probe may rise)
             const float slope = __expf((float)(-2 * P.beta * (fabs(f - 0.5) + 0.02 * gg)));
-            known = (float)(P.beta * grow) * slope > 1e-12f && grow > 1e-11 * (1 + *cmax) && 1e-4 * gg < smin * smin;
+            known = (float)(P.beta * grow) * slope > 1e-12f && grow > least && 1e-4 * gg < smin * smin;
           }
-          sdir += known ? -1.0 : (double)probe_sign(S, c, P.beta, x, y, z, inside, f, g0, g1, g2);
-          const double n0 = flip * g0, n1 = flip * g1, n2 = flip * g2;
-          const bool dn = n2 < 0;
-          if (dn) sdown += 1.0;
+          ndir += known || probe_sign(S, c, P.beta, x, y, z, inside, f, g0, g1, g2) < 0.f ? -1 : 1;
+          const bool dn = flip * g2 < 0;
+          ndown += dn;
           const bool on = (P.mode % 2 == 1) || dn;
-          const double nn = sqrt(gg);
           // off: no penalty, and zero weights unless the direction is undefined
-          if (on || !(nn > 0) || isinf(nn)) {
-            const double inner = n2 / nn / P.cosang;
+          if (on || !(gg > 0)) {
+            const double rn = rsqrt(gg), n2 = flip * g2 * rn;  // n2: the unit normal's z
+            const double inner = n2 * rcos;
             double val = 0, A = 0, B = 0;
             if (on) {
               const int m = P.mode;
@@ -838,73 +922,71 @@ __global__ void __launch_bounds__(32 * kSSRows) k_ss_rows(const Level L, SplineD
               else {
                 const double nd = exp(-P.na * (f - 0.5) * (f - 0.5));
                 const double dnd = -2 * P.na * (f - 0.5) * nd;
-                const double ex_ = exp(-(inner - P.mid) / P.sc);
-                const double ov = 2 / (1 + ex_), dov = 2 / (1 + ex_) / (1 + ex_) / P.sc * ex_;
+                const double ex_ = exp(-(inner - P.mid) * rsc), q = __drcp_rn(1 + ex_);
+                const double ov = 2 * q, dov = ov * q * rsc * ex_;
                 const double in_ = inner > 1 ? P.ia * (inner - 1) + 1 : 1, din = inner > 1 ? P.ia : 1;
                 val = nd * ov * in_; A = dnd * ov * in_; B = nd * dov * in_ + nd * ov * din;
               }
             }
             val32 = (float)val;
             if (inside) {
-              // dinner = al*(N N dN) + be*(dN N N) + ga*(N dN N)  (see compute_spline_bg_selfsupp_constraint_dcoeff)
-              const double den = nn * nn * P.cosang;
-              const double al = direction * (nn - n2 * n2 / nn) / den;
-              const double be = -direction * n2 * n0 / nn / den;
-              const double ga = -direction * n2 * n1 / nn / den;
-              wA = A; wZ = B * al; wX = B * be; wY = B * ga;
+              // dinner = al*(N N dN) + be*(dN N N) + ga*(N dN N)  (see compute_spline_bg_selfsupp_constraint_dcoeff),
+              // al = direction (nn - n2^2 / nn) / den, be = -direction n2 n0 / nn / den, den = nn^2 cosang
+              const double k = B * (direction * rn * rcos), kt = -k * n2 * (flip * rn);
+              wA = A; wZ = k * (1 - n2 * n2); wX = kt * g0; wY = kt * g1;
             }
           }
           sper += (double)val32;
         }
-        if (O.per) O.per[V.at(x, y, z)] = val32;
+        if (per) per[x] = val32;
         w[warp][0][x - xa] = wA; w[warp][1][x - xa] = wX; w[warp][2][x - xa] = wY; w[warp][3][x - xa] = wZ;
       }
       __syncwarp();
-      if (in_yz) {
-        int a0, a1;
-        seg_range(S, xa, xb, &a0, &a1);
-        for (int a = a0 + lane; a < a1; a += 32) {
-          double s = 0, sy = 0, sz = 0;
-          for (int x = max(lo[a], xa); x <= min(hi[a], xb - 1); x++) {
-            const int k = x * o + a - S.i0[x] + o;
-            const double N = S.N0[k];
-            s += w[warp][0][x - xa] * N + w[warp][1][x - xa] * S.D0[k];
-            sy += w[warp][2][x - xa] * N;
-            sz += w[warp][3][x - xa] * N;
-          }
-          O.G1[gb + a] += s;
-          O.Gy[gb + a] += sy;
-          O.Gz[gb + a] += sz;
+      for (int a = lane; a < S.nb0; a += 32) {
+        const int l0 = lo[a], ka = max(l0, xa) - l0, kb = in_yz ? min(hi[a], xb - 1) - l0 : -1;
+        double s = 0, sy = 0, sz = 0;
+        const double *bn = S.bN + a, *bd = S.bD + a;
+#pragma unroll 2
+        for (int k = ka; k <= kb; k++) {
+          const double N = bn[(long long)k * S.nb0], D = bd[(long long)k * S.nb0];
+          const int x = l0 + k - xa;
+          s = fma(w[warp][0][x], N, fma(w[warp][1][x], D, s));
+          sy = fma(w[warp][2][x], N, sy);
+          sz = fma(w[warp][3][x], N, sz);
         }
+        if (xa > 0 && kb < ka) continue;
+        const bool first = xa == 0;
+        Q.G1[gb + a] = first ? s : Q.G1[gb + a] + s;
+        Q.Gy[gb + a] = first ? sy : Q.Gy[gb + a] + sy;
+        Q.Gz[gb + a] = first ? sz : Q.Gz[gb + a] + sz;
       }
     }
   }
-  sdir = warp_add(sdir);
   sper = warp_add(sper);
-  sdown = warp_add(sdown);
+  const double sdir = (double)__reduce_add_sync(0xffffffffu, ndir), sdown = (double)__reduce_add_sync(0xffffffffu, ndown);
   if (lane == 0) { red[warp][0] = sdir; red[warp][1] = sper; red[warp][2] = sdown; }
   __syncthreads();
   if (threadIdx.x < 3) {
     double t = 0;
     for (int k = 0; k < kSSRows; k++) t += red[k][threadIdx.x];
-    O.part[threadIdx.x * (long long)gridDim.x + blockIdx.x] = t;
+    Q.part[threadIdx.x * (long long)gridDim.x + blockIdx.x] = t;
   }
 }
 // out[0..2] = the sums of probes, penalties and downward faces; out[3] the count the mean divides by
-__global__ void __launch_bounds__(512) k_ss_sums(const double* __restrict__ part, int n, int mode, double active,
+__global__ void __launch_bounds__(1024) k_ss_sums(const double* __restrict__ part, int n, int mode, double active,
                                                  double* __restrict__ out) {
-  __shared__ double sh[16];
+  __shared__ double sh[32];
   double tot[3];
   for (int k = 0; k < 3; k++) {
     double s = 0;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < n; i += 512) s += part[(long long)k * n + i];
+#pragma unroll 8
+    for (int i = threadIdx.x; i < n; i += 1024) s += part[(long long)k * n + i];
     s = warp_add(s);
     __syncthreads();
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
     __syncthreads();
     tot[k] = 0;
-    for (int q = 0; q < 16; q++) tot[k] += sh[q];
+    for (int q = 0; q < 32; q++) tot[k] += sh[q];
   }
   if (threadIdx.x == 0) {
     out[0] = tot[0];
@@ -958,9 +1040,10 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
   const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1], *r2 = h->sp.ranges[2];
   double flip = -1.0, direction = -1.0;
   for (int pass = 0; pass < 2; pass++) {
-    k_ss_rows<<<nblk, 32 * kSSRows, 0, h->stream>>>(l, S, c, R, comp, P, flip, direction, sums + 4, hcoef, smin, r0,
-                                                    r0 + S.nb0, O, view_of(l, true)); rso::note_launch();
-    k_ss_sums<<<1, 512, 0, h->stream>>>(O.part, nblk, mode, (double)l.n_active_e, sums); rso::note_launch();
+    auto rows = S.order == 2 ? k_ss_rows<2> : S.order == 3 ? k_ss_rows<3> : S.order == 4 ? k_ss_rows<4> : k_ss_rows<5>;
+    rows<<<nblk, 32 * kSSRows, 0, h->stream>>>(l, S, c, R, comp, P, flip, direction, sums + 4, hcoef, smin, r0,
+                                               r0 + S.nb0, O, view_of(l, true)); rso::note_launch();
+    k_ss_sums<<<1, 1024, 0, h->stream>>>(O.part, nblk, mode, (double)l.n_active_e, sums); rso::note_launch();
     if (dc) {
       k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, O.G1, O.Gy, r1, r1 + S.nb1, G2); rso::note_launch();
       k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, O.Gz, nullptr, r1, r1 + S.nb1, G2z); rso::note_launch();
@@ -995,6 +1078,8 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
     cudaFree(s.idx[a]); cudaFree(s.N[a]); cudaFree(s.dN[a]); cudaFree(s.ranges[a]);
   }
   cudaFree(s.knots_dev);
+  cudaFree(s.xtab);
+  s.xtab = nullptr;
   for (auto& p : s.work) { cudaFree(p); p = nullptr; }
   s.order = order;
   s.part[0] = px; s.part[1] = py; s.part[2] = pz;
@@ -1047,6 +1132,26 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
         if (!seen[b]) { rg[b] = x; seen[b] = true; }
         rg[s.nb[a] + b] = x;
       }
+    }
+    if (a == 0) {
+      // the x axis by function (see SplineDev); n and order values twice, then the supports'
+      const int nb = s.nb[0];
+      s.sup = 1;
+      for (int b = 0; b < nb; b++) s.sup = std::max(s.sup, rg[nb + b] - rg[b] + 1);
+      std::vector<double> tab(2 * ((size_t)n * order + (size_t)nb * s.sup), 0.0);
+      double *tn = tab.data(), *td = tn + (size_t)n * order, *bn = td + (size_t)n * order, *bd = bn + (size_t)nb * s.sup;
+      for (int x = 0; x < n; x++)
+        for (int q = 0; q < order; q++) {
+          const double N = s.h_N[0][(size_t)x * order + q], D = s.h_dN[0][(size_t)x * order + q];
+          tn[(size_t)q * n + x] = N;
+          td[(size_t)q * n + x] = D;
+          if (s.h_idx[0][x] < 0) continue;
+          const int b = s.h_idx[0][x] - order + q;
+          bn[(size_t)(x - rg[b]) * nb + b] = N;
+          bd[(size_t)(x - rg[b]) * nb + b] = D;
+        }
+      RSO_CHECK_CUDA(h, cudaMalloc(&s.xtab, sizeof(double) * tab.size()));
+      RSO_CHECK_CUDA(h, cudaMemcpy(s.xtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
     }
     RSO_CHECK_CUDA(h, cudaMalloc(&s.ranges[a], sizeof(int) * rg.size()));
     RSO_CHECK_CUDA(h, cudaMemcpy(s.ranges[a], rg.data(), sizeof(int) * rg.size(), cudaMemcpyHostToDevice));

@@ -79,6 +79,8 @@ struct Spline {
   long long n_coeff = 0;
   float* knots_dev = nullptr;                      // the three knot vectors back to back
   int* ranges[3] = {nullptr, nullptr, nullptr};    // per basis index: first/last element coordinate in its support
+  double* xtab = nullptr;                          // x basis tables by function (design.cu)
+  int sup = 1;                                     // longest support along x
   double* work[3] = {};                            // spline rows, adjoint stages, self-support scratch
 };
 
