@@ -1440,57 +1440,6 @@ __global__ void __cluster_dims__(BOT_CTAS, 1, 1) __launch_bounds__(BOT_THREADS, 
 // the 33^3 level of 256^3 down 174 -> 149 us (33^3 streamed, the rest held),
 // 93 x 71 x 85 110 -> 70 us, 64^3 96 -> 59 us, 49 x 38 x 56 68 -> 37 us (all
 // held), before: two-word barriers, every stencil streamed, two CTAs per SM.
-// a barrier wait gives up after this many SM clock cycles (about 2 s)
-constexpr long long kGbarCycles = 4000000000LL;
-
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid-wide barrier on bar = {arrivals, exits, gave-up flag}: one arrival per
-// CTA (a release), the arrivals counted on through the launch, so that a waiter
-// polls the very word the arrivals change (no reset, no second word to pass on:
-// 2.4 us per barrier with both, see k_bottom_grid for what is left).  goal is
-// thread 0's count of arrivals that completes its next barrier.  The last CTA to
-// leave the kernel (gbar_exit) clears the counts for the next launch.  Returns
-// false on every thread of every CTA once some wait has given up (kGbarGone in
-// the arrivals, and bar[2] for the host): the kernel then returns, and the host
-// reports it after the solve and clears all words.
-// (target, limit: the arrivals that complete the barrier and the wait's bound
-// in clock cycles; the self-test sets them, the bottom kernel keeps the grid
-// size and kGbarCycles)
-constexpr unsigned kGbarGone = 1u << 31;
-__device__ bool gbar_sync(unsigned* bar, unsigned& goal, int tid, unsigned target, long long limit = kGbarCycles) {
-  __syncthreads();
-  int bad = 0;
-  if (tid == 0) {
-    goal += target;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    const long long t0 = clock64();
-    for (;;) {
-      const unsigned v = ld_acquire_gpu(bar);
-      if (v & kGbarGone) { bad = 1; break; }
-      if (v >= goal) break;
-      if (clock64() - t0 > limit) {
-        atomicOr(bar, kGbarGone);
-        atomicExch(bar + 2, 1u);
-        bad = 1;
-        break;
-      }
-    }
-  }
-  return __syncthreads_or(bad) == 0;
-}
-// every CTA of a launch that passed all its barriers calls this once
-__device__ void gbar_exit(unsigned* bar, int tid) {
-  if (tid == 0 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
-    bar[0] = 0u;
-    bar[1] = 0u;
-  }
-}
-
 // one row-split sweep (MODE 2) or residual (MODE 0) of a level, tile by tile
 template <typename T, int MODE, bool ZERO>
 __device__ void gb_sweep_rows(const Level& L, const T* st, const T* u, const T* f, T* out, T omega, const T* uprev,

@@ -1,18 +1,18 @@
 // Svanberg MMA (the reference's mma_t: optimization/mma_t.h:159-266,
-// mma_t.cpp:18-118, mma_t.cu:15-909) in FP64 on the device.  The n-sized
-// work (asymptotes, p/q, the reduced-system sums, the step bounds and the
-// KKT residual of every line-search trial) runs in fused kernels with
-// deterministic two-pass reductions; the (m+1)^2 dual system and the
-// m-sized bookkeeping run on the host, as the reference does with Eigen.
+// mma_t.cpp:18-118, mma_t.cu:15-909) in FP64 on the device.  An update is one
+// cooperative kernel: the n-sized work (p/q, the reduced-system sums, the step
+// bounds, the KKT residual of every line-search trial, the asymptotes) with
+// deterministic grid-wide reductions, and the (m+1)^2 dual system with the
+// m-sized bookkeeping, which every CTA carries out alike.
 #include "rso_internal.cuh"
 #include <cmath>
-#include <vector>
 #include <algorithm>
+#include <string>
 
-constexpr int MMA_MAXM = 8;
-constexpr int MMA_RED = 40;   // max reductions in one pass
-constexpr int MMA_BLOCKS = 256;
-constexpr int MMA_THREADS = 256;
+constexpr int MMA_MAXM = 5;                       // constraints an update is built for
+constexpr int MMA_BLOCKS = 256, MMA_THREADS = 256;  // set-up kernels
+constexpr int MMA_UT = 512;                       // threads of a CTA of the update kernel
+constexpr int MMA_RED = MMA_MAXM * MMA_MAXM + 2 * MMA_MAXM + 6;  // most values one reduction carries
 
 struct rso_mma {
   int n = 0, m = 0;
@@ -23,87 +23,12 @@ struct rso_mma {
   double *P = nullptr, *Q = nullptr, *Dx = nullptr, *hdx = nullptr, *G = nullptr, *dx = nullptr, *dxi = nullptr,
          *deta = nullptr;
   double *part = nullptr, *res = nullptr, *h_res = nullptr;
-  std::vector<double> y, lambda, mu, s, a, c, d, b, lam_pq;
-  double z = 1, zeta = 1, a0 = 1, eps = 1;
+  unsigned* bar = nullptr;  // the update kernel's grid barrier (gbar_sync)
+  int ctas = 1;             // its CTAs, resident together: one per SM at most
   int stop_counter = 0;
 };
 
 namespace {
-
-struct MPar {
-  int n, m;
-  double eps;
-  double lam[MMA_MAXM];
-  double dl[MMA_MAXM];
-  double step;
-};
-
-__device__ __forceinline__ double wsum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ double wmax(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-  return v;
-}
-
-// reduce R values per thread over the block; op 0 sum, 1 max; partial[r * gridDim.x + block]
-template <int R>
-__device__ void block_reduce(double (&v)[R], const int* ops, int nr, double* part) {
-  __shared__ double sh[MMA_RED][MMA_THREADS / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int r = 0; r < nr; r++) {
-    const double t = ops[r] ? wmax(v[r]) : wsum(v[r]);
-    if (lane == 0) sh[r][w] = t;
-  }
-  __syncthreads();
-  if (threadIdx.x < nr) {
-    const int r = threadIdx.x;
-    double acc = ops[r] ? -1e300 : 0.0;
-    for (int k = 0; k < MMA_THREADS / 32; k++) acc = ops[r] ? fmax(acc, sh[r][k]) : acc + sh[r][k];
-    part[(long long)r * gridDim.x + blockIdx.x] = acc;
-  }
-}
-
-__global__ void k_final(const double* part, int nblocks, int nr, const int* ops_dummy, int opmask_lo,
-                        int opmask_hi, double* out) {
-  const int r = threadIdx.x;
-  if (r >= nr) return;
-  const bool mx = r < 32 ? ((opmask_lo >> r) & 1) : ((opmask_hi >> (r - 32)) & 1);
-  double acc = mx ? -1e300 : 0.0;
-  for (int b = 0; b < nblocks; b++) acc = mx ? fmax(acc, part[(long long)r * nblocks + b]) : acc + part[(long long)r * nblocks + b];
-  out[r] = acc;
-}
-
-__global__ void k_pq(int n, int m, const double* __restrict__ df, const double* __restrict__ dg,
-                     const double* __restrict__ x, const double* __restrict__ L, const double* __restrict__ U,
-                     const double* __restrict__ xmin, const double* __restrict__ xmax, double* __restrict__ P,
-                     double* __restrict__ Q) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double ux = U[i] - x[i], xl = x[i] - L[i], raa = 1e-5 / (xmax[i] - xmin[i]);
-    for (int j = 0; j <= m; j++) {
-      const double d = j == 0 ? df[i] : dg[(long long)(j - 1) * n + i];
-      const double pos = fmax(d, 0.0), neg = fmax(-d, 0.0);
-      P[(long long)j * n + i] = ux * ux * (1.001 * pos + 0.001 * neg + raa);
-      Q[(long long)j * n + i] = xl * xl * (0.001 * pos + 1.001 * neg + raa);
-    }
-  }
-}
-
-// gproxy_j = sum p_{j+1}/(U-x) + q_{j+1}/(x-L)
-__global__ void __launch_bounds__(MMA_THREADS) k_gp(MPar p, const double* __restrict__ x, const double* __restrict__ L,
-                                                    const double* __restrict__ U, const double* __restrict__ P,
-                                                    const double* __restrict__ Q, double* part) {
-  double v[MMA_MAXM] = {0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.n; i += (long long)gridDim.x * blockDim.x) {
-    const double ux = U[i] - x[i], xl = x[i] - L[i];
-    for (int j = 0; j < p.m; j++) v[j] += P[(long long)(j + 1) * p.n + i] / ux + Q[(long long)(j + 1) * p.n + i] / xl;
-  }
-  int ops[MMA_MAXM] = {0};
-  block_reduce<MMA_MAXM>(v, ops, p.m, part);
-}
 
 __global__ void k_reset(int n, double* x, const double* alpha, const double* beta, double* xi, double* eta) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -114,136 +39,394 @@ __global__ void k_reset(int n, double* x, const double* alpha, const double* bet
   }
 }
 
-// Newton system sums: A11[j][k] = sum G_j G_k / Dx, s_j = sum G_j hdx/Dx, gp_j
-__global__ void __launch_bounds__(MMA_THREADS) k_prep(MPar p, const double* __restrict__ x, const double* __restrict__ L,
-                                                      const double* __restrict__ U, const double* __restrict__ alpha,
-                                                      const double* __restrict__ beta, const double* __restrict__ xi,
-                                                      const double* __restrict__ eta, const double* __restrict__ P,
-                                                      const double* __restrict__ Q, double* __restrict__ Dx,
-                                                      double* __restrict__ hdx, double* __restrict__ G, double* part) {
-  double v[MMA_RED];
-  for (int r = 0; r < MMA_RED; r++) v[r] = 0;
-  const int m = p.m, n = p.n;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double ux = U[i] - x[i], xl = x[i] - L[i];
-    double pl = P[i], ql = Q[i];
-    for (int j = 0; j < m; j++) { pl += p.lam[j] * P[(long long)(j + 1) * n + i]; ql += p.lam[j] * Q[(long long)(j + 1) * n + i]; }
-    const double psi = 2 * pl / (ux * ux * ux) + 2 * ql / (xl * xl * xl);
-    const double dxv = psi + xi[i] / (x[i] - alpha[i]) + eta[i] / (beta[i] - x[i]);
-    const double varphi = pl / (ux * ux) - ql / (xl * xl);
-    const double h = -(p.eps / (x[i] - alpha[i]) - p.eps / (beta[i] - x[i]) - varphi);
-    Dx[i] = dxv;
-    hdx[i] = h;
-    double g[MMA_MAXM];
-    for (int j = 0; j < m; j++) {
-      g[j] = P[(long long)(j + 1) * n + i] / (ux * ux) - Q[(long long)(j + 1) * n + i] / (xl * xl);
-      G[(long long)j * n + i] = g[j];
+struct MmaArgs {
+  int n;
+  const double *df, *dg, *xmin, *xmax;
+  double *x, *L, *U, *alpha, *beta, *lastdx, *xi, *eta, *curx, *P, *Q, *Dx, *hdx, *G, *dx, *dxi, *deta;
+  double g[MMA_MAXM];
+  double* part;   // [2][MMA_RED][CTAs]
+  double* out;    // error, last step, sub-iterations, overflow, |dx|^2
+  unsigned* bar;
+};
+
+// The m-sized state of the subproblem (a = 0, a0 = 1, c = 10, d = 1:
+// optimization/mma_t.h:202-211), one copy per CTA, changed by thread 0 alone
+template <int M>
+struct Dual {
+  double lam[M], lam_pq[M], y[M], mu[M], s[M], b[M];  // multipliers and slacks; lam_pq: those p and q were last formed with
+  double dl[M], dy[M], dmu[M], ds[M], nl[M];          // search direction, and the trial's multipliers
+  double z, zeta, dz, dzeta, eps, step, old_err, new_err, err, lasterr, damp;
+  int stays, nsub, overflow, accepted, go;
+};
+constexpr double MMA_C = 10.0, MMA_D = 1.0, MMA_A0 = 1.0;
+
+// Grid-wide sums (and maxima, bit r of mx) of R values per thread into
+// res[0..R) of every CTA: shuffles and shared memory within a CTA, one partial
+// per CTA in the buffer of this reduction's parity, a grid barrier, and every
+// CTA adds the partials up in the same order.  False once a barrier wait has
+// given up.
+template <int R>
+__device__ bool grid_reduce(double (&v)[R], unsigned mx, const MmaArgs& A, int& parity, unsigned& goal, double* res,
+                            double (*sh)[MMA_UT / 32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const bool m = (mx >> r) & 1u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double t = __shfl_down_sync(0xffffffffu, v[r], o);
+      v[r] = m ? fmax(v[r], t) : v[r] + t;
     }
-    int r = 0;
-    for (int j = 0; j < m; j++)
-      for (int k = 0; k < m; k++) v[r++] += g[j] * (g[k] / dxv);
-    for (int j = 0; j < m; j++) v[r++] += g[j] * (h / dxv);
-    for (int j = 0; j < m; j++) v[r++] += P[(long long)(j + 1) * n + i] / ux + Q[(long long)(j + 1) * n + i] / xl;
+    if (lane == 0) sh[r][warp] = v[r];
   }
-  int ops[MMA_RED] = {0};
-  block_reduce<MMA_RED>(v, ops, m * m + 2 * m, part);
+  __syncthreads();
+  double* part = A.part + (long long)parity * MMA_RED * gridDim.x;
+  parity ^= 1;
+  if (threadIdx.x < R) {
+    const int r = threadIdx.x;
+    const bool m = (mx >> r) & 1u;
+    double acc = sh[r][0];
+    for (int k = 1; k < MMA_UT / 32; k++) acc = m ? fmax(acc, sh[r][k]) : acc + sh[r][k];
+    if (gridDim.x == 1) res[r] = acc;
+    else part[(long long)r * gridDim.x + blockIdx.x] = acc;
+  }
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
+  if (!rso::gbar_sync(A.bar, goal, threadIdx.x, gridDim.x)) return false;
+  for (int r = warp; r < R; r += MMA_UT / 32) {
+    const bool m = (mx >> r) & 1u;
+    double acc = m ? -1e300 : 0.0;
+    for (int k = lane; k < (int)gridDim.x; k += 32) {
+      const double t = __ldcg(part + (long long)r * gridDim.x + k);
+      acc = m ? fmax(acc, t) : acc + t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double t = __shfl_down_sync(0xffffffffu, acc, o);
+      acc = m ? fmax(acc, t) : acc + t;
+    }
+    if (lane == 0) res[r] = acc;
+  }
+  __syncthreads();
+  return true;
 }
 
-// search direction in x and the bound multipliers, with the step bounds
-__global__ void __launch_bounds__(MMA_THREADS) k_dir(MPar p, const double* __restrict__ x,
-                                                     const double* __restrict__ alpha, const double* __restrict__ beta,
-                                                     const double* __restrict__ xi, const double* __restrict__ eta,
-                                                     const double* __restrict__ Dx, const double* __restrict__ hdx,
-                                                     const double* __restrict__ G, double* __restrict__ dx,
-                                                     double* __restrict__ dxi, double* __restrict__ deta, double* part) {
-  double v[4] = {-1e300, -1e300, -1e300, -1e300};
-  const double cf = 0.99;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.n; i += (long long)gridDim.x * blockDim.x) {
-    double t = -hdx[i] / Dx[i];
-    for (int j = 0; j < p.m; j++) t -= p.dl[j] * G[(long long)j * p.n + i] / Dx[i];
-    const double xa = x[i] - alpha[i], bx = beta[i] - x[i];
-    const double di = p.eps / xa - t / xa * xi[i] - xi[i];
-    const double de = p.eps / bx + eta[i] / bx * t - eta[i];
-    dx[i] = t; dxi[i] = di; deta[i] = de;
-    v[0] = fmax(v[0], (-1 / cf) * (t / xa));
-    v[1] = fmax(v[1], (1 / cf) * (t / bx));
-    v[2] = fmax(v[2], (-1 / cf) * di / xi[i]);
-    v[3] = fmax(v[3], (-1 / cf) * de / eta[i]);
+// partial pivoting, as the host solve of earlier versions
+template <int N>
+__device__ void dense_solve(double (&A)[N][N], double (&b)[N], double (&x)[N]) {
+  for (int k = 0; k < N; k++) {
+    int piv = k;
+    for (int i = k + 1; i < N; i++)
+      if (fabs(A[i][k]) > fabs(A[piv][k])) piv = i;
+    if (piv != k) {
+      for (int j = 0; j < N; j++) { const double t = A[k][j]; A[k][j] = A[piv][j]; A[piv][j] = t; }
+      const double t = b[k]; b[k] = b[piv]; b[piv] = t;
+    }
+    for (int i = k + 1; i < N; i++) {
+      const double f = A[i][k] / A[k][k];
+      for (int j = k; j < N; j++) A[i][j] -= f * A[k][j];
+      b[i] -= f * b[k];
+    }
   }
-  int ops[4] = {1, 1, 1, 1};
-  block_reduce<4>(v, ops, 4, part);
-}
-
-// KKT residual pieces at x + step dx (step = 0: current point)
-__global__ void __launch_bounds__(MMA_THREADS) k_kkt(MPar p, const double* __restrict__ x, const double* __restrict__ L,
-                                                     const double* __restrict__ U, const double* __restrict__ alpha,
-                                                     const double* __restrict__ beta, const double* __restrict__ xi,
-                                                     const double* __restrict__ eta, const double* __restrict__ dx,
-                                                     const double* __restrict__ dxi, const double* __restrict__ deta,
-                                                     const double* __restrict__ P, const double* __restrict__ Q,
-                                                     double* part) {
-  // 0: sum rex^2, 1: sum rexsi^2, 2: sum reeta^2, 3..3+m-1: g_j; 3+m..5+m: max |.|
-  double v[3 + MMA_MAXM + 3];
-  for (int r = 0; r < 3 + MMA_MAXM + 3; r++) v[r] = 0;
-  const int m = p.m, n = p.n;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double xt = x[i] + p.step * dx[i];
-    const double xit = xi[i] + p.step * dxi[i];
-    const double et = eta[i] + p.step * deta[i];
-    const double ux = U[i] - xt, xl = xt - L[i];
-    double pl = P[i], ql = Q[i];
-    for (int j = 0; j < m; j++) { pl += p.lam[j] * P[(long long)(j + 1) * n + i]; ql += p.lam[j] * Q[(long long)(j + 1) * n + i]; }
-    const double rex = pl / (ux * ux) - ql / (xl * xl) - xit + et;
-    const double rxs = xit * (xt - alpha[i]) - p.eps;
-    const double ret = et * (beta[i] - xt) - p.eps;
-    v[0] += rex * rex; v[1] += rxs * rxs; v[2] += ret * ret;
-    for (int j = 0; j < m; j++) v[3 + j] += P[(long long)(j + 1) * n + i] / ux + Q[(long long)(j + 1) * n + i] / xl;
-    v[3 + m] = fmax(v[3 + m], fabs(rex));
-    v[4 + m] = fmax(v[4 + m], fabs(rxs));
-    v[5 + m] = fmax(v[5 + m], fabs(ret));
-  }
-  int ops[3 + MMA_MAXM + 3];
-  for (int r = 0; r < 3 + MMA_MAXM + 3; r++) ops[r] = r >= 3 + m ? 1 : 0;
-  block_reduce<3 + MMA_MAXM + 3>(v, ops, 6 + m, part);
-}
-
-__global__ void k_accept(int n, double step, double* x, double* xi, double* eta, const double* dx, const double* dxi,
-                         const double* deta) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    x[i] += step * dx[i]; xi[i] += step * dxi[i]; eta[i] += step * deta[i];
+  for (int i = N - 1; i >= 0; i--) {
+    double t = b[i];
+    for (int j = i + 1; j < N; j++) t -= A[i][j] * x[j];
+    x[i] = t / A[i][i];
   }
 }
 
-// adjust_asym (mma_t.cu:164-226) and |dx|^2
-__global__ void __launch_bounds__(MMA_THREADS) k_asym(int n, const double* __restrict__ x, const double* __restrict__ curx,
-                                                      double* __restrict__ lastdx, double* __restrict__ L,
-                                                      double* __restrict__ U, double* __restrict__ alpha,
-                                                      double* __restrict__ beta, const double* __restrict__ xmin,
-                                                      const double* __restrict__ xmax, double* part) {
-  double v[1] = {0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double d1 = x[i] - curx[i], d2 = lastdx[i];
-    double gamma = 1;
-    if (d1 * d2 > 0) gamma = 1.2;
-    if (d1 * d2 < 0) gamma = 0.7;
-    const double xv = x[i], st = xmax[i] - xmin[i];
-    double nl = xv - gamma * (xv - d1 - L[i]);
-    double nu = xv + gamma * (U[i] - xv + d1);
-    nl = fmin(fmax(nl, xv - 10 * st), xv - 0.01 * st);
-    nu = fmin(fmax(nu, xv + 0.01 * st), xv + 10 * st);
-    L[i] = nl; U[i] = nu;
-    double na = xmin[i];
-    na = fmax(na, nl + 0.1 * (xv - nl));
-    na = fmax(na, xv - 0.5 * st);
-    double nb = xmax[i];
-    nb = fmin(nb, nu - 0.1 * (nu - xv));
-    nb = fmin(nb, xv + 0.5 * st);
-    alpha[i] = na; beta[i] = nb;
-    lastdx[i] = d1;
-    v[0] += d1 * d1;
+// 2-norm and inf-norm of the KKT residual (kkt_err, mma_t.cu:574-678): the n-sized sums q[0..2], the proxies
+// gp and the n-sized maxima, and the m-sized rows
+template <int M>
+__device__ void kkt_norms(const Dual<M>& D, const double* q, const double* gp, const double* mx, const double* lam,
+                          const double* y, double z, const double* mu, double zeta, const double* s, double damp,
+                          double* e2, double* einf) {
+  double sum = q[0] + q[1] + q[2], m = fmax(-10.0, fmax(mx[0], fmax(mx[1], mx[2])));
+  auto acc = [&](double v) { sum += v * v; m = fmax(m, fabs(v)); };
+  for (int j = 0; j < M; j++) acc(MMA_C + MMA_D * y[j] - lam[j] - mu[j]);
+  acc(MMA_A0 - zeta);
+  for (int j = 0; j < M; j++) acc((gp[j] - y[j] + s[j] - D.b[j]) / damp);
+  for (int j = 0; j < M; j++) acc(mu[j] * y[j] - D.eps);
+  acc(zeta * z - D.eps);
+  for (int j = 0; j < M; j++) acc(lam[j] * s[j] - D.eps);
+  *e2 = sqrt(sum);
+  *einf = m;
+}
+
+// One update (mma_t::update) in one launch.  What bounds it is latency: some
+// thirty Newton steps of three reductions each on a few hundred kilobytes that
+// stay in L2.  As separate kernels with the dual system on the host an update of
+// 32,768 variables took 6.7 ms, 2.7 of them in single-thread final sums and most
+// of the rest in the 60 round trips.  A Newton step is three passes over the
+// variables, each ending in a grid reduction: the system's sums together with
+// the KKT residual at the current point (and the previous step taken), the
+// direction with its step bounds, and the KKT residual of a trial: 1.08 ms with
+// the copies of the design in and out.
+template <int M>
+__global__ void __launch_bounds__(MMA_UT, 1) k_mma_update(const __grid_constant__ MmaArgs A) {
+  __shared__ double sh[MMA_RED][MMA_UT / 32];
+  __shared__ double res[MMA_RED];
+  __shared__ Dual<M> D;
+  const int n = A.n, t0 = blockIdx.x * MMA_UT + threadIdx.x, ts = gridDim.x * MMA_UT;
+  int parity = 0;
+  unsigned goal = 0;
+#define MMA_REDUCE(v, mx) \
+  if (!grid_reduce(v, mx, A, parity, goal, res, sh)) return
+  // init (mma_t.cu:69-106): p, q and the proxy offsets b at the current design; reset (mma_t.cu:702-713)
+  {
+    double v[M] = {};
+    for (int i = t0; i < n; i += ts) {
+      const double x = A.x[i], ux = A.U[i] - x, xl = x - A.L[i], raa = 1e-5 / (A.xmax[i] - A.xmin[i]);
+      A.curx[i] = x;
+#pragma unroll
+      for (int j = 0; j <= M; j++) {
+        const double d = j == 0 ? A.df[i] : A.dg[(long long)(j - 1) * n + i];
+        const double pos = fmax(d, 0.0), neg = fmax(-d, 0.0);
+        const double P = ux * ux * (1.001 * pos + 0.001 * neg + raa), Q = xl * xl * (0.001 * pos + 1.001 * neg + raa);
+        A.P[(long long)j * n + i] = P;
+        A.Q[(long long)j * n + i] = Q;
+        if (j > 0) v[j - 1] += P / ux + Q / xl;
+      }
+      const double al = A.alpha[i], be = A.beta[i], xv = 0.5 * (al + be);
+      A.x[i] = xv;
+      A.xi[i] = fmax(1.0 / (xv - al), 1.0);
+      A.eta[i] = fmax(1.0 / (be - xv), 1.0);
+    }
+    MMA_REDUCE(v, 0u);
+    if (threadIdx.x == 0) {
+      for (int j = 0; j < M; j++) {
+        D.b[j] = res[j] - A.g[j];
+        D.y[j] = D.lam[j] = D.s[j] = 1;
+        D.mu[j] = fmax(MMA_C / 2, 1.0);
+        D.lam_pq[j] = 1;
+      }
+      D.z = D.zeta = 1;
+      D.eps = 1;
+      D.err = 1e30;
+      D.lasterr = 0;
+      D.step = 0;
+      D.damp = 1;
+      D.stays = D.nsub = D.overflow = D.accepted = 0;
+      D.go = 1;
+    }
+    __syncthreads();
   }
-  int ops[1] = {0};
-  block_reduce<1>(v, ops, 1, part);
+  while (D.go) {
+    // the accepted step taken; Newton system (solveLinearSystem, mma_t.cu:228-328) and KKT residual
+    {
+      constexpr int NS = M * M + 2 * M;
+      double v[NS + 6] = {};
+      const bool take = D.accepted != 0;
+      const double step = D.step, eps = D.eps;
+      for (int i = t0; i < n; i += ts) {
+        double x = A.x[i], xi = A.xi[i], eta = A.eta[i];
+        if (take) {
+          x += step * A.dx[i]; xi += step * A.dxi[i]; eta += step * A.deta[i];
+          A.x[i] = x; A.xi[i] = xi; A.eta[i] = eta;
+        }
+        const double ux = A.U[i] - x, xl = x - A.L[i], xa = x - A.alpha[i], bx = A.beta[i] - x;
+        const double iu = 1 / ux, il = 1 / xl, iu2 = iu * iu, il2 = il * il;
+        double p[M + 1], q[M + 1];
+#pragma unroll
+        for (int j = 0; j <= M; j++) { p[j] = A.P[(long long)j * n + i]; q[j] = A.Q[(long long)j * n + i]; }
+        double pl = p[0], ql = q[0], pk = p[0], qk = q[0];
+#pragma unroll
+        for (int j = 0; j < M; j++) {
+          pl += D.lam_pq[j] * p[j + 1]; ql += D.lam_pq[j] * q[j + 1];
+          pk += D.lam[j] * p[j + 1]; qk += D.lam[j] * q[j + 1];
+        }
+        const double dxv = 2 * pl * iu2 * iu + 2 * ql * il2 * il + xi / xa + eta / bx;
+        const double h = -(eps / xa - eps / bx - (pl * iu2 - ql * il2)), id = 1 / dxv;
+        A.Dx[i] = id;
+        A.hdx[i] = h;
+        double g[M];
+#pragma unroll
+        for (int j = 0; j < M; j++) {
+          g[j] = p[j + 1] * iu2 - q[j + 1] * il2;
+          A.G[(long long)j * n + i] = g[j];
+        }
+        int r = 0;
+#pragma unroll
+        for (int j = 0; j < M; j++)
+#pragma unroll
+          for (int k = 0; k < M; k++) v[r++] += g[j] * (g[k] * id);
+#pragma unroll
+        for (int j = 0; j < M; j++) v[r++] += g[j] * (h * id);
+#pragma unroll
+        for (int j = 0; j < M; j++) v[r++] += p[j + 1] * iu + q[j + 1] * il;
+        const double rex = pk * iu2 - qk * il2 - xi + eta, rxs = xi * xa - eps, ret = eta * bx - eps;
+        v[NS] += rex * rex; v[NS + 1] += rxs * rxs; v[NS + 2] += ret * ret;
+        v[NS + 3] = fmax(v[NS + 3], fabs(rex));
+        v[NS + 4] = fmax(v[NS + 4], fabs(rxs));
+        v[NS + 5] = fmax(v[NS + 5], fabs(ret));
+      }
+      MMA_REDUCE(v, 7u << (NS + 3));
+      if (threadIdx.x == 0) {
+        const double *sg = res + M * M, *gp = res + M * M + M;
+        double K[M + 1][M + 1], rhs[M + 1], sol[M + 1], hdy[M], Dy[M];
+        for (int j = 0; j < M; j++) {
+          Dy[j] = MMA_D + D.mu[j] / D.y[j];
+          hdy[j] = -(D.lam[j] + D.eps / D.y[j] - MMA_C - MMA_D * D.y[j]);
+          const double hdl = -(D.y[j] + D.b[j] - D.eps / D.lam[j] - gp[j]);
+          for (int k = 0; k < M; k++) K[j][k] = res[j * M + k];
+          K[j][j] += D.s[j] / D.lam[j] + 1 / Dy[j];
+          K[j][M] = K[M][j] = 0;  // a = 0
+          rhs[j] = hdl + hdy[j] / Dy[j] - sg[j];
+        }
+        K[M][M] = -D.zeta / D.z;
+        rhs[M] = -(D.eps / D.z - MMA_A0);
+        dense_solve<M + 1>(K, rhs, sol);
+        D.dz = sol[M];
+        for (int j = 0; j < M; j++) {
+          D.dl[j] = sol[j];
+          D.dy[j] = sol[j] / Dy[j] - hdy[j] / Dy[j];
+          D.dmu[j] = D.eps / D.y[j] - D.dy[j] * D.mu[j] / D.y[j] - D.mu[j];
+          D.ds[j] = D.eps / D.lam[j] - D.s[j] / D.lam[j] * sol[j] - D.s[j];
+          D.lam_pq[j] = D.lam[j];
+        }
+        D.dzeta = D.eps / D.z - D.zeta - (D.zeta / D.z) * D.dz;
+        double inf;
+        kkt_norms<M>(D, res + NS, gp, res + NS + 3, D.lam, D.y, D.z, D.mu, D.zeta, D.s, 1.0, &D.old_err, &inf);
+      }
+      __syncthreads();
+    }
+    // search direction and step bounds
+    {
+      double v[4] = {-1e300, -1e300, -1e300, -1e300};
+      const double cf = 0.99, eps = D.eps;
+      for (int i = t0; i < n; i += ts) {
+        const double id = A.Dx[i], x = A.x[i], xi = A.xi[i], eta = A.eta[i];
+        double t = -A.hdx[i] * id;
+#pragma unroll
+        for (int j = 0; j < M; j++) t -= D.dl[j] * A.G[(long long)j * n + i] * id;
+        const double ia = 1 / (x - A.alpha[i]), ib = 1 / (A.beta[i] - x);
+        const double di = eps * ia - t * ia * xi - xi, de = eps * ib + eta * ib * t - eta;
+        A.dx[i] = t; A.dxi[i] = di; A.deta[i] = de;
+        v[0] = fmax(v[0], (-1 / cf) * (t * ia));
+        v[1] = fmax(v[1], (1 / cf) * (t * ib));
+        v[2] = fmax(v[2], (-1 / cf) * di / xi);
+        v[3] = fmax(v[3], (-1 / cf) * de / eta);
+      }
+      MMA_REDUCE(v, 15u);
+      if (threadIdx.x == 0) {
+        double t3 = fmax(res[2], res[3]);
+        auto art = [&](double dv, double w) { t3 = fmax(t3, (-1 / cf) * dv / w); };
+        for (int j = 0; j < M; j++) {
+          art(D.dy[j], D.y[j]);
+          art(D.dl[j], D.lam[j]);
+          art(D.dmu[j], D.mu[j]);
+          art(D.ds[j], D.s[j]);
+        }
+        art(D.dz, D.z);
+        art(D.dzeta, D.zeta);
+        D.step = 1 / fmax(fmax(res[0], res[1]), fmax(t3, 1.0));
+        D.new_err = 1e30;
+        D.err = 1e30;
+        D.accepted = 0;
+        for (int j = 0; j < M; j++) D.nl[j] = D.lam[j] + D.dl[j] * D.step;
+      }
+      __syncthreads();
+    }
+    // search_step (mma_t.cu:501-571)
+    while (D.accepted == 0 && D.step > 1e-12 && D.new_err > D.old_err) {
+      double v[3 + M + 3] = {};
+      const double step = D.step, eps = D.eps;
+      for (int i = t0; i < n; i += ts) {
+        const double x = A.x[i] + step * A.dx[i], xi = A.xi[i] + step * A.dxi[i], eta = A.eta[i] + step * A.deta[i];
+        const double iu = 1 / (A.U[i] - x), il = 1 / (x - A.L[i]);
+        double pl = A.P[i], ql = A.Q[i];
+#pragma unroll
+        for (int j = 0; j < M; j++) {
+          const double p = A.P[(long long)(j + 1) * n + i], q = A.Q[(long long)(j + 1) * n + i];
+          pl += D.nl[j] * p; ql += D.nl[j] * q;
+          v[3 + j] += p * iu + q * il;
+        }
+        const double rex = pl * iu * iu - ql * il * il - xi + eta;
+        const double rxs = xi * (x - A.alpha[i]) - eps, ret = eta * (A.beta[i] - x) - eps;
+        v[0] += rex * rex; v[1] += rxs * rxs; v[2] += ret * ret;
+        v[3 + M] = fmax(v[3 + M], fabs(rex));
+        v[4 + M] = fmax(v[4 + M], fabs(rxs));
+        v[5 + M] = fmax(v[5 + M], fabs(ret));
+      }
+      MMA_REDUCE(v, 7u << (3 + M));
+      if (threadIdx.x == 0) {
+        double ny[M], nmu[M], ns[M];
+        for (int j = 0; j < M; j++) {
+          ny[j] = D.y[j] + D.dy[j] * step; nmu[j] = D.mu[j] + D.dmu[j] * step; ns[j] = D.s[j] + D.ds[j] * step;
+          D.lam_pq[j] = D.nl[j];  // the reference's kkt_err refreshes plambda/qlambda with the trial multipliers
+        }
+        const double nz = D.z + D.dz * step, nzeta = D.zeta + D.dzeta * step;
+        kkt_norms<M>(D, res, res + 3, res + 3 + M, D.nl, ny, nz, nmu, nzeta, ns, D.damp, &D.new_err, &D.err);
+        if (D.new_err < D.old_err) {
+          for (int j = 0; j < M; j++) { D.lam[j] = D.nl[j]; D.y[j] = ny[j]; D.mu[j] = nmu[j]; D.s[j] = ns[j]; }
+          D.z = nz;
+          D.zeta = nzeta;
+          D.accepted = 1;
+        } else {
+          D.step /= 2;
+          for (int j = 0; j < M; j++) D.nl[j] = D.lam[j] + D.dl[j] * D.step;
+        }
+      }
+      __syncthreads();
+    }
+    __syncthreads();  // every thread has read the loop's condition
+    if (threadIdx.x == 0) {
+      if ((D.err - D.lasterr) / D.err < 1e-5) D.stays++;
+      else D.stays = 0;
+      D.lasterr = D.err;
+      if (D.stays > 6) { D.damp *= 10; D.stays = 0; }
+      if (D.nsub++ > 80) {
+        D.overflow = 1;
+        D.go = 0;
+      } else if (!(D.err > 0.9 * D.eps)) {  // the next barrier parameter
+        D.eps *= 0.1;
+        D.damp = 1;
+        D.stays = 0;
+        D.go = D.eps > 1e-6;
+      }
+    }
+    __syncthreads();
+  }
+  // the last accepted step, adjust_asym (mma_t.cu:164-226) and |dx|^2
+  {
+    double v[1] = {};
+    const bool take = D.accepted != 0;
+    const double step = D.step;
+    for (int i = t0; i < n; i += ts) {
+      double xv = A.x[i];
+      if (take) {
+        xv += step * A.dx[i];
+        A.x[i] = xv;
+        A.xi[i] += step * A.dxi[i];
+        A.eta[i] += step * A.deta[i];
+      }
+      const double d1 = xv - A.curx[i], d2 = A.lastdx[i], lo = A.xmin[i], hi = A.xmax[i], st = hi - lo;
+      double gamma = 1;
+      if (d1 * d2 > 0) gamma = 1.2;
+      if (d1 * d2 < 0) gamma = 0.7;
+      double nl = xv - gamma * (xv - d1 - A.L[i]);
+      double nu = xv + gamma * (A.U[i] - xv + d1);
+      nl = fmin(fmax(nl, xv - 10 * st), xv - 0.01 * st);
+      nu = fmin(fmax(nu, xv + 0.01 * st), xv + 10 * st);
+      A.L[i] = nl; A.U[i] = nu;
+      A.alpha[i] = fmax(fmax(lo, nl + 0.1 * (xv - nl)), xv - 0.5 * st);
+      A.beta[i] = fmin(fmin(hi, nu - 0.1 * (nu - xv)), xv + 0.5 * st);
+      A.lastdx[i] = d1;
+      v[0] += d1 * d1;
+    }
+    MMA_REDUCE(v, 0u);
+  }
+#undef MMA_REDUCE
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    A.out[0] = D.err;
+    A.out[1] = D.step;
+    A.out[2] = D.nsub;
+    A.out[3] = D.overflow;
+    A.out[4] = res[0];
+  }
+  if (gridDim.x > 1) rso::gbar_exit(A.bar, threadIdx.x);
 }
 
 // clamp_asymptotes (mma_t.cu:747-761)
@@ -264,47 +447,10 @@ __global__ void k_clamp_asym(int n, const double* x, double* L, double* U, doubl
     if (_e != cudaSuccess) { (s)->err = cudaGetErrorString(_e); return RSO_ERR_CUDA; } \
   } while (0)
 
-// run one reduction pass's final stage and copy nr results to the host
-rso_status finish_red(rso_mma* s, int nr, unsigned long long maxmask) {
-  k_final<<<1, 64, 0, s->stream>>>(s->part, MMA_BLOCKS, nr, nullptr, (int)(maxmask & 0xffffffffu),
-                                   (int)(maxmask >> 32), s->res); rso::note_launch();
-  MMA_CHECK(s, cudaGetLastError());
-  MMA_CHECK(s, cudaMemcpyAsync(s->h_res, s->res, sizeof(double) * nr, cudaMemcpyDeviceToHost, s->stream));
-  MMA_CHECK(s, cudaStreamSynchronize(s->stream));
-  return RSO_OK;
-}
-
-void dense_solve(int N, std::vector<double> A, std::vector<double> b, std::vector<double>& x) {
-  for (int k = 0; k < N; k++) {
-    int piv = k;
-    for (int i = k + 1; i < N; i++) if (std::fabs(A[i * N + k]) > std::fabs(A[piv * N + k])) piv = i;
-    if (piv != k) { for (int j = 0; j < N; j++) std::swap(A[k * N + j], A[piv * N + j]); std::swap(b[k], b[piv]); }
-    for (int i = k + 1; i < N; i++) {
-      const double f = A[i * N + k] / A[k * N + k];
-      for (int j = k; j < N; j++) A[i * N + j] -= f * A[k * N + j];
-      b[i] -= f * b[k];
-    }
-  }
-  x.assign(N, 0.0);
-  for (int i = N - 1; i >= 0; i--) {
-    double t = b[i];
-    for (int j = i + 1; j < N; j++) t -= A[i * N + j] * x[j];
-    x[i] = t / A[i * N + i];
-  }
-}
-
-MPar mpar(rso_mma* s, const std::vector<double>& lam) {
-  MPar p;
-  p.n = s->n; p.m = s->m; p.eps = s->eps; p.step = 0;
-  for (int j = 0; j < MMA_MAXM; j++) { p.lam[j] = j < s->m ? lam[j] : 0; p.dl[j] = 0; }
-  return p;
-}
-
 }  // namespace
 
 extern "C" rso_status rso_mma_create(int n, int m, const double* xmin, const double* xmax, rso_mma** out) {
   if (!out || n <= 0 || m < 1 || m > MMA_MAXM || !xmin || !xmax) return RSO_ERR_INVALID_ARG;
-  if (m * m + 2 * m > MMA_RED) return RSO_ERR_INVALID_ARG;
   rso_mma* s = new rso_mma();
   s->n = n; s->m = m;
   auto fail = [&](rso_status st) { rso_mma_destroy(s); return st; };
@@ -316,7 +462,14 @@ extern "C" rso_status rso_mma_create(int n, int m, const double* xmin, const dou
   if (cudaMalloc(&s->P, sizeof(double) * n * (m + 1)) != cudaSuccess) return fail(RSO_ERR_OOM);
   if (cudaMalloc(&s->Q, sizeof(double) * n * (m + 1)) != cudaSuccess) return fail(RSO_ERR_OOM);
   if (cudaMalloc(&s->G, sizeof(double) * n * m) != cudaSuccess) return fail(RSO_ERR_OOM);
-  if (cudaMalloc(&s->part, sizeof(double) * MMA_RED * MMA_BLOCKS) != cudaSuccess) return fail(RSO_ERR_OOM);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return fail(RSO_ERR_CUDA);
+  s->ctas = (int)std::min<long long>(sms, rso::cdiv(n, MMA_UT));
+  if (cudaMalloc(&s->part, sizeof(double) * 2 * MMA_RED * s->ctas) != cudaSuccess) return fail(RSO_ERR_OOM);
+  if (cudaMalloc(&s->bar, sizeof(unsigned) * 4) != cudaSuccess) return fail(RSO_ERR_OOM);
+  cudaMemsetAsync(s->bar, 0, sizeof(unsigned) * 4, s->stream);
   if (cudaMalloc(&s->res, sizeof(double) * 64) != cudaSuccess) return fail(RSO_ERR_OOM);
   if (cudaMallocHost(&s->h_res, sizeof(double) * 64) != cudaSuccess) return fail(RSO_ERR_OOM);
   cudaMemcpy(s->xmin, xmin, sizeof(double) * n, cudaMemcpyHostToDevice);
@@ -331,10 +484,6 @@ extern "C" rso_status rso_mma_create(int n, int m, const double* xmin, const dou
   k_clamp_asym<<<MMA_BLOCKS, MMA_THREADS, 0, s->stream>>>(n, s->x, s->L, s->U, s->alpha, s->beta, s->xmin, s->xmax); rso::note_launch();
   k_reset<<<MMA_BLOCKS, MMA_THREADS, 0, s->stream>>>(n, s->x, s->alpha, s->beta, s->xi, s->eta); rso::note_launch();
   if (cudaStreamSynchronize(s->stream) != cudaSuccess) return fail(RSO_ERR_CUDA);
-  s->y.assign(m, 1.0); s->lambda.assign(m, 1.0); s->s.assign(m, 1.0); s->mu.assign(m, 0.0);
-  s->a.assign(m, 0.0); s->c.assign(m, 10.0); s->d.assign(m, 1.0); s->b.assign(m, 0.0);
-  for (int j = 0; j < m; j++) s->mu[j] = std::max(s->c[j] / 2, 1.0);
-  s->lam_pq = s->lambda;
   *out = s;
   return RSO_OK;
 }
@@ -402,145 +551,43 @@ extern "C" rso_status rso_mma_load(rso_mma* s, const double* state_host) {
 extern "C" rso_status rso_mma_update(rso_mma* S, const double* df, const double* dg, const double* g, int* converged,
                                      double* info) {
   if (!S || !df || (!dg && S->m > 0) || !g) return RSO_ERR_INVALID_ARG;
-  const int n = S->n, m = S->m;
-  cudaStream_t st = S->stream;
-  MMA_CHECK(S, cudaMemcpyAsync(S->curx, S->x, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  // init (mma_t.cu:69-106): p, q and the proxy offsets b at the current design
-  k_pq<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(n, m, df, dg, S->x, S->L, S->U, S->xmin, S->xmax, S->P, S->Q); rso::note_launch();
-  k_gp<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(mpar(S, S->lambda), S->x, S->L, S->U, S->P, S->Q, S->part); rso::note_launch();
-  RSO_TRY(finish_red(S, m, 0));
-  for (int j = 0; j < m; j++) S->b[j] = S->h_res[j] - g[j];
-  // reset (mma_t.cu:702-713)
-  k_reset<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(n, S->x, S->alpha, S->beta, S->xi, S->eta); rso::note_launch();
-  S->eps = 1; S->zeta = S->z = 1;
-  for (int j = 0; j < m; j++) { S->y[j] = 1; S->lambda[j] = 1; S->s[j] = 1; S->mu[j] = std::max(S->c[j] / 2, 1.0); }
-  S->lam_pq = S->lambda;
-
-  double err = 1e30, lasterr = 0, step_used = 0;
-  int nsub = 0;
-  bool overflow = false;
-  while (S->eps > 1e-6) {
-    err = 1e30;
-    double damp = 1;
-    int stays = 0;
-    while (err > 0.9 * S->eps) {
-      // Newton system (solveLinearSystem, mma_t.cu:228-328)
-      MPar p = mpar(S, S->lam_pq);
-      k_prep<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(p, S->x, S->L, S->U, S->alpha, S->beta, S->xi, S->eta, S->P, S->Q,
-                                                 S->Dx, S->hdx, S->G, S->part); rso::note_launch();
-      RSO_TRY(finish_red(S, m * m + 2 * m, 0));
-      std::vector<double> A11(m * m), sg(m), gp(m);
-      for (int i = 0; i < m * m; i++) A11[i] = S->h_res[i];
-      for (int j = 0; j < m; j++) { sg[j] = S->h_res[m * m + j]; gp[j] = S->h_res[m * m + m + j]; }
-      std::vector<double> Dy(m), Dl(m), hdy(m), hdl(m);
-      double la = 0;
-      for (int j = 0; j < m; j++) {
-        Dy[j] = S->d[j] + S->mu[j] / S->y[j];
-        Dl[j] = S->s[j] / S->lambda[j];
-        hdy[j] = -(S->lambda[j] + S->eps / S->y[j] - S->c[j] - S->d[j] * S->y[j]);
-        hdl[j] = -(S->z * S->a[j] + S->y[j] + S->b[j] - S->eps / S->lambda[j] - gp[j]);
-        la += S->lambda[j] * S->a[j];
-      }
-      const double hdz = -(la + S->eps / S->z - S->a0);
-      const int N = m + 1;
-      std::vector<double> A(N * N, 0.0), rhs(N, 0.0), sol;
-      for (int j = 0; j < m; j++) {
-        A[j * N + j] += Dl[j] + 1 / Dy[j];
-        for (int k = 0; k < m; k++) A[j * N + k] += A11[j * m + k];
-        rhs[j] = hdl[j] + hdy[j] / Dy[j] - sg[j];
-        A[j * N + m] = S->a[j];
-        A[m * N + j] = S->a[j];
-      }
-      A[m * N + m] = -S->zeta / S->z;
-      rhs[m] = hdz;
-      dense_solve(N, A, rhs, sol);
-      const double dz = sol[m];
-      std::vector<double> dl(m), dy(m), dmu(m), ds(m);
-      for (int j = 0; j < m; j++) {
-        dl[j] = sol[j];
-        dy[j] = dl[j] / Dy[j] - hdy[j] / Dy[j];
-        dmu[j] = S->eps / S->y[j] - dy[j] * S->mu[j] / S->y[j] - S->mu[j];
-        ds[j] = S->eps / S->lambda[j] - S->s[j] / S->lambda[j] * dl[j] - S->s[j];
-      }
-      const double dzeta = S->eps / S->z - S->zeta - (S->zeta / S->z) * dz;
-      for (int j = 0; j < m; j++) p.dl[j] = dl[j];
-      k_dir<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(p, S->x, S->alpha, S->beta, S->xi, S->eta, S->Dx, S->hdx, S->G, S->dx,
-                                                S->dxi, S->deta, S->part); rso::note_launch();
-      RSO_TRY(finish_red(S, 4, 0xfull));
-      const double cf = 0.99;
-      const double t1 = S->h_res[0], t2 = S->h_res[1];
-      double t3 = std::max(S->h_res[2], S->h_res[3]);
-      auto art = [&](double dv, double v) { t3 = std::max(t3, (-1 / cf) * dv / v); };
-      for (int j = 0; j < m; j++) art(dy[j], S->y[j]);
-      art(dz, S->z);
-      for (int j = 0; j < m; j++) art(dl[j], S->lambda[j]);
-      for (int j = 0; j < m; j++) art(dmu[j], S->mu[j]);
-      art(dzeta, S->zeta);
-      for (int j = 0; j < m; j++) art(ds[j], S->s[j]);
-      const double max_t = 1 / std::max(std::max(t1, t2), std::max(t3, 1.0));
-      // search_step (mma_t.cu:501-571) with kkt_err (:574-678)
-      auto kkt = [&](double step, const std::vector<double>& lam, const std::vector<double>& yv, double zv,
-                     const std::vector<double>& muv, double zetav, const std::vector<double>& sv, double dmp,
-                     double* e2, double* einf) -> rso_status {
-        MPar q = mpar(S, lam);
-        q.step = step;
-        k_kkt<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(q, S->x, S->L, S->U, S->alpha, S->beta, S->xi, S->eta, S->dx, S->dxi,
-                                                  S->deta, S->P, S->Q, S->part); rso::note_launch();
-        const unsigned long long mm = 0x7ull << (3 + m);
-        RSO_TRY(finish_red(S, 6 + m, mm));
-        S->lam_pq = lam;  // the reference's kkt_err refreshes plambda/qlambda with the trial multipliers
-        double sum = S->h_res[0] + S->h_res[1] + S->h_res[2];
-        double mx = std::max(-10.0, std::max(S->h_res[3 + m], std::max(S->h_res[4 + m], S->h_res[5 + m])));
-        auto acc = [&](double v) { sum += v * v; mx = std::max(mx, std::fabs(v)); };
-        for (int j = 0; j < m; j++) acc(S->c[j] + S->d[j] * yv[j] - lam[j] - muv[j]);
-        double l2 = 0;
-        for (int j = 0; j < m; j++) l2 += lam[j] * S->a[j];
-        acc(S->a0 - zetav - l2);
-        for (int j = 0; j < m; j++) {
-          const double r = (S->h_res[3 + j] - S->a[j] * zv - yv[j] + sv[j] - S->b[j]) / dmp;
-          acc(r);
-        }
-        for (int j = 0; j < m; j++) acc(muv[j] * yv[j] - S->eps);
-        acc(zetav * zv - S->eps);
-        for (int j = 0; j < m; j++) acc(lam[j] * sv[j] - S->eps);
-        *e2 = std::sqrt(sum);
-        *einf = mx;
-        return RSO_OK;
-      };
-      double old_err = 0, old_inf = 0;
-      RSO_TRY(kkt(0.0, S->lambda, S->y, S->z, S->mu, S->zeta, S->s, 1.0, &old_err, &old_inf));
-      double step = max_t, new_err = 1e30, new_inf = 1e30;
-      while (step > 1e-12 && new_err > old_err) {
-        std::vector<double> nl(m), ny(m), nmu(m), ns(m);
-        for (int j = 0; j < m; j++) {
-          nl[j] = S->lambda[j] + dl[j] * step; ny[j] = S->y[j] + dy[j] * step;
-          nmu[j] = S->mu[j] + dmu[j] * step; ns[j] = S->s[j] + ds[j] * step;
-        }
-        const double nz = S->z + dz * step, nzeta = S->zeta + dzeta * step;
-        RSO_TRY(kkt(step, nl, ny, nz, nmu, nzeta, ns, damp, &new_err, &new_inf));
-        if (new_err < old_err) {
-          k_accept<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(n, step, S->x, S->xi, S->eta, S->dx, S->dxi, S->deta); rso::note_launch();
-          S->lambda = nl; S->y = ny; S->mu = nmu; S->s = ns; S->z = nz; S->zeta = nzeta;
-          break;
-        }
-        step /= 2;
-      }
-      step_used = step;
-      err = new_inf;
-      if ((err - lasterr) / err < 1e-5) stays++;
-      else stays = 0;
-      lasterr = err;
-      if (stays > 6) { damp *= 10; stays = 0; }
-      if (nsub++ > 80) { overflow = true; break; }
-    }
-    if (overflow) break;
-    S->eps *= 0.1;
+  MmaArgs A;
+  A.n = S->n;
+  A.df = df; A.dg = dg; A.xmin = S->xmin; A.xmax = S->xmax;
+  A.x = S->x; A.L = S->L; A.U = S->U; A.alpha = S->alpha; A.beta = S->beta; A.lastdx = S->lastdx;
+  A.xi = S->xi; A.eta = S->eta; A.curx = S->curx; A.P = S->P; A.Q = S->Q; A.Dx = S->Dx; A.hdx = S->hdx; A.G = S->G;
+  A.dx = S->dx; A.dxi = S->dxi; A.deta = S->deta;
+  for (int j = 0; j < MMA_MAXM; j++) A.g[j] = j < S->m ? g[j] : 0.0;
+  A.part = S->part; A.out = S->res; A.bar = S->bar;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(S->ctas);
+  lc.blockDim = dim3(MMA_UT);
+  lc.stream = S->stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  void (*kernel)(MmaArgs) = S->m == 1   ? k_mma_update<1>
+                            : S->m == 2 ? k_mma_update<2>
+                            : S->m == 3 ? k_mma_update<3>
+                            : S->m == 4 ? k_mma_update<4>
+                                        : k_mma_update<5>;
+  MMA_CHECK(S, cudaLaunchKernelEx(&lc, kernel, A)); rso::note_launch();
+  // the result and the barrier's gave-up flag in one copy each, one synchronisation
+  unsigned* flag = reinterpret_cast<unsigned*>(S->h_res + 8);
+  MMA_CHECK(S, cudaMemcpyAsync(S->h_res, S->res, sizeof(double) * 5, cudaMemcpyDeviceToHost, S->stream));
+  MMA_CHECK(S, cudaMemcpyAsync(flag, S->bar + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, S->stream));
+  MMA_CHECK(S, cudaStreamSynchronize(S->stream));
+  if (*flag != 0) {
+    MMA_CHECK(S, cudaMemsetAsync(S->bar, 0, sizeof(unsigned) * 4, S->stream));
+    MMA_CHECK(S, cudaStreamSynchronize(S->stream));
+    S->err = "a grid-barrier wait of the update kernel timed out";
+    return RSO_ERR_CUDA;
   }
-  k_asym<<<MMA_BLOCKS, MMA_THREADS, 0, st>>>(n, S->x, S->curx, S->lastdx, S->L, S->U, S->alpha, S->beta, S->xmin,
-                                             S->xmax, S->part); rso::note_launch();
-  RSO_TRY(finish_red(S, 1, 0));
-  if (std::sqrt(S->h_res[0]) < 1e-3) S->stop_counter++;
-  if (info) { info[0] = err; info[1] = step_used; info[2] = nsub; info[3] = overflow; }
+  if (std::sqrt(S->h_res[4]) < 1e-3) S->stop_counter++;
+  if (info)
+    for (int k = 0; k < 4; k++) info[k] = S->h_res[k];
   if (converged) *converged = S->stop_counter > 10 ? 1 : 0;
   return RSO_OK;
 }
@@ -551,6 +598,7 @@ extern "C" void rso_mma_destroy(rso_mma* s) {
   double* vecs[] = {s->x, s->xmin, s->xmax, s->L, s->U, s->alpha, s->beta, s->lastdx, s->xi, s->eta, s->curx,
                     s->Dx, s->hdx, s->dx, s->dxi, s->deta, s->P, s->Q, s->G, s->part, s->res};
   for (double* v : vecs) cudaFree(v);
+  cudaFree(s->bar);
   if (s->h_res) cudaFreeHost(s->h_res);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;

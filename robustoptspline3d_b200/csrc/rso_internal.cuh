@@ -291,6 +291,57 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);  // a failure is the next launch_check's
 }
 
+// a barrier wait gives up after this many SM clock cycles (about 2 s)
+constexpr long long kGbarCycles = 4000000000LL;
+
+__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Grid-wide barrier on bar = {arrivals, exits, gave-up flag}: one arrival per
+// CTA (a release), the arrivals counted on through the launch, so that a waiter
+// polls the very word the arrivals change (no reset, no second word to pass on:
+// 2.4 us per barrier with both, see k_bottom_grid for what is left).  goal is
+// thread 0's count of arrivals that completes its next barrier.  The last CTA to
+// leave the kernel (gbar_exit) clears the counts for the next launch.  Returns
+// false on every thread of every CTA once some wait has given up (kGbarGone in
+// the arrivals, and bar[2] for the host): the kernel then returns, and the host
+// reports it after the solve and clears all words.
+// (target, limit: the arrivals that complete the barrier and the wait's bound
+// in clock cycles; the self-test sets them, the other kernels keep the grid
+// size and kGbarCycles)
+constexpr unsigned kGbarGone = 1u << 31;
+__device__ __forceinline__ bool gbar_sync(unsigned* bar, unsigned& goal, int tid, unsigned target, long long limit = kGbarCycles) {
+  __syncthreads();
+  int bad = 0;
+  if (tid == 0) {
+    goal += target;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    const long long t0 = clock64();
+    for (;;) {
+      const unsigned v = ld_acquire_gpu(bar);
+      if (v & kGbarGone) { bad = 1; break; }
+      if (v >= goal) break;
+      if (clock64() - t0 > limit) {
+        atomicOr(bar, kGbarGone);
+        atomicExch(bar + 2, 1u);
+        bad = 1;
+        break;
+      }
+    }
+  }
+  return __syncthreads_or(bad) == 0;
+}
+// every CTA of a launch that passed all its barriers calls this once
+__device__ __forceinline__ void gbar_exit(unsigned* bar, int tid) {
+  if (tid == 0 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
+    bar[0] = 0u;
+    bar[1] = 0u;
+  }
+}
+
 rso_status launch_check(rso_handle* h, const char* what);
 
 // reductions (reduce.cu)

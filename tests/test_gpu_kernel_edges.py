@@ -138,3 +138,25 @@ def test_sensitivity_modes(oracle, cuda, dims, penal):
     want = np.where(on, -penal * np.where(on, r, 1.0) ** (penal - 1) * q, 0.0)
     assert rel(g.computeSensitivity(t(u.ravel(), cuda)).cpu().numpy(), want) < 1e-6
     assert rel(g.elementCompliance(t(u.ravel(), cuda)).cpu().numpy(), np.where(on, r ** penal * q, 0.0)) < 1e-6
+
+
+# one CTA (no grid barrier) with a part and exactly its 512 threads, one variable more, a ragged last
+# CTA, and more variables than the GPU's threads; every number of constraints an update is built for
+@pytest.mark.parametrize("n,m", [(1, 1), (512, 2), (513, 1), (5000, 3), (5000, 4), (5000, 5), (80001, 2)])
+def test_mma_update_sizes(oracle, cuda, n, m):
+    """Three updates against the oracle, 1e-8 relative and 1e-10 absolute as in the parity test."""
+    from robustoptspline3d_b200 import MMA
+    rng = np.random.default_rng(23)
+    o, g = oracle.MMA(n, m, 0.0, 1.0), MMA(n, m, 0.0, 1.0)
+    x0 = rng.uniform(0.2, 0.8, n)
+    o.set_x(x0)
+    g.set_x(x0)
+    for k in range(3):
+        x = o.get()[0]
+        df = -np.exp(-x) * (1 + rng.uniform(0, 0.1, n))
+        dg = np.stack([np.full(n, 1.0 / n)] + [rng.standard_normal(n) * 0.1 for _ in range(m - 1)])
+        gval = np.array([x.mean() - 0.4] + [0.05 * np.sin(k + j) for j in range(m - 1)])
+        o.update(df, dg, gval)
+        g.update(t(df, cuda), t(dg, cuda), gval)
+        for a, b in zip(g.get(), o.get()):
+            assert np.allclose(a, b, rtol=1e-8, atol=1e-10)
