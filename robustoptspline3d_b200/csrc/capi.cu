@@ -56,14 +56,16 @@ extern "C" rso_status rso_element_matrix(double E, double nu, double hh, double*
   return RSO_OK;
 }
 
-// T_pos = P_pos^T K0 P_pos for every child position of a coarsening factor F
+// T_pos = P_pos^T K0 P_pos for the child positions k_galerkin_first sums over:
+// every child for factor 2, positions 0, 1.5 and 3 along each axis for factor 4
 static void galerkin_table(const double* K0, int F, std::vector<double>& T) {
-  const int np = F * F * F;
+  const int n1 = F == 4 ? 3 : F, np = n1 * n1 * n1;
+  const double at = F == 4 ? 1.5 : 1.0;
   T.assign((size_t)np * 576, 0.0);
   for (int pos = 0; pos < np; pos++) {
-    const int px = pos % F, py = (pos / F) % F, pz = pos / (F * F);
+    const double px = at * (pos % n1), py = at * (pos / n1 % n1), pz = at * (pos / (n1 * n1));
     double P[8][8];
-    auto w = [&](int o, int A) { return A ? (double)o / F : (double)(F - o) / F; };
+    auto w = [&](double o, int A) { return A ? o / F : (F - o) / F; };
     for (int a = 0; a < 8; a++)
       for (int A = 0; A < 8; A++)
         P[a][A] = w(px + (a & 1), A & 1) * w(py + ((a >> 1) & 1), (A >> 1) & 1) * w(pz + (a >> 2), A >> 2);

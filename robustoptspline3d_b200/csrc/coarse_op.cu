@@ -835,8 +835,8 @@ __global__ void __launch_bounds__(32 * PROW_WARPS) k_prolong_row(const Level Fl,
 __device__ __forceinline__ double pw(int F, int o, int A) { return A ? (double)o / F : (double)(F - o) / F; }
 
 // Support-free children enter the first-level coarse element matrices as a
-// product KE[E] = sum_pos w[E][pos] T1[pos] (w = rho^p of child pos, 0 for
-// inactive or support-touching children; T1[pos] the 576 entries of child
+// product KE[E] = sum_pos w[E][pos] T[pos] (w = rho^p of child pos, 0 for
+// inactive or support-touching children; T[pos] the 576 entries of child
 // pos's element matrix seen from the coarse element's nodes), done by
 // k_galerkin_first; the support-touching children are added by
 // k_galerkin_fix on the few coarse elements that have them.
@@ -851,174 +851,235 @@ __global__ void k_elem_fixmask(const Level Fl, uint8_t* __restrict__ efix) {
   efix[Fl.eidx(x, y, z)] = (uint8_t)m;
 }
 
-// KE (576 x ne, column per coarse element) = T1 (576 x F3) . w (F3 x ne),
-// w formed on the fly from the children's rho^p.  A CTA takes GE coarse
-// elements: their weights go to shared memory once, then the 576 rows pass
-// in chunks of 64 staged from T1; a thread accumulates 4 rows x 2 elements
-// in FP64 (each output is one ordered sum over the F3 children).
-constexpr int GE = 32, GM = 64;
+// Element matrices are stored entry by entry, KE[entry * ne + E], so that the
+// threads of a warp, which take consecutive elements of a row, read and write
+// whole sectors.
+//
+// KE = T1 . w, one ordered sum per output.  For F = 4 the 64 children enter
+// through 27 moments: an entry of a child's matrix seen from the coarse nodes is
+// a product of two trilinear weights, quadratic in the child's position along
+// each axis, so it is interpolated from three positions per axis (0, 1.5, 3:
+// T1 holds those 27 matrices) with factors phi, and the sums over the children
+// come first.  For F = 2 the eight children enter directly.  A CTA takes GE
+// coarse elements: their moments go to shared memory once, then the 576 rows
+// pass in chunks of GM staged from T1; a thread accumulates 4 rows x 4 elements
+// in FP64.  256^3: 2668 us with 64 children and 4 x 2 outputs a thread (bound by
+// shared-memory reads), 941 now.
+constexpr int GE = 64, GM = 64;
+struct Phi { double v[3][4]; };  // phi[m][pos]
 template <int F>
 __global__ void __launch_bounds__(256) k_galerkin_first(const Level Fl, const Level C, const double* __restrict__ rp,
                                                         const uint8_t* __restrict__ efix,
-                                                        const double* __restrict__ T1, double* __restrict__ KE) {
-  constexpr int F3 = F * F * F;
-  __shared__ __align__(16) double Ws[F3][GE];
-  __shared__ __align__(16) double Ts[F3][GM];
+                                                        const double* __restrict__ T1, const Phi phi,
+                                                        double* __restrict__ KE) {
+  constexpr int K = F == 4 ? 27 : 8;
+  // F = 4: the x moments of the 16 child rows first, in the memory the chunks of T1 use later
+  constexpr int SB = F == 4 && 48 * GE > K * GM ? 48 * GE : K * GM;
+  __shared__ __align__(16) double Ws[K][GE];
+  __shared__ __align__(16) double buf[SB];
   const int t = threadIdx.x;
   const long long E0 = (long long)blockIdx.x * GE;
-  for (int idx = t; idx < F3 * GE; idx += 256) {
-    const int pos = idx / GE, j = idx - pos * GE;
-    const long long E = E0 + j;
-    double r = 0.0;
-    if (E < C.ne) {
-      const int X = E % C.ex, Y = (E / C.ex) % C.ey, Z = E / ((long long)C.ex * C.ey);
-      const int x = X * F + pos % F, y = Y * F + (pos / F) % F, z = Z * F + pos / (F * F);
-      if (x < Fl.ex && y < Fl.ey && z < Fl.ez) {
-        const long long e = Fl.eidx(x, y, z);
-        if (Fl.emask[e] && !efix[e]) r = rp[e];
+  auto child = [&](long long E, int px, int py, int pz) {
+    if (E >= C.ne) return 0.0;
+    const unsigned e32 = (unsigned)E, row = e32 / (unsigned)C.ex, Z = row / (unsigned)C.ey;  // ne < 2^31
+    const int x = (int)(e32 - row * C.ex) * F + px, y = (int)(row - Z * C.ey) * F + py, z = (int)Z * F + pz;
+    if (x >= Fl.ex || y >= Fl.ey || z >= Fl.ez) return 0.0;
+    const long long e = Fl.eidx(x, y, z);
+    return Fl.emask[e] && !efix[e] ? rp[e] : 0.0;
+  };
+  if constexpr (F == 4) {
+    for (int idx = t; idx < 16 * GE; idx += 256) {
+      const int yz = idx / GE, j = idx - yz * GE;
+      double m[3] = {0, 0, 0};
+#pragma unroll
+      for (int px = 0; px < 4; px++) {
+        const double r = child(E0 + j, px, yz & 3, yz >> 2);
+#pragma unroll
+        for (int q = 0; q < 3; q++) m[q] += phi.v[q][px] * r;
       }
-    }
-    Ws[pos][j] = r;
-  }
-  const int ti = t & 15, te = t >> 4;  // rows 4 ti .. 4 ti + 3 of the chunk, elements 2 te, 2 te + 1
-  for (int m0 = 0; m0 < 576; m0 += GM) {
-    __syncthreads();  // Ws complete (first chunk); Ts free (later chunks)
-    for (int idx = t; idx < F3 * GM; idx += 256) {
-      const int k = idx / GM, i = idx - k * GM;
-      Ts[k][i] = T1[(long long)k * 576 + m0 + i];
+#pragma unroll
+      for (int q = 0; q < 3; q++) buf[(yz * 3 + q) * GE + j] = m[q];
     }
     __syncthreads();
-    double acc[4][2] = {};
-#pragma unroll 8
-    for (int k = 0; k < F3; k++) {
-      const double2 a01 = *reinterpret_cast<const double2*>(&Ts[k][4 * ti]);
-      const double2 a23 = *reinterpret_cast<const double2*>(&Ts[k][4 * ti + 2]);
-      const double2 b = *reinterpret_cast<const double2*>(&Ws[k][2 * te]);
-      const double a[4] = {a01.x, a01.y, a23.x, a23.y};
+    for (int idx = t; idx < K * GE; idx += 256) {
+      const int m = idx / GE, j = idx - m * GE, mx = m % 3, my = m / 3 % 3, mz = m / 9;
+      double s = 0;
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        acc[r][0] = fma(a[r], b.x, acc[r][0]);
-        acc[r][1] = fma(a[r], b.y, acc[r][1]);
-      }
+      for (int yz = 0; yz < 16; yz++) s += phi.v[my][yz & 3] * phi.v[mz][yz >> 2] * buf[(yz * 3 + mx) * GE + j];
+      Ws[m][j] = s;
+    }
+  } else {
+    for (int idx = t; idx < K * GE; idx += 256) {
+      const int m = idx / GE, j = idx - m * GE;
+      Ws[m][j] = child(E0 + j, m & 1, (m >> 1) & 1, m >> 2);
+    }
+  }
+  const int te = t & 15, ti = t >> 4;  // elements 4 te .. 4 te + 3, rows 4 ti .. 4 ti + 3 of the chunk
+  for (int m0 = 0; m0 < 576; m0 += GM) {
+    __syncthreads();  // Ws complete (first chunk); buf free
+    for (int idx = t; idx < K * GM; idx += 256) {
+      const int k = idx / GM, i = idx - k * GM;
+      buf[idx] = T1[(long long)k * 576 + m0 + i];
+    }
+    __syncthreads();
+    double acc[4][4] = {};
+#pragma unroll 9
+    for (int k = 0; k < K; k++) {
+      const double2 a01 = *reinterpret_cast<const double2*>(&buf[k * GM + 4 * ti]);
+      const double2 a23 = *reinterpret_cast<const double2*>(&buf[k * GM + 4 * ti + 2]);
+      const double2 b01 = *reinterpret_cast<const double2*>(&Ws[k][4 * te]);
+      const double2 b23 = *reinterpret_cast<const double2*>(&Ws[k][4 * te + 2]);
+      const double a[4] = {a01.x, a01.y, a23.x, a23.y}, b[4] = {b01.x, b01.y, b23.x, b23.y};
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[r][c] = fma(a[r], b[c], acc[r][c]);
     }
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-      const long long E = E0 + 2 * te + c;
-      if (E >= C.ne) continue;
-      double* o = KE + E * 576 + m0 + 4 * ti;
-      *reinterpret_cast<double2*>(o) = make_double2(acc[0][c], acc[1][c]);
-      *reinterpret_cast<double2*>(o + 2) = make_double2(acc[2][c], acc[3][c]);
-    }
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        if (E0 + 4 * te + c < C.ne) KE[(m0 + 4 * ti + r) * C.ne + E0 + 4 * te + c] = acc[r][c];
   }
 }
 
-// support-touching children of listed coarse elements, added to KE
+// support-touching children of listed coarse elements, added to KE: per child
+// K_c P, then P^T (K_c P), through shared memory (eight terms each; the double
+// sum over both, 64 terms with its tests inside, took 2487 us on the 4096
+// elements of a 256^3 clamped face)
 __global__ void __launch_bounds__(288) k_galerkin_fix(const Level Fl, const Level C, int F,
                                                       const double* __restrict__ rp, const double* __restrict__ K0g,
                                                       const uint8_t* __restrict__ efix, const int* __restrict__ list,
                                                       double* __restrict__ KE) {
+  __shared__ double K0[576], T[576], P[64];  // P[a * 8 + A]
   const long long E = list[blockIdx.x];
   const int X = E % C.ex, Y = (E / C.ex) % C.ey, Z = E / ((long long)C.ex * C.ey);
   const int t = threadIdx.x;
+  K0[t] = K0g[t];
+  K0[t + 288] = K0g[t + 288];
   double acc[2] = {0, 0};
-  for (int pz = 0; pz < F; pz++)
-    for (int py = 0; py < F; py++)
-      for (int px = 0; px < F; px++) {
-        const int x = X * F + px, y = Y * F + py, z = Z * F + pz;
-        if (x >= Fl.ex || y >= Fl.ey || z >= Fl.ez) continue;
-        const long long e = Fl.eidx(x, y, z);
-        const unsigned fixmask = efix[e];
-        if (!Fl.emask[e] || !fixmask) continue;
-        const double r = rp[e];
-        for (int h2 = 0; h2 < 2; h2++) {
-          const int ent = t + 288 * h2;
-          const int row = ent / 24, col = ent % 24;
-          const int A = row / 3, i = row % 3, B = col / 3, j = col % 3;
-          double s = 0;
-          for (int a = 0; a < 8; a++) {
-            const double wa = pw(F, px + (a & 1), A & 1) * pw(F, py + ((a >> 1) & 1), (A >> 1) & 1) *
-                              pw(F, pz + (a >> 2), A >> 2);
-            if (wa == 0) continue;
-            for (int b = 0; b < 8; b++) {
-              const double wb = pw(F, px + (b & 1), B & 1) * pw(F, py + ((b >> 1) & 1), (B >> 1) & 1) *
-                                pw(F, pz + (b >> 2), B >> 2);
-              if (wb == 0) continue;
-              double kv;
-              if ((fixmask >> a & 1u) || (fixmask >> b & 1u)) kv = (a == b && i == j) ? DIRICHLET_W : 0.0;
-              else kv = r * K0g[(a * 3 + i) * 24 + b * 3 + j];
-              s += wa * wb * kv;
-            }
-          }
-          acc[h2] += s;
-        }
-      }
-  KE[E * 576 + t] += acc[0];
-  KE[E * 576 + t + 288] += acc[1];
-}
-
-// dyadic recursion on element matrices
-__global__ void __launch_bounds__(288) k_galerkin_next(const Level Fl, const Level C, const double* __restrict__ KEf,
-                                                       double* __restrict__ KEc) {
-  __shared__ double K[576];
-  __shared__ double Tm[576];
-  const long long E = blockIdx.x;
-  const int X = E % C.ex, Y = (E / C.ex) % C.ey, Z = E / ((long long)C.ex * C.ey);
-  const int t = threadIdx.x;
-  double acc[2] = {0, 0};
-  if (C.emask[C.eidx(X, Y, Z)]) {
-    for (int c = 0; c < 8; c++) {
-      const int px = c & 1, py = (c >> 1) & 1, pz = c >> 2;
-      const int x = 2 * X + px, y = 2 * Y + py, z = 2 * Z + pz;
-      if (x >= Fl.ex || y >= Fl.ey || z >= Fl.ez) continue;
-      if (!Fl.emask[Fl.eidx(x, y, z)]) continue;
-      const long long ef = x + (long long)Fl.ex * (y + (long long)Fl.ey * z);
-      __syncthreads();
-      K[t] = KEf[ef * 576 + t];
-      K[t + 288] = KEf[ef * 576 + t + 288];
-      __syncthreads();
-      // Tm[(a,i),(B,j)] = sum_b K[(a,i),(b,j)] P[b][B]
-      for (int h2 = 0; h2 < 2; h2++) {
-        const int ent = t + 288 * h2;
-        const int row = ent / 24, col = ent % 24, B = col / 3, j = col % 3;
-        double s = 0;
+  for (int c = 0; c < F * F * F; c++) {
+    const int px = c % F, py = c / F % F, pz = c / (F * F);
+    const int x = X * F + px, y = Y * F + py, z = Z * F + pz;
+    if (x >= Fl.ex || y >= Fl.ey || z >= Fl.ez) continue;
+    const long long e = Fl.eidx(x, y, z);
+    const unsigned fix = efix[e];
+    if (!Fl.emask[e] || !fix) continue;  // the same for the whole CTA
+    const double r = rp[e];
+    __syncthreads();  // K0 complete; P and T free
+    if (t < 64) {
+      const int a = t >> 3, A = t & 7;
+      P[t] = pw(F, px + (a & 1), A & 1) * pw(F, py + ((a >> 1) & 1), (A >> 1) & 1) * pw(F, pz + (a >> 2), A >> 2);
+    }
+    __syncthreads();
 #pragma unroll
-        for (int b = 0; b < 8; b++) {
-          const double wb = pw(2, px + (b & 1), B & 1) * pw(2, py + ((b >> 1) & 1), (B >> 1) & 1) *
-                            pw(2, pz + (b >> 2), B >> 2);
-          s += K[row * 24 + b * 3 + j] * wb;
-        }
-        Tm[ent] = s;
-      }
-      __syncthreads();
-      for (int h2 = 0; h2 < 2; h2++) {
-        const int ent = t + 288 * h2;
-        const int row = ent / 24, col = ent % 24, A = row / 3, i = row % 3;
-        double s = 0;
+    for (int h = 0; h < 2; h++) {
+      const int ent = t + 288 * h, row = ent / 24, col = ent % 24, a = row / 3, i = row % 3, B = col / 3, j = col % 3;
+      double s = 0;
 #pragma unroll
-        for (int a = 0; a < 8; a++) {
-          const double wa = pw(2, px + (a & 1), A & 1) * pw(2, py + ((a >> 1) & 1), (A >> 1) & 1) *
-                            pw(2, pz + (a >> 2), A >> 2);
-          s += wa * Tm[(a * 3 + i) * 24 + col];
-        }
-        acc[h2] += s;
+      for (int b = 0; b < 8; b++) {
+        const bool fixed = (fix >> a & 1u) || (fix >> b & 1u);
+        const double kv = fixed ? (a == b && i == j ? DIRICHLET_W : 0.0) : r * K0[row * 24 + b * 3 + j];
+        s += kv * P[b * 8 + B];
       }
+      T[ent] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int ent = t + 288 * h, row = ent / 24, col = ent % 24, A = row / 3, i = row % 3;
+      double s = 0;
+#pragma unroll
+      for (int a = 0; a < 8; a++) s += P[a * 8 + A] * T[(a * 3 + i) * 24 + col];
+      acc[h] += s;
     }
   }
-  KEc[E * 576 + t] = acc[0];
-  KEc[E * 576 + t + 288] = acc[1];
+  KE[t * C.ne + E] += acc[0];
+  KE[(t + 288) * C.ne + E] += acc[1];
+}
+
+// Dyadic recursion on element matrices, KE_c = sum over the 8 children P^T K P.
+// A thread takes one coarse element and one pair (i, j) of components, the 8 x 8
+// block K[(a, i), (b, j)] over the nodes: row by row it interpolates along b (a
+// weight is 1 or 1/2 per axis, so a child's row is three half sums), and adds
+// the row to the coarse rows it reaches.  Consecutive lanes hold consecutive
+// elements.  The sums of an output run over the children in order.  As products
+// of 24 x 24 matrices in shared memory, one CTA per coarse element, the levels
+// below the first of 256^3 took 925 us, 451 now.
+template <int C>
+__device__ __forceinline__ void galerkin_child(const double* __restrict__ K, long long nef, int ij,
+                                               double (&acc)[8][8]) {
+  constexpr int o[3] = {C & 1, (C >> 1) & 1, C >> 2};
+#pragma unroll
+  for (int a = 0; a < 8; a++) {
+    double r[8];
+#pragma unroll
+    for (int b = 0; b < 8; b++) r[b] = K[(long long)((a * 24 + b) * 3 + ij) * nef];
+    // along each axis the child's nodes sit at o and o + 1 of 2: 0 -> (1, 0), 1 -> (1/2, 1/2), 2 -> (0, 1)
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+      for (int b = 0; b < 8; b++) {
+        if ((b >> ax) & 1) continue;
+        const int b1 = b | (1 << ax);
+        if (o[ax] == 0) { r[b] += 0.5 * r[b1]; r[b1] *= 0.5; }
+        else { r[b1] += 0.5 * r[b]; r[b] *= 0.5; }
+      }
+#pragma unroll
+    for (int A = 0; A < 8; A++) {
+      double w = 1;
+#pragma unroll
+      for (int ax = 0; ax < 3; ax++) {
+        const int p = o[ax] + ((a >> ax) & 1);  // 0, 1 or 2 halves
+        w *= (A >> ax) & 1 ? 0.5 * p : 1 - 0.5 * p;
+      }
+      if (w != 0)
+#pragma unroll
+        for (int B = 0; B < 8; B++) acc[A][B] = fma(w, r[B], acc[A][B]);
+    }
+  }
+}
+__global__ void __launch_bounds__(288, 1) k_galerkin_next(const Level Fl, const Level C, const double* __restrict__ KEf,
+                                                          double* __restrict__ KEc) {
+  const long long E = blockIdx.x * 32LL + threadIdx.x;  // blockDim (32, 9)
+  const int i = threadIdx.y / 3, j = threadIdx.y - 3 * i, ij = i * 24 + j;
+  if (E >= C.ne) return;
+  const unsigned e32 = (unsigned)E, row = e32 / (unsigned)C.ex, Zu = row / (unsigned)C.ey;
+  const int X = (int)(e32 - row * C.ex), Y = (int)(row - Zu * C.ey), Z = (int)Zu;
+  double acc[8][8] = {};
+  if (C.emask[C.eidx(X, Y, Z)]) {
+    auto base = [&](int c) -> const double* {
+      const int x = 2 * X + (c & 1), y = 2 * Y + ((c >> 1) & 1), z = 2 * Z + (c >> 2);
+      if (x >= Fl.ex || y >= Fl.ey || z >= Fl.ez || !Fl.emask[Fl.eidx(x, y, z)]) return nullptr;
+      return KEf + x + (long long)Fl.ex * (y + (long long)Fl.ey * z);
+    };
+    const double* K;
+    if ((K = base(0))) galerkin_child<0>(K, Fl.ne, ij, acc);
+    if ((K = base(1))) galerkin_child<1>(K, Fl.ne, ij, acc);
+    if ((K = base(2))) galerkin_child<2>(K, Fl.ne, ij, acc);
+    if ((K = base(3))) galerkin_child<3>(K, Fl.ne, ij, acc);
+    if ((K = base(4))) galerkin_child<4>(K, Fl.ne, ij, acc);
+    if ((K = base(5))) galerkin_child<5>(K, Fl.ne, ij, acc);
+    if ((K = base(6))) galerkin_child<6>(K, Fl.ne, ij, acc);
+    if ((K = base(7))) galerkin_child<7>(K, Fl.ne, ij, acc);
+  }
+#pragma unroll
+  for (int a = 0; a < 8; a++)
+#pragma unroll
+    for (int b = 0; b < 8; b++) KEc[(long long)((a * 24 + b) * 3 + ij) * C.ne + E] = acc[a][b];
 }
 
 // stencil assembly from element matrices: one thread per (node, neighbour d),
 // summing the 3x3 blocks of the incident elements that contain both nodes
-__global__ void k_assemble(const Level C, const double* __restrict__ KE, double* __restrict__ st64,
-                           float* __restrict__ st32) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= 27 * C.nn) return;
-  const int d = t / C.nn;
-  const long long nl = t % C.nn;
-  const int x = nl % C.nx, y = (nl / C.nx) % C.ny, z = nl / ((long long)C.nx * C.ny);
+__global__ void __launch_bounds__(256) k_assemble(const Level C, const double* __restrict__ KE,
+                                                  double* __restrict__ st64, float* __restrict__ st32) {
+  const unsigned nl = blockIdx.x * 256u + threadIdx.x;  // nn < 2^31
+  if (nl >= (unsigned)C.nn) return;
+  const int d = blockIdx.y;
+  const unsigned row = nl / (unsigned)C.nx, zu = row / (unsigned)C.ny;
+  const int x = (int)(nl - row * C.nx), y = (int)(row - zu * C.ny), z = (int)zu;
   const int dx = d % 3 - 1, dy = d / 3 % 3 - 1, dz = d / 9 - 1;
-  const long long NP = C.NP;
+  const long long NP = C.NP, ne = C.ne;
   const long long n = C.nidx(x, y, z);
   double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int k = 0; k < 8; k++) {
@@ -1026,14 +1087,13 @@ __global__ void k_assemble(const Level C, const double* __restrict__ KE, double*
     if (!((dx == kx - 1 || dx == kx) && (dy == ky - 1 || dy == ky) && (dz == kz - 1 || dz == kz))) continue;
     const int ex = x - 1 + kx, ey = y - 1 + ky, ez = z - 1 + kz;
     if (!C.emask[C.eidx(ex, ey, ez)]) continue;
-    const long long E = ex + (long long)C.ex * (ey + (long long)C.ey * ez);
     const int a = 7 - k;
     const int b = (dx - kx + 1) + 2 * (dy - ky + 1) + 4 * (dz - kz + 1);
-    const double* K = KE + E * 576;
+    const double* K = KE + (a * 72 + b * 3) * ne + ex + (long long)C.ex * (ey + (long long)C.ey * ez);
 #pragma unroll
     for (int r = 0; r < 3; r++)
 #pragma unroll
-      for (int c = 0; c < 3; c++) s[r * 3 + c] += K[(a * 3 + r) * 24 + b * 3 + c];
+      for (int c = 0; c < 3; c++) s[r * 3 + c] += K[(r * 24 + c) * ne];
   }
 #pragma unroll
   for (int i = 0; i < 9; i++) {
@@ -2129,7 +2189,7 @@ rso_status galerkin_setup(rso_handle* h) {
   if (h->L.size() < 2) return RSO_OK;
   const Level& f = h->L[0];
   const Level& c = h->L[1];
-  const int F = c.factor, F3 = F * F * F;
+  const int F = c.factor;
   RSO_CHECK_CUDA(h, cudaMalloc(&h->efix, f.NQ));
   RSO_CHECK_CUDA(h, cudaMemsetAsync(h->efix, 0, f.NQ, h->stream));
   k_elem_fixmask<<<cdiv(f.ne, 256), 256, 0, h->stream>>>(f, h->efix); rso::note_launch();
@@ -2150,7 +2210,6 @@ rso_status galerkin_setup(rso_handle* h) {
     RSO_CHECK_CUDA(h, cudaMalloc(&h->gfix, sizeof(int) * list.size()));
     RSO_CHECK_CUDA(h, cudaMemcpy(h->gfix, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
   }
-  (void)F3;
   return RSO_OK;
 }
 
@@ -2162,8 +2221,14 @@ rso_status galerkin(rso_handle* h) {
     {
       const int F = c.factor;
       const unsigned nblk = (unsigned)cdiv(c.ne, GE);
-      if (F == 4) k_galerkin_first<4><<<nblk, 256, 0, h->stream>>>(f, c, h->rp64, h->efix, h->T1, c.KE);
-      else k_galerkin_first<2><<<nblk, 256, 0, h->stream>>>(f, c, h->rp64, h->efix, h->T1, c.KE);
+      Phi phi;
+      for (int q = 0; q < 4; q++) {  // Lagrange factors on 0, 1.5, 3
+        phi.v[0][q] = (q - 1.5) * (q - 3) / 4.5;
+        phi.v[1][q] = q * (q - 3.0) / -2.25;
+        phi.v[2][q] = q * (q - 1.5) / 4.5;
+      }
+      if (F == 4) k_galerkin_first<4><<<nblk, 256, 0, h->stream>>>(f, c, h->rp64, h->efix, h->T1, phi, c.KE);
+      else k_galerkin_first<2><<<nblk, 256, 0, h->stream>>>(f, c, h->rp64, h->efix, h->T1, phi, c.KE);
       rso::note_launch();
       RSO_TRY(launch_check(h, "galerkin first level"));
       if (h->n_gfix > 0) {
@@ -2171,10 +2236,10 @@ rso_status galerkin(rso_handle* h) {
       }
     }
     else
-      k_galerkin_next<<<(unsigned)c.ne, 288, 0, h->stream>>>(f, c, f.KE, c.KE);
+      k_galerkin_next<<<(unsigned)cdiv(c.ne, 32), dim3(32, 9), 0, h->stream>>>(f, c, f.KE, c.KE);
     rso::note_launch();
     RSO_TRY(launch_check(h, "galerkin"));
-    k_assemble<<<cdiv(27 * c.nn, 256), 256, 0, h->stream>>>(c, c.KE, c.st64, c.st32); rso::note_launch();
+    k_assemble<<<dim3(cdiv(c.nn, 256), 27), 256, 0, h->stream>>>(c, c.KE, c.st64, c.st32); rso::note_launch();
     RSO_TRY(launch_check(h, "assemble"));
   }
   return RSO_OK;
@@ -2206,7 +2271,7 @@ rso_status coarsest_factor(rso_handle* h) {
   if (a_rig > 0) RSO_TRY(dense_rank_update(h, h->c_K + (size_t)N * N, N, h->c_R, 6, -1.0 / a_rig));
   int flag = 0;
   RSO_CHECK_CUDA(h, cudaMemcpyAsync(&flag, h->c_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
+  RSO_TRY(fine_stage_check(h));  // synchronises; reports a barrier wait of the inversion that gave up
   if (flag) {
     h->err = h->has_support ? "coarsest operator is not positive definite (no support node reaches it?)"
                             : "coarsest operator is singular beyond the rigid motions (disconnected parts?)";
@@ -2227,29 +2292,34 @@ __global__ void k_seed_vec(const Level L, float* v, uint64_t seed, int zero_supp
 }
 
 // lambda_max(D^-1 K) of every smoothed level: 12 power iterations in FP32
-// (the estimate only sets the smoother's step sizes and gets a 5 % margin)
+// (the estimate only sets the smoother's step sizes and gets a 5 % margin).  A
+// smoothing step with c1 = -1, omega = -1 and no right-hand side or previous
+// iterate is the iteration itself, out = u - u + D^-1 K u, so an iteration is one
+// launch; the ratio of the last two norms is the estimate, summed in FP64 and
+// read by the host once for all levels.
 rso_status estimate_lambda(rso_handle* h) {
-  const int iters = 12;
-  for (size_t li = 0; li + 1 < h->L.size() || (li == 0 && h->L.size() == 1); li++) {
+  const int iters = 12, nl = (int)h->L.size(), levels = nl == 1 ? 1 : nl - 1;
+  if (2 * levels > 24) { h->err = "too many levels"; return RSO_ERR_STATE; }
+  double* sums = h->scal + 16;  // u.u, r.r per level
+  for (int li = 0; li < levels; li++) {
     Level& l = h->L[li];
     const long long n3 = 3 * l.NP;
     k_seed_vec<<<cdiv(l.NP, 256), 256, 0, h->stream>>>(l, l.u32, 777 + li, li == 0); rso::note_launch();
     RSO_CHECK_CUDA(h, cudaMemsetAsync(l.f32, 0, sizeof(float) * n3, h->stream));
-    double lam = 1.0;
     for (int it = 0; it < iters; it++) {
-      // t = u - D^-1 K u, r = D^-1 K u
-      if (li == 0) RSO_TRY(fine_jacobi<float>(h, l.u32, l.f32, l.t32, h->rp32, 1.0));
-      else RSO_TRY(coarse_jacobi<float>(h, (int)li, l.u32, l.f32, l.t32, 1.0));
-      double uu = 0, rr = 0;
-      RSO_TRY(pow_step(h, n3, l.u32, l.t32, l.r32, &uu, &rr));
-      if (!(uu > 0)) break;
-      lam = std::sqrt(rr / uu);
-      std::swap(l.u32, l.r32);
+      if (li == 0) RSO_TRY(fine_jacobi<float>(h, l.u32, l.f32, l.t32, h->rp32, -1.0, nullptr, -1.0));
+      else RSO_TRY(coarse_jacobi<float>(h, li, l.u32, l.f32, l.t32, -1.0, nullptr, -1.0));
+      if (it + 1 == iters) RSO_TRY(norms2(h, n3, l.u32, l.t32, sums + 2 * li));
+      std::swap(l.u32, l.t32);
     }
-    l.lam = 1.05 * lam;
-    if (h->L.size() == 1) break;
   }
-  return fine_stage_check(h);
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 16, sums, 2 * levels * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  RSO_TRY(fine_stage_check(h));  // synchronises
+  for (int li = 0; li < levels; li++) {
+    const double uu = h->h_scal[16 + 2 * li], rr = h->h_scal[17 + 2 * li];
+    h->L[li].lam = 1.05 * (uu > 0 ? std::sqrt(rr / uu) : 1.0);
+  }
+  return RSO_OK;
 }
 
 template rso_status coarse_residual<double>(rso_handle*, int, const double*, const double*, double*);

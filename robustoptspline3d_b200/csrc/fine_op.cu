@@ -50,7 +50,10 @@ __global__ void k_penalise(Level L, const float* rho, float* rp32, double* rp64,
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= L.NQ) return;
   double v = 0.0;
-  if (L.emask[i]) v = pow((double)rho[i], p);
+  if (L.emask[i]) {
+    const double r = (double)rho[i];  // small whole exponents as products, a tenth of pow's instructions
+    v = p == 3.0 ? r * r * r : p == 2.0 ? r * r : p == 1.0 ? r : pow(r, p);
+  }
   rp64[i] = v;
   rp32[i] = (float)v;
 }

@@ -33,7 +33,7 @@ struct Level {
   long long n_active_e = 0, n_active_v = 0;
   uint8_t* emask = nullptr;       // padded element mask
   uint8_t* vclass = nullptr;      // padded node class
-  double* KE = nullptr;           // coarse element matrices, 576 per unpadded element
+  double* KE = nullptr;           // coarse element matrices [576][ne], ne unpadded elements
   double* st64 = nullptr;         // stencil [243][NP]
   float* st32 = nullptr;          // stencil in tiles of 128 nodes (st_at), 243 x round_up(NP, 128)
   double *u64 = nullptr, *f64 = nullptr, *r64 = nullptr, *t64 = nullptr;
@@ -108,7 +108,7 @@ struct rso_handle {
   int* load_nodes = nullptr;          // padded node ids
   double* load_normals = nullptr;     // 3 per load node
   // Galerkin tables
-  double* T1 = nullptr;               // F^3 x 576 table for the first coarsening
+  double* T1 = nullptr;               // child matrices of the first coarsening (27 for factor 4, 8 for 2) x 576
   uint8_t* efix = nullptr;            // per padded fine element: bit a set if local node a is a support node
   int* gfix = nullptr;                // coarse elements with a child that touches a support node
   int n_gfix = 0;
@@ -352,7 +352,7 @@ rso_status cg_resid_rr(rso_handle* h, long long n, const double* alpha, const do
 rso_status reduce_partials(rso_handle* h, const double* part, int n, double* dev_out);
 rso_status reduce_partials_batch(rso_handle* h, const double* part, int nper, int nb, double* dev_out,
                                  int stride = 1);
-rso_status pow_step(rso_handle* h, long long n, const float* u, const float* t, float* r, double* uu, double* rr);
+rso_status norms2(rso_handle* h, long long n, const float* u, const float* r, double* dev_out);
 rso_status dot_df(rso_handle* h, const double* a, const float* b, long long n, double* dev_out);
 rso_status dot_ff(rso_handle* h, const float* a, const float* b, long long n, double* dev_out);
 rso_status cg32_resid_rr(rso_handle* h, long long n, const double* alpha, const float* q, float* r, double* rr_dev);

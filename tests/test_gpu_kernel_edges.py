@@ -29,7 +29,7 @@ def test_fine_fp64_chunks(oracle, cuda, dims):
 # coarse levels of 2 to 17 nodes an edge: colours of one node, of fewer and of more than the 32 a CTA
 # takes, with a ragged last CTA; the ellipsoid leaves inactive nodes inside the box
 @pytest.mark.parametrize("gen", [lambda: P.cantilever(6, 4, 3), lambda: P.cantilever(30, 21, 13),
-                                 lambda: P.ellipsoid(64, 36, 28)])
+                                 lambda: P.ellipsoid(40, 24, 20)])
 @pytest.mark.parametrize("reverse", [0, 1])
 def test_coarse_gauss_seidel(oracle, cuda, gen, reverse):
     """FP64 coloured sweeps on every coarse level; 1e-12 relative, the bound of the FP64 operator pieces."""
@@ -160,3 +160,38 @@ def test_mma_update_sizes(oracle, cuda, n, m):
         g.update(t(df, cuda), t(dg, cuda), gval)
         for a, b in zip(g.get(), o.get()):
             assert np.allclose(a, b, rtol=1e-8, atol=1e-10)
+
+
+# boxes whose edges are multiples of the coarsening factors and not, with voids and clamped faces, both
+# first factors
+@pytest.mark.parametrize("dims,levels,factor", [((12, 8, 8), 2, 4), ((21, 13, 9), 3, 2), ((33, 18, 22), 3, 4)])
+def test_galerkin_operators(oracle, cuda, dims, levels, factor):
+    """Products with the assembled stencils, 1e-12 relative, as the FP64 operator pieces."""
+    g, o = make(oracle, P.voids_box(*dims, nvoids=1), n_levels=levels, first_factor=factor, smoother=1)
+    g.update_stencil()
+    o.update_stencil()
+    rng = np.random.default_rng(29)
+    for lvl in range(1, o.n_levels()):
+        mask = np.tile(o.level_masks(lvl)[1], 3)
+        u, f = (rng.standard_normal(mask.size) * mask for _ in range(2))
+        assert rel(g.coarse_residual(lvl, t(u, cuda), t(f, cuda)).cpu().numpy(), o.coarse_residual(lvl, u, f)) < 1e-12
+
+
+# coarsest systems of part of a 32-wide tile, of tiles and a remainder (N = 105, 417, 2175), and past
+# the size up to which the inversion is the blocked Gauss-Jordan kernel (N = 4707)
+@pytest.mark.parametrize("dims,levels,factor", [((12, 8, 8), 2, 4), ((21, 13, 9), 3, 2), ((16, 16, 16), 2, 2),
+                                                ((24, 20, 20), 2, 2)])
+def test_coarsest_inverse(cuda, dims, levels, factor):
+    """K x = f on the coarsest level, residual 1e-9 relative, as the coarsest solve's parity test."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.voids_box(*dims, nvoids=1)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"],
+                      Config(n_levels=levels, first_factor=factor))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    last = g.n_levels() - 1
+    mask = np.tile(g.level_masks(last)[1], 3)
+    f = np.random.default_rng(31).standard_normal(mask.size) * mask
+    x = g.solve_coarsest(t(f, cuda))
+    r = g.coarse_residual(last, x, t(f, cuda)).cpu().numpy()
+    assert np.linalg.norm(r) < 1e-9 * np.linalg.norm(f)
