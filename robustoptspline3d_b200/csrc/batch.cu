@@ -208,9 +208,12 @@ static rso_status batch_alloc(rso_handle* h, int k) {
   batch_free(h);
   const bool mixed = h->cfg.precision == RSO_MIXED;
   const size_t nl = h->L.size();
+  // zeroed: the operators read the padding of vectors of which they write the
+  // interior only
 #define BALLOC(ptr, bytes)                                                   \
   do {                                                                       \
-    if (cudaMalloc((void**)&(ptr), (bytes)) != cudaSuccess) {                \
+    if (cudaMalloc((void**)&(ptr), (bytes)) != cudaSuccess ||                \
+        cudaMemsetAsync((ptr), 0, (bytes), h->stream) != cudaSuccess) {      \
       cudaGetLastError();                                                    \
       batch_free(h);                                                         \
       h->err = "out of device memory for the batch of systems";              \

@@ -195,3 +195,22 @@ def test_coarsest_inverse(cuda, dims, levels, factor):
     x = g.solve_coarsest(t(f, cuda))
     r = g.coarse_residual(last, x, t(f, cuda)).cpu().numpy()
     assert np.linalg.norm(r) < 1e-9 * np.linalg.norm(f)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_on_used_memory(cuda, precision):
+    """The batch's slabs come from memory that held NaN before: its padding must not reach the solution."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(20, 12, 12)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None,
+                      Config(poisson_ratio=0.4, precision=precision, smoother=1, n_levels=3, first_factor=2))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    used = [cuda.full((1 << 20,), float("nan"), dtype=cuda.float64, device="cuda") for _ in range(64)]
+    cuda.cuda.synchronize()
+    del used
+    cuda.cuda.empty_cache()
+    f = t(prob["f"], cuda)
+    U, infos = g.solve_batch(cuda.stack([f, 2 * f]), tol=1e-10)
+    u, it, _, _ = g.solve(f, tol=1e-10)
+    assert rel(U[0].cpu().numpy(), u.cpu().numpy()) < 1e-8 and abs(infos[0][0] - it) <= 1
