@@ -328,8 +328,7 @@ rso_status rso_autotune(rso_handle* h, int* choices_host);
 /* Sets the launch shapes directly, in rso_autotune's format (n >= 2 ints;
  * bottom level -2 restores the built-in size rule, a row-split entry of -1
  * too), e.g. to reuse choices measured once for many handles.  The built-in
- * bottom rule, for the FP32 V-cycle of mixed precision with bottom kernel
- * kind 1: the persistent kernel from the first coarse level of at most 60,000
+ * bottom rule, with bottom kernel kind 1: the persistent kernel from the first coarse level of at most 60,000
  * nodes above the coarsest. */
 rso_status rso_set_launch_shapes(rso_handle* h, const int* choices_host, int n);
 /* Node planes per z chunk of the packed FP32 fine kernel (4, 8, 16 or 32; 0
@@ -340,7 +339,7 @@ rso_status rso_set_launch_shapes(rso_handle* h, const int* choices_host, int n);
  * use. */
 rso_status rso_set_fine_zchunk(rso_handle* h, int planes);
 int rso_fine_zchunk(const rso_handle* h);
-/* Kernel of the bottom of the FP32 V-cycle, when the launch shapes give it a
+/* Kernel of the bottom of the V-cycle, when the launch shapes give it a
  * first level (no counterpart in the reference, which launches every level's
  * kernels): kind 1 (default) one persistent cooperative kernel over the whole
  * GPU, every CTA resident at once, its phases (sweeps, residuals, transfers,
@@ -358,7 +357,7 @@ int rso_bottom_kernel(const rso_handle* h);
  * barrier state is reset afterwards, so the handle stays usable.  No fault and
  * no hang either way. */
 rso_status rso_grid_barrier_selftest(rso_handle* h, int short_by, double limit_ms, int* gave_up);
-/* Replay of the FP32 V-cycle (the mixed-precision preconditioner) from CUDA
+/* Replay of the preconditioner's V-cycle (FP32 in mixed precision, else FP64) from CUDA
  * graphs (no counterpart in the reference, which launches every kernel):
  * on by default.  The V-cycle is captured the second time its launch
  * arguments (level vectors, sizes, smoother step sizes, configuration,

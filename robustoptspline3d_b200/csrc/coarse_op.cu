@@ -1494,27 +1494,88 @@ __global__ void __cluster_dims__(BOT_CTAS, 1, 1) __launch_bounds__(BOT_THREADS, 
 // a cooperative launch (every CTA resident at once) whose phases are
 // separated by a grid-wide barrier.  FP32 sweeps run on four-node groups with
 // nine threads each and, on the levels that fit, on stencils held in shared
-// memory (below); FP64 sweeps as the row-split per-level kernel does (tiles of
-// 32 x CTY nodes, three threads per node).  What bounds it is latency: a phase
+// memory (below); FP64 sweeps with nine threads per node.  What bounds it is latency: a phase
 // is a barrier and one round of loads.  Per V-cycle, 2 + 2 Chebyshev steps: from
 // the 33^3 level of 256^3 down 174 -> 149 us (33^3 streamed, the rest held),
 // 93 x 71 x 85 110 -> 70 us, 64^3 96 -> 59 us, 49 x 38 x 56 68 -> 37 us (all
 // held), before: two-word barriers, every stencil streamed, two CTAs per SM.
-// one row-split sweep (MODE 2) or residual (MODE 0) of a level, tile by tile
-template <typename T, int MODE, bool ZERO>
-__device__ void gb_sweep_rows(const Level& L, const T* st, const T* u, const T* f, T* out, T omega, const T* uprev,
-                              T c1, T (*sres)[CTY][32]) {
-  const int tx = (L.nx + 31) / 32, ty = (L.ny + CTY - 1) / CTY;
-  const long long nt = (long long)tx * ty * L.nz * L.nb;
-  for (long long t = blockIdx.x; t < nt; t += gridDim.x) {
-    const int bx = (int)(t % tx);
-    const long long q = t / tx;
-    const int by = (int)(q % ty);
-    const long long zb = q / ty;
-    const int bsys = (int)(zb / L.nz), z = (int)(zb - (long long)bsys * L.nz);
-    coarse_r_node<T, MODE, ZERO>(L, st, u, f, out, omega, uprev, c1, bx * 32 + threadIdx.x, by * CTY + threadIdx.y,
-                                 z, bsys, sres);
-    __syncthreads();  // sres is reused by the next tile
+// FP64: a sweep (MODE 2) or residual (MODE 0) of the persistent kernel on tiles
+// of G9 consecutive nodes with nine threads each, one per neighbour row: 27
+// independent stencil loads a thread, the partial sums met in shared memory in
+// a fixed order, the first warp finishing the nodes (the split of k_coarse_gs).
+// ZERO: u read as zero (a first step from a zero iterate).
+constexpr int G9 = 32;
+template <int MODE, bool ZERO>
+__device__ void gb_sweep9(const Level& L, const double* __restrict__ st, const double* u0, const double* f0,
+                          double* out0, double omega, const double* up0, double c1, int tid, double (*part)[3][G9]) {
+  const int lane = tid % G9, row = tid / G9;
+  const long long NP = L.NP;
+  const unsigned nn = (unsigned)L.nn;
+  for (long long t = blockIdx.x; t * G9 < (long long)nn * L.nb; t += gridDim.x) {
+    const long long i = t * G9 + lane;
+    const bool in = i < (long long)nn * L.nb;
+    const unsigned b = in ? (unsigned)(i / nn) : 0u, m = in ? (unsigned)(i - (long long)b * nn) : 0u;
+    const unsigned q = m / (unsigned)L.nx, z = q / (unsigned)L.ny;
+    const long long n = L.nidx((int)(m - q * L.nx), (int)(q - z * L.ny), (int)z), vo = (long long)b * 3 * NP;
+    const bool act = in && (L.vclass[n] & NC_ACTIVE);
+    const double* u = u0 + vo;
+    double acc[3] = {0, 0, 0};
+    if (in && !ZERO) {  // zero stencil at inactive nodes
+      const long long nb = n + (row % 3 - 1) * (long long)L.px + (row / 3 - 1) * (long long)L.px * L.py;
+#pragma unroll
+      for (int e = 0; e < 3; e++) {
+        const double a0 = u[nb + e - 1], a1 = u[nb + e - 1 + NP], a2 = u[nb + e - 1 + 2 * NP];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          const double* k = st + ((3 * row + e) * 9 + 3 * r) * NP + n;
+          acc[r] = fma(k[0], a0, fma(k[NP], a1, fma(k[2 * NP], a2, acc[r])));
+        }
+      }
+    }
+    double S[9], fv[3], uo[3], pv[3];
+    if (row == 0 && in) {
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        fv[r] = f0[vo + n + r * NP];
+        uo[r] = MODE == 2 && !ZERO ? u[n + r * NP] : 0.0;
+        pv[r] = MODE == 2 && up0 ? up0[vo + n + r * NP] : 0.0;
+      }
+      if (MODE == 2) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) S[k] = st[(13 * 9 + k) * NP + n];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; r++) part[row][r][lane] = acc[r];
+    __syncthreads();
+    if (row == 0 && in) {
+      double* out = out0 + vo;
+      double res[3];
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        double s = part[0][r][lane];
+#pragma unroll
+        for (int k = 1; k < 9; k++) s += part[k][r][lane];
+        res[r] = fv[r] - (act ? s : 0.0);
+      }
+      if (MODE == 0) {
+#pragma unroll
+        for (int r = 0; r < 3; r++) out[n + r * NP] = res[r];
+      } else if (!act) {
+#pragma unroll
+        for (int r = 0; r < 3; r++) out[n + r * NP] = 0.0;
+      } else {
+        const double A = S[4] * S[8] - S[5] * S[7], B = -(S[3] * S[8] - S[5] * S[6]), C = S[3] * S[7] - S[4] * S[6];
+        const double id = omega / (S[0] * A + S[1] * B + S[2] * C);
+        const double i01 = -(S[1] * S[8] - S[2] * S[7]), i02 = S[1] * S[5] - S[2] * S[4];
+        const double i11 = S[0] * S[8] - S[2] * S[6], i12 = -(S[0] * S[5] - S[2] * S[3]);
+        const double i21 = -(S[0] * S[7] - S[1] * S[6]), i22 = S[0] * S[4] - S[1] * S[3];
+        out[n] = uo[0] + c1 * (uo[0] - pv[0]) + id * (A * res[0] + i01 * res[1] + i02 * res[2]);
+        out[n + NP] = uo[1] + c1 * (uo[1] - pv[1]) + id * (B * res[0] + i11 * res[1] + i12 * res[2]);
+        out[n + 2 * NP] = uo[2] + c1 * (uo[2] - pv[2]) + id * (C * res[0] + i21 * res[1] + i22 * res[2]);
+      }
+    }
+    __syncthreads();  // part is reused by the next tile
   }
 }
 
@@ -1528,7 +1589,6 @@ __device__ void gb_sweep_rows(const Level& L, const T* st, const T* u, const T* 
 // does (residual, or damped block Jacobi / Chebyshev step; halo rows
 // unwritten).  A team of 9 G9 threads takes a tile of G9 groups, the 128 nodes
 // of one tile of the FP32 stencil.
-constexpr int G9 = 32;
 constexpr int kTeam = 9 * G9, kTeams = 1;
 static_assert(4 * G9 == ST_TILE, "a team's tile is a tile of the stencil");
 __device__ __forceinline__ void team_sync(int team) {
@@ -1701,13 +1761,13 @@ __device__ __forceinline__ bool tile_landed(uint64_t* bar) {
   return false;
 }
 
-// threads of a CTA of the persistent kernel: two teams (FP32), 32 x CTY x 3
-// for the row-split sweeps (FP64)
+// threads of a CTA of the persistent kernel: the FP32 teams, or one thread per
+// neighbour row of G9 nodes (FP64)
 template <typename T>
-constexpr int gb_threads() { return sizeof(T) == 4 ? kTeams * kTeam : 32 * CTY * 3; }
-// shared exchange of the sweeps: [teams][9][12][G9] floats (FP32), [3][CTY][32] T (FP64)
+constexpr int gb_threads() { return sizeof(T) == 4 ? kTeams * kTeam : 9 * G9; }
+// shared exchange of the sweeps: [teams][9][12][G9] floats (FP32), [9][3][G9] doubles (FP64)
 template <typename T>
-constexpr int gb_smem() { return sizeof(T) == 4 ? kTeams * 9 * 12 * G9 * 4 : 3 * CTY * 32 * (int)sizeof(T); }
+constexpr int gb_smem() { return sizeof(T) == 4 ? kTeams * 9 * 12 * G9 * 4 : 9 * 3 * G9 * (int)sizeof(T); }
 
 template <typename T>
 __global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid_constant__ BottomArgs<T> A,
@@ -1716,7 +1776,7 @@ __global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid
   extern __shared__ __align__(128) unsigned char stile[];  // FP32: this CTA's stencil tile
   __shared__ __align__(8) uint64_t tbar;
   constexpr int NT = gb_threads<T>();
-  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int tid = threadIdx.x;
   const int g0 = blockIdx.x * NT + tid, gs = gridDim.x * NT;
   GroupPos own;
   int own_li = -1;
@@ -1768,7 +1828,7 @@ __global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid
       gb_sweep4<MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, tid, A.tile0[li], own,
                             reinterpret_cast<const float*>(stile), reinterpret_cast<float (*)[9][12][G9]>(sres));
     } else {
-      gb_sweep_rows<T, MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, reinterpret_cast<T (*)[CTY][32]>(sres));
+      gb_sweep9<MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, tid, reinterpret_cast<double (*)[3][G9]>(sres));
     }
   };
   using M0 = std::integral_constant<int, 0>;
@@ -2064,19 +2124,19 @@ rso_status coarsest_solve(rso_handle* h, const T* f, T* u) {
 // index of the first level handled by the bottom kernel (-1: none).  It needs
 // damped Jacobi or Chebyshev and at least one smoothed level above the
 // coarsest; the level is rso_autotune's choice or the built-in rule's.
-int bottom_level(const rso_handle* h, bool fp32) {
+int bottom_level(const rso_handle* h, int pre, int post) {
   const int nl = (int)h->L.size();
   if (h->cfg.smoother == RSO_SMOOTH_GS || nl < 3 || nl > BOT_MAX_LEVELS || h->nc == 0) return -1;
-  if (h->cfg.pre > BOT_MAX_SWEEPS || h->cfg.post > BOT_MAX_SWEEPS) return -1;
+  if (pre > BOT_MAX_SWEEPS || post > BOT_MAX_SWEEPS) return -1;
   // a level chosen by rso_autotune: any level from 1 to nl - 2, or none
   if (h->tune.bottom == -1) return -1;
   if (h->tune.bottom >= 1 && h->tune.bottom <= nl - 2) return h->tune.bottom;
-  // built-in rule, for the FP32 V-cycle of mixed precision (the FP64 one keeps
-  // its per-level launches): the persistent grid-wide kernel from the first
-  // level of at most kBottomMaxNodes nodes, whose sweeps are latency-bound
-  // (256^3: from 33^3, 35.2 -> 33.6 ms per solve; 64^3: from 17^3, 5.6 ->
-  // 4.2 ms); the cluster kernel only when rso_autotune finds it faster
-  if (!fp32 || h->cfg.precision != RSO_MIXED || h->tune.bottom_kind != 1) return -1;
+  // built-in rule, in both precisions: the persistent grid-wide kernel from the
+  // first level of at most kBottomMaxNodes nodes, whose sweeps are latency-bound
+  // (FP32, 256^3: from 33^3, 35.2 -> 33.6 ms per solve; 64^3: from 17^3, 5.6 ->
+  // 4.2 ms; FP64, 64 x 32 x 32: 4.2 -> 3.3 ms, 128 x 128 x 112: 17.4 -> 15.9 ms);
+  // the cluster kernel only when rso_autotune finds it faster
+  if (h->tune.bottom_kind != 1) return -1;
   for (int li = 1; li <= nl - 2; li++)
     if (h->L[li].nn <= kBottomMaxNodes) return li;
   return -1;
@@ -2138,7 +2198,7 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
   for (int li = nl - 1; li >= lb; li--) {
     const Level& l = h->L[li];
     if (sizeof(T) == 8) {
-      need = std::max(need, (long long)cdiv(l.nx, 32) * cdiv(l.ny, CTY) * l.nz * l.nb);
+      need = std::max<long long>(need, std::max(cdiv(l.nn * l.nb, G9), cdiv(3 * l.nn * l.nb, gb_threads<T>())));
       continue;
     }
     const long long tiles = cdiv(l.NP, ST_TILE);
@@ -2155,7 +2215,7 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
   const int grid = (int)std::max<long long>(1, std::min<long long>(std::max(need, held), most));
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(grid);
-  lc.blockDim = sizeof(T) == 4 ? dim3(gb_threads<T>()) : dim3(32, CTY, 3);
+  lc.blockDim = dim3(gb_threads<T>());
   lc.dynamicSmemBytes = dsm;
   lc.stream = h->stream;
   cudaLaunchAttribute at[1];

@@ -191,7 +191,7 @@ struct rso_handle {
   // vectors, reorthogonalisation sums, the force-projection vector
   double* wc_buf = nullptr;
   size_t wc_cap = 0;
-  void* vcg = nullptr;                             // captured FP32 V-cycles (solver.cu)
+  void* vcg = nullptr;                             // captured V-cycles (solver.cu)
   void* cap_prof = nullptr;                        // event pairs of the V-cycle capture in progress (prof.cu)
   bool vc_graphs = true;                           // replay captured V-cycles (rso_set_vcycle_graphs)
   // run the FP32-Krylov PCG loop as one captured graph whose iterations and
@@ -384,7 +384,8 @@ void smoother_steps(const rso_handle* h, double lam, int m, double* om, double* 
 // levels of at most this many nodes are the bottom kernels' (the built-in
 // rule's first level; the largest rso_autotune tries)
 constexpr long long kBottomMaxNodes = 60000;
-int bottom_level(const rso_handle* h, bool fp32 = true);
+int bottom_level(const rso_handle* h, int pre, int post);
+inline int bottom_level(const rso_handle* h) { return bottom_level(h, h->cfg.pre, h->cfg.post); }
 template <typename T>
 rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post);
 rso_status fine_applyK_dot(rso_handle* h, const double* u, double* f, const double* rp, double* dot_dev,
@@ -435,7 +436,10 @@ rso_status estimate_lambda(rso_handle* h);
 template <typename T>
 rso_status vcycle_levels(rso_handle* h, int pre, int post, int symmetric, bool u0_zero);
 rso_status precondition(rso_handle* h, const double* r, double* z);
+// one V-cycle from a zero iterate on L[0].f (32 or 64), the result in L[0].u, replayed from a captured graph
+// where its launches recur
 rso_status vcycle_mixed(rso_handle* h);
+rso_status vcycle_double(rso_handle* h);
 void batch_release(rso_handle* h);
 rso_status solve_pcg_batch(rso_handle* h, int k, const double* F_dense, double* U_dense, double tol, int max_iter,
                            rso_solve_info* infos);

@@ -117,7 +117,7 @@ template <typename T>
 rso_status vcycle_levels(rso_handle* h, int pre, int post, int symmetric, bool u0_zero) {
   const int nl = (int)h->L.size();
   // levels from lb down run inside one bottom kernel (bottom_vcycle)
-  const int lb = bottom_level(h, sizeof(T) == 4);
+  const int lb = bottom_level(h, pre, post);
   const int top = lb > 0 ? lb : nl;
   for (int li = 0; li < top; li++) {
     Level& l = h->L[li];
@@ -182,8 +182,7 @@ rso_status precondition(rso_handle* h, const double* r, double* z) {
     k_f2d<<<cdiv(n3, 256), 256, 0, h->stream>>>(l0.u32, z, n3); rso::note_launch();
   } else {
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(l0.f64, r, sizeof(double) * n3, cudaMemcpyDeviceToDevice, h->stream));
-    RSO_CHECK_CUDA(h, cudaMemsetAsync(l0.u64, 0, sizeof(double) * n3, h->stream));
-    RSO_TRY(vcycle_levels<double>(h, pre, post, 1, true));
+    RSO_TRY(vcycle_double(h));
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(z, l0.u64, sizeof(double) * n3, cudaMemcpyDeviceToDevice, h->stream));
   }
   return launch_check(h, "precondition");
@@ -212,19 +211,23 @@ __global__ void k_cg_step(long long n, const double* __restrict__ alpha, const d
   if (i < n) x[i] += (*alpha) * p[i];
 }
 
-// mixed precision: one FP32 V-cycle from a zero iterate on L[0].f32 (already
-// holding the FP32 residual); the result is left in L[0].u32
-static rso_status vcycle_mixed_launches(rso_handle* h) {
+// one V-cycle from a zero iterate on L[0].f (FP32 in mixed precision, already
+// holding the residual); the result is left in L[0].u
+static rso_status vcycle_launches(rso_handle* h, bool fp64) {
   Level& l0 = h->L[0];
   // the first damped-Jacobi sweep from zero reads no iterate; Gauss-Seidel does
-  if (h->cfg.smoother == RSO_SMOOTH_GS || h->cfg.pre == 0)
-    RSO_CHECK_CUDA(h, cudaMemsetAsync(l0.u32, 0, sizeof(float) * 3 * l0.NP * l0.nb, h->stream));
+  const bool clear = h->cfg.smoother == RSO_SMOOTH_GS || h->cfg.pre == 0;
+  if (fp64) {
+    if (clear) RSO_CHECK_CUDA(h, cudaMemsetAsync(l0.u64, 0, sizeof(double) * 3 * l0.NP * l0.nb, h->stream));
+    return vcycle_levels<double>(h, h->cfg.pre, h->cfg.post, 1, true);
+  }
+  if (clear) RSO_CHECK_CUDA(h, cudaMemsetAsync(l0.u32, 0, sizeof(float) * 3 * l0.NP * l0.nb, h->stream));
   return vcycle_levels<float>(h, h->cfg.pre, h->cfg.post, 1, true);
 }
 
 // ---------------------------------------------------------------- captured V-cycles
-// The FP32 V-cycle of the preconditioner is about forty launches per CG
-// iteration.  It is captured once into a CUDA graph and replayed.  What a
+// The V-cycle of the preconditioner is ten to forty launches per CG iteration,
+// a hundred with Gauss-Seidel colours.  It is captured once into a CUDA graph and replayed.  What a
 // capture freezes is the launch arguments: level vectors (the smoothers
 // rotate three per level, so successive V-cycles differ and repeat with a
 // short period), level sizes, smoother step sizes (from lambda_max), scratch
@@ -256,9 +259,14 @@ void push_bits(std::vector<uint64_t>& k, X v) {
   k.push_back(b);
 }
 
-// rotating = false leaves the rotating level vectors (u32, r32, t32) out
-std::vector<uint64_t> vc_key(const rso_handle* h, bool rotating = true) {
+// rotating = false leaves the rotating level vectors (u, r, t) out
+std::vector<uint64_t> vc_key(const rso_handle* h, bool rotating = true, bool fp64 = false) {
   std::vector<uint64_t> k;
+  push_bits(k, fp64);
+  for (const Level& l : h->L)
+    if (fp64) {
+      push_bits(k, l.u64); push_bits(k, l.f64); push_bits(k, l.r64); push_bits(k, l.t64); push_bits(k, l.st64);
+    }
   for (const Level& l : h->L) {
     push_bits(k, rotating ? l.u32 : nullptr); push_bits(k, l.f32);
     push_bits(k, rotating ? l.r32 : nullptr); push_bits(k, rotating ? l.t32 : nullptr);
@@ -267,18 +275,22 @@ std::vector<uint64_t> vc_key(const rso_handle* h, bool rotating = true) {
     push_bits(k, l.nx); push_bits(k, l.ny); push_bits(k, l.nz); push_bits(k, l.px); push_bits(k, l.py);
     push_bits(k, l.factor);
   }
-  push_bits(k, h->rp32); push_bits(k, h->xfer); push_bits(k, h->xfer_n);
+  push_bits(k, h->rp32); push_bits(k, h->rp64); push_bits(k, h->xfer); push_bits(k, h->xfer_n);
   push_bits(k, h->c_K); push_bits(k, h->c_nodes); push_bits(k, h->c_f); push_bits(k, h->c_fb); push_bits(k, h->nc);
   push_bits(k, h->cfg.smoother); push_bits(k, h->cfg.pre); push_bits(k, h->cfg.post);
   push_bits(k, h->cfg.omega); push_bits(k, h->cfg.cheb_lower); push_bits(k, h->prof_on); push_bits(k, h->vc_zdot); push_bits(k, h->vc_zdot_stride);
   push_bits(k, h->tune.fine_rows); push_bits(k, h->tune.fine_zc); push_bits(k, h->tune.bottom);
+  push_bits(k, h->tune.bottom_kind);
   for (int r : h->tune.rowsplit) push_bits(k, r);
   return k;
 }
 
 std::vector<uint64_t> vc_rotating(const rso_handle* h) {
   std::vector<uint64_t> k;
-  for (const Level& l : h->L) { push_bits(k, l.u32); push_bits(k, l.r32); push_bits(k, l.t32); }
+  for (const Level& l : h->L) {
+    push_bits(k, l.u32); push_bits(k, l.r32); push_bits(k, l.t32);
+    push_bits(k, l.u64); push_bits(k, l.r64); push_bits(k, l.t64);
+  }
   return k;
 }
 
@@ -288,6 +300,9 @@ void vc_set_rotating(rso_handle* h, const std::vector<uint64_t>& v) {
     std::memcpy(&l.u32, &v[i++], sizeof(float*));
     std::memcpy(&l.r32, &v[i++], sizeof(float*));
     std::memcpy(&l.t32, &v[i++], sizeof(float*));
+    std::memcpy(&l.u64, &v[i++], sizeof(double*));
+    std::memcpy(&l.r64, &v[i++], sizeof(double*));
+    std::memcpy(&l.t64, &v[i++], sizeof(double*));
   }
 }
 
@@ -317,12 +332,14 @@ void vcycle_graphs_free(rso_handle* h) {
   h->vcg = nullptr;
 }
 
-rso_status vcycle_mixed(rso_handle* h) {
-  if (!h->vc_graphs || h->stream == nullptr) return vcycle_mixed_launches(h);
+static rso_status vcycle_replayed(rso_handle* h, bool fp64) {
+  // a capture holds event pairs for 128 timed kernels, fewer than Gauss-Seidel's colours
+  if (!h->vc_graphs || h->stream == nullptr || (h->prof_on && h->cfg.smoother == RSO_SMOOTH_GS))
+    return vcycle_launches(h, fp64);
   if (!h->vcg) h->vcg = new VcCache();
   VcCache* c = (VcCache*)h->vcg;
-  if (c->broken) return vcycle_mixed_launches(h);
-  const std::vector<uint64_t> key = vc_key(h);
+  if (c->broken) return vcycle_launches(h, fp64);
+  const std::vector<uint64_t> key = vc_key(h, true, fp64);
   for (auto& g : c->graphs)
     if (g.key == key) {
       if (g.unread) {  // its events still hold the previous replay's times
@@ -340,7 +357,7 @@ rso_status vcycle_mixed(rso_handle* h) {
   if (!seen) {
     if (c->seen.size() >= kMaxSeen) c->seen.erase(c->seen.begin());
     c->seen.push_back(key);
-    return vcycle_mixed_launches(h);
+    return vcycle_launches(h, fp64);
   }
   // capture: the launches are recorded, not run; the graph then runs once
   const std::vector<uint64_t> before = vc_rotating(h);
@@ -353,7 +370,7 @@ rso_status vcycle_mixed(rso_handle* h) {
   if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     st = RSO_ERR_CUDA;
   } else {
-    st = vcycle_mixed_launches(h);
+    st = vcycle_launches(h, fp64);
     if (cudaStreamEndCapture(h->stream, &graph) != cudaSuccess) st = RSO_ERR_CUDA;
   }
   h->cap_prof = nullptr;
@@ -379,7 +396,7 @@ rso_status vcycle_mixed(rso_handle* h) {
     c->broken = true;
     cudaGetLastError();
     vc_set_rotating(h, before);
-    return vcycle_mixed_launches(h);
+    return vcycle_launches(h, fp64);
   }
   g.after = vc_rotating(h);
   // the captured launches were counted when they were recorded
@@ -396,6 +413,8 @@ rso_status vcycle_mixed(rso_handle* h) {
   c->graphs.push_back(std::move(g));
   return launch_check(h, "vcycle graph");
 }
+rso_status vcycle_mixed(rso_handle* h) { return vcycle_replayed(h, false); }
+rso_status vcycle_double(rso_handle* h) { return vcycle_replayed(h, true); }
 
 // reliable-update PCG: x (FP64) += alpha p (FP32), and p = z + beta p in FP32
 // (DIR_ONLY: the direction update alone, x having taken the step already)
@@ -724,7 +743,7 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
       prev = node;
       // the V-cycle and the direction update
       st = add_if(h, G, &prev, hc[i], c->cs, [&]() -> rso_status {
-        RSO_TRY(vcycle_mixed_launches(h));  // r . z into s[3] from its last fine step when h->vc_zdot says so
+        RSO_TRY(vcycle_launches(h, false));  // r . z into s[3] from its last fine step when h->vc_zdot says so
         const float* z32 = l0.u32;
         if (h->vc_zdot != s + 3) RSO_TRY(dot_ff(h, r32, z32, n3, s + 3));
         k_cg_beta<<<1, 1, 0, h->stream>>>(s);

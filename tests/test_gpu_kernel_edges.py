@@ -214,3 +214,28 @@ def test_batch_on_used_memory(cuda, precision):
     U, infos = g.solve_batch(cuda.stack([f, 2 * f]), tol=1e-10)
     u, it, _, _ = g.solve(f, tol=1e-10)
     assert rel(U[0].cpu().numpy(), u.cpu().numpy()) < 1e-8 and abs(infos[0][0] - it) <= 1
+
+
+@pytest.mark.parametrize("gen,smoother", [(lambda: P.cantilever(48, 24, 24), 2), (lambda: P.ellipsoid(40, 24, 24), 1),
+                                          (lambda: P.cantilever(33, 18, 20), 0)])
+def test_fp64_vcycle_graphs_and_bottom(cuda, gen, smoother):
+    """FP64 solves: replayed V-cycles bit-identical to plain launches; with the persistent bottom kernel
+    (nine threads per node) and without, the same solution to 1e-8 and iterations within one."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = gen()
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"],
+                      Config(precision=0, smoother=smoother, poisson_ratio=0.4, n_levels=3, first_factor=2, pre=2, post=2))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    ln = g.load_nodes()
+    f = np.zeros(3 * g.nn)
+    f[2 * g.nn + ln] = np.random.default_rng(37).standard_normal(len(ln))
+    g.set_vcycle_graphs(False)
+    plain, it, _, _ = g.solve(t(f, cuda), tol=1e-9)
+    g.set_vcycle_graphs(True)
+    for _ in range(3):
+        u, k, _, _ = g.solve(t(f, cuda), tol=1e-9)
+        assert k == it and np.array_equal(u.cpu().numpy(), plain.cpu().numpy())
+    g.set_launch_shapes(4, -1)
+    u, k, _, _ = g.solve(t(f, cuda), tol=1e-9)
+    assert abs(k - it) <= 1 and rel(u.cpu().numpy(), plain.cpu().numpy()) < 1e-8
