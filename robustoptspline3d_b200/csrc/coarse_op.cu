@@ -131,6 +131,8 @@ __global__ void __launch_bounds__(C4G * 3, 3) k_coarse4(const Level L, const flo
                                                      const float* __restrict__ u, const float* __restrict__ f,
                                                      float* __restrict__ out, float omega,
                                                      const float* __restrict__ uprev, float c1) {
+  pdl_wait(u, f, out, uprev);
+  pdl_trigger();
   __shared__ float red[2][12][C4G];
   const int tg = threadIdx.x, pz = threadIdx.y;  // neighbour plane dz = pz - 1
   const long long g = blockIdx.x * (long long)C4G + tg;
@@ -340,6 +342,8 @@ __global__ void __launch_bounds__(32 * CTY * 3) k_coarse_r(const Level L, const 
                                                            const T* __restrict__ u, const T* __restrict__ f,
                                                            T* __restrict__ out, T omega,
                                                            const T* __restrict__ uprev, T c1) {
+  pdl_wait(u, f, out, uprev);
+  pdl_trigger();
   __shared__ T sres[3][CTY][32];
   const int bsys = blockIdx.z / L.nz;
   coarse_r_node<T, MODE>(L, st, u, f, out, omega, uprev, c1, blockIdx.x * 32 + threadIdx.x,
@@ -510,6 +514,8 @@ __global__ void __launch_bounds__(GSN * 9) k_coarse_gs(const Level L, const T* _
 // Weights (F - |d|) / F per axis, d in (-F, F).
 template <typename T, int F>
 __global__ void k_restrict_z(const Level Fl, int nZ, const T* __restrict__ rf, T* __restrict__ t) {
+  pdl_wait(rf, t);
+  pdl_trigger();
   const int bsys = blockIdx.z / nZ;
   const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, Z = blockIdx.z - bsys * nZ;
   if (x >= Fl.nx || y >= Fl.ny) return;
@@ -536,6 +542,8 @@ __global__ void k_restrict_z(const Level Fl, int nZ, const T* __restrict__ rf, T
 template <int F>
 __global__ void __launch_bounds__(256) k_restrict_z_v4(const Level Fl, int nZ, const float* __restrict__ rf,
                                                        float* __restrict__ t) {
+  pdl_wait(rf, t);
+  pdl_trigger();
   const long long pxy = (long long)Fl.px * Fl.py, off = 4 * (blockIdx.x * (long long)blockDim.x + threadIdx.x);
   const int Z = blockIdx.y;
   if (off >= pxy) return;
@@ -566,6 +574,8 @@ __global__ void __launch_bounds__(256) k_restrict_z_v4(const Level Fl, int nZ, c
 template <int F>
 __global__ void __launch_bounds__(256) k_restrict_y_v4(const Level Fl, const Level C, const float* __restrict__ t,
                                                        float* __restrict__ ty) {
+  pdl_wait(t, ty);
+  pdl_trigger();
   const int ng = Fl.px / 4;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x, Z = blockIdx.y;
   if (idx >= ng * C.ny) return;
@@ -593,6 +603,8 @@ __global__ void __launch_bounds__(256) k_restrict_y_v4(const Level Fl, const Lev
 }
 template <int F>
 __global__ void k_restrict_x(const Level Fl, const Level C, const float* __restrict__ ty, float* __restrict__ fc) {
+  pdl_wait(ty, fc);
+  pdl_trigger();
   const int X = blockIdx.x * 32 + threadIdx.x, Y = blockIdx.y * 8 + threadIdx.y, Z = blockIdx.z;
   if (X >= C.nx || Y >= C.ny) return;
   const long long nC = C.nidx(X, Y, Z);
@@ -615,6 +627,8 @@ __global__ void k_restrict_x(const Level Fl, const Level C, const float* __restr
 // layout k_restrict_z_v4 writes)
 template <typename T, int F, bool PAD = false>
 __global__ void k_restrict_xy(const Level Fl, const Level C, const T* __restrict__ t, T* __restrict__ fc) {
+  pdl_wait(t, fc);
+  pdl_trigger();
   const int bsys = blockIdx.z / C.nz;
   const int X = blockIdx.x * 32 + threadIdx.x, Y = blockIdx.y * 8 + threadIdx.y, Z = blockIdx.z - bsys * C.nz;
   if (X >= C.nx || Y >= C.ny) return;
@@ -651,6 +665,8 @@ __global__ void k_restrict_xy(const Level Fl, const Level C, const T* __restrict
 // x-corners from the lanes that hold them by shuffle.
 template <typename T, int F>
 __global__ void k_prolong(const Level Fl, const Level C, const T* __restrict__ uc, T* __restrict__ uf) {
+  pdl_wait(uc, uf);
+  pdl_trigger();
   const int lane = threadIdx.x;
   const int bsys = blockIdx.z / Fl.nz;
   const int x = blockIdx.x * 32 + lane, y = blockIdx.y * 8 + threadIdx.y, z = blockIdx.z - bsys * Fl.nz;
@@ -776,6 +792,8 @@ constexpr int PROW_WARPS = 8;
 template <int F>
 __global__ void __launch_bounds__(32 * PROW_WARPS) k_prolong_row(const Level Fl, const Level C,
                                                                  const float* __restrict__ uc, float* __restrict__ uf) {
+  pdl_wait(uc, uf);
+  pdl_trigger();
   extern __shared__ float sE_all[];  // [PROW_WARPS][3][C.nx + 1]
   const int lane = threadIdx.x, w = threadIdx.y;
   const int y = blockIdx.x * PROW_WARPS + w, z = blockIdx.y;
@@ -1971,8 +1989,8 @@ rso_status coarse_residual(rso_handle* h, int level, const T* u, const T* f, T* 
   if (h->prof_on) prof_begin(h, cls, (double)l.nn);
   if (node_per_thread(h, level)) {
     if (l.nb == 1 && sizeof(T) == 4 && l.NP < (1LL << 31)) {
-      k_coarse4<0><<<cdiv(l.NP / 4, C4G), dim3(C4G, 3), 0, h->stream>>>(l, (const float*)stencil_of<T>(l), (const float*)u,
-                                                               (const float*)f, (float*)r, 0.f, nullptr, 0.f);
+      launch_pdl(k_coarse4<0>, dim3(cdiv(l.NP / 4, C4G)), dim3(C4G, 3), 0, h->stream, l,
+                 (const float*)stencil_of<T>(l), (const float*)u, (const float*)f, (float*)r, 0.f, nullptr, 0.f);
     } else if (l.nb == 1) {
       k_coarse<T, 0, 1><<<chunk_grid(l, 1), dim3(32, 8), 0, h->stream>>>(l, stencil_of<T>(l), u, f, r, T(0), (const T*)nullptr, T(0));
     } else {
@@ -1982,7 +2000,8 @@ rso_status coarse_residual(rso_handle* h, int level, const T* u, const T* f, T* 
   } else if (coarse_variant(h, level) == 2) {
     k_coarse_r9<T, 0><<<dim3(cdiv(l.nx, 32), cdiv(l.ny, CTY9), l.nz * l.nb), dim3(32, CTY9, 9), 0, h->stream>>>(l, stencil_of<T>(l), u, f, r, T(0), (const T*)nullptr, T(0)); rso::note_launch();
   } else {
-    k_coarse_r<T, 0><<<dim3(cdiv(l.nx, 32), cdiv(l.ny, CTY), l.nz * l.nb), dim3(32, CTY, 3), 0, h->stream>>>(l, stencil_of<T>(l), u, f, r, T(0), (const T*)nullptr, T(0)); rso::note_launch();
+    launch_pdl(k_coarse_r<T, 0>, dim3(cdiv(l.nx, 32), cdiv(l.ny, CTY), l.nz * l.nb), dim3(32, CTY, 3), 0,
+               h->stream, l, stencil_of<T>(l), u, f, r, T(0), (const T*)nullptr, T(0)); rso::note_launch();
   }
   if (h->prof_on) prof_end(h, cls);
   return launch_check(h, "coarse_residual");
@@ -1995,9 +2014,9 @@ rso_status coarse_jacobi(rso_handle* h, int level, const T* u_in, const T* f, T*
   if (h->prof_on) prof_begin(h, cls, (double)l.nn);
   if (node_per_thread(h, level)) {
     if (l.nb == 1 && sizeof(T) == 4 && l.NP < (1LL << 31)) {
-      k_coarse4<2><<<cdiv(l.NP / 4, C4G), dim3(C4G, 3), 0, h->stream>>>(l, (const float*)stencil_of<T>(l), (const float*)u_in,
-                                                               (const float*)f, (float*)u_out, (float)omega,
-                                                               (const float*)u_prev, (float)c1);
+      launch_pdl(k_coarse4<2>, dim3(cdiv(l.NP / 4, C4G)), dim3(C4G, 3), 0, h->stream, l,
+                 (const float*)stencil_of<T>(l), (const float*)u_in, (const float*)f, (float*)u_out, (float)omega,
+                 (const float*)u_prev, (float)c1);
     } else if (l.nb == 1) {
       k_coarse<T, 2, 1><<<chunk_grid(l, 1), dim3(32, 8), 0, h->stream>>>(l, stencil_of<T>(l), u_in, f, u_out, (T)omega, u_prev, (T)c1);
     } else {
@@ -2007,7 +2026,8 @@ rso_status coarse_jacobi(rso_handle* h, int level, const T* u_in, const T* f, T*
   } else if (coarse_variant(h, level) == 2) {
     k_coarse_r9<T, 2><<<dim3(cdiv(l.nx, 32), cdiv(l.ny, CTY9), l.nz * l.nb), dim3(32, CTY9, 9), 0, h->stream>>>(l, stencil_of<T>(l), u_in, f, u_out, (T)omega, u_prev, (T)c1); rso::note_launch();
   } else {
-    k_coarse_r<T, 2><<<dim3(cdiv(l.nx, 32), cdiv(l.ny, CTY), l.nz * l.nb), dim3(32, CTY, 3), 0, h->stream>>>(l, stencil_of<T>(l), u_in, f, u_out, (T)omega, u_prev, (T)c1); rso::note_launch();
+    launch_pdl(k_coarse_r<T, 2>, dim3(cdiv(l.nx, 32), cdiv(l.ny, CTY), l.nz * l.nb), dim3(32, CTY, 3), 0,
+               h->stream, l, stencil_of<T>(l), u_in, f, u_out, (T)omega, u_prev, (T)c1); rso::note_launch();
   }
   if (h->prof_on) prof_end(h, cls);
   return launch_check(h, "coarse_jacobi");
@@ -2020,8 +2040,8 @@ rso_status coarse_gs(rso_handle* h, int level, T* u, const T* f, int colour, int
   const long long ntot = (long long)nxc * nyc * nzc;  // 243 NP stencil entries are allocated: far below 2^31 nodes
   if (ntot == 0) return RSO_OK;
   if (h->prof_on) prof_begin(h, (sizeof(T) == 4 ? PC_COARSE32 : PC_COARSE64), (double)l.nn / 8);
-  launch_pdl(k_coarse_gs<T>, dim3(cdiv(ntot, GSN)), dim3(GSN, 9), 0, h->stream, l, stencil_of<T>(l), u, f, cx, cy, cz,
-             nxc, nyc, (int)ntot, reverse);
+  launch_pdl(k_coarse_gs<T>, dim3(cdiv(ntot, GSN)), dim3(GSN, 9), 0, h->stream, l, stencil_of<T>(l), u, f, cx, cy,
+             cz, nxc, nyc, (int)ntot, reverse);
   rso::note_launch();
   if (h->prof_on) prof_end(h, (sizeof(T) == 4 ? PC_COARSE32 : PC_COARSE64));
   return launch_check(h, "coarse_gs");
@@ -2048,30 +2068,30 @@ rso_status restrict_(rso_handle* h, int cl, const T* rf, T* fc) {
     const dim3 gy((unsigned)cdiv((long long)(f.px / 4) * c.ny, 256), c.nz);
     const dim3 gx(cdiv(c.nx, 32), cdiv(c.ny, 8), c.nz);
     if (c.factor == 4) {
-      k_restrict_z_v4<4><<<g4, 256, 0, h->stream>>>(f, c.nz, (const float*)rf, t4); rso::note_launch();
+      launch_pdl(k_restrict_z_v4<4>, g4, dim3(256), 0, h->stream, f, c.nz, (const float*)rf, t4); rso::note_launch();
       if (ty) {
-        k_restrict_y_v4<4><<<gy, 256, 0, h->stream>>>(f, c, t4, ty); rso::note_launch();
-        k_restrict_x<4><<<gx, dim3(32, 8), 0, h->stream>>>(f, c, ty, (float*)fc); rso::note_launch();
+        launch_pdl(k_restrict_y_v4<4>, gy, dim3(256), 0, h->stream, f, c, t4, ty); rso::note_launch();
+        launch_pdl(k_restrict_x<4>, gx, dim3(32, 8), 0, h->stream, f, c, ty, (float*)fc); rso::note_launch();
       } else {
-        k_restrict_xy<float, 4, true><<<node_grid(c), dim3(32, 8), 0, h->stream>>>(f, c, t4, (float*)fc); rso::note_launch();
+        launch_pdl(k_restrict_xy<float, 4, true>, node_grid(c), dim3(32, 8), 0, h->stream, f, c, t4, (float*)fc); rso::note_launch();
       }
     } else {
-      k_restrict_z_v4<2><<<g4, 256, 0, h->stream>>>(f, c.nz, (const float*)rf, t4); rso::note_launch();
+      launch_pdl(k_restrict_z_v4<2>, g4, dim3(256), 0, h->stream, f, c.nz, (const float*)rf, t4); rso::note_launch();
       if (ty) {
-        k_restrict_y_v4<2><<<gy, 256, 0, h->stream>>>(f, c, t4, ty); rso::note_launch();
-        k_restrict_x<2><<<gx, dim3(32, 8), 0, h->stream>>>(f, c, ty, (float*)fc); rso::note_launch();
+        launch_pdl(k_restrict_y_v4<2>, gy, dim3(256), 0, h->stream, f, c, t4, ty); rso::note_launch();
+        launch_pdl(k_restrict_x<2>, gx, dim3(32, 8), 0, h->stream, f, c, ty, (float*)fc); rso::note_launch();
       } else {
-        k_restrict_xy<float, 2, true><<<node_grid(c), dim3(32, 8), 0, h->stream>>>(f, c, t4, (float*)fc); rso::note_launch();
+        launch_pdl(k_restrict_xy<float, 2, true>, node_grid(c), dim3(32, 8), 0, h->stream, f, c, t4, (float*)fc); rso::note_launch();
       }
     }
     return launch_check(h, "restrict");
   }
   if (c.factor == 4) {
-    k_restrict_z<T, 4><<<gz, dim3(32, 8), 0, h->stream>>>(f, c.nz, rf, t); rso::note_launch();
-    k_restrict_xy<T, 4><<<node_grid(c), dim3(32, 8), 0, h->stream>>>(f, c, t, fc); rso::note_launch();
+    launch_pdl(k_restrict_z<T, 4>, gz, dim3(32, 8), 0, h->stream, f, c.nz, rf, t); rso::note_launch();
+    launch_pdl(k_restrict_xy<T, 4>, node_grid(c), dim3(32, 8), 0, h->stream, f, c, t, fc); rso::note_launch();
   } else if (c.factor == 2) {
-    k_restrict_z<T, 2><<<gz, dim3(32, 8), 0, h->stream>>>(f, c.nz, rf, t); rso::note_launch();
-    k_restrict_xy<T, 2><<<node_grid(c), dim3(32, 8), 0, h->stream>>>(f, c, t, fc); rso::note_launch();
+    launch_pdl(k_restrict_z<T, 2>, gz, dim3(32, 8), 0, h->stream, f, c.nz, rf, t); rso::note_launch();
+    launch_pdl(k_restrict_xy<T, 2>, node_grid(c), dim3(32, 8), 0, h->stream, f, c, t, fc); rso::note_launch();
   } else {
     h->err = "coarsening factor must be 2 or 4";
     return RSO_ERR_UNSUPPORTED;
@@ -2086,9 +2106,9 @@ rso_status prolong(rso_handle* h, int cl, const T* uc, T* uf) {
   if (sizeof(T) == 4 && f.nb == 1 && (c.factor == 4 || c.factor == 2) && row_smem <= 48 * 1024) {
     const dim3 g((unsigned)cdiv(f.ny, PROW_WARPS), f.nz);
     if (c.factor == 4)
-      k_prolong_row<4><<<g, dim3(32, PROW_WARPS), row_smem, h->stream>>>(f, c, (const float*)uc, (float*)uf);
+      launch_pdl(k_prolong_row<4>, g, dim3(32, PROW_WARPS), row_smem, h->stream, f, c, (const float*)uc, (float*)uf);
     else
-      k_prolong_row<2><<<g, dim3(32, PROW_WARPS), row_smem, h->stream>>>(f, c, (const float*)uc, (float*)uf);
+      launch_pdl(k_prolong_row<2>, g, dim3(32, PROW_WARPS), row_smem, h->stream, f, c, (const float*)uc, (float*)uf);
     rso::note_launch();
   } else if (sizeof(T) == 4 && f.nb == 1 && (c.factor == 4 || c.factor == 2)) {
     const unsigned nblk = (unsigned)cdiv(f.NP / 4, 256);
@@ -2098,9 +2118,9 @@ rso_status prolong(rso_handle* h, int cl, const T* uc, T* uf) {
       k_prolong_v4<2><<<nblk, 256, 0, h->stream>>>(f, c, (const float*)uc, (float*)uf);
     rso::note_launch();
   } else if (c.factor == 4) {
-    k_prolong<T, 4><<<node_grid(f), dim3(32, 8), 0, h->stream>>>(f, c, uc, uf); rso::note_launch();
+    launch_pdl(k_prolong<T, 4>, node_grid(f), dim3(32, 8), 0, h->stream, f, c, uc, uf); rso::note_launch();
   } else if (c.factor == 2) {
-    k_prolong<T, 2><<<node_grid(f), dim3(32, 8), 0, h->stream>>>(f, c, uc, uf); rso::note_launch();
+    launch_pdl(k_prolong<T, 2>, node_grid(f), dim3(32, 8), 0, h->stream, f, c, uc, uf); rso::note_launch();
   } else {
     h->err = "coarsening factor must be 2 or 4";
     return RSO_ERR_UNSUPPORTED;

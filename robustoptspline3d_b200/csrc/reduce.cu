@@ -37,6 +37,8 @@ __device__ __forceinline__ double block_sum(double v) {
 
 __global__ void __launch_bounds__(RED_THREADS) k_dot_partial(const double* __restrict__ a, const double* __restrict__ b,
                                                              long long n, double* __restrict__ part) {
+  pdl_wait(a, b);
+  pdl_trigger();
   double s = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     s += a[i] * b[i];
@@ -54,6 +56,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_sumf_partial(const float* __res
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_final(const double* __restrict__ part, int np, double* out) {
+  pdl_wait(part);
+  pdl_trigger();
   double s = 0;
   for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
   s = block_sum(s);
@@ -61,8 +65,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_final(const double* __restrict_
 }
 
 rso_status dot(rso_handle* h, const double* a, const double* b, long long n, double* dev_out) {
-  k_dot_partial<<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(a, b, n, h->red); rso::note_launch();
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(h->red, RED_BLOCKS, dev_out); rso::note_launch();
+  launch_pdl(k_dot_partial, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, a, b, n, h->red); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, dev_out); rso::note_launch();
   return launch_check(h, "dot");
 }
 
@@ -72,6 +76,8 @@ rso_status dot(rso_handle* h, const double* a, const double* b, long long n, dou
 __global__ void __launch_bounds__(RED_THREADS) k_cg_resid_rr(long long n, const double* __restrict__ alpha,
                                                              const double* __restrict__ q, double* __restrict__ r,
                                                              float* __restrict__ r32, double* __restrict__ part) {
+  pdl_wait(alpha, q, r);
+  pdl_trigger();
   const double a = *alpha;
   double s = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -97,8 +103,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_dot_df_partial(const double* __
 
 rso_status cg_resid_rr(rso_handle* h, long long n, const double* alpha, const double* q, double* r, float* r32,
                        double* rr_dev) {
-  k_cg_resid_rr<<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(n, alpha, q, r, r32, h->red); rso::note_launch();
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(h->red, RED_BLOCKS, rr_dev); rso::note_launch();
+  launch_pdl(k_cg_resid_rr, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, n, alpha, q, r, r32, h->red); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, rr_dev); rso::note_launch();
   return launch_check(h, "cg_resid_rr");
 }
 
@@ -108,6 +114,8 @@ rso_status cg_resid_rr(rso_handle* h, long long n, const double* alpha, const do
 __global__ void __launch_bounds__(RED_THREADS) k_cg32_resid_rr(long long n4, const double* __restrict__ alpha,
                                                                const float4* __restrict__ q, float4* __restrict__ r,
                                                                double* __restrict__ part) {
+  pdl_wait(alpha, q, r);
+  pdl_trigger();
   const float a = (float)*alpha;
   double s = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
@@ -141,10 +149,10 @@ rso_status cg32_resid_rr(rso_handle* h, long long n, const double* alpha, const 
     h->err = "cg32_resid_rr: vectors must be 16-byte aligned multiples of 4 entries";
     return RSO_ERR_STATE;
   }
-  k_cg32_resid_rr<<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(n / 4, alpha, reinterpret_cast<const float4*>(q),
-                                                              reinterpret_cast<float4*>(r), h->red);
+  launch_pdl(k_cg32_resid_rr, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, n / 4, alpha,
+             reinterpret_cast<const float4*>(q), reinterpret_cast<float4*>(r), h->red);
   rso::note_launch();
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(h->red, RED_BLOCKS, rr_dev); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, rr_dev); rso::note_launch();
   return launch_check(h, "cg32_resid_rr");
 }
 
@@ -156,13 +164,15 @@ rso_status dot_ff(rso_handle* h, const float* a, const float* b, long long n, do
   k_dot_ff_partial<<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(reinterpret_cast<const float4*>(a),
                                                                reinterpret_cast<const float4*>(b), n / 4, h->red);
   rso::note_launch();
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(h->red, RED_BLOCKS, dev_out); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, dev_out); rso::note_launch();
   return launch_check(h, "dot_ff");
 }
 
 // one sum per system: out[b * stride] = sum of part[b * nper .. (b + 1) * nper)
 __global__ void __launch_bounds__(RED_THREADS) k_final_batch(const double* __restrict__ part, int nper,
                                                              double* __restrict__ out, int stride) {
+  pdl_wait(part);
+  pdl_trigger();
   const double* p = part + (long long)blockIdx.x * nper;
   double s = 0;
   for (int i = threadIdx.x; i < nper; i += blockDim.x) s += p[i];
@@ -171,12 +181,12 @@ __global__ void __launch_bounds__(RED_THREADS) k_final_batch(const double* __res
 }
 
 rso_status reduce_partials_batch(rso_handle* h, const double* part, int nper, int nb, double* dev_out, int stride) {
-  k_final_batch<<<nb, RED_THREADS, 0, h->stream>>>(part, nper, dev_out, stride); rso::note_launch();
+  launch_pdl(k_final_batch, dim3(nb), dim3(RED_THREADS), 0, h->stream, part, nper, dev_out, stride); rso::note_launch();
   return launch_check(h, "reduce_partials_batch");
 }
 
 rso_status reduce_partials(rso_handle* h, const double* part, int n, double* dev_out) {
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(part, n, dev_out); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, part, n, dev_out); rso::note_launch();
   return launch_check(h, "reduce_partials");
 }
 
@@ -202,7 +212,7 @@ rso_status norms2(rso_handle* h, long long n, const float* u, const float* r, do
 
 rso_status dot_df(rso_handle* h, const double* a, const float* b, long long n, double* dev_out) {
   k_dot_df_partial<<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(a, b, n, h->red); rso::note_launch();
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(h->red, RED_BLOCKS, dev_out); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, dev_out); rso::note_launch();
   return launch_check(h, "dot_df");
 }
 
@@ -216,7 +226,7 @@ rso_status dot_host(rso_handle* h, const double* a, const double* b, long long n
 
 rso_status sum_float(rso_handle* h, const float* a, long long n, double* dev_out) {
   k_sumf_partial<<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(a, n, h->red); rso::note_launch();
-  k_final<<<1, RED_THREADS, 0, h->stream>>>(h->red, RED_BLOCKS, dev_out); rso::note_launch();
+  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, dev_out); rso::note_launch();
   return launch_check(h, "sum_float");
 }
 

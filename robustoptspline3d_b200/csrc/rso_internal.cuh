@@ -274,7 +274,19 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 // visible.  pdl_trigger() after it lets the successor start, so at most one
 // kernel waits ahead of the running one, and everything before the running one
 // has ended.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Pointers given to pdl_wait are reloaded after it (as far as the compiler can
+// tell they change there), so that no load through them moves ahead of the wait,
+// not even one of read-only data.
+template <typename P>
+__device__ __forceinline__ void pdl_reload(P& p) {
+  static_assert(sizeof(P) == 8, "a pointer");
+  asm volatile("" : "+l"(p)::"memory");
+}
+template <typename... P>
+__device__ __forceinline__ void pdl_wait(P&... p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (pdl_reload(p), ...);
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
 inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {

@@ -189,8 +189,14 @@ rso_status precondition(rso_handle* h, const double* r, double* z) {
 }
 
 // scalar updates on the device: s[0]=rz, s[1]=pq, s[2]=alpha, s[3]=rz_new, s[4]=beta
-__global__ void k_cg_alpha(double* s) { s[2] = s[0] / s[1]; }
+__global__ void k_cg_alpha(double* s) {
+  pdl_wait(s);
+  pdl_trigger();
+  s[2] = s[0] / s[1];
+}
 __global__ void k_cg_beta(double* s) {
+  pdl_wait(s);
+  pdl_trigger();
   s[4] = s[3] / s[0];
   s[0] = s[3];
 }
@@ -199,6 +205,8 @@ __global__ void k_cg_beta(double* s) {
 template <typename Z>
 __global__ void k_cg_step_dir(long long n, const double* __restrict__ alpha, const double* __restrict__ beta,
                               const Z* __restrict__ z, double* __restrict__ p, double* __restrict__ x) {
+  pdl_wait(alpha, beta, z, p, x);
+  pdl_trigger();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double pi = p[i];
@@ -462,6 +470,8 @@ struct StepRing {
 };
 __global__ void k_cg32_flush(long long n4, const double* __restrict__ alpha, const StepRing R, int k,
                              double2* __restrict__ x) {
+  pdl_wait(alpha, x);
+  pdl_trigger();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n4) return;
   double2 x0 = x[2 * i], x1 = x[2 * i + 1];
@@ -482,6 +492,8 @@ __global__ void k_cg32_flush(long long n4, const double* __restrict__ alpha, con
 // p_out may be p_in
 __global__ void k_cg32_dir(long long n4, const double* __restrict__ beta, const float4* __restrict__ z,
                            const float4* p_in, float4* p_out) {
+  pdl_wait(beta, z, p_in);
+  pdl_trigger();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const float4 pi = p_in[i], zi = z[i];
@@ -490,6 +502,8 @@ __global__ void k_cg32_dir(long long n4, const double* __restrict__ beta, const 
 }
 // alpha = rz / pq, also kept for the deferred step
 __global__ void k_cg_alpha_keep(double* s, double* keep) {
+  pdl_wait(s);
+  pdl_trigger();
   s[2] = s[0] / s[1];
   *keep = s[2];
 }
@@ -724,7 +738,7 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
       long long k1 = 0, kr = 0, kc = 0;
       st = add_if(h, G, prev ? &prev : nullptr, go.go[i], c->cs, [&]() -> rso_status {
         RSO_TRY(fine_applyK_dot32(h, p32, q32, s + 1));
-        k_cg_alpha<<<1, 1, 0, h->stream>>>(s);
+        launch_pdl(k_cg_alpha, dim3(1), dim3(1), 0, h->stream, s);
         RSO_TRY(cg32_resid_rr(h, n3, s + 2, q32, r32, s + 5));
         k_pcg_ctl_a<<<1, 1, 0, h->stream>>>(ctl, s, go, i, hr[i], hc[i]);
         return launch_check(h, "pcg graph");
@@ -746,7 +760,7 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
         RSO_TRY(vcycle_launches(h, false));  // r . z into s[3] from its last fine step when h->vc_zdot says so
         const float* z32 = l0.u32;
         if (h->vc_zdot != s + 3) RSO_TRY(dot_ff(h, r32, z32, n3, s + 3));
-        k_cg_beta<<<1, 1, 0, h->stream>>>(s);
+        launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s);
         k_cg32_step_dir_ctl<<<cdiv(n4, 256), 256, 0, h->stream>>>(
             n4, s + 2, s + 4, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(p32),
             reinterpret_cast<double2*>(x), ctl);
@@ -911,7 +925,8 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
       if (pend == 0) return RSO_OK;
       StepRing R;
       for (int j = 0; j < kStepRing; j++) R.p[j] = reinterpret_cast<const float4*>(ring[j < pend ? j : 0]);
-      k_cg32_flush<<<cdiv(n4, 256), 256, 0, h->stream>>>(n4, ring_alpha, R, pend, reinterpret_cast<double2*>(x));
+      launch_pdl(k_cg32_flush, dim3(cdiv(n4, 256)), dim3(256), 0, h->stream, n4, ring_alpha, R, pend,
+                 reinterpret_cast<double2*>(x));
       rso::note_launch();
       pend = 0;
       return launch_check(h, "pcg32 deferred steps");
@@ -919,10 +934,10 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
     while (it < max_iter) {
       RSO_TRY(fine_applyK_dot32(h, pc, q32, s + 1));
       if (defer) {
-        k_cg_alpha_keep<<<1, 1, 0, h->stream>>>(s, ring_alpha + pend); rso::note_launch();
+        launch_pdl(k_cg_alpha_keep, dim3(1), dim3(1), 0, h->stream, s, ring_alpha + pend); rso::note_launch();
         pend++;
       } else {
-        k_cg_alpha<<<1, 1, 0, h->stream>>>(s); rso::note_launch();
+        launch_pdl(k_cg_alpha, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
       }
       RSO_TRY(cg32_resid_rr(h, n3, s + 2, q32, r32, s + 5));
       RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 5, s + 5, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -961,13 +976,13 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
       RSO_TRY(vcycle_mixed(h));
       const float* z32 = l0.u32;
       if (!fuse) RSO_TRY(dot_ff(h, r32, z32, n3, s + 3));
-      k_cg_beta<<<1, 1, 0, h->stream>>>(s); rso::note_launch();
+      launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
       if (defer) {
         if (pend == kStepRing) RSO_TRY(flush());
         float* pn = ring[pend];  // pc itself right after a flush of one step
-        k_cg32_dir<<<cdiv(n4, 256), 256, 0, h->stream>>>(n4, s + 4, reinterpret_cast<const float4*>(z32),
-                                                         reinterpret_cast<const float4*>(pc),
-                                                         reinterpret_cast<float4*>(pn));
+        launch_pdl(k_cg32_dir, dim3(cdiv(n4, 256)), dim3(256), 0, h->stream, n4, s + 4,
+                   reinterpret_cast<const float4*>(z32), reinterpret_cast<const float4*>(pc),
+                   reinterpret_cast<float4*>(pn));
         pc = pn;
       } else if (replace) {
         k_cg32_step_dir<true><<<cdiv(n4, 256), 256, 0, h->stream>>>(
@@ -1035,7 +1050,7 @@ rso_status solve_pcg(rso_handle* h, const double* f, double* x, double tol, int 
     }
     while (it < max_iter) {
       RSO_TRY(fine_applyK_dot(h, h->p, h->q, h->rp64, s + 1));
-      k_cg_alpha<<<1, 1, 0, h->stream>>>(s); rso::note_launch();
+      launch_pdl(k_cg_alpha, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
       RSO_TRY(cg_resid_rr(h, n3, s + 2, h->q, h->r, mixed ? h->L[0].f32 : nullptr, s + 5));
       RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 5, s + 5, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
       RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -1051,13 +1066,15 @@ rso_status solve_pcg(rso_handle* h, const double* f, double* x, double tol, int 
       if (mixed) {
         RSO_TRY(vcycle_mixed(h));
         RSO_TRY(dot_df(h, h->r, h->L[0].u32, n3, s + 3));
-        k_cg_beta<<<1, 1, 0, h->stream>>>(s); rso::note_launch();
-        k_cg_step_dir<float><<<cdiv(n3, 256), 256, 0, h->stream>>>(n3, s + 2, s + 4, h->L[0].u32, h->p, x); rso::note_launch();
+        launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
+        launch_pdl(k_cg_step_dir<float>, dim3(cdiv(n3, 256)), dim3(256), 0, h->stream, n3, s + 2, s + 4,
+                   h->L[0].u32, h->p, x); rso::note_launch();
       } else {
         RSO_TRY(precondition(h, h->r, h->z));
         RSO_TRY(dot(h, h->r, h->z, n3, s + 3));
-        k_cg_beta<<<1, 1, 0, h->stream>>>(s); rso::note_launch();
-        k_cg_step_dir<double><<<cdiv(n3, 256), 256, 0, h->stream>>>(n3, s + 2, s + 4, h->z, h->p, x); rso::note_launch();
+        launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
+        launch_pdl(k_cg_step_dir<double>, dim3(cdiv(n3, 256)), dim3(256), 0, h->stream, n3, s + 2, s + 4, h->z,
+                   h->p, x); rso::note_launch();
       }
       RSO_TRY(launch_check(h, "pcg"));
     }
