@@ -593,11 +593,12 @@ constexpr int pair_slot() { return pair_rho_off<TYP>() + (36 * 2 * TYP + 31) / 3
 // it takes 8 slots rather than 6 so that slot indices and phases are a mask
 // and a shift of the stage number, not a division by 6
 constexpr int pair_slots(int mode, bool tma) { return mode == 2 && tma ? 2 * WNSLOT : WNSLOT; }
+constexpr int pair_xvals(int mode) { return mode == 2 ? 4 : 1; }  // exchanged values per component
 template <int TYP>
-constexpr int pair_smem_bytes(int nslot) {
-  // slots + corner exchange [2][4 values][3 comps][32 TYP] + 128 bytes to
-  // round the base up to a 128-byte boundary
-  return 4 * (nslot * pair_slot<TYP>() + 2 * 12 * 32 * TYP) + 128;
+constexpr int pair_smem_bytes(int mode, int nslot) {
+  // slots + corner exchange [2][values][3 comps][32 TYP] + 128 bytes to round
+  // the base up to a 128-byte boundary
+  return 4 * (nslot * pair_slot<TYP>() + 2 * pair_xvals(mode) * 3 * 32 * TYP) + 128;
 }
 
 // resident CTAs per SM (for 4 thread rows) the register budget is cut for:
@@ -621,6 +622,12 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
   constexpr int NS = pair_slots(MODE, TMA);
   static_assert((NS & (NS - 1)) == 0, "slot indices are masks of the stage number");
   constexpr bool LEAN = MODE == 2 && TMA;  // operands of the emitted plane re-read from the slots
+  // Corner exchange: the right neighbour's corners by shuffle, one value per
+  // component through shared memory to the thread row below (residual and K u:
+  // 223 -> 215 us at 256^3); the step, at its register limit, leaves all four
+  // values there (285 us; 311 with shuffles, which spill).
+  constexpr bool SHFL = MODE != 2;
+  constexpr int XV = pair_xvals(MODE);
   constexpr int RHO = pair_rho_off<TYP>(), SLOT = pair_slot<TYP>();
   constexpr uint32_t STAGE_BYTES = sizeof(float) * (3 * NPL + RX * ROWS);  // both boxes of a stage
   constexpr int CPR = RX / 4;  // 16-byte chunks per staged row
@@ -628,7 +635,7 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
   extern __shared__ __align__(128) unsigned char smem_pair[];
   // slots start on a 128-byte shared-memory address whatever the base
   float* ss = reinterpret_cast<float*>(smem_pair + ((128u - (smem_u32(smem_pair) & 127u)) & 127u));  // [NS][SLOT]
-  float* sx = ss + NS * SLOT;                  // [2][4][3][NT] corner exchange, by plane parity
+  float* sx = ss + NS * SLOT;                  // [2][XV][3][NT] corner exchange, by plane parity
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * WTX + tx;
   const int x0 = blockIdx.x * (WTX - 1), y0 = blockIdx.y * (ROWS - 1);
   // blockIdx.z = z chunk of fzc node planes + (number of chunks) * system
@@ -644,6 +651,15 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
   const int ex = x0 - 1 + tx, ey = y0 - 1 + 2 * ty;
   const int NP = (int)L.NP, px = L.px;  // 3 NP < 2^31 (checked by the launcher)
   const int nb0 = (ex + 2) + px * (ey + 2), pxy32 = px * L.py;  // node (ex + 1, ey + 1, z) at nb0 + pxy32 (z + 1)
+  // a component plane's base is the same for all threads, and a node's byte
+  // offset in it fits 32 bits: one offset serves every vector and component
+  // (256^3: step 295 -> 285 us, residual 229 -> 223 us against 64-bit indices)
+  auto rd = [&](const float* v, int c, unsigned o) {
+    return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(v + (size_t)c * NP) + o);
+  };
+  auto wr = [&](float* v, int c, unsigned o, float x) {
+    *reinterpret_cast<float*>(reinterpret_cast<char*>(v + (size_t)c * NP) + o) = x;
+  };
   const int xs = x0 & ~3, ox = x0 - xs;
 
   int goff[TMA ? 1 : KC], soff[TMA ? 1 : KC];
@@ -744,6 +760,11 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
   }
   const bool wA = tx < WTX - 1 && ex + 1 < L.nx && ey + 1 < L.ny;
   const bool wB = wA && ty < TYP - 1 && ey + 2 < L.ny;
+  // to the node above in y; a thread without a column B reads its own node again
+  // (its B lane's results are never stored), the step, short of a register for
+  // that, not at all
+  const unsigned ob = MODE == 2 || wB ? 4u * (unsigned)px : 0u;
+  auto rdB = [&](const float* v, int c, unsigned o) { return MODE != 2 || wB ? rd(v, c, o + ob) : 0.f; };
   const float2 zero2 = make_float2(0.f, 0.f);
   float2 F[4][3], Gt[4][3], uc[3], uo[3], own[3], fo[3], po[3], ra[4], rb[4];
   uint8_t clA = 0, clB = 0;
@@ -763,12 +784,17 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
     float2 acc[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      acc[c] = p_add(own[c], make_float2(xb[(0 * 3 + c) * NT + tid + 1], xb[(1 * 3 + c) * NT + tid + 1]));
-      if (wB) acc[c].y += xb[(2 * 3 + c) * NT + tid + WTX] + xb[(3 * 3 + c) * NT + tid + WTX + 1];
+      if constexpr (SHFL) {  // own holds the right neighbour's share already
+        acc[c] = own[c];
+        if (wB) acc[c].y += xb[c * NT + tid + WTX];
+      } else {
+        acc[c] = p_add(own[c], make_float2(xb[(0 * 3 + c) * NT + tid + 1], xb[(1 * 3 + c) * NT + tid + 1]));
+        if (wB) acc[c].y += xb[(2 * 3 + c) * NT + tid + WTX] + xb[(3 * 3 + c) * NT + tid + WTX + 1];
+      }
     }
-    const int n = nb0 + pxy32 * (zo + 1);  // L.nidx(ex + 1, ey + 1, zo) in 32 bits
-    const bool workA = (clA & NC_ACTIVE) && !(clA & NC_SUPPORT);
-    const bool workB = (clB & NC_ACTIVE) && !(clB & NC_SUPPORT);
+    const unsigned n = 4u * (unsigned)(nb0 + pxy32 * (zo + 1));  // byte offset of node (ex + 1, ey + 1, zo)
+    const bool workA = (clA & (NC_ACTIVE | NC_SUPPORT)) == NC_ACTIVE;
+    const bool workB = (clB & (NC_ACTIVE | NC_SUPPORT)) == NC_ACTIVE;
     float2 res[3];
     if (MODE == 0) {
 #pragma unroll
@@ -796,6 +822,7 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
         for (int c = 0; c < 3; c++) uo[c] = make_float2(pu[c * NPL + RX + 1], pu[c * NPL + 2 * RX + 1]);
         ra[0] = make_float2(pa[0], pa[RX]);
         ra[1] = make_float2(pa[1], pa[RX + 1]);
+        // the last thread row has no column B, and its layer no row for one
         ra[2] = make_float2(pa[RX], wB ? pa[2 * RX] : 0.f);
         ra[3] = make_float2(pa[RX + 1], wB ? pa[2 * RX + 1] : 0.f);
         rb[0] = make_float2(pb[0], pb[RX]);
@@ -838,8 +865,8 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      out[n + c * NP] = res[c].x;
-      if (wB) out[n + px + c * NP] = res[c].y;
+      wr(out, c, n, res[c].x);
+      if (wB) wr(out, c, n + ob, res[c].y);
     }
   };
 
@@ -855,17 +882,17 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
       __syncthreads();
       issue(z + 1 + WPD);
     }
-    if (z - 1 >= z0) emit(z - 1, sx + ((z - 1) & 1) * 12 * NT);
+    if (z - 1 >= z0) emit(z - 1, sx + ((z - 1) & 1) * XV * 3 * NT);
     if (wA && z >= z0) {
-      const int n = nb0 + pxy32 * (z + 1);
-      clA = L.vclass[n];
-      if (wB) clB = L.vclass[n + px];
+      const unsigned m = (unsigned)(nb0 + pxy32 * (z + 1)), n = 4u * m;
+      clA = L.vclass[m];
+      if (MODE != 2 || wB) clB = L.vclass[m + ob / 4u];
       if (MODE != 1) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) fo[c] = make_float2(f[n + c * NP], wB ? f[n + px + c * NP] : 0.f);
+        for (int c = 0; c < 3; c++) fo[c] = make_float2(rd(f, c, n), rdB(f, c, n));
         if (MODE == 2 && uprev != nullptr) {
 #pragma unroll
-          for (int c = 0; c < 3; c++) po[c] = make_float2(uprev[n + c * NP], wB ? uprev[n + px + c * NP] : 0.f);
+          for (int c = 0; c < 3; c++) po[c] = make_float2(rd(uprev, c, n), rdB(uprev, c, n));
         }
       }
     }
@@ -958,17 +985,25 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
         Gt[q][c] = p_add(v[q][c], v[q + 4][c]);
       }
     if (z >= z0) {
-      float* xb = sx + (z & 1) * 12 * NT;
+      float* xb = sx + (z & 1) * XV * 3 * NT;
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const float2 e0 = p_sub(tot[0][c], tot[1][c]), e1 = p_add(tot[0][c], tot[1][c]);
         const float2 g0 = p_sub(tot[2][c], tot[3][c]), g1 = p_add(tot[2][c], tot[3][c]);
         const float2 c00 = p_sub(e0, g0), c10 = p_sub(e1, g1), c01 = p_add(e0, g0), c11 = p_add(e1, g1);
-        xb[(0 * 3 + c) * NT + tid] = c01.x + c00.y;  // A (0,1) + B (0,0): node (ex, ey + 1)
-        xb[(1 * 3 + c) * NT + tid] = c01.y;          // B (0,1): node (ex, ey + 2)
-        xb[(2 * 3 + c) * NT + tid] = c10.x;          // A (1,0): node (ex + 1, ey)
-        xb[(3 * 3 + c) * NT + tid] = c00.x;          // A (0,0): node (ex, ey)
         own[c] = make_float2(c11.x + c10.y, c11.y);  // nodes (ex + 1, ey + 1), (ex + 1, ey + 2)
+        const float sA = c01.x + c00.y;  // A (0,1) + B (0,0): node (ex, ey + 1)
+        if constexpr (SHFL) {
+          const float rA = __shfl_down_sync(0xffffffffu, sA, 1), rB = __shfl_down_sync(0xffffffffu, c01.y, 1);
+          const float r0 = __shfl_down_sync(0xffffffffu, c00.x, 1);
+          own[c] = p_add(own[c], make_float2(rA, rB));
+          xb[c * NT + tid] = c10.x + r0;         // A (1,0) and the right neighbour's A (0,0): node (ex + 1, ey)
+        } else {
+          xb[(0 * 3 + c) * NT + tid] = sA;
+          xb[(1 * 3 + c) * NT + tid] = c01.y;    // B (0,1): node (ex, ey + 2)
+          xb[(2 * 3 + c) * NT + tid] = c10.x;    // A (1,0): node (ex + 1, ey)
+          xb[(3 * 3 + c) * NT + tid] = c00.x;    // A (0,0): node (ex, ey)
+        }
       }
     }
     if constexpr (!LEAN) {
@@ -980,7 +1015,7 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
     }
   }
   __syncthreads();
-  emit(z1 - 1, sx + ((z1 - 1) & 1) * 12 * NT);
+  emit(z1 - 1, sx + ((z1 - 1) & 1) * XV * 3 * NT);
   if constexpr (DOT) pq = (double)zq.x + (wB ? (double)zq.y : 0.0);
   if ((MODE == 1 || DOT) && dotp != nullptr) {
     __shared__ double sred[TYP];
@@ -1366,9 +1401,9 @@ static rso_status launch_fine(rso_handle* h, const T* u, const T* f, T* out, con
   // column per thread, staged by cp.async
   constexpr bool packed = sizeof(T) == 4;
   const int pty = fine_pty(h);
-  const int smem = packed ? (pty == 2   ? pair_smem_bytes<2>(pair_slots(MODE, kPairTMA))
-                             : pty == 8 ? pair_smem_bytes<8>(pair_slots(MODE, kPairTMA))
-                                        : pair_smem_bytes<4>(pair_slots(MODE, kPairTMA)))
+  const int smem = packed ? (pty == 2   ? pair_smem_bytes<2>(MODE, pair_slots(MODE, kPairTMA))
+                             : pty == 8 ? pair_smem_bytes<8>(MODE, pair_slots(MODE, kPairTMA))
+                                        : pair_smem_bytes<4>(MODE, pair_slots(MODE, kPairTMA)))
                           : walsh_smem_bytes<T, WTY>();
   // MODE 2 with dotp: the instantiation that also sums f . out
   const bool jdot = MODE == 2 && dotp != nullptr;

@@ -26,6 +26,24 @@ def test_fine_fp64_chunks(oracle, cuda, dims):
     assert rel(jac, o.smooth(0, u, f, kind=1, omega=0.3, sweeps=1)) < 1e-12
 
 
+# the packed FP32 kernel's tiles (31 nodes by 3, 7 or 15): one short of, on and past a tile edge in x
+# and y, where a thread's second column or its right neighbour is missing
+@pytest.mark.parametrize("rows", [2, 4, 8])
+@pytest.mark.parametrize("dims", [(6, 4, 3), (29, 13, 9), (30, 14, 10), (31, 15, 17), (33, 6, 12)])
+def test_fine_fp32_tile_edges(oracle, cuda, dims, rows):
+    """FP32 K u, residual and Chebyshev step; 2e-5 relative, the bound of the FP32 operator pieces."""
+    g, o = make(oracle, P.cantilever(*dims), n_levels=2, first_factor=2)
+    g.set_launch_shapes(fine_rows=rows)
+    rng = np.random.default_rng(9)
+    cls = o.node_class()
+    fix = np.tile(((cls & 4) > 0) | ((cls & 1) == 0), 3)
+    u, f, up = (np.where(fix, 0.0, rng.standard_normal(3 * o.nn)) for _ in range(3))
+    assert rel(g.fine_sweep_fp32(1, t(u, cuda)).cpu().numpy(), o.apply_K(u)) < 2e-5
+    assert rel(g.fine_sweep_fp32(0, t(u, cuda), t(f, cuda)).cpu().numpy(), o.residual(u, f)) < 2e-5
+    step = o.smooth(0, u, f, kind=1, omega=0.3, sweeps=1) + 0.7 * (u - up)
+    assert rel(g.fine_sweep_fp32(2, t(u, cuda), t(f, cuda), t(up, cuda), omega=0.3, c1=0.7).cpu().numpy(), step) < 2e-5
+
+
 # coarse levels of 2 to 17 nodes an edge: colours of one node, of fewer and of more than the 32 a CTA
 # takes, with a ragged last CTA; the ellipsoid leaves inactive nodes inside the box
 @pytest.mark.parametrize("gen", [lambda: P.cantilever(6, 4, 3), lambda: P.cantilever(30, 21, 13),
