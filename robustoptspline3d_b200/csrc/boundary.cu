@@ -10,18 +10,20 @@
 //  - regions and fields: the range and field classes of
 //    boundary/BoundaryCondition.h, evaluated at node positions in
 //    computeProjectionMatrix (grid/Grid.cpp:2694-2760).
-// Here each is one FP64 kernel: a block per face for the shell (an element
+// Here each is one FP64 kernel: a warp per face for the shell (an element
 // in a face's index box within w of that face is within w of the mesh, and an
 // element within w of the mesh lies in the index box of its nearest face, so
-// the union over faces is the reference's set), a thread per point for the
+// the union over faces is the reference's set), a warp per point for the
 // normals (the nearest face with the lowest index on a tie, found by a ring
 // search over a uniform face grid, or by scanning all faces of small meshes),
-// a thread per node or point for the regions and fields.  The file is compiled without
+// a warp per row of nodes or a thread per point for the regions and fields.  The file is compiled without
 // multiply-add contraction so every product and sum rounds as in the host
 // restatement the tests compare with.
 #include "rso_internal.cuh"
+#include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <numeric>
 #include <utility>
 #include <vector>
 
@@ -74,37 +76,144 @@ __device__ __forceinline__ D3 vertex(const float* __restrict__ vtx, int i) {
   return {(double)vtx[3 * i], (double)vtx[3 * i + 1], (double)vtx[3 * i + 2]};
 }
 
-// one block per face: the face's grown index box, element centres within w of it
-__global__ void k_shell(const float* __restrict__ vtx, const int* __restrict__ faces, int nf, double b0x, double b0y,
-                        double b0z, double eh, double wshell, int R, const uint8_t* __restrict__ solid,
-                        uint8_t* __restrict__ shell) {
-  const int f = blockIdx.x;
-  if (f >= nf) return;
+// Shell elements.  Every element of a byte array (rows of `pitch` bytes, a
+// multiple of 8) is 0 (void), 1 (solid) or 2 (shell).  A warp takes a face: its
+// lanes take rows of the face's grown index box, read eight elements at a time
+// and compute distances for those still 1 only, since a face need not look at
+// what another has marked (a stale 1 only costs the distance again, and every
+// store to a byte stores the same 2).  Faces about the size of an element
+// overlap in some hundred boxes, and nearly all of the FP64 work was there: one
+// CTA a face testing every solid element took 3.2 ms for 262144 faces on 256^3
+// elements, this 0.58 ms.  Faces whose box has more than kShellRows rows go to a
+// list that a second launch works off with the whole grid per face.
+constexpr int kShellRows = 2048;
+
+struct ShellGrid {
+  double b0[3], eh, w;
+  int R, pitch;
+};
+
+// the index box of a face grown by the shell's width (all lanes of the warp together); 0 rows if it is empty
+struct FaceBox {
+  D3 a, b, c;
+  double lo[3], hi[3];
+  int lid[3], rid[3];
+  double lim;  // squared distance to the face's bounding box from which an element is out
+};
+
+__device__ int face_box(const float* __restrict__ vtx, const int* __restrict__ faces, int f, const ShellGrid& G,
+                        FaceBox* B) {
   const D3 a = vertex(vtx, faces[3 * f]), b = vertex(vtx, faces[3 * f + 1]), c = vertex(vtx, faces[3 * f + 2]);
-  const double b0[3] = {b0x, b0y, b0z};
+  B->a = a, B->b = b, B->c = c;
   const double lo[3] = {fmin(fmin(a.x, b.x), c.x), fmin(fmin(a.y, b.y), c.y), fmin(fmin(a.z, b.z), c.z)};
   const double hi[3] = {fmax(fmax(a.x, b.x), c.x), fmax(fmax(a.y, b.y), c.y), fmax(fmax(a.z, b.z), c.z)};
-  int lid[3], rid[3];
-  for (int j = 0; j < 3; j++) {
-    const double ql = (lo[j] - wshell * 1.3 - b0[j] - 0.5 * eh) / eh;
-    const double qr = (hi[j] + wshell * 1.3 - b0[j] - 0.5 * eh) / eh + 1;
+  {  // lane j: the lower bound of axis j, lane 3 + j: its upper bound
+    const int lane = threadIdx.x & 31, j = lane % 3;
+    const bool up = lane >= 3;
+    const double o = j == 0 ? G.b0[0] : (j == 1 ? G.b0[1] : G.b0[2]);
+    const double l = j == 0 ? lo[0] : (j == 1 ? lo[1] : lo[2]), u = j == 0 ? hi[0] : (j == 1 ? hi[1] : hi[2]);
+    double q = ((up ? u + G.w * 1.3 : l - G.w * 1.3) - o - 0.5 * G.eh) / G.eh;
+    if (up) q += 1;
     // int conversion truncates; out-of-range quotients saturate before the clamp
-    lid[j] = (int)fmax(fmin(ql, 2147483647.0), -2147483648.0);
-    rid[j] = (int)fmax(fmin(qr, 2147483647.0), -2147483648.0);
-    lid[j] = min(max(lid[j], 0), R - 1);
-    rid[j] = min(max(rid[j], 0), R - 1);
+    const int id = min(max((int)fmax(fmin(q, 2147483647.0), -2147483648.0), 0), G.R - 1);
+    for (int k = 0; k < 3; k++) {
+      B->lid[k] = __shfl_sync(0xffffffffu, id, k);
+      B->rid[k] = __shfl_sync(0xffffffffu, id, 3 + k);
+    }
   }
-  const int nbx = rid[0] - lid[0], nby = rid[1] - lid[1], nbz = rid[2] - lid[2];
-  if (nbx <= 0 || nby <= 0 || nbz <= 0) return;
-  const double sh2 = wshell * wshell;
-  const long long nbox = (long long)nbx * nby * nbz;
-  for (long long k = threadIdx.x; k < nbox; k += blockDim.x) {
-    const int x = lid[0] + (int)(k % nbx), y = lid[1] + (int)((k / nbx) % nby), z = lid[2] + (int)(k / ((long long)nbx * nby));
-    const long long e = (long long)x + (long long)R * (y + (long long)R * z);
-    if (!solid[e]) continue;
-    const D3 p = {(x + 0.5) * eh + b0x, (y + 0.5) * eh + b0y, (z + 0.5) * eh + b0z};
-    const D3 d = sub(p, closest_on_triangle(p, a, b, c));
-    if (dot(d, d) < sh2) shell[e] = 1;
+  double m2 = 0;  // (largest distance from an element of the box to a point of the face)^2
+  for (int j = 0; j < 3; j++) {
+    B->lo[j] = lo[j], B->hi[j] = hi[j];
+    const double m = hi[j] - lo[j] + 1.3 * G.w + G.eh;
+    m2 += m * m;
+  }
+  // Elements further than w from the face's bounding box need no distance if
+  // the computed closest point lies on the face.  Rounding moves it off by at
+  // most about 80 eps L^3 M^2 / |n|^2 (L the longest edge, M the distance, n
+  // the face's normal: the barycentric sums cancel on slivers), so that is
+  // kept below w / 1000 against the hundredth of w taken as margin; slivers
+  // beyond it compute every distance.
+  const D3 ab = sub(b, a), ac = sub(c, a), bc = sub(c, b), n = cross(ab, ac);
+  const double l2 = fmax(dot(ab, ab), fmax(dot(ac, ac), dot(bc, bc)));
+  const bool fit = dot(n, n) * G.w > 1e-10 * l2 * sqrt(l2) * m2;
+  B->lim = fit ? 1.02 * G.w * G.w : INFINITY;
+  const int nbx = B->rid[0] - B->lid[0], nby = B->rid[1] - B->lid[1], nbz = B->rid[2] - B->lid[2];
+  return nbx > 0 && nby > 0 && nbz > 0 ? nby * nbz : 0;
+}
+
+__device__ __forceinline__ double outside(double x, double lo, double hi) {
+  return x < lo ? lo - x : (x > hi ? x - hi : 0.0);
+}
+
+// rows r0, r0 + step, .. of the box
+__device__ __forceinline__ void shell_rows(const FaceBox& B, const ShellGrid& G, int rows, int r0, int step,
+                                           uint8_t* state) {
+  const int nby = B.rid[1] - B.lid[1];
+  const double sh2 = G.w * G.w;
+  for (int r = r0; r < rows; r += step) {
+    const int y = B.lid[1] + r % nby, z = B.lid[2] + r / nby;
+    const double py = (y + 0.5) * G.eh + G.b0[1], pz = (z + 0.5) * G.eh + G.b0[2];
+    const double oy = outside(py, B.lo[1], B.hi[1]), oz = outside(pz, B.lo[2], B.hi[2]), ryz = oy * oy + oz * oz;
+    if (ryz > B.lim) continue;
+    uint8_t* row = state + ((size_t)z * G.R + y) * G.pitch;
+    for (int x8 = B.lid[0] & ~7; x8 < B.rid[0]; x8 += 8) {
+      unsigned long long todo =
+          __ldcg(reinterpret_cast<const unsigned long long*>(row + x8)) & 0x0101010101010101ull;
+      if (x8 < B.lid[0]) todo &= ~0ull << (8 * (B.lid[0] - x8));
+      if (x8 + 8 > B.rid[0]) todo &= ~0ull >> (8 * (x8 + 8 - B.rid[0]));
+      for (; todo != 0; todo &= todo - 1) {
+        const int x = x8 + (__ffsll((long long)todo) - 1) / 8;
+        const D3 p = {(x + 0.5) * G.eh + G.b0[0], py, pz};
+        const double ox = outside(p.x, B.lo[0], B.hi[0]);
+        if (ox * ox + ryz > B.lim) continue;
+        const D3 d = sub(p, closest_on_triangle(p, B.a, B.b, B.c));
+        if (dot(d, d) < sh2) row[x] = 2;
+      }
+    }
+  }
+}
+
+// A warp per face, in steps of `stride` (coprime to nf): neighbours in the list
+// are neighbours in space, and in list order the warps at work together would
+// all compute the distances of the same elements (1.29 ms; 0.75 ms in steps;
+// 0.58 ms with the registers cut for six CTAs an SM).  `big` = {number, faces..}
+// of those left to k_shell_big.
+__global__ void __launch_bounds__(128, 6) k_shell(const float* __restrict__ vtx, const int* __restrict__ faces, int nf,
+                                               int stride, ShellGrid G, uint8_t* state, int* __restrict__ big) {
+  const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
+  if (wid >= nf) return;
+  const long long f = wid * stride % nf;
+  FaceBox B;
+  const int rows = face_box(vtx, faces, (int)f, G, &B), lane = threadIdx.x & 31;
+  if (rows > kShellRows) {
+    if (lane == 0) big[1 + atomicAdd(big, 1)] = (int)f;
+    return;
+  }
+  shell_rows(B, G, rows, lane, 32, state);
+}
+
+// all threads of the grid on the rows of one listed face after the other
+__global__ void __launch_bounds__(128) k_shell_big(const float* __restrict__ vtx, const int* __restrict__ faces,
+                                                   ShellGrid G, uint8_t* state, const int* __restrict__ big) {
+  const int nb = big[0];
+  for (int k = 0; k < nb; k++) {
+    FaceBox B;
+    const int rows = face_box(vtx, faces, big[1 + k], G, &B);
+    shell_rows(B, G, rows, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, state);
+  }
+}
+
+// a warp per row: user's solid bytes (any non-zero is solid) to states, and states to shell bytes
+template <bool IN>
+__global__ void k_shell_bytes(uint8_t* __restrict__ user, uint8_t* __restrict__ state, int R, int pitch) {
+  const int lane = threadIdx.x & 31;
+  for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32; row < (long long)R * R;
+       row += (long long)gridDim.x * blockDim.x / 32) {
+    uint8_t *u = user + row * R, *s = state + row * pitch;
+    if (IN)
+      for (int x = lane; x < pitch; x += 32) s[x] = x < R && u[x] ? 1 : 0;
+    else
+      for (int x = lane; x < R; x += 32) u[x] = s[x] >> 1;
   }
 }
 
@@ -195,7 +304,7 @@ __device__ __forceinline__ void face_cells(const FaceGrid& G, D3 a, D3 b, D3 c, 
   }
 }
 
-// FILL false: count the faces of every cell; true: write them (cursor per cell)
+// FILL false: count the faces of every cell; true: write them (counts: the next item per cell)
 template <bool FILL>
 __global__ void k_bin_faces(const float* __restrict__ vtx, const int* __restrict__ faces, int nf, FaceGrid G,
                             int* __restrict__ counts, int* __restrict__ items) {
@@ -208,56 +317,83 @@ __global__ void k_bin_faces(const float* __restrict__ vtx, const int* __restrict
       for (int x = c0[0]; x <= c1[0]; x++) {
         const long long cell = x + (long long)G.g[0] * (y + (long long)G.g[1] * z);
         const int slot = atomicAdd(&counts[cell], 1);
-        if (FILL) items[G.start[cell] + slot] = f;
+        if (FILL) items[slot] = f;
       }
 }
 
-// one thread per point: cells in rings of growing Chebyshev radius around the
+// One warp per point: cells in rings of growing Chebyshev radius around the
 // point's cell, until no face outside the visited block can come as close as
 // the best so far (the faces that could still tie or win lie within the
 // bound); the best is the lexicographic minimum of (squared distance, face
-// index), the brute-force scan's answer
-__global__ void k_normals_grid(const float* __restrict__ vtx, const int* __restrict__ faces, FaceGrid G,
-                               const double* __restrict__ pts, int np, double* __restrict__ nrm) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// index), the brute-force scan's answer.  The cells of a row are consecutive,
+// so a ring is a list of runs of items: each lane fetches one run's bounds, and
+// all lanes share out the runs' faces.  Bound by the chain of distances of a
+// point: a thread per point ran 128 CTAs with tens of FP64 distances one after
+// the other (16384 points, 262144 faces: 1379 us), the warp takes 32 at once
+// (177 us).
+__global__ void __launch_bounds__(128) k_normals_grid(const float* __restrict__ vtx, const int* __restrict__ faces,
+                                                      FaceGrid G, const double* __restrict__ pts, int np,
+                                                      double* __restrict__ nrm) {
+  const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32), lane = threadIdx.x & 31;
   if (i >= np) return;
-  const D3 p = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
+  const D3 p = {pts[3 * (size_t)i], pts[3 * (size_t)i + 1], pts[3 * (size_t)i + 2]};
   const double pc[3] = {p.x, p.y, p.z};
   int c[3];
   for (int j = 0; j < 3; j++) c[j] = cell_of(pc[j], G.lo[j], G.cs[j], G.g[j]);
   double best = INFINITY;
-  D3 bq = p;
   int bf = 0x7fffffff;
   const int rmax = max(G.g[0], max(G.g[1], G.g[2]));
-  auto visit = [&](int x, int y, int z) {
-    const long long cell = x + (long long)G.g[0] * (y + (long long)G.g[1] * z);
-    for (int k = G.start[cell]; k < G.start[cell + 1]; k++) {
-      const int f = G.items[k];
-      const D3 a = vertex(vtx, faces[3 * f]), b = vertex(vtx, faces[3 * f + 1]), cc = vertex(vtx, faces[3 * f + 2]);
-      const D3 q = closest_on_triangle(p, a, b, cc);
-      const D3 d = sub(q, p);
-      const double d2 = dot(d, d);
-      if (d2 < best || (d2 == best && f < bf)) {
-        best = d2;
-        bq = q;
-        bf = f;
-      }
-    }
-  };
   for (int r = 0; r <= rmax; r++) {
     const int z0 = max(c[2] - r, 0), z1 = min(c[2] + r, G.g[2] - 1);
     const int y0 = max(c[1] - r, 0), y1 = min(c[1] + r, G.g[1] - 1);
     const int x0 = max(c[0] - r, 0), x1 = min(c[0] + r, G.g[0] - 1);
-    for (int z = z0; z <= z1; z++) {
-      const bool zs = z == c[2] - r || z == c[2] + r;
-      for (int y = y0; y <= y1; y++) {
-        const bool ys = zs || y == c[1] - r || y == c[1] + r;
-        if (ys) {
-          for (int x = x0; x <= x1; x++) visit(x, y, z);
-        } else {
-          if (c[0] - r >= 0) visit(c[0] - r, y, z);
-          if (r > 0 && c[0] + r < G.g[0]) visit(c[0] + r, y, z);
+    const int ny = y1 - y0 + 1, nrun = 2 * ny * (z1 - z0 + 1);
+    for (int s0 = 0; s0 < nrun; s0 += 32) {
+      // run s: row s / 2 of the block, whole on the ring's faces (s even), else its two end cells
+      int from = 0, len = 0;
+      if (s0 + lane < nrun) {
+        const int side = (s0 + lane) & 1, y = y0 + ((s0 + lane) >> 1) % ny, z = z0 + ((s0 + lane) >> 1) / ny;
+        const bool whole = z == c[2] - r || z == c[2] + r || y == c[1] - r || y == c[1] + r;
+        const int xa = whole ? x0 : (side ? c[0] + r : c[0] - r), xb = whole ? x1 : xa;
+        if ((!whole || !side) && xa >= 0 && xb < G.g[0]) {
+          const long long row = (long long)G.g[0] * (y + (long long)G.g[1] * z);
+          from = G.start[row + xa];
+          len = G.start[row + xb + 1] - from;
         }
+      }
+      int end = len;  // inclusive prefix sum: the runs laid end to end
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, end, 31);
+      for (int k0 = 0; k0 < total; k0 += 32) {
+        const int k = k0 + lane;
+        int run = 0;  // first run that ends after k
+        for (int o = 16; o > 0; o >>= 1) {
+          const int v = __shfl_sync(0xffffffffu, end, run + o - 1);
+          if (v <= k) run += o;
+        }
+        const int re = __shfl_sync(0xffffffffu, end, run), rl = __shfl_sync(0xffffffffu, len, run);
+        const int rf = __shfl_sync(0xffffffffu, from, run);
+        if (k < total) {
+          const int f = G.items[rf + (k - (re - rl))];
+          const D3 d = sub(closest_on_triangle(p, vertex(vtx, faces[3 * f]), vertex(vtx, faces[3 * f + 1]),
+                                               vertex(vtx, faces[3 * f + 2])), p);
+          const double d2 = dot(d, d);
+          if (d2 < best || (d2 == best && f < bf)) {
+            best = d2;
+            bf = f;
+          }
+        }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double d2 = __shfl_xor_sync(0xffffffffu, best, o);
+      const int f = __shfl_xor_sync(0xffffffffu, bf, o);
+      if (d2 < best || (d2 == best && f < bf)) {
+        best = d2;
+        bf = f;
       }
     }
     // lower bound on the distance from p to cells outside the block: the
@@ -283,7 +419,89 @@ __global__ void k_normals_grid(const float* __restrict__ vtx, const int* __restr
     const double bd = bound - G.slack;
     if (bd > 0.0 && best < bd * bd * (1.0 - 1e-12)) break;
   }
-  emit_normal(vtx, faces, bf == 0x7fffffff ? 0 : bf, bq, p, nrm + 3 * i);
+  if (lane != 0) return;
+  D3 bq = p;  // face 0 when no distance compares (degenerate faces only)
+  if (bf != 0x7fffffff)
+    bq = closest_on_triangle(p, vertex(vtx, faces[3 * bf]), vertex(vtx, faces[3 * bf + 1]), vertex(vtx, faces[3 * bf + 2]));
+  emit_normal(vtx, faces, bf == 0x7fffffff ? 0 : bf, bq, p, nrm + 3 * (size_t)i);
+}
+
+// Bounding box of the faces' vertices, {lo, hi} of each CTA (fminf and fmaxf
+// pass over NaN).  On the host, three random reads a face through the whole
+// list took 9 ms for 262144 faces.
+__global__ void __launch_bounds__(256) k_face_bounds(const float* __restrict__ vtx, const int* __restrict__ faces,
+                                                     long long nv, float* __restrict__ out) {
+  float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  for (long long k = blockIdx.x * 256ll + threadIdx.x; k < nv; k += gridDim.x * 256ll)
+    for (int a = 0; a < 3; a++) {
+      const float x = vtx[3 * (size_t)faces[k] + a];
+      v[a] = fminf(v[a], x);
+      v[3 + a] = fmaxf(v[3 + a], x);
+    }
+  __shared__ float part[8][6];
+  for (int a = 0; a < 6; a++) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const float x = __shfl_xor_sync(0xffffffffu, v[a], o);
+      v[a] = a < 3 ? fminf(v[a], x) : fmaxf(v[a], x);
+    }
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x / 32][a] = v[a];
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    float x = part[0][threadIdx.x];
+    for (int w = 1; w < 8; w++)
+      x = threadIdx.x < 3 ? fminf(x, part[w][threadIdx.x]) : fmaxf(x, part[w][threadIdx.x]);
+    out[6 * blockIdx.x + threadIdx.x] = x;
+  }
+}
+
+// Exclusive scan of the cells' counts in two launches: the sums of 1024 cells,
+// then every CTA adds up the sums before its own.  start saturates at
+// INT32_MAX; the last CTA leaves the total.
+__device__ __forceinline__ long long cta_sum(long long v, long long* sh) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x / 32] = v;
+  __syncthreads();
+  v = 0;
+  for (int w = 0; w < (int)blockDim.x / 32; w++) v += sh[w];
+  __syncthreads();
+  return v;
+}
+
+__global__ void __launch_bounds__(1024) k_cell_sums(const int* __restrict__ counts, long long ncell,
+                                                    long long* __restrict__ sums) {
+  __shared__ long long sh[32];
+  const long long c = blockIdx.x * 1024ll + threadIdx.x;
+  const long long s = cta_sum(c < ncell ? counts[c] : 0, sh);
+  if (threadIdx.x == 0) sums[blockIdx.x] = s;
+}
+
+// the counts become cursors: the next item of every cell
+__global__ void __launch_bounds__(1024) k_cell_start(int* __restrict__ counts, long long ncell,
+                                                     const long long* __restrict__ sums, int* __restrict__ start,
+                                                     long long* __restrict__ total) {
+  __shared__ long long sh[32], wsum[32];
+  long long base = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += 1024) base += sums[b];
+  base = cta_sum(base, sh);
+  const long long c = blockIdx.x * 1024ll + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+  const long long n = c < ncell ? counts[c] : 0;
+  long long v = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long x = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += x;
+  }
+  if (lane == 31) wsum[warp] = v;
+  __syncthreads();
+  for (int w = 0; w < warp; w++) base += wsum[w];
+  if (c < ncell) {
+    counts[c] = start[c] = (int)min(base + v - n, 0x7fffffffll);
+    if (c == ncell - 1) {
+      start[ncell] = (int)min(base + v, 0x7fffffffll);
+      *total = base + v;
+    }
+  }
 }
 
 __device__ bool region_contains(const rso_region& r, D3 p) {
@@ -323,15 +541,21 @@ __device__ bool region_contains(const rso_region& r, D3 p) {
   return in != (r.complement != 0);
 }
 
+// a warp per row of nodes: the row's y and z are divided out once, not per node
+// (257^3 nodes: 113 -> 68 us)
 __global__ void k_region_mask(const rso_region* __restrict__ regions, int nr, double ox, double oy, double oz,
-                              double h, int nx, int ny, long long nn, uint8_t* __restrict__ mask) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= nn) return;
-  const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((long long)nx * ny));
-  const D3 p = {ox + x * h, oy + y * h, oz + z * h};
-  bool in = false;
-  for (int k = 0; k < nr; k++) in |= region_contains(regions[k], p);
-  mask[i] = in ? 1 : 0;
+                              double h, int nx, int ny, long long rows, uint8_t* __restrict__ mask) {
+  for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32; r < rows;
+       r += (long long)gridDim.x * blockDim.x / 32) {
+    const int y = (int)(r % ny), z = (int)(r / ny);
+    uint8_t* row = mask + r * nx;
+    for (long long x = threadIdx.x & 31; x < nx; x += 32) {
+      const D3 p = {ox + (int)x * h, oy + y * h, oz + z * h};
+      bool in = false;
+      for (int k = 0; k < nr; k++) in |= region_contains(regions[k], p);
+      row[x] = in ? 1 : 0;
+    }
+  }
 }
 
 __device__ double field_norm(const rso_field& f, D3 p) {
@@ -388,12 +612,6 @@ __global__ void k_region_field(const rso_field* __restrict__ fields, int nfld, c
   out[3 * i + 2] = s.z;
 }
 
-// device copies of a host array; frees everything it allocated on destruction
-// Device blocks of these entry points, cached per device in power-of-two
-// size classes between calls: repeated calls reuse them instead of
-// allocating and freeing (a free lets the driver unmap the memory and the
-// next allocation map it again, which made the call times vary by tens of
-// milliseconds).  At most kCacheCap bytes per device stay cached.
 constexpr int kCacheDevices = 64;
 constexpr size_t kCacheCap = size_t(1) << 30;
 struct BlockCache {
@@ -402,6 +620,8 @@ struct BlockCache {
   size_t held[kCacheDevices] = {};
 };
 BlockCache g_blocks;
+
+}  // namespace
 
 cudaError_t block_get(int dev, size_t bytes, void** p, size_t* cls) {
   size_t c = 256;
@@ -433,37 +653,7 @@ void block_put(int dev, size_t cls, void* p) {
   cudaFree(p);
 }
 
-// device copies of host arrays and work buffers for one call; the blocks go
-// back to the cache when the call returns (every kernel of the call has
-// finished by then: each entry point ends with a synchronous copy)
-struct Scratch {
-  struct Block {
-    void* p;
-    size_t cls;
-  };
-  std::vector<Block> blocks;
-  int dev = -1;
-  cudaError_t err = cudaSuccess;
-  Scratch() { err = cudaGetDevice(&dev); }
-  template <typename T>
-  T* upload(const T* host, size_t n) {
-    if (err != cudaSuccess) return nullptr;
-    void* p = nullptr;
-    size_t cls = 0;
-    err = block_get(dev, sizeof(T) * (n ? n : 1), &p, &cls);
-    if (err != cudaSuccess) return nullptr;
-    blocks.push_back({p, cls});
-    if (host && n) err = cudaMemcpy(p, host, sizeof(T) * n, cudaMemcpyHostToDevice);
-    return static_cast<T*>(p);
-  }
-  template <typename T>
-  T* alloc(size_t n) { return upload<T>(nullptr, n); }
-  ~Scratch() {
-    // a failed call may have left work in flight on the device
-    if (err != cudaSuccess) cudaDeviceSynchronize();
-    for (const Block& b : blocks) block_put(dev, b.cls, b.p);
-  }
-};
+namespace {
 
 static_assert(sizeof(rso_region) == 80 && sizeof(rso_field) == 192, "rso_region / rso_field layout is part of the ABI");
 
@@ -498,11 +688,24 @@ extern "C" rso_status rso_shell_elements(const float* vertices_host, int n_verti
   Scratch s;
   const float* dv = s.upload(vertices_host, 3 * (size_t)n_vertices);
   const int* df = s.upload(faces_host, 3 * (size_t)n_faces);
-  const uint8_t* dsolid = s.upload(solid_host, (size_t)nvox);
-  uint8_t* dshell = s.alloc<uint8_t>((size_t)nvox);
-  if (s.err == cudaSuccess) s.err = cudaMemset(dshell, 0, (size_t)nvox);
-  if (s.err == cudaSuccess && wshell > 0) {
-    k_shell<<<n_faces, 256>>>(dv, df, n_faces, box_host[0], box_host[1], box_host[2], eh, wshell, R, dsolid, dshell);
+  uint8_t* dshell = s.upload(solid_host, (size_t)nvox);  // the solid bytes, then the shell's
+  ShellGrid G{{box_host[0], box_host[1], box_host[2]}, eh, wshell, R, (R + 7) & ~7};
+  uint8_t* state = s.alloc<uint8_t>((size_t)R * R * G.pitch);
+  int* big = s.alloc<int>(1 + (size_t)n_faces);
+  if (s.err == cudaSuccess) s.err = cudaMemset(big, 0, sizeof(int));
+  if (s.err == cudaSuccess) {
+    const unsigned rows = (unsigned)std::min(((long long)R * R + 7) / 8, 148LL * 64);
+    k_shell_bytes<true><<<rows, 256>>>(dshell, state, R, G.pitch);
+    note_launch();
+    if (wshell > 0) {
+      int stride = (int)(0.618 * n_faces) + 1;
+      while (std::gcd(stride, n_faces) != 1) stride++;
+      k_shell<<<(unsigned)cdiv(n_faces, 4), 128>>>(dv, df, n_faces, stride, G, state, big);
+      note_launch();
+      k_shell_big<<<148 * 8, 128>>>(dv, df, G, state, big);
+      note_launch();
+    }
+    k_shell_bytes<false><<<rows, 256>>>(dshell, state, R, G.pitch);
     note_launch();
     s.err = cudaGetLastError();
   }
@@ -527,20 +730,27 @@ extern "C" rso_status rso_mesh_normals(const float* vertices_host, int n_vertice
   FaceGrid G{};
   if (s.err == cudaSuccess && n_faces >= 256) {
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (long long k = 0; k < 3LL * n_faces; k++) {
-      const int v = faces_host[k];
-      for (int a = 0; a < 3; a++) {
-        lo[a] = std::fmin(lo[a], (double)vertices_host[3 * v + a]);
-        hi[a] = std::fmax(hi[a], (double)vertices_host[3 * v + a]);
-      }
+    constexpr int kParts = 148;
+    float part[6 * kParts];
+    float* dpart = s.alloc<float>(6 * kParts);
+    if (s.err == cudaSuccess) {
+      k_face_bounds<<<kParts, 256>>>(dv, df, 3LL * n_faces, dpart);
+      note_launch();
+      s.err = cudaGetLastError();
     }
+    if (s.err == cudaSuccess) s.err = cudaMemcpy(part, dpart, sizeof(part), cudaMemcpyDeviceToHost);
+    for (int k = 0; k < kParts && s.err == cudaSuccess; k++)
+      for (int a = 0; a < 3; a++) {
+        lo[a] = std::fmin(lo[a], (double)part[6 * k + a]);
+        hi[a] = std::fmax(hi[a], (double)part[6 * k + 3 + a]);
+      }
     double ext[3], emax = 0, mag = 0;
     for (int a = 0; a < 3; a++) {
       ext[a] = hi[a] - lo[a];
       emax = std::fmax(emax, ext[a]);
       mag = std::fmax(mag, std::fmax(std::fabs(lo[a]), std::fabs(hi[a])));
     }
-    if (emax > 0 && std::isfinite(emax) && std::isfinite(mag)) {
+    if (s.err == cudaSuccess && emax > 0 && std::isfinite(emax) && std::isfinite(mag)) {
       const double target = std::min(std::max(n_faces / 2.0, 1.0), (double)(1 << 21));
       double vol = 1;
       for (int a = 0; a < 3; a++) vol *= std::fmax(ext[a], 1e-3 * emax);
@@ -562,19 +772,19 @@ extern "C" rso_status rso_mesh_normals(const float* vertices_host, int n_vertice
         note_launch();
         s.err = cudaGetLastError();
       }
-      std::vector<int> hc((size_t)ncell);
-      if (s.err == cudaSuccess) s.err = cudaMemcpy(hc.data(), counts, sizeof(int) * ncell, cudaMemcpyDeviceToHost);
-      std::vector<int> hs((size_t)ncell + 1, 0);
+      const int nsum = (int)cdiv(ncell, 1024);
+      long long* sums = s.alloc<long long>((size_t)nsum + 1);  // + the total
+      int* start = s.alloc<int>((size_t)ncell + 1);
       long long total = 0;
-      for (long long cidx = 0; cidx < ncell; cidx++) {
-        hs[cidx] = (int)std::min(total, (long long)INT32_MAX);
-        total += hc[cidx];
+      if (s.err == cudaSuccess) {
+        k_cell_sums<<<nsum, 1024>>>(counts, ncell, sums);
+        note_launch();
+        k_cell_start<<<nsum, 1024>>>(counts, ncell, sums, start, sums + nsum);
+        note_launch();
+        s.err = cudaMemcpy(&total, sums + nsum, sizeof(total), cudaMemcpyDeviceToHost);
       }
-      hs[ncell] = (int)std::min(total, (long long)INT32_MAX);
       if (s.err == cudaSuccess && total <= (1LL << 25)) {
-        int* start = s.upload(hs.data(), hs.size());
         int* items = s.alloc<int>((size_t)std::max(total, 1LL));
-        if (s.err == cudaSuccess) s.err = cudaMemset(counts, 0, sizeof(int) * ncell);
         if (s.err == cudaSuccess) {
           G.start = start;
           G.items = items;
@@ -587,7 +797,7 @@ extern "C" rso_status rso_mesh_normals(const float* vertices_host, int n_vertice
     }
   }
   if (s.err == cudaSuccess && grid) {
-    k_normals_grid<<<cdiv(n_points, 128), 128>>>(dv, df, G, dp, n_points, dn);
+    k_normals_grid<<<(unsigned)cdiv((long long)n_points, 4), 128>>>(dv, df, G, dp, n_points, dn);
     note_launch();
     s.err = cudaGetLastError();
   } else if (s.err == cudaSuccess) {
@@ -610,8 +820,9 @@ extern "C" rso_status rso_region_mask(const rso_region* regions_host, int n_regi
   const rso_region* dr = s.upload(regions_host, (size_t)n_regions);
   uint8_t* dm = s.alloc<uint8_t>((size_t)nn);
   if (s.err == cudaSuccess) {
-    k_region_mask<<<cdiv(nn, 256), 256>>>(dr, n_regions, origin_host[0], origin_host[1], origin_host[2], h, nx, ny,
-                                          nn, dm);
+    const long long rows = (long long)ny * nz;
+    k_region_mask<<<(unsigned)std::min((rows + 7) / 8, 148LL * 64), 256>>>(dr, n_regions, origin_host[0], origin_host[1],
+                                                                         origin_host[2], h, nx, ny, rows, dm);
     note_launch();
     s.err = cudaGetLastError();
   }

@@ -504,6 +504,46 @@ rso_status worst_case(rso_handle* h, int steps, int cf, double tol, uint64_t see
 rso_status modified_pm(rso_handle* h, int cf, uint64_t seed, int max_itn, double* f_pad, double* u_pad,
                        double* c_worst, int* itn);
 
+// Device blocks of the mesh input's entry points (boundary.cu, voxelize.cu), cached per device in power-of-two
+// size classes between calls: repeated calls reuse them instead of
+// allocating and freeing (a free lets the driver unmap the memory and the
+// next allocation map it again, which made the call times vary by tens of
+// milliseconds).  At most kCacheCap bytes per device stay cached.
+cudaError_t block_get(int dev, size_t bytes, void** p, size_t* cls);
+void block_put(int dev, size_t cls, void* p);
+
+// device copies of host arrays and work buffers for one call; the blocks go
+// back to the cache when the call returns (every kernel of the call has
+// finished by then: each entry point ends with a synchronous copy)
+struct Scratch {
+  struct Block {
+    void* p;
+    size_t cls;
+  };
+  std::vector<Block> blocks;
+  int dev = -1;
+  cudaError_t err = cudaSuccess;
+  Scratch() { err = cudaGetDevice(&dev); }
+  template <typename T>
+  T* upload(const T* host, size_t n) {
+    if (err != cudaSuccess) return nullptr;
+    void* p = nullptr;
+    size_t cls = 0;
+    err = block_get(dev, sizeof(T) * (n ? n : 1), &p, &cls);
+    if (err != cudaSuccess) return nullptr;
+    blocks.push_back({p, cls});
+    if (host && n) err = cudaMemcpy(p, host, sizeof(T) * n, cudaMemcpyHostToDevice);
+    return static_cast<T*>(p);
+  }
+  template <typename T>
+  T* alloc(size_t n) { return upload<T>(nullptr, n); }
+  ~Scratch() {
+    // a failed call may have left work in flight on the device
+    if (err != cudaSuccess) cudaDeviceSynchronize();
+    for (const Block& b : blocks) block_put(dev, b.cls, b.p);
+  }
+};
+
 // MMA state accessors (mma.cu)
 double* mma_x(rso_mma* s);
 int mma_n(rso_mma* s);

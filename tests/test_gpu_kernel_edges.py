@@ -3,6 +3,7 @@ remainders, the smallest and largest of a range), against the FP64 oracle."""
 import numpy as np
 import pytest
 
+import mesh_shapes as M
 import problems as P
 from test_gpu_00_parity import make, rel, t
 
@@ -257,3 +258,64 @@ def test_fp64_vcycle_graphs_and_bottom(cuda, gen, smoother):
     g.set_launch_shapes(4, -1)
     u, k, _, _ = g.solve(t(f, cuda), tol=1e-9)
     assert abs(k - it) <= 1 and rel(u.cpu().numpy(), plain.cpu().numpy()) < 1e-8
+
+
+# grids of 2, 4 and 8 voxels (several columns to a word or a warp), of one warp's words a column (128)
+# and of more (256)
+@pytest.mark.parametrize("pref", [1, 2, 6, 100, 130])
+def test_voxel_columns(cuda, pref):
+    """Solid voxels of every column layout of the parity scan; the same bytes."""
+    from oracle import voxel
+    from robustoptspline3d_b200.voxelize import voxelize
+    v, f = M.icosphere(1, 5.0, rotation_seed=3)
+    got, R, _ = voxelize(v, f, pref)
+    want, Ro, _ = voxel.voxelize(v, f, pref)
+    assert R == Ro and np.array_equal(got, want), int(np.sum(got != want))
+
+
+# boxes of more rows than a warp takes (the cube), rows that are no multiple of eight bytes, and slivers
+# whose closest points are too inexact for the bounding-box test (the flattened sphere)
+@pytest.mark.parametrize("shape,R,width,flat", [("cube", 71, 3.5, 1.0), ("icosphere", 37, 2.2, 1.0),
+                                                ("icosphere", 24, 1.3, 1e-7), ("icosphere", 8, 9.0, 1.0)])
+def test_shell_rows(cuda, shape, R, width, flat):
+    """Shell elements for any non-zero solid byte; the same bytes."""
+    from oracle import boundary as OB
+    from robustoptspline3d_b200 import boundary as B
+    v, f = M.cube(4.0) if shape == "cube" else M.icosphere(2, 4.0, rotation_seed=2)
+    v = (np.asarray(v, np.float64) * [1.0, 1.0, flat]).astype(np.float32)
+    lo, size = v.min(0), 1.1 * float(np.ptp(v, axis=0).max())
+    lo = (0.5 * (v.min(0) + v.max(0)) - 0.5 * size).astype(np.float32)
+    box = np.concatenate([lo, lo + np.float32(size)]).astype(np.float32)
+    solid = np.random.default_rng(1).choice(np.array([0, 1, 2, 255], np.uint8), size=(R, R, R))
+    got = B.shell_elements(v, f, box, R, width, solid)
+    want = OB.shell_elements(v, f, box, R, width, (solid > 0).astype(np.uint8))
+    assert np.array_equal(got, want), int(np.sum(got != want))
+    assert got.sum() > 0
+
+
+@pytest.mark.parametrize("flat", [1.0, 0.0])
+def test_normals_rings(cuda, flat):
+    """Normals at points in the mesh's box, far outside it (many rings) and on vertices (ties), of a
+    sphere and of a flat disc; 1e-12, the bound of the normals test."""
+    from oracle import boundary as OB
+    from robustoptspline3d_b200 import boundary as B
+    v, f = M.icosphere(3, 1.0, rotation_seed=5)
+    v = (np.asarray(v, np.float64) * [1.0, 1.0, flat]).astype(np.float32)
+    rng = np.random.default_rng(8)
+    P = np.concatenate([rng.uniform(-1.2, 1.2, (301, 3)), rng.uniform(-40, 40, (70, 3)), v[:33].astype(np.float64)])
+    if flat == 0.0:
+        P = P[:371]  # both layers of the disc tie at a vertex and have opposite planes
+    got, want = B.mesh_normals(v, f, P), OB.mesh_normals(v, f, P)
+    assert np.max(np.abs(got - want)) <= 1e-12
+
+
+@pytest.mark.parametrize("dims", [(1, 5, 3), (31, 3, 2), (33, 7, 5), (257, 2, 3)])
+def test_region_rows(cuda, dims):
+    """Region masks on rows shorter than, equal to and longer than a warp; the same bytes."""
+    from robustoptspline3d_b200 import boundary as B
+    r = [B.sphere((0.4, 0.3, 0.2), 0.9), B.halfspace(1, 0.5, -1, -9.0)]
+    got = B.region_mask(r, (-0.5, -0.4, -0.3), 0.2, dims)
+    z, y, x = np.meshgrid(*(np.arange(n) for n in dims[::-1]), indexing="ij")
+    x, y, z = -0.5 + x * 0.2, -0.4 + y * 0.2, -0.3 + z * 0.2
+    want = ((x - 0.4) ** 2 + (y - 0.3) ** 2 + (z - 0.2) ** 2 < 0.9 ** 2) | (x + 0.5 * y - z - 9.0 > 0)
+    assert np.array_equal(got, want.astype(np.uint8))
