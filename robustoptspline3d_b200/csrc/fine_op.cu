@@ -1086,9 +1086,11 @@ __global__ void __launch_bounds__(256) k_fine_jacobi0(const Level L, const T* __
 // FP32 first Jacobi step from zero with four consecutive padded nodes per
 // thread (px is a multiple of 4): f, out and the node classes move as 16-byte
 // vectors, and the 20 rho^p values of the group's elements (5 per row of
-// elements) as one 16-byte and one scalar load per row.  Same arithmetic, in
-// the same order, as k_fine_jacobi0<float>.  Halo rows are skipped; the halo
-// nodes of a group are written as zero.
+// elements) as one 16-byte and one scalar load per row.  The diagonal block
+// comes from signed sums of the rows' pair sums and differences, as in
+// k_fine_p.  Bound by the bytes (28 a node) since the block takes 20 additions
+// and not 48 multiply-adds a node (256^3: 124 -> 104 us).  Halo rows are
+// skipped; the halo nodes of a group are written as zero.
 __global__ void __launch_bounds__(256) k_fine_jacobi0_v4(const Level L, const float* __restrict__ f,
                                                          float* __restrict__ out, const float* __restrict__ rp,
                                                          float omega) {
@@ -1147,25 +1149,21 @@ __global__ void __launch_bounds__(256) k_fine_jacobi0_v4(const Level L, const fl
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (!work[k]) continue;
-      float D[6] = {0, 0, 0, 0, 0, 0};
+      // per element row (y side + 2 (z side)): sum and difference of its two elements
+      float S[4], T[4];
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        // element q of the node: (a, b, c) = (q & 1, q >> 1 & 1, q >> 2)
-        const float r = rr[((q >> 1) & 1) + 2 * (q >> 2)][k + (q & 1)];
-        const int vi = 7 - q;
-        D[0] += r * k0<float>((vi * 3 + 0) * 24 + vi * 3 + 0);
-        D[1] += r * k0<float>((vi * 3 + 0) * 24 + vi * 3 + 1);
-        D[2] += r * k0<float>((vi * 3 + 0) * 24 + vi * 3 + 2);
-        D[3] += r * k0<float>((vi * 3 + 1) * 24 + vi * 3 + 1);
-        D[4] += r * k0<float>((vi * 3 + 1) * 24 + vi * 3 + 2);
-        D[5] += r * k0<float>((vi * 3 + 2) * 24 + vi * 3 + 2);
+      for (int row = 0; row < 4; row++) {
+        S[row] = rr[row][k + 1] + rr[row][k];
+        T[row] = rr[row][k + 1] - rr[row][k];
       }
+      const float a = cWp[W_DA].x * ((S[0] + S[1]) + (S[2] + S[3]));
+      const float b = cWp[W_DB].x * ((T[1] - T[0]) + (T[3] - T[2]));  // xy
+      const float c = cWp[W_DB].x * ((T[2] - T[0]) + (T[3] - T[1]));  // xz
+      const float e = cWp[W_DB].x * ((S[3] - S[2]) - (S[1] - S[0]));  // yz
       const float r0 = fv[0][k], r1 = fv[1][k], r2 = fv[2][k];
-      const float a = D[0], b = D[1], c = D[2], d = D[3], e = D[4], gg = D[5];
-      const float A = d * gg - e * e, B = c * e - b * gg, C = b * e - c * d;
-      const float det = a * A + b * B + c * C;
-      const float id = omega / det;
-      const float E = a * gg - c * c, F = b * c - a * e, I = a * d - b * b;
+      const float A = a * a - e * e, B = c * e - b * a, C = b * e - c * a;
+      const float id = omega / (a * A + b * B + c * C);
+      const float E = a * a - c * c, F = b * c - a * e, I = a * a - b * b;
       o[0][k] = id * (A * r0 + B * r1 + C * r2);
       o[1][k] = id * (B * r0 + E * r1 + F * r2);
       o[2][k] = id * (C * r0 + F * r1 + I * r2);

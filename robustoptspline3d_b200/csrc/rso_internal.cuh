@@ -425,7 +425,10 @@ template <typename T>
 rso_status coarse_residual(rso_handle* h, int level, const T* u, const T* f, T* r);
 template <typename T>
 rso_status coarse_jacobi(rso_handle* h, int level, const T* u_in, const T* f, T* u_out, double omega,
-                         const T* u_prev = nullptr, double c1 = 0.0);
+                         const T* u_prev = nullptr, double c1 = 0.0, bool rev = false);
+// the first step from a zero iterate
+template <typename T>
+rso_status coarse_jacobi0(rso_handle* h, int level, const T* f, T* u_out, double omega);
 template <typename T>
 rso_status coarse_gs(rso_handle* h, int level, T* u, const T* f, int colour, int reverse);
 template <typename T>

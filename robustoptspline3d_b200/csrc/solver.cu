@@ -60,8 +60,8 @@ void smoother_steps(const rso_handle* h, double lam, int m, double* om, double* 
   }
 }
 
-// zero: the iterate is known to be zero before the first sweep (the first
-// sweep on the fine level then needs no operator application).  Jacobi and
+// zero: the iterate is known to be zero before the first sweep, and is not
+// read: a Jacobi or Chebyshev sweep from it needs no operator application.  Jacobi and
 // Chebyshev steps rotate three level vectors: u (current), t (next) and r
 // (previous iterate; free while the level is being smoothed).
 // last_dot (FP32 fine level only): the last step also sums f . u into it
@@ -91,7 +91,8 @@ static rso_status smooth(rso_handle* h, int li, int sweeps, int reverse, bool ze
         RSO_TRY(fine_jacobi_dot32(h, LV<T>::u(l), LV<T>::f(l), LV<T>::t(l), om[s], prev, c1[s], last_dot,
                                   h->vc_zdot_stride));
     } else if (li == 0) RSO_TRY(fine_jacobi<T>(h, LV<T>::u(l), LV<T>::f(l), LV<T>::t(l), LV<T>::rp(h), om[s], prev, c1[s]));
-    else RSO_TRY(coarse_jacobi<T>(h, li, LV<T>::u(l), LV<T>::f(l), LV<T>::t(l), om[s], prev, c1[s]));
+    else if (zero && s == 0) RSO_TRY(coarse_jacobi0<T>(h, li, LV<T>::f(l), LV<T>::t(l), om[0]));
+    else RSO_TRY(coarse_jacobi<T>(h, li, LV<T>::u(l), LV<T>::f(l), LV<T>::t(l), om[s], prev, c1[s], zero != (s & 1)));
     if (cheb) {  // previous <- current <- next
       T* old_prev = LV<T>::r(l);
       LV<T>::r(l) = LV<T>::u(l);
@@ -124,7 +125,8 @@ rso_status vcycle_levels(rso_handle* h, int pre, int post, int symmetric, bool u
     if (li > 0) {
       RSO_TRY(level_residual<T>(h, li - 1));
       RSO_TRY(restrict_<T>(h, li, LV<T>::r(h->L[li - 1]), LV<T>::f(l)));
-      RSO_CHECK_CUDA(h, cudaMemsetAsync(LV<T>::u(l), 0, sizeof(T) * 3 * l.NP * l.nb, h->stream));
+      if (h->cfg.smoother == RSO_SMOOTH_GS || pre == 0 || li == nl - 1)
+        RSO_CHECK_CUDA(h, cudaMemsetAsync(LV<T>::u(l), 0, sizeof(T) * 3 * l.NP * l.nb, h->stream));
     }
     const bool zero = li > 0 || u0_zero;
     if (li < nl - 1) RSO_TRY(smooth<T>(h, li, pre, 0, zero));
