@@ -614,7 +614,9 @@ constexpr int pair_min_blocks(int mode, int typ) {
 // otherwise every thread stages 16-byte chunks with cp.async.
 // DOT (MODE 2 only): also sum f . out into per-CTA partials (dotp); a
 // separate instantiation so the plain step carries none of it
-template <int MODE, int TYP, bool TMA, bool DOT = false>
+// PREV (MODE 2 only): the previous iterate (zero without uprev) enters with
+// weight c1; likewise
+template <int MODE, int TYP, bool TMA, bool DOT = false, bool PREV = false>
 __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
     k_fine_p(const Level L, const float* u, const float* f, float* out, const float* __restrict__ rp, float omega,
              double* dotp, const float* uprev, float c1, int fzc, const __grid_constant__ CUtensorMap tmu, const __grid_constant__ CUtensorMap tmr) {
@@ -625,7 +627,8 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
   // Corner exchange: the right neighbour's corners by shuffle, one value per
   // component through shared memory to the thread row below (residual and K u:
   // 223 -> 215 us at 256^3); the step, at its register limit, leaves all four
-  // values there (285 us; 311 with shuffles, which spill).
+  // values there (255 us; 256 with shuffles, 311 with the previous iterate too,
+  // which spills).
   constexpr bool SHFL = MODE != 2;
   constexpr int XV = pair_xvals(MODE);
   constexpr int RHO = pair_rho_off<TYP>(), SLOT = pair_slot<TYP>();
@@ -852,7 +855,7 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
       dl[2] = p_fma(C, r0, p_fma(Fm, r1, p_mul(I, r2)));
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        const float2 v = p_fma(id, dl[c], p_fma(cc1, p_sub(uo[c], po[c]), uo[c]));
+        const float2 v = p_fma(id, dl[c], PREV ? p_fma(cc1, p_sub(uo[c], po[c]), uo[c]) : uo[c]);
         res[c] = make_float2(workA ? v.x : 0.f, workB ? v.y : 0.f);
       }
       // DOT: this thread's share of f . out (the CG step's r . z when this
@@ -890,7 +893,7 @@ __global__ void __launch_bounds__(32 * TYP, pair_min_blocks(MODE, TYP))
       if (MODE != 1) {
 #pragma unroll
         for (int c = 0; c < 3; c++) fo[c] = make_float2(rd(f, c, n), rdB(f, c, n));
-        if (MODE == 2 && uprev != nullptr) {
+        if (PREV && uprev != nullptr) {
 #pragma unroll
           for (int c = 0; c < 3; c++) po[c] = make_float2(rd(uprev, c, n), rdB(uprev, c, n));
         }
@@ -1381,6 +1384,23 @@ rso_status fine_stage_check(rso_handle* h) {
   return RSO_OK;
 }
 
+using PairKernel = void (*)(const Level, const float*, const float*, float*, const float*, float, double*,
+                            const float*, float, int, const CUtensorMap, const CUtensorMap);
+template <int MODE, int TYP>
+static PairKernel pair_variant(bool dot, bool prev) {
+  if constexpr (MODE == 2) {
+    if (dot) return prev ? k_fine_p<2, TYP, kPairTMA, true, true> : k_fine_p<2, TYP, kPairTMA, true, false>;
+    if (prev) return k_fine_p<2, TYP, kPairTMA, false, true>;
+  }
+  return k_fine_p<MODE, TYP, kPairTMA>;
+}
+template <int MODE>
+static PairKernel pair_kernel(int rows, bool dot, bool prev) {
+  return rows == 2   ? pair_variant<MODE, 2>(dot, prev)
+         : rows == 8 ? pair_variant<MODE, 8>(dot, prev)
+                     : pair_variant<MODE, 4>(dot, prev);
+}
+
 template <typename T, int MODE>
 static rso_status launch_fine(rso_handle* h, const T* u, const T* f, T* out, const T* rp, double omega, int cls,
                               const char* what, double* dotp = nullptr, const T* uprev = nullptr, double c1 = 0.0,
@@ -1403,18 +1423,11 @@ static rso_status launch_fine(rso_handle* h, const T* u, const T* f, T* out, con
                              : pty == 8 ? pair_smem_bytes<8>(MODE, pair_slots(MODE, kPairTMA))
                                         : pair_smem_bytes<4>(MODE, pair_slots(MODE, kPairTMA)))
                           : walsh_smem_bytes<T, WTY>();
-  // MODE 2 with dotp: the instantiation that also sums f . out
-  const bool jdot = MODE == 2 && dotp != nullptr;
+  // MODE 2: the instantiations that also sum f . out, and that weigh the previous iterate
+  const bool jdot = MODE == 2 && dotp != nullptr, jprev = MODE == 2 && (uprev != nullptr || c1 != 0.0);
   const void* kern;
   if constexpr (packed) {
-    if (jdot)
-      kern = pty == 2   ? reinterpret_cast<const void*>(k_fine_p<MODE, 2, kPairTMA, true>)
-             : pty == 8 ? reinterpret_cast<const void*>(k_fine_p<MODE, 8, kPairTMA, true>)
-                        : reinterpret_cast<const void*>(k_fine_p<MODE, 4, kPairTMA, true>);
-    else
-      kern = pty == 2   ? reinterpret_cast<const void*>(k_fine_p<MODE, 2, kPairTMA>)
-             : pty == 8 ? reinterpret_cast<const void*>(k_fine_p<MODE, 8, kPairTMA>)
-                        : reinterpret_cast<const void*>(k_fine_p<MODE, 4, kPairTMA>);
+    kern = reinterpret_cast<const void*>(pair_kernel<MODE>(pty, jdot, jprev));
   } else if (MODE == 0 && out32 != nullptr) {
     kern = reinterpret_cast<const void*>(k_fine_w<T, MODE, WTY, true>);
   } else {
@@ -1422,10 +1435,10 @@ static rso_status launch_fine(rso_handle* h, const T* u, const T* f, T* out, con
   }
   // the shared-memory opt-in is per device and kernel; setting it twice from
   // racing threads is harmless, so an atomic flag per device suffices
-  static std::atomic<bool> attr[3][2][64];
+  static std::atomic<bool> attr[3][4][64];
   const int ti = pty == 2 ? 0 : pty == 4 ? 1 : 2;
-  const bool second = jdot || (MODE == 0 && out32 != nullptr);  // the instantiation with the extra outputs
-  std::atomic<bool>* done = (h->device >= 0 && h->device < 64) ? &attr[ti][second ? 1 : 0][h->device] : nullptr;
+  const int variant = (jdot || (MODE == 0 && out32 != nullptr) ? 1 : 0) + (packed && jprev ? 2 : 0);
+  std::atomic<bool>* done = (h->device >= 0 && h->device < 64) ? &attr[ti][variant][h->device] : nullptr;
   if (!done || !done->load(std::memory_order_acquire)) {
     RSO_CHECK_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (done) done->store(true, std::memory_order_release);
@@ -1435,25 +1448,8 @@ static rso_status launch_fine(rso_handle* h, const T* u, const T* f, T* out, con
     CUtensorMap mu{}, mr{};
     if (kPairTMA) RSO_TRY(pair_tensor_maps(h, l, u, rp, 2 * pty, &mu, &mr));
     if (h->prof_on) prof_begin(h, cls, (double)l.nn);
-    if (jdot) {
-      if (pty == 2)
-        launch_pdl(k_fine_p<MODE, 2, kPairTMA, true>, pair_grid(l, 2, fzc), dim3(WTX, 2), smem, h->stream, l, u, f,
-                   out, rp, (float)omega, dotp, uprev, (float)c1, fzc, mu, mr);
-      else if (pty == 8)
-        launch_pdl(k_fine_p<MODE, 8, kPairTMA, true>, pair_grid(l, 8, fzc), dim3(WTX, 8), smem, h->stream, l, u, f,
-                   out, rp, (float)omega, dotp, uprev, (float)c1, fzc, mu, mr);
-      else
-        launch_pdl(k_fine_p<MODE, 4, kPairTMA, true>, pair_grid(l, 4, fzc), dim3(WTX, 4), smem, h->stream, l, u, f,
-                   out, rp, (float)omega, dotp, uprev, (float)c1, fzc, mu, mr);
-    } else if (pty == 2)
-      launch_pdl(k_fine_p<MODE, 2, kPairTMA>, pair_grid(l, 2, fzc), dim3(WTX, 2), smem, h->stream, l, u, f, out,
-                 rp, (float)omega, MODE == 2 ? nullptr : dotp, uprev, (float)c1, fzc, mu, mr);
-    else if (pty == 8)
-      launch_pdl(k_fine_p<MODE, 8, kPairTMA>, pair_grid(l, 8, fzc), dim3(WTX, 8), smem, h->stream, l, u, f, out,
-                 rp, (float)omega, MODE == 2 ? nullptr : dotp, uprev, (float)c1, fzc, mu, mr);
-    else
-      launch_pdl(k_fine_p<MODE, 4, kPairTMA>, pair_grid(l, 4, fzc), dim3(WTX, 4), smem, h->stream, l, u, f, out,
-                 rp, (float)omega, MODE == 2 ? nullptr : dotp, uprev, (float)c1, fzc, mu, mr);
+    launch_pdl(pair_kernel<MODE>(pty, jdot, jprev), pair_grid(l, pty, fzc), dim3(WTX, pty), smem, h->stream, l, u, f,
+               out, rp, (float)omega, MODE == 2 && !jdot ? nullptr : dotp, uprev, (float)c1, fzc, mu, mr);
   } else {
     if (h->prof_on) prof_begin(h, cls, (double)l.nn);
     if (MODE == 0 && out32 != nullptr)

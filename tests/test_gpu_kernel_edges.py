@@ -319,3 +319,30 @@ def test_region_rows(cuda, dims):
     x, y, z = -0.5 + x * 0.2, -0.4 + y * 0.2, -0.3 + z * 0.2
     want = ((x - 0.4) ** 2 + (y - 0.3) ** 2 + (z - 0.2) ** 2 < 0.9 ** 2) | (x + 0.5 * y - z - 9.0 > 0)
     assert np.array_equal(got, want.astype(np.uint8))
+
+
+@pytest.mark.parametrize("sweeps", [1, 2, 3, 4])
+def test_chebyshev_sweeps(oracle, cuda, sweeps):
+    """FP64 Chebyshev smoothing of a single level (two sweeps take the factored form, others the
+    recurrence) against the recurrence on the oracle's operator; 1e-11 relative, ten times the bound of
+    the operator pieces for up to four of them in a row."""
+    g, o = make(oracle, P.cantilever(9, 6, 5), n_levels=1, smoother=2)
+    g.update_stencil()
+    rng = np.random.default_rng(21)
+    cls = o.node_class()
+    fix = np.tile(((cls & 4) > 0) | ((cls & 1) == 0), 3)
+    u, f = (np.where(fix, 0.0, rng.standard_normal(3 * o.nn)) for _ in range(2))
+    got, _ = g.v_cycle(t(u, cuda), t(f, cuda), pre=sweeps, post=0)
+    lam, lower = g.level_lambda(0), 0.25
+    theta, delta = 0.5 * lam * (1 + lower), 0.5 * lam * (1 - lower)
+    rho, step = delta / theta, 0.0
+    for k in range(sweeps):
+        d = o.smooth(0, u, f, kind=1, omega=1.0, sweeps=1) - u  # D^-1 (f - K u)
+        if k == 0:
+            step = d / theta
+        else:
+            new = 1.0 / (2.0 * theta / delta - rho)
+            step = new * rho * step + 2.0 * new / delta * d
+            rho = new
+        u = u + step
+    assert rel(got.cpu().numpy(), u) < 1e-11
