@@ -742,145 +742,74 @@ __global__ void k_prolong(const Level Fl, const Level C, const T* __restrict__ u
   uf[n + 2 * Fl.NP] = u2 + (w0 * e0[2] + w1 * e1[2]);
 }
 
-// FP32, single system: four consecutive padded fine nodes per thread (px is a
-// multiple of 4), the fine vector and node classes as 16-byte vectors, the
-// yz-interpolated coarse values of the (at most four) coarse columns the group
-// touches computed once.  Same arithmetic, in the same order, as k_prolong.
+// FP32, single system: four consecutive padded fine nodes a thread in the F
+// planes from one coarse plane to the next.  The group's two corners a node
+// lie on three coarse columns, folded along y once and along z per plane; all
+// loads of the F planes go out together, as 16-byte vectors, which is what
+// keeps enough bytes in flight (24 a fine node, the bound: 256^3 97 -> 78 us
+// against a warp per fine row with the coarse row folded in shared memory).
+constexpr int PRO_T = 128;
 template <int F>
-__global__ void __launch_bounds__(256) k_prolong_v4(const Level Fl, const Level C, const float* __restrict__ uc,
-                                                    float* __restrict__ uf) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long NP = Fl.NP, px = Fl.px, pxy = (long long)Fl.px * Fl.py;
-  const long long p0 = 4 * g;
-  if (p0 >= NP) return;
-  const int zp = (int)(p0 / pxy);
-  const long long rem = p0 - zp * pxy;
-  const int yp = (int)(rem / px), xp = (int)(rem - yp * px);
-  if (zp < 1 || zp > Fl.nz || yp < 1 || yp > Fl.ny) return;
-  const uchar4 cl4 = *reinterpret_cast<const uchar4*>(Fl.vclass + p0);
-  const uint8_t cls[4] = {cl4.x, cl4.y, cl4.z, cl4.w};
-  bool upd[4];
-  bool any = false;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int x = xp - 1 + k;
-    upd[k] = x >= 0 && x < Fl.nx && (cls[k] & NC_ACTIVE) && !(cls[k] & NC_SUPPORT);
-    any = any || upd[k];
-  }
-  if (!any) return;
-  const int y = yp - 1, z = zp - 1;
-  const int Y0 = y / F, Z0 = z / F, oy = y - F * Y0, oz = z - F * Z0;
-  const float wy[2] = {(float)(F - oy) / (float)F, (float)oy / (float)F};
-  const float wz[2] = {(float)(F - oz) / (float)F, (float)oz / (float)F};
-  const int x_first = max(xp - 1, 0), x_last = min(xp + 2, Fl.nx - 1);
-  const int Xa = x_first / F, Xb = x_last / F + 1;
-  const long long cpx = C.px, cpxy = (long long)C.px * C.py;
-  float E[4][3];
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const int X = Xa + j;
-#pragma unroll
-    for (int c = 0; c < 3; c++) E[j][c] = 0.f;
-    if (X <= Xb && X <= C.nx) {  // index C.nx is the padded halo (zero)
-      const long long c0 = C.nidx(X, Y0, Z0);
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        float s = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) s += wy[k & 1] * wz[k >> 1] * uc[c0 + (k & 1) * cpx + (k >> 1) * cpxy + c * C.NP];
-        E[j][c] = s;
-      }
-    }
-  }
-  float u[3][4];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const float4 m = *reinterpret_cast<const float4*>(uf + p0 + c * NP);
-    u[c][0] = m.x; u[c][1] = m.y; u[c][2] = m.z; u[c][3] = m.w;
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    if (!upd[k]) continue;
-    const int x = xp - 1 + k, X0 = x / F, ox = x - F * X0, j = X0 - Xa;
-    const float w1 = (float)ox / (float)F, w0 = (float)(F - ox) / (float)F;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float e0 = 0.f, e1 = 0.f;
-#pragma unroll
-      for (int q = 0; q < 3; q++)
-        if (q == j) { e0 = E[q][c]; e1 = E[q + 1][c]; }
-      u[c][k] = u[c][k] + (w0 * e0 + w1 * e1);
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++)
-    *reinterpret_cast<float4*>(uf + p0 + c * NP) = make_float4(u[c][0], u[c][1], u[c][2], u[c][3]);
-}
-
-// FP32, single system: one warp per fine row (y, z).  The lanes first fold the
-// row's coarse columns along y and z into shared memory (E[c][X], X = 0..C.nx,
-// index C.nx the zero halo), then update four consecutive padded fine nodes
-// each with 16-byte loads and stores, taking every node's two x-corners from
-// E: 12 coarse loads per coarse column instead of up to 36 per four nodes.
-// Same arithmetic, in the same order, as k_prolong.
-constexpr int PROW_WARPS = 8;
-template <int F>
-__global__ void __launch_bounds__(32 * PROW_WARPS) k_prolong_row(const Level Fl, const Level C,
-                                                                 const float* __restrict__ uc, float* __restrict__ uf) {
+__global__ void __launch_bounds__(PRO_T) k_prolong_slab(const Level Fl, const Level C, const float* __restrict__ uc,
+                                                        float* __restrict__ uf) {
   pdl_wait(uc, uf);
   pdl_trigger();
-  extern __shared__ float sE_all[];  // [PROW_WARPS][3][C.nx + 1]
-  const int lane = threadIdx.x, w = threadIdx.y;
-  const int y = blockIdx.x * PROW_WARPS + w, z = blockIdx.y;
-  if (y >= Fl.ny) return;  // whole warp
-  const int ncol = C.nx + 1;
-  float* sE = sE_all + w * 3 * ncol;
-  const int Y0 = y / F, Z0 = z / F, oy = y - F * Y0, oz = z - F * Z0;
-  const float wy[2] = {(float)(F - oy) / (float)F, (float)oy / (float)F};
-  const float wz[2] = {(float)(F - oz) / (float)F, (float)oz / (float)F};
-  const long long cpx = C.px, cpxy = (long long)C.px * C.py;
-  for (int X = lane; X < ncol; X += 32) {
-    const long long c0 = C.nidx(X, Y0, Z0);
+  const unsigned ng = (unsigned)Fl.px / 4, idx = blockIdx.x * PRO_T + threadIdx.x;
+  const int y = (int)(idx / ng), g = (int)(idx - (unsigned)y * ng), Z0 = blockIdx.y;
+  if (y >= Fl.ny) return;
+  const long long NP = Fl.NP, pxy = (long long)Fl.px * Fl.py;
+  const long long p0 = 4 * g + (long long)Fl.px * (y + 1) + pxy * (F * Z0 + 1);
+  const int nz = min(F, Fl.nz - F * Z0);
+  float4 u[F][3];
+  uchar4 cl[F];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float s = 0;
+  for (int j = 0; j < F; j++) {
+    if (j >= nz) break;
+    cl[j] = *reinterpret_cast<const uchar4*>(Fl.vclass + p0 + j * pxy);
 #pragma unroll
-      for (int k = 0; k < 4; k++) s += wy[k & 1] * wz[k >> 1] * uc[c0 + (k & 1) * cpx + (k >> 1) * cpxy + c * C.NP];
-      sE[c * ncol + X] = s;
-    }
+    for (int c = 0; c < 3; c++) u[j][c] = *reinterpret_cast<const float4*>(uf + p0 + j * pxy + c * NP);
   }
-  __syncwarp();
-  const long long NP = Fl.NP, rb = (long long)Fl.px * ((y + 1) + (long long)Fl.py * (z + 1));
-  for (int gq = lane; 4 * gq < Fl.px; gq += 32) {
-    const long long p0 = rb + 4 * gq;
-    const uchar4 cl4 = *reinterpret_cast<const uchar4*>(Fl.vclass + p0);
-    const uint8_t cls[4] = {cl4.x, cl4.y, cl4.z, cl4.w};
+  // coarse columns XB, XB + 1, XB + 2 (halo ones are zero) at the two planes, folded along y
+  const int XB = F == 4 ? g - 1 : 2 * g - 1, Y0 = y / F, oy = y - F * Y0;
+  const float wy1 = (float)oy / (float)F, wy0 = (float)(F - oy) / (float)F;
+  float e[2][3][3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const long long c0 = C.nidx(min(XB + i, C.nx), Y0, Z0);
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const float* q = uc + c0 + (long long)k * C.px * C.py + c * C.NP;
+        e[k][i][c] = wy0 * q[0] + wy1 * q[C.px];
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < F; j++) {
+    if (j >= nz) break;
+    const uint8_t cls[4] = {cl[j].x, cl[j].y, cl[j].z, cl[j].w};
     bool upd[4];
-    bool any = false;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const int x = 4 * gq - 1 + k;
-      upd[k] = x >= 0 && x < Fl.nx && (cls[k] & NC_ACTIVE) && !(cls[k] & NC_SUPPORT);
-      any = any || upd[k];
+      const int x = 4 * g - 1 + k;
+      upd[k] = x >= 0 && x < Fl.nx && (cls[k] & (NC_ACTIVE | NC_SUPPORT)) == NC_ACTIVE;
     }
-    if (!any) continue;
-    float u[3][4];
+    if (!(upd[0] || upd[1] || upd[2] || upd[3])) continue;
+    const float w1 = (float)j / (float)F, w0 = (float)(F - j) / (float)F;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      const float4 m = *reinterpret_cast<const float4*>(uf + p0 + c * NP);
-      u[c][0] = m.x; u[c][1] = m.y; u[c][2] = m.z; u[c][3] = m.w;
+      float E[3], v[4] = {u[j][c].x, u[j][c].y, u[j][c].z, u[j][c].w};
+#pragma unroll
+      for (int i = 0; i < 3; i++) E[i] = w0 * e[0][i][c] + w1 * e[1][i][c];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        // node 4 g - 1 + k lies ox past column XB + i
+        const int t = F - 1 + k, i = t / F, ox = t - F * i;
+        const float a = (float)(F - ox) / (float)F, b = (float)ox / (float)F;
+        if (upd[k]) v[k] += ox == 0 ? E[i] : a * E[i] + b * E[min(i + 1, 2)];
+      }
+      *reinterpret_cast<float4*>(uf + p0 + j * pxy + c * NP) = make_float4(v[0], v[1], v[2], v[3]);
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (!upd[k]) continue;
-      const int x = 4 * gq - 1 + k, X0 = x / F, ox = x - F * X0;
-      const float w1 = (float)ox / (float)F, w0 = (float)(F - ox) / (float)F;
-#pragma unroll
-      for (int c = 0; c < 3; c++) u[c][k] = u[c][k] + (w0 * sE[c * ncol + X0] + w1 * sE[c * ncol + X0 + 1]);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-      *reinterpret_cast<float4*>(uf + p0 + c * NP) = make_float4(u[c][0], u[c][1], u[c][2], u[c][3]);
   }
 }
 
@@ -2145,20 +2074,12 @@ template <typename T>
 rso_status prolong(rso_handle* h, int cl, const T* uc, T* uf) {
   const Level& f = h->L[cl - 1];
   const Level& c = h->L[cl];
-  const size_t row_smem = sizeof(float) * PROW_WARPS * 3 * (c.nx + 1);
-  if (sizeof(T) == 4 && f.nb == 1 && (c.factor == 4 || c.factor == 2) && row_smem <= 48 * 1024) {
-    const dim3 g((unsigned)cdiv(f.ny, PROW_WARPS), f.nz);
+  if (sizeof(T) == 4 && f.nb == 1 && (c.factor == 4 || c.factor == 2)) {
+    const dim3 g((unsigned)cdiv((long long)(f.px / 4) * f.ny, PRO_T), cdiv(f.nz, c.factor));
     if (c.factor == 4)
-      launch_pdl(k_prolong_row<4>, g, dim3(32, PROW_WARPS), row_smem, h->stream, f, c, (const float*)uc, (float*)uf);
+      launch_pdl(k_prolong_slab<4>, g, dim3(PRO_T), 0, h->stream, f, c, (const float*)uc, (float*)uf);
     else
-      launch_pdl(k_prolong_row<2>, g, dim3(32, PROW_WARPS), row_smem, h->stream, f, c, (const float*)uc, (float*)uf);
-    rso::note_launch();
-  } else if (sizeof(T) == 4 && f.nb == 1 && (c.factor == 4 || c.factor == 2)) {
-    const unsigned nblk = (unsigned)cdiv(f.NP / 4, 256);
-    if (c.factor == 4)
-      k_prolong_v4<4><<<nblk, 256, 0, h->stream>>>(f, c, (const float*)uc, (float*)uf);
-    else
-      k_prolong_v4<2><<<nblk, 256, 0, h->stream>>>(f, c, (const float*)uc, (float*)uf);
+      launch_pdl(k_prolong_slab<2>, g, dim3(PRO_T), 0, h->stream, f, c, (const float*)uc, (float*)uf);
     rso::note_launch();
   } else if (c.factor == 4) {
     launch_pdl(k_prolong<T, 4>, node_grid(f), dim3(32, 8), 0, h->stream, f, c, uc, uf); rso::note_launch();

@@ -1092,8 +1092,8 @@ __global__ void __launch_bounds__(256) k_fine_jacobi0(const Level L, const T* __
 // elements) as one 16-byte and one scalar load per row.  The diagonal block
 // comes from signed sums of the rows' pair sums and differences, as in
 // k_fine_p.  Bound by the bytes (28 a node) since the block takes 20 additions
-// and not 48 multiply-adds a node (256^3: 124 -> 104 us).  Halo rows are
-// skipped; the halo nodes of a group are written as zero.
+// and not 48 multiply-adds a node and all loads go out together (256^3: 124 ->
+// 92 us).  Halo rows are skipped; the halo nodes of a group are written as zero.
 __global__ void __launch_bounds__(256) k_fine_jacobi0_v4(const Level L, const float* __restrict__ f,
                                                          float* __restrict__ out, const float* __restrict__ rp,
                                                          float omega) {
@@ -1109,68 +1109,60 @@ __global__ void __launch_bounds__(256) k_fine_jacobi0_v4(const Level L, const fl
   const unsigned rem = p0u - (unsigned)zp * pxyu;
   const int yp = (int)(rem / pxu), xp = (int)(rem - (unsigned)yp * pxu);
   if (zp < 1 || zp > L.nz || yp < 1 || yp > L.ny) return;
+  // all loads of the group go out together, whatever its nodes' classes
   const uchar4 cl4 = *reinterpret_cast<const uchar4*>(L.vclass + p0);
-  const uint8_t cls[4] = {cl4.x, cl4.y, cl4.z, cl4.w};
-  bool work[4];
-  bool any = false;
+  float fv[3][4];
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int x = xp + k - 1;
-    work[k] = x >= 0 && x < L.nx && (cls[k] & NC_ACTIVE) && !(cls[k] & NC_SUPPORT);
-    any = any || work[k];
+  for (int c = 0; c < 3; c++) {
+    const float4 m = *reinterpret_cast<const float4*>(f + p0 + c * NP);
+    fv[c][0] = m.x; fv[c][1] = m.y; fv[c][2] = m.z; fv[c][3] = m.w;
   }
+  // element rows (y-1+b, z-1+c) of the nodes' 8 elements; element x of node
+  // x + a - 1 ... padded element index xp + j - 1 for j = 0..4
+  const long long qx = L.qx, qxy = (long long)L.qx * L.qy;
+  float rr[4][5];
+#pragma unroll
+  for (int row = 0; row < 4; row++) {
+    const long long e = (long long)(yp - 1 + (row & 1)) * qx + (long long)(zp - 1 + (row >> 1)) * qxy;
+    // padded element x index xp - 1 + j: elements x - 1 + a of node x = xp - 1 + k
+    const float* rowp = rp + e + xp;
+    rr[row][0] = xp > 0 ? rowp[-1] : 0.f;
+    if (xp + 4 <= L.qx) {
+      const float4 m = *reinterpret_cast<const float4*>(rowp);
+      rr[row][1] = m.x; rr[row][2] = m.y; rr[row][3] = m.z; rr[row][4] = m.w;
+    } else {
+#pragma unroll
+      for (int j = 1; j < 5; j++) rr[row][j] = (xp + j - 1 < L.qx) ? rowp[j - 1] : 0.f;
+    }
+  }
+  const uint8_t cls[4] = {cl4.x, cl4.y, cl4.z, cl4.w};
   float o[3][4];
 #pragma unroll
   for (int c = 0; c < 3; c++)
 #pragma unroll
     for (int k = 0; k < 4; k++) o[c][k] = 0.f;
-  if (any) {
-    // element rows (y-1+b, z-1+c) of the nodes' 8 elements; element x of node
-    // x + a - 1 ... padded element index xp + j - 1 for j = 0..4
-    const long long qx = L.qx, qxy = (long long)L.qx * L.qy;
-    float rr[4][5];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int x = xp + k - 1;
+    if (!(x >= 0 && x < L.nx && (cls[k] & (NC_ACTIVE | NC_SUPPORT)) == NC_ACTIVE)) continue;
+    // per element row (y side + 2 (z side)): sum and difference of its two elements
+    float S[4], T[4];
 #pragma unroll
     for (int row = 0; row < 4; row++) {
-      const long long e = (long long)(yp - 1 + (row & 1)) * qx + (long long)(zp - 1 + (row >> 1)) * qxy;
-      // padded element x index xp - 1 + j: elements x - 1 + a of node x = xp - 1 + k
-      const float* rowp = rp + e + xp;
-      rr[row][0] = xp > 0 ? rowp[-1] : 0.f;
-      if (xp + 4 <= L.qx) {
-        const float4 m = *reinterpret_cast<const float4*>(rowp);
-        rr[row][1] = m.x; rr[row][2] = m.y; rr[row][3] = m.z; rr[row][4] = m.w;
-      } else {
-#pragma unroll
-        for (int j = 1; j < 5; j++) rr[row][j] = (xp + j - 1 < L.qx) ? rowp[j - 1] : 0.f;
-      }
+      S[row] = rr[row][k + 1] + rr[row][k];
+      T[row] = rr[row][k + 1] - rr[row][k];
     }
-    float fv[3][4];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float4 m = *reinterpret_cast<const float4*>(f + p0 + c * NP);
-      fv[c][0] = m.x; fv[c][1] = m.y; fv[c][2] = m.z; fv[c][3] = m.w;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (!work[k]) continue;
-      // per element row (y side + 2 (z side)): sum and difference of its two elements
-      float S[4], T[4];
-#pragma unroll
-      for (int row = 0; row < 4; row++) {
-        S[row] = rr[row][k + 1] + rr[row][k];
-        T[row] = rr[row][k + 1] - rr[row][k];
-      }
-      const float a = cWp[W_DA].x * ((S[0] + S[1]) + (S[2] + S[3]));
-      const float b = cWp[W_DB].x * ((T[1] - T[0]) + (T[3] - T[2]));  // xy
-      const float c = cWp[W_DB].x * ((T[2] - T[0]) + (T[3] - T[1]));  // xz
-      const float e = cWp[W_DB].x * ((S[3] - S[2]) - (S[1] - S[0]));  // yz
-      const float r0 = fv[0][k], r1 = fv[1][k], r2 = fv[2][k];
-      const float A = a * a - e * e, B = c * e - b * a, C = b * e - c * a;
-      const float id = omega / (a * A + b * B + c * C);
-      const float E = a * a - c * c, F = b * c - a * e, I = a * a - b * b;
-      o[0][k] = id * (A * r0 + B * r1 + C * r2);
-      o[1][k] = id * (B * r0 + E * r1 + F * r2);
-      o[2][k] = id * (C * r0 + F * r1 + I * r2);
-    }
+    const float a = cWp[W_DA].x * ((S[0] + S[1]) + (S[2] + S[3]));
+    const float b = cWp[W_DB].x * ((T[1] - T[0]) + (T[3] - T[2]));  // xy
+    const float c = cWp[W_DB].x * ((T[2] - T[0]) + (T[3] - T[1]));  // xz
+    const float e = cWp[W_DB].x * ((S[3] - S[2]) - (S[1] - S[0]));  // yz
+    const float r0 = fv[0][k], r1 = fv[1][k], r2 = fv[2][k];
+    const float A = a * a - e * e, B = c * e - b * a, C = b * e - c * a;
+    const float id = omega / (a * A + b * B + c * C);
+    const float E = a * a - c * c, F = b * c - a * e, I = a * a - b * b;
+    o[0][k] = id * (A * r0 + B * r1 + C * r2);
+    o[1][k] = id * (B * r0 + E * r1 + F * r2);
+    o[2][k] = id * (C * r0 + F * r1 + I * r2);
   }
 #pragma unroll
   for (int c = 0; c < 3; c++)

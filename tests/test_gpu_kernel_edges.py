@@ -346,3 +346,22 @@ def test_chebyshev_sweeps(oracle, cuda, sweeps):
             rho = new
         u = u + step
     assert rel(got.cpu().numpy(), u) < 1e-11
+
+
+# boxes whose planes, rows and groups of four do not divide by the coarsening, one to three coarse columns wide
+@pytest.mark.parametrize("dims,factor", [((7, 5, 3), 2), ((13, 9, 6), 4), ((21, 10, 7), 2), ((33, 18, 11), 4)])
+def test_prolongation_and_first_step_fp32(oracle, cuda, dims, factor):
+    """FP32 prolongation and the fine level's step from zero; 2e-5 relative, the bound of the FP32 pieces."""
+    g, o = make(oracle, P.cantilever(*dims), n_levels=2, first_factor=factor)
+    g.update_stencil()
+    rng = np.random.default_rng(13)
+    cls = o.node_class()
+    fix = np.tile(((cls & 4) > 0) | ((cls & 1) == 0), 3)
+    _, vm = o.level_masks(1)
+    uc = rng.standard_normal(3 * vm.size) * np.tile(vm, 3)
+    uf = np.where(fix, 0.0, rng.standard_normal(3 * o.nn))
+    want = np.where(fix, 0.0, o.prolong(1, uc, uf))
+    assert rel(g.prolong_fp32(1, t(uc, cuda), t(uf, cuda)).cpu().numpy(), want) < 2e-5
+    z = np.zeros(3 * o.nn)
+    got = g.fine_sweep_fp32(3, t(z, cuda), t(uf, cuda), omega=0.3).cpu().numpy()
+    assert rel(got, o.smooth(0, z, uf, kind=1, omega=0.3, sweeps=1)) < 2e-5
