@@ -35,15 +35,55 @@ __device__ __forceinline__ double block_sum(double v) {
   return v;
 }
 
-__global__ void __launch_bounds__(RED_THREADS) k_dot_partial(const double* __restrict__ a, const double* __restrict__ b,
-                                                             long long n, double* __restrict__ part) {
+// Sum over the grid of every CTA's s (valid in thread 0): the last CTA to
+// arrive adds the partials, in an order that does not depend on arrival, and
+// resets the ticket.  A second launch for that cost 2 to 3 us, a fiftieth of a
+// CG iteration on 100 thousand nodes.
+__device__ __forceinline__ void grid_sum(double s, double* part, unsigned* ticket, double* out) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) s += __ldcg(part + i);
+  s = block_sum(s);
+  if (threadIdx.x == 0) {
+    *out = s;
+    *ticket = 0;
+  }
+}
+static unsigned* ticket_of(rso_handle* h) { return reinterpret_cast<unsigned*>(h->scal + 62); }
+
+// alpha = rz / pq for every thread of the CTA; CTA 0 keeps it, and rz as the
+// old one of the next beta (s: the scalars of solve_pcg_k32)
+__device__ __forceinline__ double cg_alpha(double* s, double* keep) {
+  __shared__ double sa;
+  if (threadIdx.x == 0) {
+    const double rz = s[3], a = rz / s[1];
+    sa = a;
+    if (blockIdx.x == 0) {
+      s[0] = rz;
+      s[2] = a;
+      if (keep) *keep = a;
+    }
+  }
+  __syncthreads();
+  return sa;
+}
+
+__global__ void __launch_bounds__(RED_THREADS) k_dot(const double* __restrict__ a, const double* __restrict__ b,
+                                                     long long n, double* part, unsigned* ticket, double* out) {
   pdl_wait(a, b);
   pdl_trigger();
   double s = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     s += a[i] * b[i];
-  s = block_sum(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(block_sum(s), part, ticket, out);
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_sumf_partial(const float* __restrict__ a, long long n,
@@ -65,20 +105,20 @@ __global__ void __launch_bounds__(RED_THREADS) k_final(const double* __restrict_
 }
 
 rso_status dot(rso_handle* h, const double* a, const double* b, long long n, double* dev_out) {
-  launch_pdl(k_dot_partial, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, a, b, n, h->red); rso::note_launch();
-  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, dev_out); rso::note_launch();
+  launch_pdl(k_dot, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, a, b, n, h->red, ticket_of(h), dev_out);
+  rso::note_launch();
   return launch_check(h, "dot");
 }
 
-// CG residual step fused with its norm: r -= a q, sum r.r, and (mixed
-// precision) the FP32 copy of r that the V-cycle smooths.  The matching
-// x += a p is deferred to the direction update, which reads p anyway.
-__global__ void __launch_bounds__(RED_THREADS) k_cg_resid_rr(long long n, const double* __restrict__ alpha,
-                                                             const double* __restrict__ q, double* __restrict__ r,
-                                                             float* __restrict__ r32, double* __restrict__ part) {
-  pdl_wait(alpha, q, r);
+// CG residual step fused with its scalars: alpha, r -= alpha q, r . r, and
+// (mixed precision) the FP32 copy of r that the V-cycle smooths.  The matching
+// x += alpha p is deferred to the direction update, which reads p anyway.
+__global__ void __launch_bounds__(RED_THREADS) k_cg_resid_rr(long long n, double* sc, const double* __restrict__ q,
+                                                             double* __restrict__ r, float* __restrict__ r32,
+                                                             double* part, unsigned* ticket) {
+  pdl_wait(sc, q, r);
   pdl_trigger();
-  const double a = *alpha;
+  const double a = cg_alpha(sc, nullptr);
   double s = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const double ri = r[i] - a * q[i];
@@ -86,8 +126,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_resid_rr(long long n, const 
     if (r32) r32[i] = (float)ri;
     s += ri * ri;
   }
-  s = block_sum(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(block_sum(s), part, ticket, sc + 5);
 }
 
 // sum a.b with b in FP32 (the mixed-precision preconditioned residual)
@@ -101,22 +140,21 @@ __global__ void __launch_bounds__(RED_THREADS) k_dot_df_partial(const double* __
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-rso_status cg_resid_rr(rso_handle* h, long long n, const double* alpha, const double* q, double* r, float* r32,
-                       double* rr_dev) {
-  launch_pdl(k_cg_resid_rr, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, n, alpha, q, r, r32, h->red); rso::note_launch();
-  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, rr_dev); rso::note_launch();
+rso_status cg_resid_rr(rso_handle* h, long long n, double* s, const double* q, double* r, float* r32) {
+  launch_pdl(k_cg_resid_rr, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, n, s, q, r, r32, h->red, ticket_of(h));
+  rso::note_launch();
   return launch_check(h, "cg_resid_rr");
 }
 
 // FP32 Krylov recurrence (reliable-update PCG): r -= a q in FP32 with the
 // sum r.r in FP64, and a.b of two FP32 vectors summed in FP64; 16-byte
 // vectors (3 NP is a multiple of 4 and the buffers are 256-byte aligned)
-__global__ void __launch_bounds__(RED_THREADS) k_cg32_resid_rr(long long n4, const double* __restrict__ alpha,
+__global__ void __launch_bounds__(RED_THREADS) k_cg32_resid_rr(long long n4, double* sc, double* keep,
                                                                const float4* __restrict__ q, float4* __restrict__ r,
-                                                               double* __restrict__ part) {
-  pdl_wait(alpha, q, r);
+                                                               double* part, unsigned* ticket) {
+  pdl_wait(sc, q, r);
   pdl_trigger();
-  const float a = (float)*alpha;
+  const float a = (float)cg_alpha(sc, keep);
   double s = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     const float4 qi = q[i];
@@ -128,8 +166,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg32_resid_rr(long long n4, con
     r[i] = ri;
     s += (double)ri.x * ri.x + (double)ri.y * ri.y + (double)ri.z * ri.z + (double)ri.w * ri.w;
   }
-  s = block_sum(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(block_sum(s), part, ticket, sc + 5);
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_dot_ff_partial(const float4* __restrict__ a,
@@ -144,15 +181,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_dot_ff_partial(const float4* __
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-rso_status cg32_resid_rr(rso_handle* h, long long n, const double* alpha, const float* q, float* r, double* rr_dev) {
+rso_status cg32_resid_rr(rso_handle* h, long long n, double* s, double* keep, const float* q, float* r) {
   if ((n & 3) || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(r)) & 15)) {
     h->err = "cg32_resid_rr: vectors must be 16-byte aligned multiples of 4 entries";
     return RSO_ERR_STATE;
   }
-  launch_pdl(k_cg32_resid_rr, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, n / 4, alpha,
-             reinterpret_cast<const float4*>(q), reinterpret_cast<float4*>(r), h->red);
+  launch_pdl(k_cg32_resid_rr, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h->stream, n / 4, s, keep,
+             reinterpret_cast<const float4*>(q), reinterpret_cast<float4*>(r), h->red, ticket_of(h));
   rso::note_launch();
-  launch_pdl(k_final, dim3(1), dim3(RED_THREADS), 0, h->stream, h->red, RED_BLOCKS, rr_dev); rso::note_launch();
   return launch_check(h, "cg32_resid_rr");
 }
 

@@ -359,15 +359,15 @@ rso_status launch_check(rso_handle* h, const char* what);
 // reductions (reduce.cu)
 rso_status dot(rso_handle* h, const double* a, const double* b, long long n, double* dev_out);
 rso_status dot_host(rso_handle* h, const double* a, const double* b, long long n, double* out);
-rso_status cg_resid_rr(rso_handle* h, long long n, const double* alpha, const double* q, double* r, float* r32,
-                       double* rr_dev);
+// s: the CG scalars (solve_pcg_k32): alpha = s[3] / s[1] to s[2] (and *keep), s[3] to s[0], r . r to s[5]
+rso_status cg_resid_rr(rso_handle* h, long long n, double* s, const double* q, double* r, float* r32);
 rso_status reduce_partials(rso_handle* h, const double* part, int n, double* dev_out);
 rso_status reduce_partials_batch(rso_handle* h, const double* part, int nper, int nb, double* dev_out,
                                  int stride = 1);
 rso_status norms2(rso_handle* h, long long n, const float* u, const float* r, double* dev_out);
 rso_status dot_df(rso_handle* h, const double* a, const float* b, long long n, double* dev_out);
 rso_status dot_ff(rso_handle* h, const float* a, const float* b, long long n, double* dev_out);
-rso_status cg32_resid_rr(rso_handle* h, long long n, const double* alpha, const float* q, float* r, double* rr_dev);
+rso_status cg32_resid_rr(rso_handle* h, long long n, double* s, double* keep, const float* q, float* r);
 rso_status fine_applyK_dot32(rso_handle* h, const float* u, float* f, double* dot_dev, int stride = 1);
 rso_status sum_float(rso_handle* h, const float* a, long long n, double* dev_out);
 

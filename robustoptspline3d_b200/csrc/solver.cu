@@ -203,30 +203,27 @@ rso_status precondition(rso_handle* h, const double* r, double* z) {
   return launch_check(h, "precondition");
 }
 
-// scalar updates on the device: s[0]=rz, s[1]=pq, s[2]=alpha, s[3]=rz_new, s[4]=beta
-__global__ void k_cg_alpha(double* s) {
-  pdl_wait(s);
-  pdl_trigger();
-  s[2] = s[0] / s[1];
-}
-__global__ void k_cg_beta(double* s) {
-  pdl_wait(s);
-  pdl_trigger();
-  s[4] = s[3] / s[0];
-  s[0] = s[3];
+// CG scalars on the device: s[0]=rz of the step before, s[1]=pq, s[2]=alpha, s[3]=rz, s[5]=rr
+// beta = rz / rz of the iteration before, for every thread of the CTA
+__device__ __forceinline__ double cg_beta(const double* s) {
+  __shared__ double sb;
+  if (threadIdx.x == 0) sb = s[3] / s[0];
+  __syncthreads();
+  return sb;
 }
 
 // x += alpha p (the step of the previous iteration); p = z + beta p
 template <typename Z>
-__global__ void k_cg_step_dir(long long n, const double* __restrict__ alpha, const double* __restrict__ beta,
-                              const Z* __restrict__ z, double* __restrict__ p, double* __restrict__ x) {
-  pdl_wait(alpha, beta, z, p, x);
+__global__ void k_cg_step_dir(long long n, const double* __restrict__ s, const Z* __restrict__ z,
+                              double* __restrict__ p, double* __restrict__ x) {
+  pdl_wait(s, z, p, x);
   pdl_trigger();
+  const double beta = cg_beta(s);
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double pi = p[i];
-  x[i] += (*alpha) * pi;
-  p[i] = (double)z[i] + (*beta) * pi;
+  x[i] += s[2] * pi;
+  p[i] = (double)z[i] + beta * pi;
 }
 __global__ void k_cg_step(long long n, const double* __restrict__ alpha, const double* __restrict__ p,
                           double* __restrict__ x) {
@@ -442,13 +439,14 @@ rso_status vcycle_double(rso_handle* h) { return vcycle_replayed(h, true); }
 // reliable-update PCG: x (FP64) += alpha p (FP32), and p = z + beta p in FP32
 // (DIR_ONLY: the direction update alone, x having taken the step already)
 template <bool DIR_ONLY>
-__global__ void k_cg32_step_dir(long long n4, const double* __restrict__ alpha, const double* __restrict__ beta,
-                                const float4* __restrict__ z, float4* __restrict__ p, double2* __restrict__ x) {
+__global__ void k_cg32_step_dir(long long n4, const double* __restrict__ s, const float4* __restrict__ z,
+                                float4* __restrict__ p, double2* __restrict__ x) {
+  const float b = (float)cg_beta(s);
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const float4 pi = p[i], zi = z[i];
   if (!DIR_ONLY) {
-    const double a = *alpha;
+    const double a = s[2];
     double2 x0 = x[2 * i], x1 = x[2 * i + 1];
     x0.x += a * pi.x;
     x0.y += a * pi.y;
@@ -457,7 +455,6 @@ __global__ void k_cg32_step_dir(long long n4, const double* __restrict__ alpha, 
     x[2 * i] = x0;
     x[2 * i + 1] = x1;
   }
-  const float b = (float)*beta;
   p[i] = make_float4(zi.x + b * pi.x, zi.y + b * pi.y, zi.z + b * pi.z, zi.w + b * pi.w);
 }
 __global__ void k_cg32_step(long long n4, const double* __restrict__ alpha, const float4* __restrict__ p,
@@ -505,22 +502,16 @@ __global__ void k_cg32_flush(long long n4, const double* __restrict__ alpha, con
 }
 // p_out = z + beta p_in in FP32 (the direction update of k_cg32_step_dir);
 // p_out may be p_in
-__global__ void k_cg32_dir(long long n4, const double* __restrict__ beta, const float4* __restrict__ z,
+__global__ void k_cg32_dir(long long n4, const double* __restrict__ s, const float4* __restrict__ z,
                            const float4* p_in, float4* p_out) {
-  pdl_wait(beta, z, p_in);
+  pdl_wait(s, z, p_in);
   pdl_trigger();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  float4 pi, zi;
+  if (i < n4) { pi = p_in[i]; zi = z[i]; }  // in flight during the division
+  const float b = (float)cg_beta(s);
   if (i >= n4) return;
-  const float4 pi = p_in[i], zi = z[i];
-  const float b = (float)*beta;
   p_out[i] = make_float4(zi.x + b * pi.x, zi.y + b * pi.y, zi.z + b * pi.z, zi.w + b * pi.w);
-}
-// alpha = rz / pq, also kept for the deferred step
-__global__ void k_cg_alpha_keep(double* s, double* keep) {
-  pdl_wait(s);
-  pdl_trigger();
-  s[2] = s[0] / s[1];
-  *keep = s[2];
 }
 
 // Mixed-precision PCG with the Krylov recurrence in FP32 (no counterpart in
@@ -631,14 +622,14 @@ __global__ void k_pcg_ctl_b(PcgCtl* c, const double* s, PcgGo g, int i, cudaGrap
 
 // the direction update of k_cg32_step_dir with the step taken or not as the
 // control block says (after a replacement x has taken it already)
-__global__ void k_cg32_step_dir_ctl(long long n4, const double* __restrict__ alpha, const double* __restrict__ beta,
-                                    const float4* __restrict__ z, float4* __restrict__ p, double2* __restrict__ x,
-                                    const PcgCtl* __restrict__ c) {
+__global__ void k_cg32_step_dir_ctl(long long n4, const double* __restrict__ s, const float4* __restrict__ z,
+                                    float4* __restrict__ p, double2* __restrict__ x, const PcgCtl* __restrict__ c) {
+  const float b = (float)cg_beta(s);
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const float4 pi = p[i], zi = z[i];
   if (!c->replace) {
-    const double a = *alpha;
+    const double a = s[2];
     double2 x0 = x[2 * i], x1 = x[2 * i + 1];
     x0.x += a * pi.x;
     x0.y += a * pi.y;
@@ -647,7 +638,6 @@ __global__ void k_cg32_step_dir_ctl(long long n4, const double* __restrict__ alp
     x[2 * i] = x0;
     x[2 * i + 1] = x1;
   }
-  const float b = (float)*beta;
   p[i] = make_float4(zi.x + b * pi.x, zi.y + b * pi.y, zi.z + b * pi.z, zi.w + b * pi.w);
 }
 
@@ -753,8 +743,7 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
       long long k1 = 0, kr = 0, kc = 0;
       st = add_if(h, G, prev ? &prev : nullptr, go.go[i], c->cs, [&]() -> rso_status {
         RSO_TRY(fine_applyK_dot32(h, p32, q32, s + 1));
-        launch_pdl(k_cg_alpha, dim3(1), dim3(1), 0, h->stream, s);
-        RSO_TRY(cg32_resid_rr(h, n3, s + 2, q32, r32, s + 5));
+        RSO_TRY(cg32_resid_rr(h, n3, s, nullptr, q32, r32));
         k_pcg_ctl_a<<<1, 1, 0, h->stream>>>(ctl, s, go, i, hr[i], hc[i]);
         return launch_check(h, "pcg graph");
       }, &node, &k1);
@@ -775,9 +764,8 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
         RSO_TRY(vcycle_launches(h, false));  // r . z into s[3] from its last fine step when h->vc_zdot says so
         const float* z32 = l0.u32;
         if (h->vc_zdot != s + 3) RSO_TRY(dot_ff(h, r32, z32, n3, s + 3));
-        launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s);
         k_cg32_step_dir_ctl<<<cdiv(n4, 256), 256, 0, h->stream>>>(
-            n4, s + 2, s + 4, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(p32),
+            n4, s, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(p32),
             reinterpret_cast<double2*>(x), ctl);
         return launch_check(h, "pcg graph");
       }, &node, &kc);
@@ -795,7 +783,7 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
   return st;
 }
 
-// Runs the loop from the state solve_pcg_k32 prepared (p, r32, q, s[0] = r.z)
+// Runs the loop from the state solve_pcg_k32 prepared (p, r32, q, s[3] = r.z)
 // on the device.  Returns RSO_ERR_UNSUPPORTED when no graph could be made
 // (nothing has run then; the host loop takes over).
 static rso_status pcg32_graph(rso_handle* h, const double* f, double* x, double tol, int max_iter, double fn,
@@ -862,7 +850,7 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
                                 rso_solve_info* info, bool* stalled, int* used, bool x_zero) {
   Level& l0 = h->L[0];
   const long long n3 = 3 * l0.NP, n4 = n3 / 4;
-  double* s = h->scal;  // s[0]=rz, s[1]=pq, s[2]=alpha, s[3]=rz_new, s[4]=beta, s[5]=rr
+  double* s = h->scal;  // s[0]=rz of the step before, s[1]=pq, s[2]=alpha, s[3]=rz, s[5]=rr
   float* r32 = l0.f32;  // the V-cycle's right-hand side (not rotated by the smoothers)
   // the V-cycle's result is L[0].u32, a pointer the Chebyshev and Jacobi
   // smoothers rotate: read it after every V-cycle
@@ -915,11 +903,10 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
       rso_handle* h;
       ~ZdotReset() { h->vc_zdot = nullptr; }
     } zreset{h};
-    h->vc_zdot = fuse ? s + 0 : nullptr;
+    h->vc_zdot = fuse ? s + 3 : nullptr;
     RSO_TRY(vcycle_mixed(h));
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(p32, l0.u32, sizeof(float) * n3, cudaMemcpyDeviceToDevice, h->stream));
-    if (!fuse) RSO_TRY(dot_ff(h, r32, l0.u32, n3, s + 0));
-    h->vc_zdot = fuse ? s + 3 : nullptr;
+    if (!fuse) RSO_TRY(dot_ff(h, r32, l0.u32, n3, s + 3));
     rso_status gs = RSO_ERR_UNSUPPORTED;
     if (h->solve_graphs && h->vc_graphs && !h->prof_on && h->stream && max_iter > 0)
       gs = pcg32_graph(h, f, x, tol, max_iter, fn, rbase, &it, &rel, stalled);
@@ -948,13 +935,8 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
     };
     while (it < max_iter) {
       RSO_TRY(fine_applyK_dot32(h, pc, q32, s + 1));
-      if (defer) {
-        launch_pdl(k_cg_alpha_keep, dim3(1), dim3(1), 0, h->stream, s, ring_alpha + pend); rso::note_launch();
-        pend++;
-      } else {
-        launch_pdl(k_cg_alpha, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
-      }
-      RSO_TRY(cg32_resid_rr(h, n3, s + 2, q32, r32, s + 5));
+      RSO_TRY(cg32_resid_rr(h, n3, s, defer ? ring_alpha + pend : nullptr, q32, r32));
+      if (defer) pend++;
       RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 5, s + 5, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
       RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
       vcycle_graphs_harvest(h);
@@ -991,21 +973,20 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
       RSO_TRY(vcycle_mixed(h));
       const float* z32 = l0.u32;
       if (!fuse) RSO_TRY(dot_ff(h, r32, z32, n3, s + 3));
-      launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
       if (defer) {
         if (pend == kStepRing) RSO_TRY(flush());
         float* pn = ring[pend];  // pc itself right after a flush of one step
-        launch_pdl(k_cg32_dir, dim3(cdiv(n4, 256)), dim3(256), 0, h->stream, n4, s + 4,
+        launch_pdl(k_cg32_dir, dim3(cdiv(n4, 256)), dim3(256), 0, h->stream, n4, s,
                    reinterpret_cast<const float4*>(z32), reinterpret_cast<const float4*>(pc),
                    reinterpret_cast<float4*>(pn));
         pc = pn;
       } else if (replace) {
         k_cg32_step_dir<true><<<cdiv(n4, 256), 256, 0, h->stream>>>(
-            n4, s + 2, s + 4, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(pc),
+            n4, s, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(pc),
             reinterpret_cast<double2*>(x));
       } else {
         k_cg32_step_dir<false><<<cdiv(n4, 256), 256, 0, h->stream>>>(
-            n4, s + 2, s + 4, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(pc),
+            n4, s, reinterpret_cast<const float4*>(z32), reinterpret_cast<float4*>(pc),
             reinterpret_cast<double2*>(x));
       }
       rso::note_launch();
@@ -1057,16 +1038,15 @@ rso_status solve_pcg(rso_handle* h, const double* f, double* x, double tol, int 
       k_d2f<<<cdiv(n3, 256), 256, 0, h->stream>>>(h->r, h->L[0].f32, n3); rso::note_launch();
       RSO_TRY(vcycle_mixed(h));
       k_f2d<<<cdiv(n3, 256), 256, 0, h->stream>>>(h->L[0].u32, h->p, n3); rso::note_launch();
-      RSO_TRY(dot_df(h, h->r, h->L[0].u32, n3, s + 0));
+      RSO_TRY(dot_df(h, h->r, h->L[0].u32, n3, s + 3));
     } else {
       RSO_TRY(precondition(h, h->r, h->z));
       RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->p, h->z, sizeof(double) * n3, cudaMemcpyDeviceToDevice, h->stream));
-      RSO_TRY(dot(h, h->r, h->z, n3, s + 0));
+      RSO_TRY(dot(h, h->r, h->z, n3, s + 3));
     }
     while (it < max_iter) {
       RSO_TRY(fine_applyK_dot(h, h->p, h->q, h->rp64, s + 1));
-      launch_pdl(k_cg_alpha, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
-      RSO_TRY(cg_resid_rr(h, n3, s + 2, h->q, h->r, mixed ? h->L[0].f32 : nullptr, s + 5));
+      RSO_TRY(cg_resid_rr(h, n3, s, h->q, h->r, mixed ? h->L[0].f32 : nullptr));
       RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 5, s + 5, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
       RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
       vcycle_graphs_harvest(h);
@@ -1081,14 +1061,12 @@ rso_status solve_pcg(rso_handle* h, const double* f, double* x, double tol, int 
       if (mixed) {
         RSO_TRY(vcycle_mixed(h));
         RSO_TRY(dot_df(h, h->r, h->L[0].u32, n3, s + 3));
-        launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
-        launch_pdl(k_cg_step_dir<float>, dim3(cdiv(n3, 256)), dim3(256), 0, h->stream, n3, s + 2, s + 4,
+        launch_pdl(k_cg_step_dir<float>, dim3(cdiv(n3, 256)), dim3(256), 0, h->stream, n3, s,
                    h->L[0].u32, h->p, x); rso::note_launch();
       } else {
         RSO_TRY(precondition(h, h->r, h->z));
         RSO_TRY(dot(h, h->r, h->z, n3, s + 3));
-        launch_pdl(k_cg_beta, dim3(1), dim3(1), 0, h->stream, s); rso::note_launch();
-        launch_pdl(k_cg_step_dir<double>, dim3(cdiv(n3, 256)), dim3(256), 0, h->stream, n3, s + 2, s + 4, h->z,
+        launch_pdl(k_cg_step_dir<double>, dim3(cdiv(n3, 256)), dim3(256), 0, h->stream, n3, s, h->z,
                    h->p, x); rso::note_launch();
       }
       RSO_TRY(launch_check(h, "pcg"));
