@@ -207,7 +207,7 @@ __global__ void k_filter(const Level L, const FOff* __restrict__ off, int noff, 
   }
 }
 
-// Radii from 1 to under 5.  A CTA of 32 x 16 threads marches along z through a
+// Radii from 1 to under 5.  A CTA of 32 x 8 threads marches along z through a
 // tile of columns.  Each plane, with its halo of RZ elements, is staged once in
 // shared memory as FP64 (so a value is converted once, not once per tap).  The
 // weight depends on the three distances alone, so the neighbour columns at the
@@ -220,8 +220,11 @@ __global__ void k_filter(const Level L, const FOff* __restrict__ off, int noff, 
 // (inside the box and all active) its part of the weight sum is known; else the
 // mask is summed as the values are.  256^3, R = 2: 1007 us with a thread walking
 // a tap table (loads and conversions), 464 with the columns' weights read from
-// shared memory, 241 now (the next plane's loads in flight during a plane's taps).
-constexpr int FTX = 32, FTY = 16, kFiltRZ = 4;
+// shared memory, 241 with the next plane's loads in flight during a plane's taps
+// and 16 rows a CTA, 209 now: with 8 rows an SM has four barriers to wait at in
+// turn instead of two, which is worth the wider halo, and a class is summed two
+// by two instead of in a chain.
+constexpr int FTX = 32, FTY = 8, kFiltRZ = 4;
 constexpr int fclass(int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; }
 constexpr int kFClasses = fclass(kFiltRZ, kFiltRZ) + 1;
 struct FPlan {
@@ -239,14 +242,22 @@ __device__ __forceinline__ void filter_taps(const FPlan& P, const T* p, double (
     for (int b = 0; b <= a; b++) {
       const int reach = P.reach[fclass(a, b)];
       if (reach < 0) continue;
-      T t = 0;  // FP32 for the mask: small whole numbers
+      // the class's columns, two by two (FP32 for the mask: small whole numbers)
+      T v[8];
+      int n = 0;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const int sx = q & 1 ? 1 : -1, sy = q & 2 ? 1 : -1;
         if ((a == 0 && sx > 0) || (b == 0 && sy > 0)) continue;
-        t += p[sy * b * WX + sx * a];
-        if (a != b) t += p[sx * a * WX + sy * b];
+        v[n++] = p[sy * b * WX + sx * a];
+        if (a != b) v[n++] = p[sx * a * WX + sy * b];
       }
+#pragma unroll
+      for (int m = 1; m < 8; m *= 2)
+#pragma unroll
+        for (int i = 0; i + m < 8; i += 2 * m)
+          if (i + m < n) v[i] += v[i + m];
+      const T t = v[0];
       const double s = (double)t;
 #pragma unroll
       for (int j = 0; j <= RZ; j++)
@@ -358,7 +369,7 @@ static rso_status filter_tiles(rso_handle* h, double R, const float* in, float* 
   const FPlan P = filter_plan(R, RZ);
   // planes per chunk: each chunk stages 2 RZ planes more than it writes, so
   // chunks are as long as the grid still has two CTAs per SM with them
-  int zc = 64;
+  int zc = 32;
   while (zc > 8 && (long long)cdiv(l.ex, FTX) * cdiv(l.ey, FTY) * cdiv(l.ez, zc) < 2 * 148) zc /= 2;
   const dim3 g(cdiv(l.ex, FTX), cdiv(l.ey, FTY), cdiv(l.ez, zc)), b(FTX, FTY);
   if (!adjoint) {
