@@ -21,9 +21,13 @@
 // restatement the tests compare with.
 #include "rso_internal.cuh"
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <numeric>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -653,6 +657,91 @@ void block_put(int dev, size_t cls, void* p) {
   cudaFree(p);
 }
 
+// Copies of tens of megabytes into ordinary host memory.  The driver's copy
+// moves them through its own staging buffer on one core, which also takes the
+// page faults of a destination that was never touched: 2.2 ms for 17 MB, where
+// the transfer needs 0.3 ms (four 17 MB results of the mesh input, 19 -> 13 ms
+// with the computations between them).  Here pieces go through a pinned ring, and a few
+// threads carry them on to the destination, each piece's slot being refilled
+// as soon as it is empty.  The ring (8 MB) is made on first use and kept; a
+// call that finds it in use, or any failure to get threads or pinned memory,
+// takes the driver's copy.
+namespace {
+constexpr size_t kPiece = size_t(1) << 20;
+constexpr int kSlots = 8, kCarriers = 4;
+struct HostRing {
+  std::mutex m;
+  char* slots = nullptr;
+};
+HostRing g_ring;
+
+struct Carry {
+  char* dst;
+  const char* src;
+  size_t n;
+  int dev;
+  cudaEvent_t landed[kSlots];
+  std::atomic<int> failed{0};
+  cudaError_t fetch(size_t piece) {  // piece into its slot, after everything before it on the default stream
+    const int slot = (int)(piece % kSlots);
+    const size_t o = piece * kPiece;
+    cudaError_t e = cudaMemcpyAsync(g_ring.slots + slot * kPiece, src + o, std::min(kPiece, n - o),
+                                    cudaMemcpyDeviceToHost, 0);
+    if (e == cudaSuccess) e = cudaEventRecord(landed[slot], 0);
+    return e;
+  }
+  // carrier t takes the pieces of slots t, t + kCarriers, ..: no other carrier touches them
+  void run(int t, int carriers) {
+    cudaError_t e = cudaSetDevice(dev);
+    const size_t np = (n + kPiece - 1) / kPiece;
+    for (size_t k = t; k < np && e == cudaSuccess; k++) {
+      const int slot = (int)(k % kSlots);
+      if (slot % carriers != t) continue;
+      e = cudaEventSynchronize(landed[slot]);
+      if (e != cudaSuccess) break;
+      std::memcpy(dst + k * kPiece, g_ring.slots + slot * kPiece, std::min(kPiece, n - k * kPiece));
+      if (k + kSlots < np) e = fetch(k + kSlots);
+    }
+    if (e != cudaSuccess) failed = (int)e;
+  }
+};
+}  // namespace
+
+cudaError_t copy_to_host(void* dst, const void* src, size_t n) {
+  cudaPointerAttributes at{};
+  std::unique_lock<std::mutex> lk(g_ring.m, std::defer_lock);
+  if (n < 4 * kPiece || cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type != cudaMemoryTypeUnregistered ||
+      !lk.try_lock() ||
+      (!g_ring.slots && cudaHostAlloc((void**)&g_ring.slots, kSlots * kPiece, cudaHostAllocPortable) != cudaSuccess)) {
+    cudaGetLastError();
+    return cudaMemcpy(dst, src, n, cudaMemcpyDeviceToHost);
+  }
+  Carry c;
+  c.dst = (char*)dst, c.src = (const char*)src, c.n = n;
+  cudaError_t e = cudaGetDevice(&c.dev);
+  int made = 0;
+  for (; made < kSlots && e == cudaSuccess; made++) {
+    e = cudaEventCreateWithFlags(&c.landed[made], cudaEventDisableTiming);
+    if (e != cudaSuccess) break;
+  }
+  for (size_t k = 0; k < (size_t)kSlots && k * kPiece < n && e == cudaSuccess; k++) e = c.fetch(k);
+  if (e == cudaSuccess) {
+    std::thread helper[kCarriers - 1];
+    int helpers = 0;
+    try {  // std::thread throws when the system has no thread to give
+      for (; helpers < kCarriers - 1; helpers++) helper[helpers] = std::thread(&Carry::run, &c, helpers + 1, kCarriers);
+    } catch (const std::system_error&) {
+    }
+    c.run(0, kCarriers);
+    for (int t = helpers + 1; t < kCarriers; t++) c.run(t, kCarriers);  // those without a thread of their own
+    for (int t = 0; t < helpers; t++) helper[t].join();
+    e = (cudaError_t)c.failed.load();
+  }
+  if (e != cudaSuccess) cudaStreamSynchronize(0);  // no copy into the ring outlives the call
+  for (int i = 0; i < made; i++) cudaEventDestroy(c.landed[i]);
+  return e;
+}
+
 namespace {
 
 static_assert(sizeof(rso_region) == 80 && sizeof(rso_field) == 192, "rso_region / rso_field layout is part of the ABI");
@@ -709,7 +798,7 @@ extern "C" rso_status rso_shell_elements(const float* vertices_host, int n_verti
     note_launch();
     s.err = cudaGetLastError();
   }
-  if (s.err == cudaSuccess) s.err = cudaMemcpy(shell_host, dshell, (size_t)nvox, cudaMemcpyDeviceToHost);
+  if (s.err == cudaSuccess) s.err = copy_to_host(shell_host, dshell, (size_t)nvox);
   return s.err == cudaSuccess ? RSO_OK : RSO_ERR_CUDA;
 }
 
@@ -826,7 +915,7 @@ extern "C" rso_status rso_region_mask(const rso_region* regions_host, int n_regi
     note_launch();
     s.err = cudaGetLastError();
   }
-  if (s.err == cudaSuccess) s.err = cudaMemcpy(mask_host, dm, (size_t)nn, cudaMemcpyDeviceToHost);
+  if (s.err == cudaSuccess) s.err = copy_to_host(mask_host, dm, (size_t)nn);
   return s.err == cudaSuccess ? RSO_OK : RSO_ERR_CUDA;
 }
 

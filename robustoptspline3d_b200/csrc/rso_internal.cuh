@@ -514,6 +514,8 @@ rso_status modified_pm(rso_handle* h, int cf, uint64_t seed, int max_itn, double
 // milliseconds).  At most kCacheCap bytes per device stay cached.
 cudaError_t block_get(int dev, size_t bytes, void** p, size_t* cls);
 void block_put(int dev, size_t cls, void* p);
+// device to ordinary host memory, after the default stream's work; returns when the bytes are there
+cudaError_t copy_to_host(void* dst, const void* src, size_t n);
 
 // device copies of host arrays and work buffers for one call; the blocks go
 // back to the cache when the call returns (every kernel of the call has

@@ -173,6 +173,6 @@ extern "C" rso_status rso_voxelize(const float* vertices_host, int n_vertices, c
     note_launch();
     s.err = cudaGetLastError();
   }
-  if (s.err == cudaSuccess) s.err = cudaMemcpy(solid_host, words, (size_t)nvox, cudaMemcpyDeviceToHost);
+  if (s.err == cudaSuccess) s.err = copy_to_host(solid_host, words, (size_t)nvox);
   return s.err == cudaSuccess ? RSO_OK : RSO_ERR_CUDA;
 }

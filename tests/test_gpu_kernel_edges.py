@@ -365,3 +365,18 @@ def test_prolongation_and_first_step_fp32(oracle, cuda, dims, factor):
     z = np.zeros(3 * o.nn)
     got = g.fine_sweep_fp32(3, t(z, cuda), t(uf, cuda), omega=0.3).cpu().numpy()
     assert rel(got, o.smooth(0, z, uf, kind=1, omega=0.3, sweeps=1)) < 2e-5
+
+
+@pytest.mark.parametrize("threads", [1, 3])
+@pytest.mark.parametrize("dims", [(160, 162, 161), (160, 163, 162), (256, 256, 257)])
+def test_large_masks_to_host(cuda, dims, threads):
+    """Results of 4 MB (just under and over the size that takes the pinned ring) and 17 MB (each slot of it
+    refilled) in ordinary memory, from one caller and from several at once; the same bytes."""
+    from concurrent.futures import ThreadPoolExecutor
+    from robustoptspline3d_b200 import boundary as B
+    z, y, x = np.meshgrid(*(np.arange(n) for n in dims[::-1]), indexing="ij", sparse=True)
+    want = ((x * 0.5 + y * 0.25 - z * 0.125 - 20.0) > 0).astype(np.uint8)
+    with ThreadPoolExecutor(threads) as pool:
+        got = list(pool.map(lambda _: B.region_mask([B.halfspace(0.5, 0.25, -0.125, -20.0)], (0, 0, 0), 1.0, dims),
+                            range(2 * threads)))
+    assert all(np.array_equal(m, want) for m in got)
