@@ -845,8 +845,9 @@ __global__ void k_elem_fixmask(const Level Fl, uint8_t* __restrict__ efix) {
 // come first.  For F = 2 the eight children enter directly.  A CTA takes GE
 // coarse elements: their moments go to shared memory once, then the 576 rows
 // pass in chunks of GM staged from T1; a thread accumulates 4 rows x 4 elements
-// in FP64.  256^3: 2668 us with 64 children and 4 x 2 outputs a thread (bound by
-// shared-memory reads), 941 now.
+// in FP64, 16 elements apart so that a store fills whole sectors.  256^3: 2668 us
+// with 64 children and 4 x 2 outputs a thread (bound by shared-memory reads),
+// 941 with the moments and four elements in a row, 642 now.
 constexpr int GE = 64, GM = 64;
 struct Phi { double v[3][4]; };  // phi[m][pos]
 template <int F>
@@ -896,7 +897,7 @@ __global__ void __launch_bounds__(256) k_galerkin_first(const Level Fl, const Le
       Ws[m][j] = child(E0 + j, m & 1, (m >> 1) & 1, m >> 2);
     }
   }
-  const int te = t & 15, ti = t >> 4;  // elements 4 te .. 4 te + 3, rows 4 ti .. 4 ti + 3 of the chunk
+  const int te = t & 15, ti = t >> 4;  // elements te, te + 16, .. (whole sectors a store), rows 4 ti .. 4 ti + 3 of the chunk
   for (int m0 = 0; m0 < 576; m0 += GM) {
     __syncthreads();  // Ws complete (first chunk); buf free
     for (int idx = t; idx < K * GM; idx += 256) {
@@ -909,9 +910,8 @@ __global__ void __launch_bounds__(256) k_galerkin_first(const Level Fl, const Le
     for (int k = 0; k < K; k++) {
       const double2 a01 = *reinterpret_cast<const double2*>(&buf[k * GM + 4 * ti]);
       const double2 a23 = *reinterpret_cast<const double2*>(&buf[k * GM + 4 * ti + 2]);
-      const double2 b01 = *reinterpret_cast<const double2*>(&Ws[k][4 * te]);
-      const double2 b23 = *reinterpret_cast<const double2*>(&Ws[k][4 * te + 2]);
-      const double a[4] = {a01.x, a01.y, a23.x, a23.y}, b[4] = {b01.x, b01.y, b23.x, b23.y};
+      const double a[4] = {a01.x, a01.y, a23.x, a23.y};
+      const double b[4] = {Ws[k][te], Ws[k][te + 16], Ws[k][te + 32], Ws[k][te + 48]};
 #pragma unroll
       for (int r = 0; r < 4; r++)
 #pragma unroll
@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(256) k_galerkin_first(const Level Fl, const Le
     for (int r = 0; r < 4; r++)
 #pragma unroll
       for (int c = 0; c < 4; c++)
-        if (E0 + 4 * te + c < C.ne) KE[(m0 + 4 * ti + r) * C.ne + E0 + 4 * te + c] = acc[r][c];
+        if (E0 + te + 16 * c < C.ne) KE[(m0 + 4 * ti + r) * C.ne + E0 + te + 16 * c] = acc[r][c];
   }
 }
 
