@@ -524,10 +524,8 @@ __global__ void k_spline_axis(int n, int order, int nb, float bmin, float step, 
 __device__ bool axis_basis(double u, int order, int nb, float bmin, float step, const float* knots, int* I,
                            double* N) {
   const float pf = (float)u;
-  const int i = (int)__fdiv_rn(__fsub_rn(pf, bmin), step) + order;
-  *I = i;
-  if (i < order || i > nb) return false;
-  const int span = i - 1, p = order - 1;
+  if (!knot_index(__fdiv_rn(__fsub_rn(pf, bmin), step), order, nb, I)) return false;
+  const int span = *I - 1, p = order - 1;
   double left[6], right[6];
   N[0] = 1.0;
   for (int j = 1; j <= p; j++) {

@@ -303,6 +303,17 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);  // a failure is the next launch_check's
 }
 
+// First-knot index trunc(q) + order of q = (coordinate - first knot) / step;
+// false outside the knots.  The range is tested before the conversion: a
+// coordinate past the integers (where an infinite coefficient's gradient sends
+// a probe) would overflow the sum, pass for an index inside and be read far out
+// of range.  NaN gives `order`, an index inside.
+__device__ __forceinline__ bool knot_index(float q, int order, int nb, int* i) {
+  if (q <= -1.f || q >= (float)(nb - order + 1)) return false;
+  *i = (int)q + order;
+  return true;
+}
+
 // a barrier wait gives up after this many SM clock cycles (about 2 s)
 constexpr long long kGbarCycles = 4000000000LL;
 

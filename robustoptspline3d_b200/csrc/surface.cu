@@ -70,10 +70,8 @@ struct MCGrid {
 __device__ bool basis_vd(const SplineP& S, int a, double u, int* I, double* N, double* dN) {
   const int o = S.order, p = o - 1;
   const float pf = __double2float_rn(u);
-  const int i = (int)__fdiv_rn(__fsub_rn(pf, S.bmin[a]), S.step[a]) + o;
-  *I = i;
-  if (i < o || i > S.nb[a]) return false;
-  const int span = i - 1;
+  if (!knot_index(__fdiv_rn(__fsub_rn(pf, S.bmin[a]), S.step[a]), o, S.nb[a], I)) return false;
+  const int span = *I - 1;
   const float* K = S.kn[a];
   double ndu[5][5], left[5], right[5];
   ndu[0][0] = 1.0;

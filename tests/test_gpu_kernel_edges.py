@@ -380,3 +380,30 @@ def test_large_masks_to_host(cuda, dims, threads):
         got = list(pool.map(lambda _: B.region_mask([B.halfspace(0.5, 0.25, -0.125, -20.0)], (0, 0, 0), 1.0, dims),
                             range(2 * threads)))
     assert all(np.array_equal(m, want) for m in got)
+
+
+@pytest.mark.parametrize("order", [2, 3, 4, 5])
+def test_probe_past_the_integers(oracle, cuda, order):
+    """Probes and surface points at coordinates past the integers lie outside the knots: probe sums and
+    counts equal to the oracle's for finite coefficients, and no error, with the same results
+    afterwards, for infinite ones and points."""
+    g, o = make(oracle, P.voids_box(12, 10, 8, nvoids=1), n_levels=2, first_factor=2)
+    n = o.spline_setup(order, (3, 2, 4))
+    assert g.set_spline_partition(3, 2, 4, order) == n
+    c = np.random.default_rng(41).normal(0.5, 0.15, n).astype(np.float32)
+    big = (np.float32(1e15) * (c - np.float32(0.5))).astype(np.float32)
+    _, _, _, cnt, ds = g.deal_background_points(big, 8.0, 4)
+    _, _, _, cnto, dso = o.selfsupport(big.astype(np.float64), 8.0, 4)
+    assert cnt == cnto and ds == dso
+    before = g.deal_background_points(c, 8.0, 4)
+    inf = c.copy()
+    inf[n // 2] = np.inf
+    inf[n // 3] = -np.inf
+    g.deal_background_points(inf, 8.0, 4)
+    after = g.deal_background_points(c, 8.0, 4)
+    assert all(cuda.equal(a, b) if isinstance(a, cuda.Tensor) else a == b for a, b in zip(before, after))
+    pts = np.random.default_rng(43).uniform(1, 7, (3, 40)).astype(np.float32)
+    g.uploadSurfacePoints(pts)
+    want = g.deal_surface_points(c, 8.0, 5)[1]
+    g.uploadSurfacePoints(np.concatenate([pts, np.array([[1e12, 3e38, np.inf], [2, -np.inf, 3], [3, 2, 1e12]], np.float32)], 1))
+    assert cuda.equal(g.deal_surface_points(c, 8.0, 5)[1][:40], want)
