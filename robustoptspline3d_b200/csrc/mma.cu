@@ -66,12 +66,13 @@ constexpr double MMA_C = 10.0, MMA_D = 1.0, MMA_A0 = 1.0;
 // CTA adds the partials up in the same order.  False once a barrier wait has
 // given up.
 template <int R>
-__device__ bool grid_reduce(double (&v)[R], unsigned mx, const MmaArgs& A, int& parity, unsigned& goal, double* res,
+__device__ bool grid_reduce(double (&v)[R], unsigned long long mx, const MmaArgs& A, int& parity, unsigned& goal, double* res,
                             double (*sh)[MMA_UT / 32]) {
+  static_assert(R <= MMA_RED && R <= 64, "a bit of the maxima mask and a slot per value");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const bool m = (mx >> r) & 1u;
+    const bool m = (mx >> r) & 1ull;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const double t = __shfl_down_sync(0xffffffffu, v[r], o);
@@ -84,7 +85,7 @@ __device__ bool grid_reduce(double (&v)[R], unsigned mx, const MmaArgs& A, int& 
   parity ^= 1;
   if (threadIdx.x < R) {
     const int r = threadIdx.x;
-    const bool m = (mx >> r) & 1u;
+    const bool m = (mx >> r) & 1ull;
     double acc = sh[r][0];
     for (int k = 1; k < MMA_UT / 32; k++) acc = m ? fmax(acc, sh[r][k]) : acc + sh[r][k];
     if (gridDim.x == 1) res[r] = acc;
@@ -96,7 +97,7 @@ __device__ bool grid_reduce(double (&v)[R], unsigned mx, const MmaArgs& A, int& 
   }
   if (!rso::gbar_sync(A.bar, goal, threadIdx.x, gridDim.x)) return false;
   for (int r = warp; r < R; r += MMA_UT / 32) {
-    const bool m = (mx >> r) & 1u;
+    const bool m = (mx >> r) & 1ull;
     double acc = m ? -1e300 : 0.0;
     for (int k = lane; k < (int)gridDim.x; k += 32) {
       const double t = __ldcg(part + (long long)r * gridDim.x + k);
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(MMA_UT, 1) k_mma_update(const __grid_constant_
       A.xi[i] = fmax(1.0 / (xv - al), 1.0);
       A.eta[i] = fmax(1.0 / (be - xv), 1.0);
     }
-    MMA_REDUCE(v, 0u);
+    MMA_REDUCE(v, 0ull);
     if (threadIdx.x == 0) {
       for (int j = 0; j < M; j++) {
         D.b[j] = res[j] - A.g[j];
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(MMA_UT, 1) k_mma_update(const __grid_constant_
         v[NS + 4] = fmax(v[NS + 4], fabs(rxs));
         v[NS + 5] = fmax(v[NS + 5], fabs(ret));
       }
-      MMA_REDUCE(v, 7u << (NS + 3));
+      MMA_REDUCE(v, 7ull << (NS + 3));
       if (threadIdx.x == 0) {
         const double *sg = res + M * M, *gp = res + M * M + M;
         double K[M + 1][M + 1], rhs[M + 1], sol[M + 1], hdy[M], Dy[M];
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(MMA_UT, 1) k_mma_update(const __grid_constant_
         v[2] = fmax(v[2], (-1 / cf) * di / xi);
         v[3] = fmax(v[3], (-1 / cf) * de / eta);
       }
-      MMA_REDUCE(v, 15u);
+      MMA_REDUCE(v, 15ull);
       if (threadIdx.x == 0) {
         double t3 = fmax(res[2], res[3]);
         auto art = [&](double dv, double w) { t3 = fmax(t3, (-1 / cf) * dv / w); };
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(MMA_UT, 1) k_mma_update(const __grid_constant_
         v[4 + M] = fmax(v[4 + M], fabs(rxs));
         v[5 + M] = fmax(v[5 + M], fabs(ret));
       }
-      MMA_REDUCE(v, 7u << (3 + M));
+      MMA_REDUCE(v, 7ull << (3 + M));
       if (threadIdx.x == 0) {
         double ny[M], nmu[M], ns[M];
         for (int j = 0; j < M; j++) {
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(MMA_UT, 1) k_mma_update(const __grid_constant_
       A.lastdx[i] = d1;
       v[0] += d1 * d1;
     }
-    MMA_REDUCE(v, 0u);
+    MMA_REDUCE(v, 0ull);
   }
 #undef MMA_REDUCE
   if (blockIdx.x == 0 && threadIdx.x == 0) {
