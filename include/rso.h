@@ -357,6 +357,11 @@ int rso_bottom_kernel(const rso_handle* h);
  * barrier state is reset afterwards, so the handle stays usable.  No fault and
  * no hang either way. */
 rso_status rso_grid_barrier_selftest(rso_handle* h, int short_by, double limit_ms, int* gave_up);
+/* For tests of the error path: leaves the handle's barrier as a wait that gave
+ * up leaves it.  Every CTA of the next kernel with a grid barrier returns at
+ * its first one, and the entry point that launched it fails with RSO_ERR_CUDA
+ * and clears the state. */
+rso_status rso_grid_barrier_give_up(rso_handle* h);
 /* Replay of the preconditioner's V-cycle (FP32 in mixed precision, else FP64) from CUDA
  * graphs (no counterpart in the reference, which launches every kernel):
  * on by default.  The V-cycle is captured the second time its launch

@@ -419,7 +419,7 @@ rso_status solve_pcg_batch(rso_handle* h, int k, const double* F, double* U, dou
           it[b] = iter;
           since[b]++;
           const double rn = std::sqrt(B.h_scal[b * KS + 5]);
-          if (!std::isfinite(rn)) { h->err = "non-finite residual in batched PCG"; return RSO_ERR_NONFINITE; }
+          if (!std::isfinite(rn)) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in batched PCG");
           rel[b] = rn / fn[b];
           rrec[b] = rn;
           if (rn < tol * fn[b] || rn < h->krylov32 * rbase[b] || iter >= max_iter || since[b] >= kCycleMax)
@@ -444,7 +444,7 @@ rso_status solve_pcg_batch(rso_handle* h, int k, const double* F, double* U, dou
             if (!((ask >> b) & 1ULL)) { left++; continue; }
             const double rtrue = std::sqrt(B.h_scal[b * KS + 5]);
             rel[b] = rtrue / fn[b];
-            if (!std::isfinite(rel[b])) { h->err = "non-finite residual in batched PCG"; return RSO_ERR_NONFINITE; }
+            if (!std::isfinite(rel[b])) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in batched PCG");
             if (rel[b] < tol) { done[b] = 1; continue; }
             cycles[b]++;
             if (rtrue > stall_ratio(h->krylov32, rrec[b] / rbase[b]) * rbase[b] ||
@@ -505,7 +505,7 @@ rso_status solve_pcg_batch(rso_handle* h, int k, const double* F, double* U, dou
           if (done[b]) continue;
           it[b] = used + iter;
           rel[b] = std::sqrt(B.h_scal[b * KS + 5]) / fn[b];
-          if (!std::isfinite(rel[b])) { h->err = "non-finite residual in batched PCG"; return RSO_ERR_NONFINITE; }
+          if (!std::isfinite(rel[b])) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in batched PCG");
           if (rel[b] < tol) done[b] = 2;  // converged in this iteration: x still takes this step
           else left++;
         }

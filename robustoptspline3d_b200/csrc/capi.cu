@@ -678,8 +678,7 @@ extern "C" rso_status rso_vcycle(rso_handle* h, double* u, const double* f, int 
   RSO_TRY(zero_support(h, h->w));
   RSO_TRY(vcycle_fp64(h, h->x, h->w, pre, post, symmetric, rel));
   RSO_TRY(unpad_nodes(h, 0, h->x, u));
-  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
-  return RSO_OK;
+  return fine_stage_check(h);  // synchronises; reports a barrier wait of the bottom kernel that gave up
 }
 
 extern "C" rso_status rso_solve(rso_handle* h, const double* f, double* u, double tol, int max_iter, int method,

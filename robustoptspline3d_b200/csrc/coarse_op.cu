@@ -2417,3 +2417,15 @@ extern "C" rso_status rso_grid_barrier_selftest(rso_handle* h, int short_by, dou
   *gave_up = flag != 0;
   return RSO_OK;
 }
+
+extern "C" rso_status rso_grid_barrier_give_up(rso_handle* h) {
+  if (!h) return RSO_ERR_INVALID_ARG;
+  if (!h->gbar) {
+    h->err = "grid barrier state not allocated";
+    return RSO_ERR_STATE;
+  }
+  const unsigned gone[4] = {kGbarGone, 0u, 1u, 0u};
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->gbar, gone, sizeof(gone), cudaMemcpyHostToDevice, h->stream));
+  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
+  return RSO_OK;
+}

@@ -1376,6 +1376,12 @@ rso_status fine_stage_check(rso_handle* h) {
   return RSO_OK;
 }
 
+rso_status solve_failed(rso_handle* h, rso_status st, const char* what) {
+  RSO_TRY(fine_stage_check(h));
+  h->err = what;
+  return st;
+}
+
 using PairKernel = void (*)(const Level, const float*, const float*, float*, const float*, float, double*,
                             const float*, float, int, const CUtensorMap, const CUtensorMap);
 template <int MODE, int TYP>

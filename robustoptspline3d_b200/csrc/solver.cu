@@ -841,7 +841,7 @@ static rso_status pcg32_graph(rso_handle* h, const double* f, double* x, double 
   note_launches(g->k_iter * hc.it + g->k_rep * hc.n_rep + g->k_cont * hc.n_cont);
   *it = hc.it;
   *rel = hc.rel;
-  if (hc.status == PCG_NONFINITE) { h->err = "non-finite residual in PCG"; return RSO_ERR_NONFINITE; }
+  if (hc.status == PCG_NONFINITE) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in PCG");
   *stalled = hc.status == PCG_STALLED;
   return RSO_OK;
 }
@@ -943,7 +943,7 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
       it++;
       since++;
       const double rnorm = std::sqrt(h->h_scal[5]);
-      if (!std::isfinite(rnorm)) { h->err = "non-finite residual in PCG"; return RSO_ERR_NONFINITE; }
+      if (!std::isfinite(rnorm)) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in PCG");
       const bool replace =
           rnorm < h->krylov32 * rbase || rnorm < tol * fn || it >= max_iter || since >= kCycleMax;
       if (replace) {
@@ -957,7 +957,7 @@ static rso_status solve_pcg_k32(rso_handle* h, const double* f, double* x, doubl
         RSO_TRY(true_residual_rr(&rn2));
         const double rtrue = std::sqrt(rn2);
         rel = rtrue / fn;
-        if (!std::isfinite(rel)) { h->err = "non-finite residual in PCG"; return RSO_ERR_NONFINITE; }
+        if (!std::isfinite(rel)) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in PCG");
         if (rel < tol || it >= max_iter) break;
         cycles++;
         if (rtrue > stall_ratio(h->krylov32, rnorm / rbase) * rbase ||
@@ -1053,7 +1053,7 @@ rso_status solve_pcg(rso_handle* h, const double* f, double* x, double tol, int 
       rn2 = h->h_scal[5];
       it++;
       rel = std::sqrt(rn2) / fn;
-      if (!std::isfinite(rel)) { h->err = "non-finite residual in PCG"; return RSO_ERR_NONFINITE; }
+      if (!std::isfinite(rel)) return solve_failed(h, RSO_ERR_NONFINITE, "non-finite residual in PCG");
       if (rel < tol || it >= max_iter) {
         k_cg_step<<<cdiv(n3, 256), 256, 0, h->stream>>>(n3, s + 2, h->p, x); rso::note_launch();
         break;
@@ -1098,7 +1098,7 @@ rso_status solve_vcycles(rso_handle* h, const double* f, double* x, double tol, 
     RSO_TRY(dot_host(h, h->r, h->r, n3, &rn2));
     rel = std::sqrt(rn2) / fn;
     it++;
-    if (!std::isfinite(rel) || rel > 1e4) { h->err = "defect correction diverged"; return RSO_ERR_DIVERGED; }
+    if (!std::isfinite(rel) || rel > 1e4) return solve_failed(h, RSO_ERR_DIVERGED, "defect correction diverged");
   }
   RSO_TRY(displacement_project(h, x));
   RSO_TRY(fine_stage_check(h));

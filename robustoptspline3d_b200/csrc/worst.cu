@@ -273,7 +273,7 @@ rso_status modified_pm(rso_handle* h, int cf, uint64_t seed, int max_itn, double
   int itn = 0;
   while (itn++ < max_itn && (fch > 1e-4 || rr > 1e-2)) {
     RSO_TRY(vcycle_fp64(h, u, f, 1, 1, 0, &rr));
-    if (!std::isfinite(rr) || rr > 1e4) { h->err = "modified power method diverged"; return RSO_ERR_DIVERGED; }
+    if (!std::isfinite(rr) || rr > 1e4) return solve_failed(h, RSO_ERR_DIVERGED, "modified power method diverged");
     RSO_TRY(displacement_project(h, u));  // support-free problems (optimization.cpp:284-286)
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(f, u, sizeof(double) * n3, cudaMemcpyDeviceToDevice, h->stream));
     RSO_TRY(force_project(h, f, cf));
@@ -290,7 +290,7 @@ rso_status modified_pm(rso_handle* h, int cf, uint64_t seed, int max_itn, double
   }
   if (itn_out) *itn_out = itn;
   if (c_worst) RSO_TRY(dot_host(h, f, u, n3, c_worst));
-  return RSO_OK;
+  return fine_stage_check(h);
 }
 
 }  // namespace rso

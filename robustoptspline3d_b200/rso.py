@@ -118,6 +118,7 @@ SIGNATURES = {
     "rso_set_bottom_kernel": (_ci, [_vp, _ci]),
     "rso_bottom_kernel": (_ci, [_vp]),
     "rso_grid_barrier_selftest": (_ci, [_vp, _ci, _cd, _pi]),
+    "rso_grid_barrier_give_up": (_ci, [_vp]),
     "rso_set_krylov_fp32": (_ci, [_vp, _cd]),
     "rso_set_krylov_fp32_cycles": (_ci, [_vp, _ci]),
     "rso_displacement_project": (_ci, [_vp, _vp]),
@@ -559,6 +560,10 @@ class HierarchyGrid:
         self._chk(self.lib.rso_grid_barrier_selftest(self.h, int(short_by), float(limit_ms), ctypes.byref(out)),
                   "rso_grid_barrier_selftest")
         return int(out.value)
+
+    def grid_barrier_give_up(self):
+        """Leave the grid barrier as a wait that gave up leaves it (for tests of the error path)."""
+        self._chk(self.lib.rso_grid_barrier_give_up(self.h), "rso_grid_barrier_give_up")
 
     def set_solve_graphs(self, on):
         """Run the mixed PCG loop as one device-controlled CUDA graph per solve."""

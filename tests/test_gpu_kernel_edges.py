@@ -407,3 +407,29 @@ def test_probe_past_the_integers(oracle, cuda, order):
     want = g.deal_surface_points(c, 8.0, 5)[1]
     g.uploadSurfacePoints(np.concatenate([pts, np.array([[1e12, 3e38, np.inf], [2, -np.inf, 3], [3, 2, 1e12]], np.float32)], 1))
     assert cuda.equal(g.deal_surface_points(c, 8.0, 5)[1][:40], want)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_barrier_that_gave_up_is_reported(cuda, precision):
+    """Every entry point that runs the persistent kernels reports a grid-barrier wait that gave up, once,
+    and computes the same as before on its next call."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    from robustoptspline3d_b200.rso import RSOError
+    prob = P.cantilever(32, 16, 16)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None,
+                      Config(poisson_ratio=0.4, precision=precision, n_levels=3, first_factor=2))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    f = t(prob["f"], cuda)
+    z = cuda.zeros_like(f)
+    calls = [lambda: g.v_cycle(z, f, 2, 2)[0], lambda: g.solve(f, tol=1e-8)[0],
+             lambda: g.solve(f, tol=1e-3, max_iter=100, method=0)[0],
+             lambda: g.solve_batch(cuda.stack([f, 2 * f]), tol=1e-8)[0], lambda: g.modifiedPM(0, max_itn=5)[2],
+             lambda: (g.update_stencil(), g.stencil(1))[1]]
+    for i, call in enumerate(calls):
+        call()  # past the first capture of a V-cycle
+        want = call()
+        g.grid_barrier_give_up()
+        with pytest.raises(RSOError, match="grid-barrier"):
+            call()
+        assert cuda.equal(call(), want), i
