@@ -305,24 +305,24 @@ std::vector<uint64_t> vc_key(const rso_handle* h, bool rotating = true, bool fp6
   return k;
 }
 
-std::vector<uint64_t> vc_rotating(const rso_handle* h) {
+// the level vectors that a V-cycle of the precision rotates; those of the other
+// are not in its key, and a replay leaves them alone
+std::vector<uint64_t> vc_rotating(const rso_handle* h, bool fp64) {
   std::vector<uint64_t> k;
   for (const Level& l : h->L) {
-    push_bits(k, l.u32); push_bits(k, l.r32); push_bits(k, l.t32);
-    push_bits(k, l.u64); push_bits(k, l.r64); push_bits(k, l.t64);
+    if (fp64) { push_bits(k, l.u64); push_bits(k, l.r64); push_bits(k, l.t64); }
+    else { push_bits(k, l.u32); push_bits(k, l.r32); push_bits(k, l.t32); }
   }
   return k;
 }
 
-void vc_set_rotating(rso_handle* h, const std::vector<uint64_t>& v) {
+void vc_set_rotating(rso_handle* h, const std::vector<uint64_t>& v, bool fp64) {
   size_t i = 0;
   for (Level& l : h->L) {
-    std::memcpy(&l.u32, &v[i++], sizeof(float*));
-    std::memcpy(&l.r32, &v[i++], sizeof(float*));
-    std::memcpy(&l.t32, &v[i++], sizeof(float*));
-    std::memcpy(&l.u64, &v[i++], sizeof(double*));
-    std::memcpy(&l.r64, &v[i++], sizeof(double*));
-    std::memcpy(&l.t64, &v[i++], sizeof(double*));
+    static_assert(sizeof(float*) == sizeof(uint64_t) && sizeof(double*) == sizeof(uint64_t), "a pointer an entry");
+    std::memcpy(fp64 ? (void*)&l.u64 : (void*)&l.u32, &v[i++], sizeof(uint64_t));
+    std::memcpy(fp64 ? (void*)&l.r64 : (void*)&l.r32, &v[i++], sizeof(uint64_t));
+    std::memcpy(fp64 ? (void*)&l.t64 : (void*)&l.t32, &v[i++], sizeof(uint64_t));
   }
 }
 
@@ -368,7 +368,7 @@ static rso_status vcycle_replayed(rso_handle* h, bool fp64) {
       }
       RSO_CHECK_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
       note_launches(g.kernels);
-      vc_set_rotating(h, g.after);
+      vc_set_rotating(h, g.after, fp64);
       g.unread = prof_pairs_used(g.pairs);
       return launch_check(h, "vcycle graph");
     }
@@ -380,7 +380,7 @@ static rso_status vcycle_replayed(rso_handle* h, bool fp64) {
     return vcycle_launches(h, fp64);
   }
   // capture: the launches are recorded, not run; the graph then runs once
-  const std::vector<uint64_t> before = vc_rotating(h);
+  const std::vector<uint64_t> before = vc_rotating(h, fp64);
   VcGraph g;
   g.key = key;
   if (h->prof_on) g.pairs = prof_pairs_new(128);
@@ -415,10 +415,10 @@ static rso_status vcycle_replayed(rso_handle* h, bool fp64) {
     vc_drop(g);
     c->broken = true;
     cudaGetLastError();
-    vc_set_rotating(h, before);
+    vc_set_rotating(h, before, fp64);
     return vcycle_launches(h, fp64);
   }
-  g.after = vc_rotating(h);
+  g.after = vc_rotating(h, fp64);
   // the captured launches were counted when they were recorded
   RSO_CHECK_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
   g.unread = prof_pairs_used(g.pairs);
@@ -725,7 +725,7 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
   float* p32 = reinterpret_cast<float*>(h->z);
   float* q32 = reinterpret_cast<float*>(h->q);
   PcgCtl* ctl = c->ctl;
-  const std::vector<uint64_t> rot = vc_rotating(h);
+  const std::vector<uint64_t> rot = vc_rotating(h, false);
   cudaGraph_t G = nullptr;
   rso_status st = RSO_OK;
   do {
@@ -771,14 +771,14 @@ static rso_status build_solve_graph(rso_handle* h, SolveGraphs* c, const double*
       }, &node, &kc);
       if (st != RSO_OK) break;
       prev = node;
-      vc_set_rotating(h, rot);  // every unrolled V-cycle starts from the same vectors
+      vc_set_rotating(h, rot, false);  // every unrolled V-cycle starts from the same vectors
       g->k_iter = k1; g->k_rep = kr; g->k_cont = kc;
     }
     if (st != RSO_OK) break;
     if (cudaGraphInstantiate(&g->exec, G, 0) != cudaSuccess) { g->exec = nullptr; st = RSO_ERR_CUDA; }
   } while (false);
   if (G) cudaGraphDestroy(G);
-  vc_set_rotating(h, rot);
+  vc_set_rotating(h, rot, false);
   cudaGetLastError();  // a failed capture leaves its error here
   return st;
 }
