@@ -383,6 +383,9 @@ rso_status rso_set_vcycle_graphs(rso_handle* h, int on);
  * are on and per-kernel profiling is off; a failed capture falls back to the
  * host-driven loop.  Off by default. */
 rso_status rso_set_solve_graphs(rso_handle* h, int on);
+/* How many V-cycle graphs and solve graphs the handle has launched; NULL for
+ * either.  A count that stands still shows a fall-back to plain launches. */
+rso_status rso_graph_launches(const rso_handle* h, long long* vcycles, long long* solves);
 /* Krylov recurrence of the mixed-precision PCG (no counterpart in the
  * reference, whose CG is FP64).  0 < replace_factor < 1 (1e-2 by default in
  * mixed precision): the recurrence runs in FP32 (FP32 operator, FP32

@@ -532,6 +532,13 @@ extern "C" rso_status rso_set_solve_graphs(rso_handle* h, int on) {
   return RSO_OK;
 }
 
+extern "C" rso_status rso_graph_launches(const rso_handle* h, long long* vcycles, long long* solves) {
+  if (!h) return RSO_ERR_INVALID_ARG;
+  if (vcycles) *vcycles = h->graph_launches[0];
+  if (solves) *solves = h->graph_launches[1];
+  return RSO_OK;
+}
+
 extern "C" rso_status rso_set_krylov_fp32(rso_handle* h, double replace_factor) {
   if (!h || !(replace_factor >= 0.0) || !(replace_factor < 1.0)) return RSO_ERR_INVALID_ARG;
   h->krylov32 = replace_factor;

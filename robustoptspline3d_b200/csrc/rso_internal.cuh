@@ -194,6 +194,7 @@ struct rso_handle {
   void* vcg = nullptr;                             // captured V-cycles (solver.cu)
   void* cap_prof = nullptr;                        // event pairs of the V-cycle capture in progress (prof.cu)
   bool vc_graphs = true;                           // replay captured V-cycles (rso_set_vcycle_graphs)
+  long long graph_launches[2] = {0, 0};            // of V-cycle and solve graphs (rso_graph_launches)
   // run the FP32-Krylov PCG loop as one captured graph whose iterations and
   // residual replacements are decided on the device (rso_set_solve_graphs)
   bool solve_graphs = false;

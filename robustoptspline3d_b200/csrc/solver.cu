@@ -367,6 +367,7 @@ static rso_status vcycle_replayed(rso_handle* h, bool fp64) {
         vcycle_graphs_harvest(h);
       }
       RSO_CHECK_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
+      h->graph_launches[0]++;
       note_launches(g.kernels);
       vc_set_rotating(h, g.after, fp64);
       g.unread = prof_pairs_used(g.pairs);
@@ -421,6 +422,7 @@ static rso_status vcycle_replayed(rso_handle* h, bool fp64) {
   g.after = vc_rotating(h, fp64);
   // the captured launches were counted when they were recorded
   RSO_CHECK_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
+  h->graph_launches[0]++;
   g.unread = prof_pairs_used(g.pairs);
   if (c->graphs.size() >= kMaxGraphs) {
     if (c->graphs.front().unread) {
@@ -833,6 +835,7 @@ static rso_status pcg32_graph(rso_handle* h, const double* f, double* x, double 
   const int max_launches = max_iter / kSolveUnroll + 2;
   for (int launch = 0;; launch++) {
     RSO_CHECK_CUDA(h, cudaGraphLaunch(g->exec, h->stream));
+    h->graph_launches[1]++;
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(c->h_ctl, c->ctl, sizeof(PcgCtl), cudaMemcpyDeviceToHost, h->stream));
     RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
     if (hc.done) break;

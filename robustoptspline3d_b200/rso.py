@@ -113,6 +113,7 @@ SIGNATURES = {
     "rso_fine_sweep_fp32": (_ci, [_vp, _ci, _vp, _vp, _vp, ctypes.c_double, ctypes.c_double, _vp]),
     "rso_set_vcycle_graphs": (_ci, [_vp, _ci]),
     "rso_set_solve_graphs": (_ci, [_vp, _ci]),
+    "rso_graph_launches": (_ci, [_vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]),
     "rso_set_fine_zchunk": (_ci, [_vp, _ci]),
     "rso_fine_zchunk": (_ci, [_vp]),
     "rso_set_bottom_kernel": (_ci, [_vp, _ci]),
@@ -568,6 +569,12 @@ class HierarchyGrid:
     def set_solve_graphs(self, on):
         """Run the mixed PCG loop as one device-controlled CUDA graph per solve."""
         self._chk(self.lib.rso_set_solve_graphs(self.h, 1 if on else 0), "rso_set_solve_graphs")
+
+    def graph_launches(self):
+        """(V-cycle graphs, solve graphs) launched so far on this handle."""
+        v, s = ctypes.c_longlong(0), ctypes.c_longlong(0)
+        self._chk(self.lib.rso_graph_launches(self.h, ctypes.byref(v), ctypes.byref(s)), "rso_graph_launches")
+        return v.value, s.value
 
     def fine_sweep_fp32(self, op, u, f=None, uprev=None, omega=1.0, c1=0.0):
         """One FP32 fine-level sweep (op 0 residual, 1 K u, 2 Jacobi/Chebyshev step), FP64 in and out."""

@@ -433,3 +433,30 @@ def test_barrier_that_gave_up_is_reported(cuda, precision):
         with pytest.raises(RSOError, match="grid-barrier"):
             call()
         assert cuda.equal(call(), want), i
+
+
+@pytest.mark.parametrize("precision,smoother", [(0, 0), (0, 1), (0, 2), (1, 0), (1, 1), (1, 2)])
+def test_graphs_are_launched(cuda, precision, smoother):
+    """V-cycles are replayed from graphs, all but the first few of a second solve, and a mixed solve under
+    device control launches its own graph: none of them has fallen back to plain launches."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(48, 24, 24)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None,
+                      Config(precision=precision, smoother=smoother, poisson_ratio=0.4, n_levels=3, first_factor=2))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    f = t(prob["f"], cuda)
+    want, it, _, _ = g.solve(f, tol=1e-9)
+    v0, _ = g.graph_launches()
+    u, k, _, _ = g.solve(f, tol=1e-9)
+    v1, s1 = g.graph_launches()
+    assert k == it and cuda.equal(u, want)
+    assert v1 - v0 >= it - 4 and s1 == 0
+    g.set_vcycle_graphs(False)
+    g.solve(f, tol=1e-9)
+    assert g.graph_launches() == (v1, 0)
+    if precision == 1:
+        g.set_vcycle_graphs(True)
+        g.set_solve_graphs(True)
+        u, k, _, _ = g.solve(f, tol=1e-9)
+        assert g.graph_launches()[1] > 0 and k == it and cuda.equal(u, want)
