@@ -2340,12 +2340,14 @@ __global__ void k_seed_vec(const Level L, float* v, uint64_t seed, int zero_supp
 // smoothing step with c1 = -1, omega = -1 and no right-hand side or previous
 // iterate is the iteration itself, out = u - u + D^-1 K u, so an iteration is one
 // launch; the ratio of the last two norms is the estimate, summed in FP64 and
-// read by the host once for all levels.
+// read by the host once for kLamGroup levels (all of them but for a hierarchy
+// that was asked to go on past its last element).
+constexpr int kLamGroup = 12;
 rso_status estimate_lambda(rso_handle* h) {
   const int iters = 12, nl = (int)h->L.size(), levels = nl == 1 ? 1 : nl - 1;
-  if (2 * levels > 24) { h->err = "too many levels"; return RSO_ERR_STATE; }
-  double* sums = h->scal + 16;  // u.u, r.r per level
+  double* sums = h->scal + 16;  // u.u, r.r per level of the group
   for (int li = 0; li < levels; li++) {
+    const int slot = li % kLamGroup;
     Level& l = h->L[li];
     const long long n3 = 3 * l.NP;
     k_seed_vec<<<cdiv(l.NP, 256), 256, 0, h->stream>>>(l, l.u32, 777 + li, li == 0); rso::note_launch();
@@ -2353,15 +2355,16 @@ rso_status estimate_lambda(rso_handle* h) {
     for (int it = 0; it < iters; it++) {
       if (li == 0) RSO_TRY(fine_jacobi<float>(h, l.u32, l.f32, l.t32, h->rp32, -1.0, nullptr, -1.0));
       else RSO_TRY(coarse_jacobi<float>(h, li, l.u32, l.f32, l.t32, -1.0, nullptr, -1.0));
-      if (it + 1 == iters) RSO_TRY(norms2(h, n3, l.u32, l.t32, sums + 2 * li));
+      if (it + 1 == iters) RSO_TRY(norms2(h, n3, l.u32, l.t32, sums + 2 * slot));
       std::swap(l.u32, l.t32);
     }
-  }
-  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 16, sums, 2 * levels * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  RSO_TRY(fine_stage_check(h));  // synchronises
-  for (int li = 0; li < levels; li++) {
-    const double uu = h->h_scal[16 + 2 * li], rr = h->h_scal[17 + 2 * li];
-    h->L[li].lam = 1.05 * (uu > 0 ? std::sqrt(rr / uu) : 1.0);
+    if (slot + 1 < kLamGroup && li + 1 < levels) continue;
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 16, sums, 2 * (slot + 1) * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    RSO_TRY(fine_stage_check(h));  // synchronises
+    for (int k = 0; k <= slot; k++) {
+      const double uu = h->h_scal[16 + 2 * k], rr = h->h_scal[17 + 2 * k];
+      h->L[li - slot + k].lam = 1.05 * (uu > 0 ? std::sqrt(rr / uu) : 1.0);
+    }
   }
   return RSO_OK;
 }

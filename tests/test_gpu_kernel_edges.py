@@ -460,3 +460,24 @@ def test_graphs_are_launched(cuda, precision, smoother):
         g.set_solve_graphs(True)
         u, k, _, _ = g.solve(f, tol=1e-9)
         assert g.graph_launches()[1] > 0 and k == it and cuda.equal(u, want)
+
+
+@pytest.mark.parametrize("smoother", [0, 1, 2])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("levels", [12, 13, 14, 15])
+def test_more_levels_than_elements(cuda, levels, precision, smoother):
+    """A level count past the last element is accepted, as any other: the solution of two levels to 1e-6
+    relative (both solved to 1e-9), and a step size for every level."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(12, 8, 8)
+    u = []
+    for nl in (2, levels):
+        g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None,
+                          Config(precision=precision, smoother=smoother, n_levels=nl, first_factor=2))
+        g.set_density(prob["rho"].astype(np.float32).ravel())
+        g.update_stencil()
+        assert g.n_levels() == nl
+        u.append(g.solve(t(prob["f"], cuda), tol=1e-9, max_iter=400)[0].cpu().numpy())
+        if smoother != 0:
+            assert all(0 < g.level_lambda(i) < 10 for i in range(nl - 1))
+    assert rel(u[1], u[0]) < 1e-6
