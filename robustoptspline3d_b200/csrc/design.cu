@@ -121,11 +121,16 @@ rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens, int ener
 // eta), den = t0 + tanh(beta (1 - eta)), the same for every element.  One
 // exponential serves both maps: with E = exp(-2 |x|), tanh x = sign(x) (1 - E) /
 // (1 + E) and its slope is 4 E / (1 + E)^2, without the cancellation of
-// 1 - tanh^2 in the tails.  (256^3: 122 us with tanh and a thread per
+// 1 - tanh^2 in the tails.  1 - E cancels towards x = 0, an error of 2e-16 in
+// values of the size of beta / 2: below |beta| = 1e-3 (kStepSmall; 2e-13 there, an
+// FP32 result's last bit is 6e-8) the step takes tanh, and divides by den, whose
+// reciprocal may overflow.  (256^3: 122 us with tanh and a thread per
 // element, bound by instructions and by each thread's two dependent loads, 70 so,
 // a thread loading four elements of its column at once.)
-template <bool CHAIN>
-__global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* in, double beta, double t0, double rden,
+// scale: 1 / den, for the chain beta / den; SMALL: den
+constexpr double kStepSmall = 1e-3;
+template <bool CHAIN, bool SMALL = false>
+__global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* in, double beta, double t0, double scale,
                                                    double rmin, const uint8_t* shell, const float* gin, float* out,
                                                    const View V, int zc) {
   const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
@@ -148,12 +153,15 @@ __global__ void __launch_bounds__(256) k_heaviside(const Level L, const float* i
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       if (z + j >= n) break;
-      const double s = beta * ((double)a[j] - 0.5), E = exp(-2 * fabs(s)), q = __drcp_rn(1 + E);
+      const double s = beta * ((double)a[j] - 0.5);
       double v;
-      if (CHAIN) {
-        v = (double)g[j] * beta * (4 * E * q * q) * rden;
+      if constexpr (SMALL) {
+        v = (t0 + tanh(s)) / scale;
       } else {
-        v = (t0 + copysign((1 - E) * q, s)) * rden;
+        const double E = exp(-2 * fabs(s)), q = __drcp_rn(1 + E);
+        v = CHAIN ? (double)g[j] * (4 * E * q * q) * scale : (t0 + copysign((1 - E) * q, s)) * scale;
+      }
+      if (!CHAIN) {
         v = one[j] ? 1.0 : fmin(fmax(v, rmin), 1.0);
       }
       out[o0 + (z + j) * V.sz] = on[j] ? (float)v : 0.f;
@@ -165,8 +173,10 @@ rso_status heaviside(rso_handle* h, const float* in, double beta, const uint8_t*
   const Level& l = h->L[0];
   const double t0 = std::tanh(beta * 0.5), den = t0 + std::tanh(beta * (1 - 0.5));
   const int zc = column_chunk(l);
-  k_heaviside<false><<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, in, beta, t0, 1 / den, h->cfg.rho_min, shell,
-                                                                        nullptr, out, view_of(l, dense), zc); rso::note_launch();
+  const bool small = std::fabs(beta) < kStepSmall;
+  auto k = small ? k_heaviside<false, true> : k_heaviside<false>;
+  k<<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, in, beta, t0, small ? den : 1 / den, h->cfg.rho_min, shell,
+                                                       nullptr, out, view_of(l, dense), zc); rso::note_launch();
   return launch_check(h, "heaviside");
 }
 
@@ -174,7 +184,7 @@ rso_status heaviside_chain(rso_handle* h, const float* rho, double beta, const f
   const Level& l = h->L[0];
   const double t0 = std::tanh(beta * 0.5), den = t0 + std::tanh(beta * (1 - 0.5));
   const int zc = column_chunk(l);
-  k_heaviside<true><<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, rho, beta, t0, 1 / den, 0.0, nullptr, gin,
+  k_heaviside<true><<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, rho, beta, t0, beta / den, 0.0, nullptr, gin,
                                                                        gout, view_of(l, dense), zc); rso::note_launch();
   return launch_check(h, "heaviside_chain");
 }

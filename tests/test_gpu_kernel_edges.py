@@ -481,3 +481,24 @@ def test_more_levels_than_elements(cuda, levels, precision, smoother):
         if smoother != 0:
             assert all(0 < g.level_lambda(i) < 10 for i in range(nl - 1))
     assert rel(u[1], u[0]) < 1e-6
+
+
+@pytest.mark.parametrize("beta", [1e-310, 1e-14, 1e-9, 9.9e-4, 1e-3, 0.1, 8.0, 300.0, 1e5, -1e-12, -2.0])
+def test_heaviside_slopes(cuda, beta):
+    """The step and its slope against tanh in FP64, from nearly linear (where differences of exponentials
+    cancel) to a jump; one FP32 rounding, 1e-7 relative to one."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.voids_box(21, 13, 11, nvoids=1)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"],
+                      Config(n_levels=2, first_factor=2, rho_min=1e-3))
+    rng = np.random.default_rng(47)
+    x, gin = rng.uniform(0, 1, g.ne).astype(np.float32), rng.standard_normal(g.ne).astype(np.float32)
+    x[:9] = [0, 1, 0.5, 0.5 + 2.0 ** -24, 0.5 - 2.0 ** -25, 0.25, 0.75, 2, -1]
+    on = prob["emask"].ravel() > 0
+    s, th = beta * (x.astype(np.float64) - 0.5), np.tanh
+    den = 2 * th(beta * 0.5)
+    want = np.where(on, np.clip((th(beta * 0.5) + th(s)) / den, 1e-3, 1.0), 0.0)
+    assert np.max(np.abs(g.projectDensities(x, beta).cpu().numpy() - want)) < 1e-7
+    slope = np.where(on, gin * (beta / den) / np.cosh(np.minimum(np.abs(s), 300.0)) ** 2, 0.0)
+    got = g.projectSensitivity(x, beta, gin).cpu().numpy()
+    assert np.max(np.abs(got - slope)) < 1e-7 * max(1.0, np.max(np.abs(slope)))
