@@ -89,8 +89,18 @@ __device__ __forceinline__ D3 vertex(const float* __restrict__ vtx, int i) {
 // overlap in some hundred boxes, and nearly all of the FP64 work was there: one
 // CTA a face testing every solid element took 3.2 ms for 262144 faces on 256^3
 // elements, this 0.58 ms.  Faces whose box has more than kShellRows rows go to a
-// list that a second launch works off with the whole grid per face.
-constexpr int kShellRows = 2048;
+// list that a second launch works off by words of eight elements, its CTAs shared
+// out over the list (one face after the other on the whole grid, a thread a row,
+// left most threads idle: 277 ms for 40000 faces and w = 20 on 256^3, 12.6 so).
+// Meshes of fewer faces than the GPU holds warps (kShellFew; on grids of under 32
+// elements an edge, which all warps crowd on, kShellFewSmall) take one launch over
+// all of them, a thread an element, the CTAs shared out likewise: no states and no
+// list, whose three launches a coarse mesh does not earn back, and no lane walks a
+// row alone.  A call, with its copies, so and by warps: 12 faces, 128^3, w = 3,
+// 0.53 and 2.8 ms; 320 faces, 256^3, w = 10, 2.5 and 13.6 ms; 5120 faces, 128^3, w =
+// 8, 1.01 and 0.93 ms, but 16^3, w = 3, 0.14 and 0.20 ms; 262144 faces, 256^3, w = 3,
+// 5.6 and 4.3 ms.
+constexpr int kShellRows = 2048, kShellFew = 148 * 24, kShellFewSmall = 8192, kShellCtas = 148 * 8;
 
 struct ShellGrid {
   double b0[3], eh, w;
@@ -149,31 +159,34 @@ __device__ __forceinline__ double outside(double x, double lo, double hi) {
   return x < lo ? lo - x : (x > hi ? x - hi : 0.0);
 }
 
-// rows r0, r0 + step, .. of the box
-__device__ __forceinline__ void shell_rows(const FaceBox& B, const ShellGrid& G, int rows, int r0, int step,
-                                           uint8_t* state) {
-  const int nby = B.rid[1] - B.lid[1];
+// row r of the box: its bytes and centre, and its distance^2 from the face's bounding box in y and z
+struct ShellRow {
+  uint8_t* row;
+  double py, pz, ryz;
+};
+__device__ __forceinline__ ShellRow shell_row(const FaceBox& B, const ShellGrid& G, int r, uint8_t* state) {
+  const int nby = B.rid[1] - B.lid[1], y = B.lid[1] + r % nby, z = B.lid[2] + r / nby;
+  ShellRow W;
+  W.row = state + ((size_t)z * G.R + y) * G.pitch;
+  W.py = (y + 0.5) * G.eh + G.b0[1], W.pz = (z + 0.5) * G.eh + G.b0[2];
+  const double oy = outside(W.py, B.lo[1], B.hi[1]), oz = outside(W.pz, B.lo[2], B.hi[2]);
+  W.ryz = oy * oy + oz * oz;
+  return W;
+}
+// its elements x8 .. x8 + 7 that lie in the box
+__device__ __forceinline__ void shell_word(const FaceBox& B, const ShellGrid& G, const ShellRow& W, int x8) {
   const double sh2 = G.w * G.w;
-  for (int r = r0; r < rows; r += step) {
-    const int y = B.lid[1] + r % nby, z = B.lid[2] + r / nby;
-    const double py = (y + 0.5) * G.eh + G.b0[1], pz = (z + 0.5) * G.eh + G.b0[2];
-    const double oy = outside(py, B.lo[1], B.hi[1]), oz = outside(pz, B.lo[2], B.hi[2]), ryz = oy * oy + oz * oz;
-    if (ryz > B.lim) continue;
-    uint8_t* row = state + ((size_t)z * G.R + y) * G.pitch;
-    for (int x8 = B.lid[0] & ~7; x8 < B.rid[0]; x8 += 8) {
-      unsigned long long todo =
-          __ldcg(reinterpret_cast<const unsigned long long*>(row + x8)) & 0x0101010101010101ull;
-      if (x8 < B.lid[0]) todo &= ~0ull << (8 * (B.lid[0] - x8));
-      if (x8 + 8 > B.rid[0]) todo &= ~0ull >> (8 * (x8 + 8 - B.rid[0]));
-      for (; todo != 0; todo &= todo - 1) {
-        const int x = x8 + (__ffsll((long long)todo) - 1) / 8;
-        const D3 p = {(x + 0.5) * G.eh + G.b0[0], py, pz};
-        const double ox = outside(p.x, B.lo[0], B.hi[0]);
-        if (ox * ox + ryz > B.lim) continue;
-        const D3 d = sub(p, closest_on_triangle(p, B.a, B.b, B.c));
-        if (dot(d, d) < sh2) row[x] = 2;
-      }
-    }
+  unsigned long long todo =
+      __ldcg(reinterpret_cast<const unsigned long long*>(W.row + x8)) & 0x0101010101010101ull;
+  if (x8 < B.lid[0]) todo &= ~0ull << (8 * (B.lid[0] - x8));
+  if (x8 + 8 > B.rid[0]) todo &= ~0ull >> (8 * (x8 + 8 - B.rid[0]));
+  for (; todo != 0; todo &= todo - 1) {
+    const int x = x8 + (__ffsll((long long)todo) - 1) / 8;
+    const D3 p = {(x + 0.5) * G.eh + G.b0[0], W.py, W.pz};
+    const double ox = outside(p.x, B.lo[0], B.hi[0]);
+    if (ox * ox + W.ryz > B.lim) continue;
+    const D3 d = sub(p, closest_on_triangle(p, B.a, B.b, B.c));
+    if (dot(d, d) < sh2) W.row[x] = 2;
   }
 }
 
@@ -193,17 +206,80 @@ __global__ void __launch_bounds__(128, 6) k_shell(const float* __restrict__ vtx,
     if (lane == 0) big[1 + atomicAdd(big, 1)] = (int)f;
     return;
   }
-  shell_rows(B, G, rows, lane, 32, state);
+  for (int r = lane; r < rows; r += 32) {
+    const ShellRow W = shell_row(B, G, r, state);
+    if (W.ryz > B.lim) continue;
+    for (int x8 = B.lid[0] & ~7; x8 < B.rid[0]; x8 += 8) shell_word(B, G, W, x8);
+  }
 }
 
-// all threads of the grid on the rows of one listed face after the other
+// The grid's CTAs shared out over n faces: teams of `size` CTAs, this CTA being
+// number `rank` of team `team`.  A team takes every teams-th face.
+struct Team { int size, team, teams, rank; };
+__device__ __forceinline__ Team team_of(int n, int least) {
+  Team t;
+  t.size = min(max((int)gridDim.x / max(n, 1), least), (int)gridDim.x);
+  t.teams = gridDim.x / t.size;
+  t.team = blockIdx.x / t.size;
+  t.rank = blockIdx.x - t.team * t.size;
+  return t;
+}
+
+// the listed faces, by words of eight elements
 __global__ void __launch_bounds__(128) k_shell_big(const float* __restrict__ vtx, const int* __restrict__ faces,
                                                    ShellGrid G, uint8_t* state, const int* __restrict__ big) {
   const int nb = big[0];
-  for (int k = 0; k < nb; k++) {
+  const Team T = team_of(nb, 8);
+  if (T.team >= T.teams) return;
+  for (int k = T.team; k < nb; k += T.teams) {
     FaceBox B;
     const int rows = face_box(vtx, faces, big[1 + k], G, &B);
-    shell_rows(B, G, rows, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, state);
+    const int first = B.lid[0] & ~7;
+    const unsigned nw = (B.rid[0] - first + 7) / 8;  // rows * nw <= 2048^3 / 8
+    for (unsigned u = T.rank * 128 + threadIdx.x; u < rows * nw; u += T.size * 128) {
+      const unsigned r = u / nw;
+      const ShellRow W = shell_row(B, G, (int)r, state);
+      if (!(W.ryz > B.lim)) shell_word(B, G, W, first + 8 * (int)(u - r * nw));
+    }
+  }
+}
+
+// all faces of a small mesh, by elements; an element that already is shell is left out (a stale byte
+// only costs its distance again)
+__global__ void __launch_bounds__(256) k_shell_few(const float* __restrict__ vtx, const int* __restrict__ faces, int nf,
+                                                   ShellGrid G, const uint8_t* __restrict__ solid, uint8_t* shell) {
+  const Team T = team_of(nf, 1);
+  const double sh2 = G.w * G.w;
+  if (T.team >= T.teams) return;
+  for (int f = T.team; f < nf; f += T.teams) {
+    FaceBox B;
+    const int rows = face_box(vtx, faces, f, G, &B);
+    const unsigned nbx = B.rid[0] - B.lid[0], nby = B.rid[1] - B.lid[1];
+    if (rows == 0) continue;
+    auto element = [&](unsigned x0, unsigned y0, unsigned z0) {
+      const int x = B.lid[0] + (int)x0, y = B.lid[1] + (int)y0, z = B.lid[2] + (int)z0;
+      const size_t e = ((size_t)z * G.R + y) * G.R + x;
+      if (!solid[e] || shell[e]) return;
+      const D3 p = {(x + 0.5) * G.eh + G.b0[0], (y + 0.5) * G.eh + G.b0[1], (z + 0.5) * G.eh + G.b0[2]};
+      const double ox = outside(p.x, B.lo[0], B.hi[0]), oy = outside(p.y, B.lo[1], B.hi[1]),
+                   oz = outside(p.z, B.lo[2], B.hi[2]);
+      if (ox * ox + (oy * oy + oz * oz) > B.lim) return;
+      const D3 d = sub(p, closest_on_triangle(p, B.a, B.b, B.c));
+      if (dot(d, d) < sh2) shell[e] = 1;
+    };
+    const unsigned long long n = (unsigned long long)rows * nbx;
+    const unsigned step = T.size * 256, start = T.rank * 256 + threadIdx.x;
+    if (n < (1ull << 31)) {  // 32-bit divisions
+      for (unsigned k = start; k < (unsigned)n; k += step) {
+        const unsigned r = k / nbx, z = r / nby;
+        element(k - r * nbx, r - z * nby, z);
+      }
+    } else {
+      for (unsigned long long k = start; k < n; k += step) {
+        const unsigned r = (unsigned)(k / nbx), z = r / nby;
+        element((unsigned)(k - (unsigned long long)r * nbx), r - z * nby, z);
+      }
+    }
   }
 }
 
@@ -777,8 +853,20 @@ extern "C" rso_status rso_shell_elements(const float* vertices_host, int n_verti
   Scratch s;
   const float* dv = s.upload(vertices_host, 3 * (size_t)n_vertices);
   const int* df = s.upload(faces_host, 3 * (size_t)n_faces);
-  uint8_t* dshell = s.upload(solid_host, (size_t)nvox);  // the solid bytes, then the shell's
+  uint8_t* dsolid = s.upload(solid_host, (size_t)nvox);
+  uint8_t* dshell = dsolid;  // many faces: the shell's bytes take the solid ones' place
   ShellGrid G{{box_host[0], box_host[1], box_host[2]}, eh, wshell, R, (R + 7) & ~7};
+  if (n_faces < (R < 32 ? kShellFewSmall : kShellFew)) {
+    dshell = s.alloc<uint8_t>((size_t)nvox);
+    if (s.err == cudaSuccess) s.err = cudaMemset(dshell, 0, (size_t)nvox);
+    if (s.err == cudaSuccess && wshell > 0) {
+      k_shell_few<<<std::max(kShellCtas, n_faces), 256>>>(dv, df, n_faces, G, dsolid, dshell);
+      note_launch();
+      s.err = cudaGetLastError();
+    }
+    if (s.err == cudaSuccess) s.err = copy_to_host(shell_host, dshell, (size_t)nvox);
+    return s.err == cudaSuccess ? RSO_OK : RSO_ERR_CUDA;
+  }
   uint8_t* state = s.alloc<uint8_t>((size_t)R * R * G.pitch);
   int* big = s.alloc<int>(1 + (size_t)n_faces);
   if (s.err == cudaSuccess) s.err = cudaMemset(big, 0, sizeof(int));
@@ -791,7 +879,7 @@ extern "C" rso_status rso_shell_elements(const float* vertices_host, int n_verti
       while (std::gcd(stride, n_faces) != 1) stride++;
       k_shell<<<(unsigned)cdiv(n_faces, 4), 128>>>(dv, df, n_faces, stride, G, state, big);
       note_launch();
-      k_shell_big<<<148 * 8, 128>>>(dv, df, G, state, big);
+      k_shell_big<<<kShellCtas, 128>>>(dv, df, G, state, big);
       note_launch();
     }
     k_shell_bytes<false><<<rows, 256>>>(dshell, state, R, G.pitch);

@@ -502,3 +502,32 @@ def test_heaviside_slopes(cuda, beta):
     slope = np.where(on, gin * (beta / den) / np.cosh(np.minimum(np.abs(s), 300.0)) ** 2, 0.0)
     got = g.projectSensitivity(x, beta, gin).cpu().numpy()
     assert np.max(np.abs(got - slope)) < 1e-7 * max(1.0, np.max(np.abs(slope)))
+
+
+# the kernel of few faces: one face, more faces than CTAs, boxes of a row and of the whole grid, several
+# teams to a face; that of many: faces in the list (all of 48 rows), boxes clipped at the grid's edge
+@pytest.mark.parametrize("subdiv,R,width,keep", [(0, 40, 30.0, 1.0), (3, 33, 1.1, 1.0), (3, 20, 4.0, 1.0),
+                                                 (4, 17, 0.4, 1.0), (4, 30, 2.5, 0.5), (4, 49, 60.0, 0.002)])
+@pytest.mark.parametrize("nfaces", [1, None])
+def test_shell_faces(cuda, subdiv, R, width, keep, nfaces):
+    """Shell elements of meshes of one to 5120 faces; the same bytes."""
+    from oracle import boundary as OB
+    from robustoptspline3d_b200 import boundary as B
+    v, f = M.icosphere(subdiv, 4.0, rotation_seed=6)
+    f = f[:nfaces]
+    box = np.array([-4.2, -4.3, -4.4, 4.4, 4.3, 4.2], np.float32)
+    solid = (np.random.default_rng(3).random((R, R, R)) < keep).astype(np.uint8) * 7
+    got = B.shell_elements(v, f, box, R, width, solid)
+    want = OB.shell_elements(v, f, box, R, width, (solid > 0).astype(np.uint8))
+    assert np.array_equal(got, want), int(np.sum(got != want))
+
+
+def test_shell_of_many_wide_faces(cuda):
+    """Every face of 5120 in the list of large boxes: as the union of the shells of parts of few faces."""
+    from robustoptspline3d_b200 import boundary as B
+    v, f = M.icosphere(4, 4.0, rotation_seed=6)
+    box = np.array([-4.2, -4.3, -4.4, 4.4, 4.3, 4.2], np.float32)
+    solid = np.ones((64, 64, 64), np.uint8)
+    got = B.shell_elements(v, f, box, 64, 19.0, solid)
+    want = np.max([B.shell_elements(v, part, box, 64, 19.0, solid) for part in np.array_split(f, 2)], axis=0)
+    assert np.array_equal(got, want) and 0 < got.sum() < got.size
