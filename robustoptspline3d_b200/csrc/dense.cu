@@ -16,7 +16,7 @@
 //            triangular; k_fwd_tiles forms the right-hand side of a tile row,
 //            k_trsm_rows solves it with the diagonal tile), then X = Y^T Y
 //            (k_gram_tiles, lower tiles mirrored to the upper triangle).
-// Small matrices (up to kJordanMax, every hierarchy that coarsens by itself) take
+// Matrices up to kJordanMax (every hierarchy that coarsens by itself) take
 // k_jordan instead, a blocked Gauss-Jordan inversion in one cooperative launch:
 // the steps above are a chain of short launches (five per 64 rows), 1.4 ms for
 // the 375 unknowns below 256^3.
@@ -291,8 +291,11 @@ static int ntiles(int N) { return (N + DT - 1) / DT; }
 // memory) and forms D A_kj for its tiles' columns.  The last step writes X.
 // Rows past N are read as the identity's.  flag is set on a pivot that is not
 // positive.  Bound by the latency of the pivot tiles: 161 us for N = 375 (the
-// launches above: 1.4 ms), 1.39 ms for N = 1152 (4.9 ms).
-constexpr int JT = 32, kJordanMax = 3072;
+// launches above: 1.4 ms), 1.39 ms for N = 1152 (4.9 ms).  It does twice the
+// operations, a step of them at a time with the pivot tile's chain in front, so the
+// launches win from about N = 2500 (an operator update with N = 2430: 13.9 against
+// 15.1 ms; N = 2700: 20.4 against 17.6; N = 3000: 27.7 against 20.3).
+constexpr int JT = 32, kJordanMax = 2432;
 __global__ void __launch_bounds__(256, 1) k_jordan(double* A, double* X, double* Y, int N, int* flag, unsigned* bar) {
   __shared__ double D[JT][JT + 1], B[JT][JT + 1], C[JT][JT + 1], piv[2];
   const int t = threadIdx.x, c = t & 31, r0 = t >> 5;  // column c, rows r0 + 8 q
@@ -412,7 +415,7 @@ static rso_status jordan_inverse(rso_handle* h, double* A, double* X, double* Y,
   return launch_check(h, "coarsest dense inverse");
 }
 
-// K (N x N in A, overwritten by its Cholesky factor in the lower triangle),
+// K (N x N in A, overwritten: past kJordanMax by its Cholesky factor in the lower triangle),
 // X = K^-1, Y scratch (N x N); flag set on a pivot that is not positive
 rso_status dense_spd_inverse(rso_handle* h, double* A, double* X, double* Y, int N, int* flag) {
   const long long NN = (long long)N * N;

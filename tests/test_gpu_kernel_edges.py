@@ -531,3 +531,19 @@ def test_shell_of_many_wide_faces(cuda):
     got = B.shell_elements(v, f, box, 64, 19.0, solid)
     want = np.max([B.shell_elements(v, part, box, 64, 19.0, solid) for part in np.array_split(f, 2)], axis=0)
     assert np.array_equal(got, want) and 0 < got.sum() < got.size
+
+
+@pytest.mark.parametrize("dims,n", [((18, 16, 16), 2430), ((18, 18, 16), 2700)])
+def test_coarsest_inverse_line(cuda, dims, n):
+    """The largest coarsest systems below and the next above the line between the two inversions: residual
+    1e-9 relative, as the coarsest solve's parity test."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(*dims)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None, Config(n_levels=2, first_factor=2))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    mask = np.tile(g.level_masks(1)[1], 3)
+    assert int(mask.sum()) == n
+    f = np.random.default_rng(53).standard_normal(mask.size) * mask
+    x = g.solve_coarsest(t(f, cuda))
+    assert np.linalg.norm(g.coarse_residual(1, x, t(f, cuda)).cpu().numpy()) < 1e-9 * np.linalg.norm(f)
