@@ -547,3 +547,12 @@ def test_coarsest_inverse_line(cuda, dims, n):
     f = np.random.default_rng(53).standard_normal(mask.size) * mask
     x = g.solve_coarsest(t(f, cuda))
     assert np.linalg.norm(g.coarse_residual(1, x, t(f, cuda)).cpu().numpy()) < 1e-9 * np.linalg.norm(f)
+
+
+@pytest.mark.parametrize("dims", [(203, 203, 203), (203, 204, 203)])
+def test_masks_at_the_ring_line(cuda, dims):
+    """Results just under and over the 8 MB from which they go through the pinned ring; the same bytes."""
+    from robustoptspline3d_b200 import boundary as B
+    z, y, x = np.meshgrid(*(np.arange(n) for n in dims[::-1]), indexing="ij", sparse=True)
+    want = ((x * 0.5 - y * 0.25 + z * 0.125 - 30.0) > 0).astype(np.uint8)
+    assert np.array_equal(B.region_mask([B.halfspace(0.5, -0.25, 0.125, -30.0)], (0, 0, 0), 1.0, dims), want)
