@@ -556,3 +556,15 @@ def test_masks_at_the_ring_line(cuda, dims):
     z, y, x = np.meshgrid(*(np.arange(n) for n in dims[::-1]), indexing="ij", sparse=True)
     want = ((x * 0.5 - y * 0.25 + z * 0.125 - 30.0) > 0).astype(np.uint8)
     assert np.array_equal(B.region_mask([B.halfspace(0.5, -0.25, 0.125, -30.0)], (0, 0, 0), 1.0, dims), want)
+
+
+@pytest.mark.parametrize("nx", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32])
+def test_region_short_rows(cuda, nx):
+    """Region masks with 1 to 32 lanes a row, whole and ragged; the same bytes."""
+    from robustoptspline3d_b200 import boundary as B
+    dims = (nx, 37, 53)
+    got = B.region_mask([B.sphere((0.4, 0.3, 0.2), 0.9), B.halfspace(1, 0.5, -1, -1.0)], (-0.5, -0.4, -0.3), 0.1, dims)
+    z, y, x = np.meshgrid(*(np.arange(n) for n in dims[::-1]), indexing="ij")
+    x, y, z = -0.5 + x * 0.1, -0.4 + y * 0.1, -0.3 + z * 0.1
+    want = ((x - 0.4) ** 2 + (y - 0.3) ** 2 + (z - 0.2) ** 2 < 0.9 ** 2) | (x + 0.5 * y - z - 1.0 > 0)
+    assert np.array_equal(got, want.astype(np.uint8)) and 0 < got.sum() < got.size
