@@ -874,6 +874,7 @@ __global__ void __launch_bounds__(1024) k_max_abs(long long n, const double* __r
 // it does not.
 struct SSOut { double *G1, *Gy, *Gz; float* per; double* part; };
 constexpr int kSSRows = 4, kSSSeg = 128;
+static int ss_blocks(const Level& l) { return cdiv((long long)l.ey * l.ez, kSSRows); }
 template <int O>
 __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, SplineDev S, const double* __restrict__ c,
                                                              const double* __restrict__ R, long long comp, const SSPar P,
@@ -1031,9 +1032,7 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
   P.ia = 15.0;
   const long long comp = (long long)S.nb0 * l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
                   t3 = (long long)S.nb0 * S.nb1 * S.nb2;
-  const int nblk = cdiv((long long)l.ey * l.ez, kSSRows);
-  if (!h->sp.work[2])  // the rows of value and derivatives, and the partial sums, made on first use
-    RSO_CHECK_CUDA(h, cudaMalloc(&h->sp.work[2], sizeof(double) * (3 * comp + 3LL * nblk)));
+  const int nblk = ss_blocks(l);
   double* R = h->sp.work[2];
   double* sums = h->scal + 48;
   // H / M of the probe's bound
@@ -1177,8 +1176,10 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
   }
   s.n_coeff = (long long)s.nb[0] * s.nb[1] * s.nb[2];
   // work[0]: spline rows, or stage 1 of the adjoints (three weights); work[1]: the two arrays of the
-  // other stage; work[2] is the self-support constraint's, made on its first call
-  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * 3 * (size_t)s.nb[0] * l.ey * l.ez));
+  // other stage; work[2]: the self-support constraint's rows of value and derivatives, and its partial sums
+  const size_t comp = (size_t)s.nb[0] * l.ey * l.ez;
+  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * 3 * comp));
+  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[2], sizeof(double) * (3 * comp + 3 * (size_t)ss_blocks(l))));
   RSO_CHECK_CUDA(h, cudaMalloc(&s.work[1], sizeof(double) * 2 * (size_t)s.nb[0] * s.nb[1] * l.ez));
   cudaFree(h->coef_a); cudaFree(h->coef_b); cudaFree(h->coef_c);
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_a, sizeof(double) * s.n_coeff));

@@ -568,3 +568,18 @@ def test_region_short_rows(cuda, nx):
     x, y, z = -0.5 + x * 0.1, -0.4 + y * 0.1, -0.3 + z * 0.1
     want = ((x - 0.4) ** 2 + (y - 0.3) ** 2 + (z - 0.2) ** 2 < 0.9 ** 2) | (x + 0.5 * y - z - 1.0 > 0)
     assert np.array_equal(got, want.astype(np.uint8)) and 0 < got.sum() < got.size
+
+
+def test_spline_set_up_allocates_for_the_constraint(cuda):
+    """The first overhang call after a spline set-up allocates no device memory: what it needs is there."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(96, 96, 96)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None, Config())
+    n = g.set_spline_partition(28, 28, 28, 4)  # rows of 3 x 32 x 96 x 96 doubles: 7 MB
+    c = t(np.random.default_rng(59).normal(0.5, 0.15, n).astype(np.float32), cuda)
+    per, dc = cuda.empty(g.ne, device="cuda"), cuda.empty(n, device="cuda")
+    cuda.cuda.synchronize()
+    free, _ = cuda.cuda.mem_get_info()
+    assert g.lib.rso_selfsupport(g.h, c.data_ptr(), 8.0, 4, 2.36, 2.36, per.data_ptr(), dc.data_ptr(), None, None,
+                                 None) == 0
+    assert cuda.cuda.mem_get_info()[0] == free
