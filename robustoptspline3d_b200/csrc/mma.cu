@@ -445,7 +445,7 @@ __global__ void k_clamp_asym(int n, const double* x, double* L, double* U, doubl
 #define MMA_CHECK(s, call)                                                         \
   do {                                                                             \
     cudaError_t _e = (call);                                                       \
-    if (_e != cudaSuccess) { (s)->err = cudaGetErrorString(_e); return RSO_ERR_CUDA; } \
+    if (_e != cudaSuccess) { cudaGetLastError(); (s)->err = cudaGetErrorString(_e); return RSO_ERR_CUDA; } \
   } while (0)
 
 }  // namespace
@@ -454,7 +454,7 @@ extern "C" rso_status rso_mma_create(int n, int m, const double* xmin, const dou
   if (!out || n <= 0 || m < 1 || m > MMA_MAXM || !xmin || !xmax) return RSO_ERR_INVALID_ARG;
   rso_mma* s = new rso_mma();
   s->n = n; s->m = m;
-  auto fail = [&](rso_status st) { rso_mma_destroy(s); return st; };
+  auto fail = [&](rso_status st) { rso_mma_destroy(s); cudaGetLastError(); return st; };
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(RSO_ERR_CUDA);
   double** vecs[] = {&s->x, &s->xmin, &s->xmax, &s->L, &s->U, &s->alpha, &s->beta, &s->lastdx, &s->xi, &s->eta,
                      &s->curx, &s->Dx, &s->hdx, &s->dx, &s->dxi, &s->deta};

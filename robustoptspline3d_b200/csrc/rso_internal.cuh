@@ -247,10 +247,12 @@ rso_status surface_selfsupport(rso_handle* h, const double* c, double beta, int 
 }  // namespace rso
 
 // ---------------------------------------------------------------- helpers
+// (an error that is reported here is not left for the next call's launch check)
 #define RSO_CHECK_CUDA(h, call)                                                          \
   do {                                                                                   \
     cudaError_t _e = (call);                                                             \
     if (_e != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                \
       (h)->err = std::string(#call) + ": " + cudaGetErrorString(_e);                      \
       return RSO_ERR_CUDA;                                                               \
     }                                                                                    \
@@ -557,8 +559,11 @@ struct Scratch {
   template <typename T>
   T* alloc(size_t n) { return upload<T>(nullptr, n); }
   ~Scratch() {
-    // a failed call may have left work in flight on the device
-    if (err != cudaSuccess) cudaDeviceSynchronize();
+    // a failed call may have left work in flight on the device, and its error for the next launch check
+    if (err != cudaSuccess) {
+      cudaDeviceSynchronize();
+      cudaGetLastError();
+    }
     for (const Block& b : blocks) block_put(dev, b.cls, b.p);
   }
 };

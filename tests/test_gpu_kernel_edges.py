@@ -583,3 +583,15 @@ def test_spline_set_up_allocates_for_the_constraint(cuda):
     assert g.lib.rso_selfsupport(g.h, c.data_ptr(), 8.0, 4, 2.36, 2.36, per.data_ptr(), dc.data_ptr(), None, None,
                                  None) == 0
     assert cuda.cuda.mem_get_info()[0] == free
+
+
+def test_reported_errors_are_not_left_over(cuda):
+    """A call that failed for lack of memory leaves no error for the next launch, ours or the caller's."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    from robustoptspline3d_b200.rso import RSOError
+    prob = P.cantilever(12, 10, 8)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None, Config(n_levels=2, first_factor=2))
+    with pytest.raises(RSOError):
+        g.set_spline_partition(100000, 100000, 100000, 4)
+    assert float((cuda.ones(4, device="cuda") + 1).sum()) == 8.0
+    g.update_stencil()
