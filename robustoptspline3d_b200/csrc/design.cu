@@ -1092,14 +1092,16 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
   if (order < 2 || order > 5 || px < 0 || py < 0 || pz < 0) return RSO_ERR_INVALID_ARG;
   Spline& s = h->sp;
   const Level& l = h->L[0];
+  // not set up (order 0: the entry points refuse) until every buffer is there
+  s.order = 0;
+  auto drop = [](auto*& p) { cudaFree(p); p = nullptr; };
   for (int a = 0; a < 3; a++) {
-    cudaFree(s.idx[a]); cudaFree(s.N[a]); cudaFree(s.dN[a]); cudaFree(s.ranges[a]);
+    drop(s.idx[a]); drop(s.N[a]); drop(s.dN[a]); drop(s.ranges[a]);
   }
-  cudaFree(s.knots_dev);
-  cudaFree(s.xtab);
-  s.xtab = nullptr;
-  for (auto& p : s.work) { cudaFree(p); p = nullptr; }
-  s.order = order;
+  drop(s.knots_dev);
+  drop(s.xtab);
+  for (auto& p : s.work) drop(p);
+  drop(h->coef_a); drop(h->coef_b); drop(h->coef_c);
   s.part[0] = px; s.part[1] = py; s.part[2] = pz;
   const int edim[3] = {l.ex, l.ey, l.ez};
   std::vector<float> allk;
@@ -1181,10 +1183,10 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
   RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * 3 * comp));
   RSO_CHECK_CUDA(h, cudaMalloc(&s.work[2], sizeof(double) * (3 * comp + 3 * (size_t)ss_blocks(l))));
   RSO_CHECK_CUDA(h, cudaMalloc(&s.work[1], sizeof(double) * 2 * (size_t)s.nb[0] * s.nb[1] * l.ez));
-  cudaFree(h->coef_a); cudaFree(h->coef_b); cudaFree(h->coef_c);
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_a, sizeof(double) * s.n_coeff));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_b, sizeof(double) * s.n_coeff));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_c, sizeof(double) * s.n_coeff));
+  s.order = order;
   return RSO_OK;
 }
 

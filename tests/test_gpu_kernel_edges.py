@@ -595,3 +595,23 @@ def test_reported_errors_are_not_left_over(cuda):
         g.set_spline_partition(100000, 100000, 100000, 4)
     assert float((cuda.ones(4, device="cuda") + 1).sum()) == 8.0
     g.update_stencil()
+
+
+def test_spline_set_up_that_failed(cuda):
+    """A set-up whose coefficients do not fit the device fails, and the maps are refused until one succeeds,
+    with the results of before."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    from robustoptspline3d_b200.rso import RSOError
+    prob = P.cantilever(12, 10, 8)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None, Config(n_levels=2, first_factor=2))
+    n = g.set_spline_partition(3, 2, 4, 4)
+    c = np.random.default_rng(61).normal(0.5, 0.15, n).astype(np.float32)
+    want = g.coeff2density(c)
+    with pytest.raises(RSOError):
+        g.set_spline_partition(100000, 100000, 100000, 4)
+    for call in (lambda: g.coeff2density(c), lambda: g.ddensity2dcoeff(want), lambda: g.deal_background_points(c, 8.0),
+                 lambda: g.updateCoeff(c, -c, 0.3)):
+        with pytest.raises(RSOError):
+            call()
+    assert g.set_spline_partition(3, 2, 4, 4) == n
+    assert cuda.equal(g.coeff2density(c), want)
