@@ -1102,6 +1102,7 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
   drop(s.xtab);
   for (auto& p : s.work) drop(p);
   drop(h->coef_a); drop(h->coef_b); drop(h->coef_c);
+  drop(h->coef_df); drop(h->coef_dg);  // the design iteration makes them in the new size
   s.part[0] = px; s.part[1] = py; s.part[2] = pz;
   const int edim[3] = {l.ex, l.ey, l.ez};
   std::vector<float> allk;

@@ -101,8 +101,8 @@ rso_status design_iteration(rso_handle* h, rso_mma* mma, const rso_iter_params* 
   const bool ss = prm->ss_mode >= 0;
   if (m != (ss ? 2 : 1)) { h->err = "MMA needs 1 constraint (volume) or 2 (volume, self-support)"; return RSO_ERR_INVALID_ARG; }
   if (!h->coef_df) {
+    if (!h->coef_dg) RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_dg, sizeof(double) * nc * 2));
     RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_df, sizeof(double) * nc));
-    RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_dg, sizeof(double) * nc * 2));
   }
   DesignEval ev;
   RSO_TRY(evaluate_design(h, mma_x(mma), prm, &ev));

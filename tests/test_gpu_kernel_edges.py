@@ -615,3 +615,21 @@ def test_spline_set_up_that_failed(cuda):
             call()
     assert g.set_spline_partition(3, 2, 4, 4) == n
     assert cuda.equal(g.coeff2density(c), want)
+
+
+def test_design_iteration_after_a_finer_spline(cuda):
+    """A design iteration on a spline set up anew with more coefficients: as on a handle that only ever had
+    that spline."""
+    from robustoptspline3d_b200 import MMA, Config, HierarchyGrid, IterParams
+    prob = P.top_loaded_cube(12)
+    out = []
+    for first in (True, False):
+        g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None, Config(n_levels=2, first_factor=2, smoother=1))
+        for parts in ((1, 1, 1), (9, 8, 7)) if first else ((9, 8, 7),):
+            n = g.set_spline_partition(*parts, 4)
+            m = MMA(n, 2, 0.0, 1.0)
+            m.set_x(np.random.default_rng(67).uniform(0.3, 0.7, n))
+            g.design_iteration(m, IterParams(lanczos_steps=4, filter_radius=1.5))
+        out.append(m.get())
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
