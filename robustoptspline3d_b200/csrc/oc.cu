@@ -212,7 +212,7 @@ extern "C" rso_status rso_oc_update_coeff(rso_handle* h, float* coeff_dev, const
   float gmax = 0;
   RSO_TRY(maxabs(h, nc, 0, csens_dev, &gmax));
   // the search varies the coefficients from a copy of the incoming ones
-  float* copy = h->e_c;  // holds NQ >= n_coeff floats
+  float* copy = reinterpret_cast<float*>(h->coef_c);  // n_coeff doubles, unused by the maps
   RSO_CHECK_CUDA(h, cudaMemcpyAsync(copy, coeff_dev, sizeof(float) * nc, cudaMemcpyDeviceToDevice, h->stream));
   const float goal = (float)vgoal, st = (float)step, dp = (float)damp, lo_c = (float)cmin, hi_c = (float)cmax;
   float lo = 0.f, hi = gmax, g = (lo + hi) / 2, V = 2.f;

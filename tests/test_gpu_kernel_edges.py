@@ -633,3 +633,20 @@ def test_design_iteration_after_a_finer_spline(cuda):
         out.append(m.get())
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("parts", [(9, 8, 7), (40, 30, 30)])
+def test_oc_with_more_coefficients_than_elements(oracle, cuda, parts):
+    """The OC coefficient update on a box of 12 x 10 x 8 elements with fewer and with far more coefficients,
+    against the oracle's at the bounds of its parity test."""
+    from oracle import oc
+    g, o = make(oracle, P.cantilever(12, 10, 8), n_levels=2, first_factor=2)
+    n = o.spline_setup(4, parts)
+    assert g.set_spline_partition(*parts, 4) == n
+    rng = np.random.default_rng(71)
+    c, s = rng.uniform(0.4, 0.6, n).astype(np.float32), -rng.uniform(0.5, 1.5, n).astype(np.float32)
+    new, rho, info = g.updateCoeff(c, s, 0.5, step=0.1, damp=0.5, cmin=0.0, cmax=1.0)
+    co, ro, go, vo, to = oc.update_coeff(o, c, s, 0.5, 0.1, 0.5, 0.0, 1.0)
+    assert info["trials"] == to and abs(info["g"] - go) <= 1e-5 * go and abs(info["volume"] - vo) <= 1e-5
+    assert np.max(np.abs(new.cpu().numpy() - co)) <= 1e-5
+    assert np.max(np.abs(rho.cpu().numpy() - ro)) <= 1e-5
