@@ -112,6 +112,8 @@ rso_status design_iteration(rso_handle* h, rso_mma* mma, const rso_iter_params* 
   k_scale_into<<<cdiv(nc, 256), 256, 0, h->stream>>>(nc, prm->vol_scale, h->coef_c, h->coef_dg); rso::note_launch();
   if (ss) { k_scale_into<<<cdiv(nc, 256), 256, 0, h->stream>>>(nc, prm->ss_scale, h->coef_b, h->coef_dg + nc); rso::note_launch(); }
   RSO_TRY(launch_check(h, "MMA inputs"));
+  // the update runs on the MMA's own stream
+  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
   double g[2] = {prm->vol_scale * (ev.volume - prm->volume_ratio), prm->ss_scale * ev.ss};
   int conv = 0;
   double minfo[4];

@@ -650,3 +650,29 @@ def test_oc_with_more_coefficients_than_elements(oracle, cuda, parts):
     assert info["trials"] == to and abs(info["g"] - go) <= 1e-5 * go and abs(info["volume"] - vo) <= 1e-5
     assert np.max(np.abs(new.cpu().numpy() - co)) <= 1e-5
     assert np.max(np.abs(rho.cpu().numpy() - ro)) <= 1e-5
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_design_iteration_is_reproducible(cuda, precision):
+    """The design iteration's update reads its gradients on another stream than they were written on: forty
+    iterations from the same coefficients end in the same bits, those of the gradients passed by hand."""
+    from robustoptspline3d_b200 import MMA, Config, HierarchyGrid, IterParams
+    prob = P.top_loaded_cube(12)
+    p = IterParams(lanczos_steps=4, filter_radius=1.5)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None,
+                      Config(n_levels=2, first_factor=2, smoother=2, precision=precision))
+    n = g.set_spline_partition(9, 8, 7, 4)
+    x = np.random.default_rng(67).uniform(0.3, 0.7, n)
+    v, gl, gv, gs = g.design_gradient(t(x, cuda), p)
+    ref = MMA(n, 2, 0.0, 1.0)
+    ref.set_x(x)
+    ref.update(p.sens_scale * gl, cuda.stack([p.vol_scale * gv, p.ss_scale * gs]),
+               np.array([p.vol_scale * (v["volume"] - p.volume_ratio), p.ss_scale * v["ss"]]))
+    for _ in range(40):
+        m = MMA(n, 2, 0.0, 1.0)
+        m.set_x(x)
+        g.design_iteration(m, p)
+        assert all(np.array_equal(a, b) for a, b in zip(m.get(), ref.get()))
+        m.close()
+    ref.close()
+    g.close()
