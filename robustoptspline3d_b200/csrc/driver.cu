@@ -165,6 +165,7 @@ extern "C" rso_status rso_design_iteration_host(rso_handle* h, rso_mma* mma, con
                                                 rso_iter_info* info) {
   if (!h || !mma || !prm) return RSO_ERR_INVALID_ARG;
   const long long nc = h->sp.n_coeff;
+  if (!h->sp.order || mma_n(mma) != nc) return design_iteration(h, mma, prm, info);  // refuses, before any copy
   if (cin) RSO_CHECK_CUDA(h, cudaMemcpyAsync(mma_x(mma), cin, sizeof(double) * nc, cudaMemcpyHostToDevice, h->stream));
   RSO_TRY(design_iteration(h, mma, prm, info));
   if (cout) RSO_CHECK_CUDA(h, cudaMemcpy(cout, mma_x(mma), sizeof(double) * nc, cudaMemcpyDeviceToHost));

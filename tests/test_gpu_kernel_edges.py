@@ -676,3 +676,19 @@ def test_design_iteration_is_reproducible(cuda, precision):
         m.close()
     ref.close()
     g.close()
+
+
+def test_host_iteration_of_another_size(cuda):
+    """The host form of the design iteration refuses an MMA of another size before it copies anything."""
+    from robustoptspline3d_b200 import MMA, Config, HierarchyGrid, IterParams
+    from robustoptspline3d_b200.rso import RSOError
+    prob = P.top_loaded_cube(12)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], None, Config(n_levels=2, first_factor=2))
+    m = MMA(9, 2, 0.0, 1.0)
+    x0 = m.get()[0]
+    with pytest.raises(RSOError, match="not set up"):
+        g.design_iteration_host(m, np.ones(9), IterParams())
+    n = g.set_spline_partition(9, 8, 7, 4)
+    with pytest.raises(RSOError, match="size differs"):
+        g.design_iteration_host(m, np.ones(n), IterParams())
+    assert np.array_equal(m.get()[0], x0)
