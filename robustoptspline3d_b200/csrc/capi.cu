@@ -149,14 +149,14 @@ static rso_status setup(rso_handle* h, int ex, int ey, int ez, const uint8_t* em
   h->own_stream = true;
   RSO_TRY(rso_element_matrix(h->cfg.youngs_modulus, h->cfg.poisson_ratio, 1.0, h->K0));
   ALLOC(h->K0_dev, sizeof(double) * 576);
-  RSO_CHECK_CUDA(h, cudaMemcpy(h->K0_dev, h->K0, sizeof(double) * 576, cudaMemcpyHostToDevice));
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->K0_dev, h->K0, sizeof(double) * 576, cudaMemcpyHostToDevice, h->stream));
   RSO_TRY(upload_K0(h));
   ALLOC(h->red, sizeof(double) * 4096);
   ALLOC(h->gbar, sizeof(unsigned) * 4);
-  RSO_CHECK_CUDA(h, cudaMemset(h->gbar, 0, sizeof(unsigned) * 4));
+  RSO_CHECK_CUDA(h, cudaMemsetAsync(h->gbar, 0, sizeof(unsigned) * 4, h->stream));
   ALLOC(h->scal, sizeof(double) * 64);
   RSO_CHECK_CUDA(h, cudaMallocHost((void**)&h->h_scal, sizeof(double) * 64));
-  RSO_CHECK_CUDA(h, cudaMemset(h->scal, 0, sizeof(double) * 64));
+  RSO_CHECK_CUDA(h, cudaMemsetAsync(h->scal, 0, sizeof(double) * 64, h->stream));
   h->L.push_back(make_level(ex, ey, ez, 0));
   RSO_TRY(build_topology(h, em, fa, la, ln));
   {
@@ -177,40 +177,41 @@ static rso_status setup(rso_handle* h, int ex, int ey, int ez, const uint8_t* em
                                                        (long long)cdiv(f0.ny, 7) * cdiv(f0.nz, kFineZc64Min));
     ALLOC(h->fpart, sizeof(double) * h->fpart_n);
   }
-  // per-level buffers
+  // per-level buffers; every copy and fill of a handle goes to its own stream, which does not
+  // wait for the default one
   for (size_t li = 0; li < h->L.size(); li++) {
     Level& l = h->L[li];
     const size_t v64 = sizeof(double) * 3 * l.NP, v32 = sizeof(float) * 3 * l.NP;
     ALLOC(l.u64, v64); ALLOC(l.f64, v64); ALLOC(l.r64, v64); ALLOC(l.t64, v64);
     ALLOC(l.u32, v32); ALLOC(l.f32, v32); ALLOC(l.r32, v32); ALLOC(l.t32, v32);
-    RSO_CHECK_CUDA(h, cudaMemset(l.u64, 0, v64)); RSO_CHECK_CUDA(h, cudaMemset(l.f64, 0, v64));
-    RSO_CHECK_CUDA(h, cudaMemset(l.r64, 0, v64)); RSO_CHECK_CUDA(h, cudaMemset(l.t64, 0, v64));
-    RSO_CHECK_CUDA(h, cudaMemset(l.u32, 0, v32)); RSO_CHECK_CUDA(h, cudaMemset(l.f32, 0, v32));
-    RSO_CHECK_CUDA(h, cudaMemset(l.r32, 0, v32)); RSO_CHECK_CUDA(h, cudaMemset(l.t32, 0, v32));
+    RSO_CHECK_CUDA(h, cudaMemsetAsync(l.u64, 0, v64, h->stream)); RSO_CHECK_CUDA(h, cudaMemsetAsync(l.f64, 0, v64, h->stream));
+    RSO_CHECK_CUDA(h, cudaMemsetAsync(l.r64, 0, v64, h->stream)); RSO_CHECK_CUDA(h, cudaMemsetAsync(l.t64, 0, v64, h->stream));
+    RSO_CHECK_CUDA(h, cudaMemsetAsync(l.u32, 0, v32, h->stream)); RSO_CHECK_CUDA(h, cudaMemsetAsync(l.f32, 0, v32, h->stream));
+    RSO_CHECK_CUDA(h, cudaMemsetAsync(l.r32, 0, v32, h->stream)); RSO_CHECK_CUDA(h, cudaMemsetAsync(l.t32, 0, v32, h->stream));
     if (li > 0) {
       ALLOC(l.KE, sizeof(double) * 576 * l.ne);
       ALLOC(l.st64, sizeof(double) * 243 * l.NP);
       ALLOC(l.st32, sizeof(float) * st32_len(l.NP));
-      RSO_CHECK_CUDA(h, cudaMemset(l.KE, 0, sizeof(double) * 576 * l.ne));
-      RSO_CHECK_CUDA(h, cudaMemset(l.st64, 0, sizeof(double) * 243 * l.NP));
-      RSO_CHECK_CUDA(h, cudaMemset(l.st32, 0, sizeof(float) * st32_len(l.NP)));
+      RSO_CHECK_CUDA(h, cudaMemsetAsync(l.KE, 0, sizeof(double) * 576 * l.ne, h->stream));
+      RSO_CHECK_CUDA(h, cudaMemsetAsync(l.st64, 0, sizeof(double) * 243 * l.NP, h->stream));
+      RSO_CHECK_CUDA(h, cudaMemsetAsync(l.st32, 0, sizeof(float) * st32_len(l.NP), h->stream));
     }
   }
   Level& l0 = h->L[0];
   ALLOC(h->rho, sizeof(float) * l0.NQ); ALLOC(h->rp32, sizeof(float) * l0.NQ); ALLOC(h->rp64, sizeof(double) * l0.NQ);
-  RSO_CHECK_CUDA(h, cudaMemset(h->rho, 0, sizeof(float) * l0.NQ));
+  RSO_CHECK_CUDA(h, cudaMemsetAsync(h->rho, 0, sizeof(float) * l0.NQ, h->stream));
   const size_t v64 = sizeof(double) * 3 * l0.NP;
   ALLOC(h->x, v64); ALLOC(h->r, v64); ALLOC(h->p, v64); ALLOC(h->q, v64); ALLOC(h->z, v64); ALLOC(h->w, v64);
-  for (double* p : {h->x, h->r, h->p, h->q, h->z, h->w}) RSO_CHECK_CUDA(h, cudaMemset(p, 0, v64));
+  for (double* p : {h->x, h->r, h->p, h->q, h->z, h->w}) RSO_CHECK_CUDA(h, cudaMemsetAsync(p, 0, v64, h->stream));
   ALLOC(h->e_a, sizeof(float) * l0.NQ); ALLOC(h->e_b, sizeof(float) * l0.NQ); ALLOC(h->e_c, sizeof(float) * l0.NQ);
   ALLOC(h->e_d, sizeof(float) * l0.NQ); ALLOC(h->e_rhohat, sizeof(float) * l0.NQ);
-  for (float* p : {h->e_a, h->e_b, h->e_c, h->e_d, h->e_rhohat}) RSO_CHECK_CUDA(h, cudaMemset(p, 0, sizeof(float) * l0.NQ));
+  for (float* p : {h->e_a, h->e_b, h->e_c, h->e_d, h->e_rhohat}) RSO_CHECK_CUDA(h, cudaMemsetAsync(p, 0, sizeof(float) * l0.NQ, h->stream));
   // default density 1 on active elements
   {
     std::vector<float> ones(l0.ne, 1.0f);
     float* d = nullptr;
     ALLOC(d, sizeof(float) * l0.ne);
-    RSO_CHECK_CUDA(h, cudaMemcpy(d, ones.data(), sizeof(float) * l0.ne, cudaMemcpyHostToDevice));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(d, ones.data(), sizeof(float) * l0.ne, cudaMemcpyHostToDevice, h->stream));
     RSO_TRY(pad_elems_f(h, d, h->rho));
     RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
     cudaFree(d);
@@ -221,7 +222,7 @@ static rso_status setup(rso_handle* h, int ex, int ey, int ez, const uint8_t* em
     std::vector<double> T;
     galerkin_table(h->K0, h->L[1].factor, T);
     ALLOC(h->T1, sizeof(double) * T.size());
-    RSO_CHECK_CUDA(h, cudaMemcpy(h->T1, T.data(), sizeof(double) * T.size(), cudaMemcpyHostToDevice));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->T1, T.data(), sizeof(double) * T.size(), cudaMemcpyHostToDevice, h->stream));
     RSO_TRY(galerkin_setup(h));
     // coarsest node list + node->row map
     const Level& c = h->L.back();
@@ -241,7 +242,7 @@ static rso_status setup(rso_handle* h, int ex, int ey, int ez, const uint8_t* em
     std::vector<int> packed(nodes);
     packed.insert(packed.end(), crow.begin(), crow.end());
     ALLOC(h->c_nodes, sizeof(int) * packed.size());
-    RSO_CHECK_CUDA(h, cudaMemcpy(h->c_nodes, packed.data(), sizeof(int) * packed.size(), cudaMemcpyHostToDevice));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->c_nodes, packed.data(), sizeof(int) * packed.size(), cudaMemcpyHostToDevice, h->stream));
     const size_t N = 3 * (size_t)h->nc;
     ALLOC(h->c_K, sizeof(double) * 3 * N * N);  // factor, inverse, L^-1 scratch
     ALLOC(h->c_f, sizeof(double) * N);

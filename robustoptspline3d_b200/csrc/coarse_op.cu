@@ -2252,7 +2252,7 @@ rso_status galerkin_setup(rso_handle* h) {
   h->n_gfix = (int)list.size();
   if (h->n_gfix) {
     RSO_CHECK_CUDA(h, cudaMalloc(&h->gfix, sizeof(int) * list.size()));
-    RSO_CHECK_CUDA(h, cudaMemcpy(h->gfix, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->gfix, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, h->stream));
   }
   return RSO_OK;
 }

@@ -1124,7 +1124,7 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
     allk.insert(allk.end(), K.begin(), K.end());
   }
   RSO_CHECK_CUDA(h, cudaMalloc(&s.knots_dev, sizeof(float) * allk.size()));
-  RSO_CHECK_CUDA(h, cudaMemcpy(s.knots_dev, allk.data(), sizeof(float) * allk.size(), cudaMemcpyHostToDevice));
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(s.knots_dev, allk.data(), sizeof(float) * allk.size(), cudaMemcpyHostToDevice, h->stream));
   size_t koff = 0;
   for (int a = 0; a < 3; a++) {
     const int n = edim[a];
@@ -1172,10 +1172,10 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
           bd[(size_t)(x - rg[b]) * nb + b] = D;
         }
       RSO_CHECK_CUDA(h, cudaMalloc(&s.xtab, sizeof(double) * tab.size()));
-      RSO_CHECK_CUDA(h, cudaMemcpy(s.xtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+      RSO_CHECK_CUDA(h, cudaMemcpyAsync(s.xtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, h->stream));
     }
     RSO_CHECK_CUDA(h, cudaMalloc(&s.ranges[a], sizeof(int) * rg.size()));
-    RSO_CHECK_CUDA(h, cudaMemcpy(s.ranges[a], rg.data(), sizeof(int) * rg.size(), cudaMemcpyHostToDevice));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(s.ranges[a], rg.data(), sizeof(int) * rg.size(), cudaMemcpyHostToDevice, h->stream));
   }
   s.n_coeff = (long long)s.nb[0] * s.nb[1] * s.nb[2];
   // work[0]: spline rows, or stage 1 of the adjoints (three weights); work[1]: the two arrays of the

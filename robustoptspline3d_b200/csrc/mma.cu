@@ -473,14 +473,15 @@ extern "C" rso_status rso_mma_create(int n, int m, const double* xmin, const dou
   cudaMemsetAsync(s->bar, 0, sizeof(unsigned) * 4, s->stream);
   if (cudaMalloc(&s->res, sizeof(double) * 64) != cudaSuccess) return fail(RSO_ERR_OOM);
   if (cudaMallocHost(&s->h_res, sizeof(double) * 64) != cudaSuccess) return fail(RSO_ERR_OOM);
-  cudaMemcpy(s->xmin, xmin, sizeof(double) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(s->xmax, xmax, sizeof(double) * n, cudaMemcpyHostToDevice);
+  // on the MMA's own stream: copies and fills on the default one may still be under way when they return
+  cudaMemcpyAsync(s->xmin, xmin, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(s->xmax, xmax, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
   // set_bound (mma_t.cu:809-819) and init_subproblem_variable (:797-807)
-  cudaMemcpy(s->alpha, xmin, sizeof(double) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(s->beta, xmax, sizeof(double) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(s->L, xmin, sizeof(double) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(s->U, xmax, sizeof(double) * n, cudaMemcpyHostToDevice);
-  cudaMemset(s->lastdx, 0, sizeof(double) * n);
+  cudaMemcpyAsync(s->alpha, xmin, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(s->beta, xmax, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(s->L, xmin, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(s->U, xmax, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemsetAsync(s->lastdx, 0, sizeof(double) * n, s->stream);
   k_reset<<<MMA_BLOCKS, MMA_THREADS, 0, s->stream>>>(n, s->x, s->alpha, s->beta, s->xi, s->eta); rso::note_launch();
   k_clamp_asym<<<MMA_BLOCKS, MMA_THREADS, 0, s->stream>>>(n, s->x, s->L, s->U, s->alpha, s->beta, s->xmin, s->xmax); rso::note_launch();
   k_reset<<<MMA_BLOCKS, MMA_THREADS, 0, s->stream>>>(n, s->x, s->alpha, s->beta, s->xi, s->eta); rso::note_launch();

@@ -113,15 +113,17 @@ rso_status rigid_setup(rso_handle* h) {
     pos[3 * k + 1] = (double)(n / l0.nx % l0.ny);
     pos[3 * k + 2] = (double)(n / ((long long)l0.nx * l0.ny));
   }
-  RSO_CHECK_CUDA(h, cudaMemcpy(nrm.data(), h->load_normals, sizeof(double) * nrm.size(), cudaMemcpyDeviceToHost));
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(nrm.data(), h->load_normals, sizeof(double) * nrm.size(), cudaMemcpyDeviceToHost,
+                                    h->stream));
+  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->rigid_q, sizeof(double) * 2 * 6 * ls));
-  RSO_CHECK_CUDA(h, cudaMemset(h->rigid_q, 0, sizeof(double) * 2 * 6 * ls));
+  RSO_CHECK_CUDA(h, cudaMemsetAsync(h->rigid_q, 0, sizeof(double) * 2 * 6 * ls, h->stream));
   for (int cf = 0; cf < 2; cf++) {
     std::vector<double> Q;
     h->rigid_k[cf] = nl ? rigid_mgs(pos, cf ? nrm.data() : nullptr, true, Q) : 0;
     if (h->rigid_k[cf])
-      RSO_CHECK_CUDA(h, cudaMemcpy(h->rigid_q + (size_t)cf * 6 * ls, Q.data(), sizeof(double) * Q.size(),
-                                   cudaMemcpyHostToDevice));
+      RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->rigid_q + (size_t)cf * 6 * ls, Q.data(), sizeof(double) * Q.size(),
+                                        cudaMemcpyHostToDevice, h->stream));
   }
   // fine nodes: centroid and inverse Gram matrix of the motions about it
   const std::vector<uint8_t>& vm = h->h_vmask[0];
@@ -147,7 +149,7 @@ rso_status rigid_setup(rso_handle* h) {
   if (!inv6(G, M)) { h->err = "rigid motions of the active nodes are degenerate"; return RSO_ERR_INVALID_ARG; }
   M[36] = ctr[0]; M[37] = ctr[1]; M[38] = ctr[2];
   RSO_CHECK_CUDA(h, cudaMalloc(&h->rigid_m, sizeof(M)));
-  RSO_CHECK_CUDA(h, cudaMemcpy(h->rigid_m, M, sizeof(M), cudaMemcpyHostToDevice));
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->rigid_m, M, sizeof(M), cudaMemcpyHostToDevice, h->stream));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->rigid_scr, sizeof(double) * 6 * RG_BLOCKS));
   // coarsest nodes: orthonormal motions (coarse node coordinates: positions
   // scaled by a common factor span the same motions)
@@ -170,7 +172,7 @@ rso_status rigid_setup(rso_handle* h) {
     for (int j = 0; j < k; j++)
       for (size_t i = 0; i < N; i++) Rrow[i * 6 + j] = Q[j * N + i];
     RSO_CHECK_CUDA(h, cudaMalloc(&h->c_R, sizeof(double) * Rrow.size()));
-    RSO_CHECK_CUDA(h, cudaMemcpy(h->c_R, Rrow.data(), sizeof(double) * Rrow.size(), cudaMemcpyHostToDevice));
+    RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->c_R, Rrow.data(), sizeof(double) * Rrow.size(), cudaMemcpyHostToDevice, h->stream));
   }
   return RSO_OK;
 }

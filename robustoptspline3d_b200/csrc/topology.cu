@@ -406,7 +406,7 @@ rso_status build_topology(rso_handle* h, const uint8_t* emask, const uint8_t* fi
     for (long long k = 0; k < nl; k++)
       for (int c = 0; c < 3; c++) nrm[3 * k + c] = load_normals[3 * (long long)h->h_load_nodes[k] + c];
   RSO_CHECK_CUDA(h, cudaMalloc(&h->load_normals, sizeof(double) * nrm.size()));
-  RSO_CHECK_CUDA(h, cudaMemcpy(h->load_normals, nrm.data(), sizeof(double) * nrm.size(), cudaMemcpyHostToDevice));
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->load_normals, nrm.data(), sizeof(double) * nrm.size(), cudaMemcpyHostToDevice, h->stream));
   return RSO_OK;
 }
 
