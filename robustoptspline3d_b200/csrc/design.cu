@@ -697,17 +697,33 @@ rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, f
 // side) serve both rows.  256^3, 32 coefficients: 202 us with a thread per
 // (a, y, z) reading the fields directly, 205 with one row per warp and the values
 // looked up through the span table, 88 now.
+// Boxes with few rows cut them in chunks of x (XSplit), a warp each, which write
+// sums of their own, `stride` apart; stage 2 adds up those a function's support meets.
 constexpr int kSeg = 256, kAdjRows = 2, kAdjWarps = 4;
+struct XSplit { int chunks, len; };
+// Rows are cut where whole ones make fewer than four warps an SM, into pieces of 32
+// elements at least, until there are eight an SM.  1500 x 6 x 6 elements, 32
+// coefficients along x: adjoint 0.146 -> 0.057 ms a call, overhang constraint 0.644
+// -> 0.125 (a thread an element or a sum, as before both: 0.100 and 0.317).
+static XSplit x_split(const Level& l, int rows_per_warp, int seg) {
+  const long long warps = cdiv((long long)l.ey * l.ez, rows_per_warp);
+  int len = seg;
+  if (warps >= 4 * 148) return {1, l.ex};
+  while (len > 32 && warps * cdiv(l.ex, len) < 8 * 148) len /= 2;
+  return l.ex <= len ? XSplit{1, l.ex} : XSplit{cdiv(l.ex, len), len};
+}
 __global__ void __launch_bounds__(32 * kAdjWarps) k_adj_x(const Level L, SplineDev S, const float* __restrict__ g,
                                                           const uint8_t* __restrict__ shell, const View V,
                                                           const int* __restrict__ lo, const int* __restrict__ hi,
-                                                          double* __restrict__ G1) {
+                                                          int len, long long stride, double* __restrict__ G1) {
   __shared__ double w[kAdjWarps][kAdjRows][kSeg];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rows = L.ey * L.ez, r0 = (blockIdx.x * kAdjWarps + warp) * kAdjRows;
   if (r0 >= rows) return;
-  for (int xa = 0; xa < L.ex; xa += kSeg) {
-    const int xb = min(xa + kSeg, L.ex);
+  const int x0 = blockIdx.y * len, x1 = min(x0 + len, L.ex);
+  G1 += blockIdx.y * stride;
+  for (int xa = x0; xa < x1; xa += kSeg) {
+    const int xb = min(xa + kSeg, x1);
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < kAdjRows; j++) {
@@ -736,28 +752,46 @@ __global__ void __launch_bounds__(32 * kAdjWarps) k_adj_x(const Level L, SplineD
       for (int j = 0; j < kAdjRows; j++)
         if (r0 + j < rows) {
           double* G = G1 + (long long)S.nb0 * (r0 + j) + a;
-          *G = xa == 0 ? s[j] : *G + s[j];
+          *G = xa == x0 ? s[j] : *G + s[j];
         }
     }
   }
 }
-// Stage 2, y: G2[z][b][a] = sum_y G1[z][y][a] N_b(y) (+ Gd[z][y][a] D_b(y))
+// Stage 2, y: G2[z][b][a] = sum_y G1[z][y][a] N_b(y) (+ Gd[z][y][a] D_b(y)); SPLIT: stage 1 in chunks of len
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_adj_y(SplineDev S, int ey, int ez, const double* __restrict__ G1,
                                                const double* __restrict__ Gd, const int* __restrict__ lo,
-                                               const int* __restrict__ hi, double* __restrict__ G2) {
+                                               const int* __restrict__ hi, const int* __restrict__ xlo,
+                                               const int* __restrict__ xhi, int len, long long stride,
+                                               double* __restrict__ G2) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long pl = (long long)S.nb0 * S.nb1;
   if (t >= pl * ez) return;
   const int z = (int)(t / pl), ab = (int)(t - pl * z), b = ab / S.nb0, a = ab - b * S.nb0;
+  const int c0 = SPLIT ? xlo[a] / len : 0, c1 = SPLIT ? xhi[a] / len : 0;
+  auto stage1 = [&](const double* G, long long g) {
+    double v = G[g + c0 * stride];
+    if (SPLIT)
+      for (int c = c0 + 1; c <= c1; c++) v += G[g + c * stride];
+    return v;
+  };
   double s = 0;
 #pragma unroll 4
   for (int y = lo[b]; y <= hi[b]; y++) {
     const long long g = a + (long long)S.nb0 * (y + (long long)ey * z);
     const int k = y * S.order + b - S.i1[y] + S.order;
-    s += G1[g] * S.N1[k];
-    if (Gd) s += Gd[g] * S.D1[k];
+    s += stage1(G1, g) * S.N1[k];
+    if (Gd) s += stage1(Gd, g) * S.D1[k];
   }
   G2[t] = s;
+}
+static void adj_y(rso_handle* h, const SplineDev& S, const XSplit& X, long long stride, const double* G1,
+                  const double* Gd, double* G2) {
+  const Level& l = h->L[0];
+  const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1];
+  auto k = X.chunks > 1 ? k_adj_y<true> : k_adj_y<false>;
+  k<<<cdiv((long long)S.nb0 * S.nb1 * l.ez, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, G1, Gd, r1, r1 + S.nb1, r0,
+                                                                       r0 + S.nb0, X.len, stride, G2); rso::note_launch();
 }
 // Stage 3, z: dc[c][b][a] = scale (sum_z G2[z][b][a] N_c(z) (+ Gd[z][b][a] D_c(z))); scale from
 // *count (its reciprocal, 0 for 0) when given.  The supports are a fifth of the box or
@@ -792,12 +826,13 @@ rso_status density2coeff(rso_handle* h, const float* g, const uint8_t* shell, do
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
   const SplineDev S = spline_dev(h, h->sp.knots_dev);
   double *G1 = h->sp.work[0], *G2 = h->sp.work[1];
-  const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1], *r2 = h->sp.ranges[2];
-  const long long rows = (long long)l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
-                  t3 = (long long)S.nb0 * S.nb1 * S.nb2;
-  k_adj_x<<<cdiv(rows, kAdjRows * kAdjWarps), 32 * kAdjWarps, 0, h->stream>>>(l, S, g, shell, view_of(l, dense), r0,
-                                                                               r0 + S.nb0, G1); rso::note_launch();
-  k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, G1, nullptr, r1, r1 + S.nb1, G2); rso::note_launch();
+  const int *r0 = h->sp.ranges[0], *r2 = h->sp.ranges[2];
+  const long long rows = (long long)l.ey * l.ez, t3 = (long long)S.nb0 * S.nb1 * S.nb2, stride = S.nb0 * rows;
+  const XSplit X = x_split(l, kAdjRows, kSeg);
+  const dim3 grid(cdiv(rows, kAdjRows * kAdjWarps), X.chunks);
+  k_adj_x<<<grid, 32 * kAdjWarps, 0, h->stream>>>(l, S, g, shell, view_of(l, dense), r0, r0 + S.nb0, X.len, stride, G1);
+  rso::note_launch();
+  adj_y(h, S, X, stride, G1, nullptr, G2);
   k_adj_z<<<cdiv(t3, 32), dim3(32, 8), 0, h->stream>>>(S, G2, nullptr, r2, r2 + S.nb2, nullptr, dc); rso::note_launch();
   return launch_check(h, "density2coeff");
 }
@@ -881,7 +916,7 @@ __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, Spli
                                                              double flip, double direction,
                                                              const double* __restrict__ cmax, double hcoef, double smin,
                                                              const int* __restrict__ lo, const int* __restrict__ hi,
-                                                             const SSOut Q, const View V) {
+                                                             int len, SSOut Q, const View V) {
   __shared__ double w[kSSRows][4][kSSSeg];
   __shared__ double red[kSSRows][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -897,8 +932,10 @@ __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, Spli
     const uint8_t* mask = L.emask + L.eidx(0, y, z);
     const double *r0 = R + gb - O, *r1 = r0 + comp, *r2 = r1 + comp;
     float* per = Q.per ? Q.per + V.at(0, y, z) : nullptr;
-    for (int xa = 0; xa < L.ex; xa += kSSSeg) {
-      const int xb = min(xa + kSSSeg, L.ex);
+    const int x0 = blockIdx.y * len, x1 = min(x0 + len, L.ex);
+    Q.G1 += blockIdx.y * 3 * comp, Q.Gy += blockIdx.y * 3 * comp, Q.Gz += blockIdx.y * 3 * comp;
+    for (int xa = x0; xa < x1; xa += kSSSeg) {
+      const int xb = min(xa + kSSSeg, x1);
       __syncwarp();
       for (int x = xa + lane; x < xb; x += 32) {
         double wA = 0, wX = 0, wY = 0, wZ = 0;
@@ -974,8 +1011,8 @@ __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, Spli
           sy = fma(w[warp][2][x], N, sy);
           sz = fma(w[warp][3][x], N, sz);
         }
-        if (xa > 0 && kb < ka) continue;
-        const bool first = xa == 0;
+        if (xa > x0 && kb < ka) continue;
+        const bool first = xa == x0;
         Q.G1[gb + a] = first ? s : Q.G1[gb + a] + s;
         Q.Gy[gb + a] = first ? sy : Q.Gy[gb + a] + sy;
         Q.Gz[gb + a] = first ? sz : Q.Gz[gb + a] + sz;
@@ -989,7 +1026,7 @@ __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, Spli
   if (threadIdx.x < 3) {
     double t = 0;
     for (int k = 0; k < kSSRows; k++) t += red[k][threadIdx.x];
-    Q.part[threadIdx.x * (long long)gridDim.x + blockIdx.x] = t;
+    Q.part[(threadIdx.x * (long long)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = t;
   }
 }
 // out[0..2] = the sums of probes, penalties and downward faces; out[3] the count the mean divides by
@@ -1032,7 +1069,8 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
   P.ia = 15.0;
   const long long comp = (long long)S.nb0 * l.ey * l.ez, t2 = (long long)S.nb0 * S.nb1 * l.ez,
                   t3 = (long long)S.nb0 * S.nb1 * S.nb2;
-  const int nblk = ss_blocks(l);
+  const XSplit X = x_split(l, 1, kSSSeg);
+  const dim3 grid(ss_blocks(l), X.chunks);
   double* R = h->sp.work[2];
   double* sums = h->scal + 48;
   // H / M of the probe's bound
@@ -1055,16 +1093,16 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
   O.per = per_dense;
   O.part = R + 3 * comp;
   double *G2 = h->sp.work[1], *G2z = G2 + t2;
-  const int *r0 = h->sp.ranges[0], *r1 = h->sp.ranges[1], *r2 = h->sp.ranges[2];
+  const int *r0 = h->sp.ranges[0], *r2 = h->sp.ranges[2];
   double flip = -1.0, direction = -1.0;
   for (int pass = 0; pass < 2; pass++) {
     auto rows = S.order == 2 ? k_ss_rows<2> : S.order == 3 ? k_ss_rows<3> : S.order == 4 ? k_ss_rows<4> : k_ss_rows<5>;
-    rows<<<nblk, 32 * kSSRows, 0, h->stream>>>(l, S, c, R, comp, P, flip, direction, sums + 4, hcoef, smin, r0,
-                                               r0 + S.nb0, O, view_of(l, true)); rso::note_launch();
-    k_ss_sums<<<1, 1024, 0, h->stream>>>(O.part, nblk, mode, (double)l.n_active_e, sums); rso::note_launch();
+    rows<<<grid, 32 * kSSRows, 0, h->stream>>>(l, S, c, R, comp, P, flip, direction, sums + 4, hcoef, smin, r0,
+                                               r0 + S.nb0, X.len, O, view_of(l, true)); rso::note_launch();
+    k_ss_sums<<<1, 1024, 0, h->stream>>>(O.part, (int)(grid.x * grid.y), mode, (double)l.n_active_e, sums); rso::note_launch();
     if (dc) {
-      k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, O.G1, O.Gy, r1, r1 + S.nb1, G2); rso::note_launch();
-      k_adj_y<<<cdiv(t2, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, O.Gz, nullptr, r1, r1 + S.nb1, G2z); rso::note_launch();
+      adj_y(h, S, X, 3 * comp, O.G1, O.Gy, G2);
+      adj_y(h, S, X, 3 * comp, O.Gz, nullptr, G2z);
       k_adj_z<<<cdiv(t3, 32), dim3(32, 8), 0, h->stream>>>(S, G2, G2z, r2, r2 + S.nb2, sums + 3, dc); rso::note_launch();
     }
     RSO_TRY(launch_check(h, "selfsupport"));
@@ -1178,11 +1216,13 @@ rso_status spline_setup(rso_handle* h, int order, int px, int py, int pz) {
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(s.ranges[a], rg.data(), sizeof(int) * rg.size(), cudaMemcpyHostToDevice, h->stream));
   }
   s.n_coeff = (long long)s.nb[0] * s.nb[1] * s.nb[2];
-  // work[0]: spline rows, or stage 1 of the adjoints (three weights); work[1]: the two arrays of the
-  // other stage; work[2]: the self-support constraint's rows of value and derivatives, and its partial sums
+  // work[0]: spline rows, or stage 1 of the adjoints (one or three weights, every chunk of x); work[1]: the
+  // two arrays of the other stage; work[2]: the self-support constraint's rows of value and derivatives, and
+  // its partial sums
   const size_t comp = (size_t)s.nb[0] * l.ey * l.ez;
-  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * 3 * comp));
-  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[2], sizeof(double) * (3 * comp + 3 * (size_t)ss_blocks(l))));
+  const size_t ca = x_split(l, kAdjRows, kSeg).chunks, cs = x_split(l, 1, kSSSeg).chunks;
+  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[0], sizeof(double) * std::max(ca, 3 * cs) * comp));
+  RSO_CHECK_CUDA(h, cudaMalloc(&s.work[2], sizeof(double) * (3 * comp + 3 * cs * ss_blocks(l))));
   RSO_CHECK_CUDA(h, cudaMalloc(&s.work[1], sizeof(double) * 2 * (size_t)s.nb[0] * s.nb[1] * l.ez));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_a, sizeof(double) * s.n_coeff));
   RSO_CHECK_CUDA(h, cudaMalloc(&h->coef_b, sizeof(double) * s.n_coeff));

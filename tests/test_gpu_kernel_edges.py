@@ -692,3 +692,27 @@ def test_host_iteration_of_another_size(cuda):
     with pytest.raises(RSOError, match="size differs"):
         g.design_iteration_host(m, np.ones(n), IterParams())
     assert np.array_equal(m.get()[0], x0)
+
+
+# few rows, cut in chunks of 32 to 128 elements with a ragged last one: supports inside a chunk, over
+# several, over all; and rows just too many for it
+@pytest.mark.parametrize("dims,order,parts", [((1000, 4, 3), 4, (200, 2, 1)), ((333, 5, 4), 3, (2, 0, 1)),
+                                              ((65, 8, 9), 5, (12, 3, 3)), ((129, 25, 24), 4, (9, 4, 5)),
+                                              ((97, 40, 30), 2, (40, 3, 3)), ((33, 2, 2), 4, (0, 0, 0))])
+@pytest.mark.parametrize("amplitude", [1.0, 3000.0])
+def test_spline_rows_in_chunks(oracle, cuda, dims, order, parts, amplitude):
+    """Adjoint 1e-6, constraint value 1e-5 and gradient 1e-4 relative, counts and probe sums equal: the
+    bounds of these maps in the parity tests."""
+    g, o = make(oracle, P.cantilever(*dims), n_levels=4, first_factor=2)
+    n = o.spline_setup(order, parts)
+    assert g.set_spline_partition(*parts, order) == n
+    rng = np.random.default_rng(73)
+    c = (amplitude * rng.normal(0.5, 0.15, n)).astype(np.float32)
+    x = rng.standard_normal(o.ne).astype(np.float32)
+    assert rel(g.ddensity2dcoeff(x).cpu().numpy(), o.density2coeff_adjoint(x.astype(np.float64))) < 1e-6
+    for mode in (4, 5):
+        v, per, dc, cnt, ds = g.deal_background_points(c, 8.0, mode)
+        vo, pero, dco, cnto, dso = o.selfsupport(c.astype(np.float64), 8.0, mode)
+        assert cnt == cnto and ds == dso and abs(v - vo) <= 1e-5 * max(abs(vo), 1e-12)
+        assert rel(per.cpu().numpy(), pero) < 1e-5
+        assert rel(dc.cpu().numpy(), dco) < 1e-4
