@@ -906,11 +906,11 @@ __global__ void __launch_bounds__(1024) k_max_abs(long long n, const double* __r
 // The penalty needs the sign `flip` that the sum of all probes gives.  It is
 // taken as -1 (`direction` likewise), which the sum confirms in every design
 // whose density grows along its gradient; the caller runs the pass again when
-// it does not.
+// it does not, without the probes (PROBE false), which cost most of it there.
 struct SSOut { double *G1, *Gy, *Gz; float* per; double* part; };
 constexpr int kSSRows = 4, kSSSeg = 128;
 static int ss_blocks(const Level& l) { return cdiv((long long)l.ey * l.ez, kSSRows); }
-template <int O>
+template <int O, bool PROBE>
 __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, SplineDev S, const double* __restrict__ c,
                                                              const double* __restrict__ R, long long comp, const SSPar P,
                                                              double flip, double direction,
@@ -956,14 +956,14 @@ __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, Spli
             }
           }
           const double gg = g0 * g0 + g1 * g1 + g2 * g2;
-          bool known = false;
-          if (O >= 3 && tH < 1.0 && inside) {
+          bool known = !PROBE;
+          if (PROBE && O >= 3 && tH < 1.0 && inside) {
             const double grow = 0.01 * gg * (1 - 0.5 * tH);
             // sech^2(s) >= exp(-2 |s|), s up to beta (|v - 1/2| + what the probe may rise)
             const float slope = __expf((float)(-2 * P.beta * (fabs(f - 0.5) + 0.02 * gg)));
             known = (float)(P.beta * grow) * slope > 1e-12f && grow > least && 1e-4 * gg < smin * smin;
           }
-          ndir += known || probe_sign(S, c, P.beta, x, y, z, inside, f, g0, g1, g2) < 0.f ? -1 : 1;
+          if (PROBE) ndir += known || probe_sign(S, c, P.beta, x, y, z, inside, f, g0, g1, g2) < 0.f ? -1 : 1;
           const bool dn = flip * g2 < 0;
           ndown += dn;
           const bool on = (P.mode % 2 == 1) || dn;
@@ -1029,6 +1029,12 @@ __global__ void __launch_bounds__(32 * kSSRows, 5) k_ss_rows(const Level L, Spli
     Q.part[(threadIdx.x * (long long)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = t;
   }
 }
+template <bool PROBE>
+static auto ss_rows_of(int order) {
+  return order == 2 ? k_ss_rows<2, PROBE> : order == 3 ? k_ss_rows<3, PROBE> : order == 4 ? k_ss_rows<4, PROBE>
+                                                                                          : k_ss_rows<5, PROBE>;
+}
+static auto ss_rows(int order, bool probe) { return probe ? ss_rows_of<true>(order) : ss_rows_of<false>(order); }
 // out[0..2] = the sums of probes, penalties and downward faces; out[3] the count the mean divides by
 __global__ void __launch_bounds__(1024) k_ss_sums(const double* __restrict__ part, int n, int mode, double active,
                                                  double* __restrict__ out) {
@@ -1094,9 +1100,9 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
   O.part = R + 3 * comp;
   double *G2 = h->sp.work[1], *G2z = G2 + t2;
   const int *r0 = h->sp.ranges[0], *r2 = h->sp.ranges[2];
-  double flip = -1.0, direction = -1.0;
+  double flip = -1.0, direction = -1.0, ds = 0;
   for (int pass = 0; pass < 2; pass++) {
-    auto rows = S.order == 2 ? k_ss_rows<2> : S.order == 3 ? k_ss_rows<3> : S.order == 4 ? k_ss_rows<4> : k_ss_rows<5>;
+    auto rows = ss_rows(S.order, pass == 0);
     rows<<<grid, 32 * kSSRows, 0, h->stream>>>(l, S, c, R, comp, P, flip, direction, sums + 4, hcoef, smin, r0,
                                                r0 + S.nb0, X.len, O, view_of(l, true)); rso::note_launch();
     k_ss_sums<<<1, 1024, 0, h->stream>>>(O.part, (int)(grid.x * grid.y), mode, (double)l.n_active_e, sums); rso::note_launch();
@@ -1108,14 +1114,14 @@ rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, do
     RSO_TRY(launch_check(h, "selfsupport"));
     RSO_CHECK_CUDA(h, cudaMemcpyAsync(h->h_scal + 48, sums, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
-    const double ds = h->h_scal[48];
+    if (pass == 0) ds = h->h_scal[48];
     const double f = ds < 0 ? -1.0 : 1.0, d = ds > 0 ? 1.0 : -1.0;
     if (f == flip && d == direction) break;
     flip = f;
     direction = d;
   }
   const double sum = h->h_scal[49], cnt = h->h_scal[51];
-  if (dirsum) *dirsum = h->h_scal[48];
+  if (dirsum) *dirsum = ds;
   if (count) *count = cnt;
   double v = 0;
   if (cnt != 0) v = (mode <= 1) ? std::pow(sum / cnt, 1 / P.fpara) - 1 : sum / cnt;

@@ -716,3 +716,24 @@ def test_spline_rows_in_chunks(oracle, cuda, dims, order, parts, amplitude):
         assert cnt == cnto and ds == dso and abs(v - vo) <= 1e-5 * max(abs(vo), 1e-12)
         assert rel(per.cpu().numpy(), pero) < 1e-5
         assert rel(dc.cpu().numpy(), dco) < 1e-4
+
+
+@pytest.mark.parametrize("dims,order,parts,seed", [((40, 24, 20), 3, (3, 5, 2), 0), ((33, 9, 70), 4, (3, 5, 2), 1),
+                                                   ((33, 9, 70), 5, (3, 5, 2), 0), ((12, 10, 8), 4, (30, 1, 12), 2)])
+def test_overhang_with_a_positive_probe_sum(oracle, cuda, dims, order, parts, seed):
+    """Coefficients so large that most probes land beyond the box or on the other side: the sum of the probes
+    is not negative and the pass runs again; the bounds of the constraint's parity test."""
+    g, o = make(oracle, P.cantilever(*dims), n_levels=2, first_factor=2)
+    n = o.spline_setup(order, parts)
+    assert g.set_spline_partition(*parts, order) == n
+    positive = 0
+    for k in range(4):
+        c = (3e5 * np.random.default_rng(seed + 10 * k).normal(0.5, 0.15, n)).astype(np.float32)
+        for mode in (0, 2, 4, 5):
+            v, per, dc, cnt, ds = g.deal_background_points(c, 8.0, mode)
+            vo, pero, dco, cnto, dso = o.selfsupport(c.astype(np.float64), 8.0, mode)
+            assert cnt == cnto and ds == dso
+            assert abs(v - vo) <= 1e-5 * max(abs(vo), 1e-12)
+            assert rel(per.cpu().numpy(), pero) < 1e-5 and rel(dc.cpu().numpy(), dco) < 1e-4
+        positive += ds >= 0
+    assert positive > 0
