@@ -737,3 +737,14 @@ def test_overhang_with_a_positive_probe_sum(oracle, cuda, dims, order, parts, se
             assert rel(per.cpu().numpy(), pero) < 1e-5 and rel(dc.cpu().numpy(), dco) < 1e-4
         positive += ds >= 0
     assert positive > 0
+
+
+@pytest.mark.parametrize("dims", [(1, 9, 40), (2, 33, 30), (5, 8, 50), (8, 8, 40), (9, 40, 9), (16, 5, 20), (17, 9, 9)])
+@pytest.mark.parametrize("radius", [0.6, 6.2])
+def test_general_filter_on_narrow_boxes(oracle, cuda, dims, radius):
+    """FP64 sums rounded to FP32 once: 1e-6 relative, on tiles of every width."""
+    g, o = make(oracle, P.cantilever(*dims), n_levels=2, first_factor=2)
+    x = np.random.default_rng(83).standard_normal(o.ne).astype(np.float32)
+    assert rel(g.filterSensitivity(radius, x).cpu().numpy(), o.filter(radius, x.astype(np.float64))) < 1e-6
+    assert rel(g.densityFilter(radius, x, adjoint=True).cpu().numpy(),
+               o.density_filter_adjoint(radius, x.astype(np.float64))) < 1e-6
