@@ -1788,14 +1788,15 @@ __global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid
       landed = false;
     }
   }
-  // every CTA with a tile waits for it before the tile's first use
+  // every CTA with a tile waits for it before the tile's first use; after a wait
+  // that gave up, the next barrier ends the kernel, and leave() waits once more
   auto need_tile = [&](int li) {
     if (li != own_li || landed) return;
-    if (!tile_landed(&tbar)) {
+    landed = tile_landed(&tbar);
+    if (!landed) {
       atomicOr(bar, kGbarGone);
       atomicExch(bar + 2, 1u);
     }
-    landed = true;
   };
   // leaving early: not before the tile's copy has ended
   auto leave = [&]() {
