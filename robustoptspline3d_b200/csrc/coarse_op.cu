@@ -1263,8 +1263,8 @@ __device__ void bot_restrict(const Level& Fl, const Level& C, const T* rf0, T* f
 template <typename T, int F>
 __device__ void bot_restrict3(const Level& Fl, const Level& C, const T* rf0, T* fc0, const T* __restrict__ st,
                               T* first0, T om, int g0, int gs) {
-  // the levels of the persistent kernel are below 2^31 nodes (checked by its
-  // launcher): 32-bit index arithmetic
+  // 4 nn nb and one step of the grid stay below 2^32 (kBottomNodes, checked by
+  // the launcher): 32-bit index arithmetic
   const unsigned nn = (unsigned)C.nn, nx = (unsigned)C.nx, ny = (unsigned)C.ny, all = nn * (unsigned)C.nb;
   for (unsigned it = g0; it < ((4u * all + 31u) & ~31u); it += gs) {  // whole warps: the quads shuffle
     const unsigned ib = it >> 2, c = it & 3u;
@@ -2127,6 +2127,11 @@ int bottom_level(const rso_handle* h, int pre, int post) {
   return -1;
 }
 
+// Padded nodes of a level, all systems, that the persistent kernel's 32-bit indices
+// take: bot_restrict3 counts to 4 a node in steps of the grid's threads, fewer than
+// 2^22, and the sweeps to 4 a group of four nodes.
+constexpr long long kBottomNodes = (1LL << 30) - (1LL << 20);
+static_assert(4ull * kBottomNodes + (1ull << 22) <= 1ull << 32, "no index of the persistent kernel wraps");
 template <typename T>
 rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
   BottomArgs<T> A;
@@ -2155,8 +2160,8 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
     return launch_check(h, "bottom_vcycle");
   }
   for (int li = lb; li < nl; li++)
-    if (h->L[li].NP * h->L[li].nb >= (1LL << 31)) {
-      h->err = "the persistent bottom kernel takes levels below 2^31 padded nodes";
+    if (h->L[li].NP * h->L[li].nb > kBottomNodes) {
+      h->err = "the persistent bottom kernel takes levels of at most 2^30 - 2^20 padded nodes";
       return RSO_ERR_UNSUPPORTED;
     }
   // the persistent kernel: at most as many CTAs as are resident at once (a
