@@ -104,6 +104,12 @@ typedef struct {
 rso_status rso_voxelize(const float* vertices_host, int n_vertices, const int* faces_host, int n_faces,
                         int preferred_resolution, uint8_t* solid_host, int* resolution_out, float* box_out);
 
+/* The mesh input's entry points (rso_voxelize to rso_region_field) keep device
+ * blocks between calls, at most 1 GiB a device, and a pinned ring of 8 MB for
+ * their results: this gives all of it back.  Calls under way in other threads
+ * keep what they hold, and later calls allocate again. */
+rso_status rso_release_mesh_memory(void);
+
 /* Shell elements of a voxelised mesh (HierarchyGrid::setSolidShellElement,
  * grid/Grid.cpp:253-322): with h = (box max x - box min x) / R (FP32
  * quotient) and w = shell_width * h, solid element e = (x, y, z) of the R^3

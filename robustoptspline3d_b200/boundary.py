@@ -276,6 +276,11 @@ def _check(st, what):
         raise RSOError(f"{what}: status {st}")
 
 
+def release_memory():
+    """Give back the device blocks and the pinned ring that the mesh input keeps between calls."""
+    _check(load_library().rso_release_mesh_memory(), "rso_release_mesh_memory")
+
+
 def region_mask(regions, origin, h, dims):
     """Union of `regions` on the node grid origin + (i, j, k) h, dims = (nx, ny, nz);
     (nz, ny, nx) uint8 array."""

@@ -720,7 +720,25 @@ cudaError_t block_get(int dev, size_t bytes, void** p, size_t* cls) {
         return cudaSuccess;
       }
   }
+  const cudaError_t e = cudaMalloc(p, c);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();  // the blocks of other sizes may be what is missing
+  blocks_release(dev);
   return cudaMalloc(p, c);
+}
+
+// frees the cached blocks of a device, or of all (dev < 0)
+void blocks_release(int dev) {
+  for (int k = 0; k < kCacheDevices; k++) {
+    if (dev >= 0 && k != dev) continue;
+    std::vector<std::pair<size_t, void*>> v;
+    {
+      std::lock_guard<std::mutex> lk(g_blocks.m);
+      v.swap(g_blocks.blocks[k]);
+      g_blocks.held[k] = 0;
+    }
+    for (const auto& b : v) cudaFree(b.second);
+  }
 }
 
 void block_put(int dev, size_t cls, void* p) {
@@ -741,8 +759,8 @@ void block_put(int dev, size_t cls, void* p) {
 // the transfer needs 0.3 ms (four 17 MB results of the mesh input, 19 -> 13 ms
 // with the computations between them).  Here pieces go through a pinned ring, and a few
 // threads carry them on to the destination, each piece's slot being refilled
-// as soon as it is empty.  The ring (8 MB) is made on first use and kept; a
-// call that finds it in use, or any failure to get threads or pinned memory,
+// as soon as it is empty.  The ring (8 MB) is made on first use and kept until
+// rso_release_mesh_memory; a call that finds it in use, or any failure to get threads or pinned memory,
 // takes the driver's copy.  Starting the threads takes 0.1 to 0.4 ms, more or less
 // from call to call, so copies below kRingLeast take the driver's too (region masks,
 // medians of 25 calls: 5.3 MB 0.95 and 0.78 ms through the ring, 0.77 and 0.87 by
@@ -787,6 +805,13 @@ struct Carry {
   }
 };
 }  // namespace
+
+// frees the ring, after the call that uses it
+static void ring_release() {
+  std::lock_guard<std::mutex> lk(g_ring.m);
+  if (g_ring.slots) cudaFreeHost(g_ring.slots);
+  g_ring.slots = nullptr;
+}
 
 cudaError_t copy_to_host(void* dst, const void* src, size_t n) {
   cudaPointerAttributes at{};
@@ -843,6 +868,12 @@ bool regions_valid(const rso_region* r, int n) {
 }  // namespace rso
 
 using namespace rso;
+
+extern "C" rso_status rso_release_mesh_memory(void) {
+  blocks_release(-1);
+  ring_release();
+  return RSO_OK;
+}
 
 extern "C" rso_status rso_shell_elements(const float* vertices_host, int n_vertices, const int* faces_host,
                                          int n_faces, const float* box_host, int resolution, double shell_width,

@@ -527,9 +527,11 @@ rso_status modified_pm(rso_handle* h, int cf, uint64_t seed, int max_itn, double
 // size classes between calls: repeated calls reuse them instead of
 // allocating and freeing (a free lets the driver unmap the memory and the
 // next allocation map it again, which made the call times vary by tens of
-// milliseconds).  At most kCacheCap bytes per device stay cached.
+// milliseconds).  At most kCacheCap bytes per device stay cached, until
+// rso_release_mesh_memory or an allocation that fails for lack of memory.
 cudaError_t block_get(int dev, size_t bytes, void** p, size_t* cls);
 void block_put(int dev, size_t cls, void* p);
+void blocks_release(int dev);
 // device to ordinary host memory, after the default stream's work; returns when the bytes are there
 cudaError_t copy_to_host(void* dst, const void* src, size_t n);
 

@@ -114,6 +114,7 @@ SIGNATURES = {
     "rso_set_vcycle_graphs": (_ci, [_vp, _ci]),
     "rso_set_solve_graphs": (_ci, [_vp, _ci]),
     "rso_graph_launches": (_ci, [_vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]),
+    "rso_release_mesh_memory": (_ci, []),
     "rso_set_fine_zchunk": (_ci, [_vp, _ci]),
     "rso_fine_zchunk": (_ci, [_vp]),
     "rso_set_bottom_kernel": (_ci, [_vp, _ci]),

@@ -748,3 +748,29 @@ def test_general_filter_on_narrow_boxes(oracle, cuda, dims, radius):
     assert rel(g.filterSensitivity(radius, x).cpu().numpy(), o.filter(radius, x.astype(np.float64))) < 1e-6
     assert rel(g.densityFilter(radius, x, adjoint=True).cpu().numpy(),
                o.density_filter_adjoint(radius, x.astype(np.float64))) < 1e-6
+
+
+def test_mesh_memory_is_given_back(cuda):
+    """The mesh input's cached blocks and pinned ring go back on request, also while other threads call, and
+    calls after it give the same bytes."""
+    from concurrent.futures import ThreadPoolExecutor
+    from robustoptspline3d_b200 import boundary as B
+    from robustoptspline3d_b200.voxelize import voxelize
+    v, f = M.icosphere(3, 4.0)
+
+    def run(_=None):
+        solid, R, box = voxelize(v, f, 140)
+        return solid, B.shell_elements(v, f, box, R, 2.0, solid)
+
+    B.release_memory()
+    cuda.cuda.synchronize()
+    free = cuda.cuda.mem_get_info()[0]
+    want = run()
+    assert cuda.cuda.mem_get_info()[0] < free
+    B.release_memory()
+    assert cuda.cuda.mem_get_info()[0] >= free
+    with ThreadPoolExecutor(4) as pool:
+        jobs = [pool.submit(run) if k % 3 else pool.submit(B.release_memory) for k in range(12)]
+        got = [j.result() for j in jobs]
+    for g in got:
+        assert g is None or all(np.array_equal(a, b) for a, b in zip(g, want))
