@@ -26,7 +26,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
-#include <system_error>
+#include <new>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -744,11 +744,12 @@ void blocks_release(int dev) {
 void block_put(int dev, size_t cls, void* p) {
   if (dev >= 0 && dev < kCacheDevices) {
     std::lock_guard<std::mutex> lk(g_blocks.m);
-    if (g_blocks.held[dev] + cls <= kCacheCap) {
-      g_blocks.blocks[dev].push_back({cls, p});
-      g_blocks.held[dev] += cls;
-      return;
-    }
+    if (g_blocks.held[dev] + cls <= kCacheCap) try {
+        g_blocks.blocks[dev].push_back({cls, p});
+        g_blocks.held[dev] += cls;
+        return;
+      } catch (const std::bad_alloc&) {  // no room in the list: freed
+      }
   }
   cudaFree(p);
 }
@@ -834,9 +835,9 @@ cudaError_t copy_to_host(void* dst, const void* src, size_t n) {
   if (e == cudaSuccess) {
     std::thread helper[kCarriers - 1];
     int helpers = 0;
-    try {  // std::thread throws when the system has no thread to give
+    try {  // std::thread throws when the system has no thread, or no memory, to give
       for (; helpers < kCarriers - 1; helpers++) helper[helpers] = std::thread(&Carry::run, &c, helpers + 1, kCarriers);
-    } catch (const std::system_error&) {
+    } catch (...) {
     }
     c.run(0, kCarriers);
     for (int t = helpers + 1; t < kCarriers; t++) c.run(t, kCarriers);  // those without a thread of their own

@@ -543,18 +543,20 @@ struct Scratch {
     void* p;
     size_t cls;
   };
-  std::vector<Block> blocks;
-  int dev = -1;
+  static constexpr int kMost = 16;  // blocks a call takes (an entry point takes ten at most)
+  Block blocks[kMost];
+  int taken = 0, dev = -1;
   cudaError_t err = cudaSuccess;
   Scratch() { err = cudaGetDevice(&dev); }
   template <typename T>
   T* upload(const T* host, size_t n) {
+    if (err == cudaSuccess && taken == kMost) err = cudaErrorMemoryAllocation;
     if (err != cudaSuccess) return nullptr;
     void* p = nullptr;
     size_t cls = 0;
     err = block_get(dev, sizeof(T) * (n ? n : 1), &p, &cls);
     if (err != cudaSuccess) return nullptr;
-    blocks.push_back({p, cls});
+    blocks[taken++] = {p, cls};
     if (host && n) err = cudaMemcpy(p, host, sizeof(T) * n, cudaMemcpyHostToDevice);
     return static_cast<T*>(p);
   }
@@ -566,7 +568,7 @@ struct Scratch {
       cudaDeviceSynchronize();
       cudaGetLastError();
     }
-    for (const Block& b : blocks) block_put(dev, b.cls, b.p);
+    for (int k = 0; k < taken; k++) block_put(dev, blocks[k].cls, blocks[k].p);
   }
 };
 
