@@ -19,12 +19,16 @@ static rso_status finish(rso_handle* h) {
   return RSO_OK;
 }
 
-// The maps read and write the caller's arrays directly.  An output may overlap
-// an input: the input (n floats) is then read from a copy in a scratch field.
-static rso_status apart(rso_handle* h, const float** in, long long n, const float* out, long long n_out, float* scratch) {
-  if (*in >= out + n_out || *in + n <= out) return RSO_OK;
-  RSO_CHECK_CUDA(h, cudaMemcpyAsync(scratch, *in, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream));
-  *in = scratch;
+// The maps read and write the caller's arrays directly.  An output (ne floats) may
+// overlap an input, the shell mask too: the input (ne entries, or none) is then read
+// from a copy in a scratch field.
+template <typename T>
+static rso_status apart(rso_handle* h, const T** in, const float* out, float* scratch) {
+  const size_t ne = (size_t)h->L[0].ne;
+  const char *a = (const char*)*in, *b = (const char*)out;
+  if (!a || a >= b + sizeof(float) * ne || a + sizeof(T) * ne <= b) return RSO_OK;
+  RSO_CHECK_CUDA(h, cudaMemcpyAsync(scratch, *in, sizeof(T) * ne, cudaMemcpyDeviceToDevice, h->stream));
+  *in = reinterpret_cast<const T*>(scratch);
   return RSO_OK;
 }
 
@@ -45,25 +49,23 @@ extern "C" rso_status rso_element_energy(rso_handle* h, const double* u, float* 
 
 extern "C" rso_status rso_heaviside(rso_handle* h, const float* in, double beta, const uint8_t* shell, float* out) {
   if (!h || !in || !out) return RSO_ERR_INVALID_ARG;
-  const long long ne = h->L[0].ne;
-  RSO_TRY(apart(h, &in, ne, out, ne, h->e_a));
+  RSO_TRY(apart(h, &in, out, h->e_a));
+  RSO_TRY(apart(h, &shell, out, h->e_b));
   RSO_TRY(heaviside(h, in, beta, shell, out, true));
   return finish(h);
 }
 
 extern "C" rso_status rso_heaviside_chain(rso_handle* h, const float* rho, double beta, const float* gin, float* gout) {
   if (!h || !rho || !gin || !gout) return RSO_ERR_INVALID_ARG;
-  const long long ne = h->L[0].ne;
-  RSO_TRY(apart(h, &rho, ne, gout, ne, h->e_a));
-  RSO_TRY(apart(h, &gin, ne, gout, ne, h->e_b));
+  RSO_TRY(apart(h, &rho, gout, h->e_a));
+  RSO_TRY(apart(h, &gin, gout, h->e_b));
   RSO_TRY(heaviside_chain(h, rho, beta, gin, gout, true));
   return finish(h);
 }
 
 static rso_status filter_api(rso_handle* h, double R, const float* in, float* out, int adjoint) {
   if (!h || !in || !out || !(R > 0)) return RSO_ERR_INVALID_ARG;
-  const long long ne = h->L[0].ne;
-  RSO_TRY(apart(h, &in, ne, out, ne, h->e_a));
+  RSO_TRY(apart(h, &in, out, h->e_a));
   RSO_TRY(filter(h, R, in, out, adjoint, true));
   return finish(h);
 }
@@ -103,6 +105,7 @@ extern "C" rso_status rso_coeff2density(rso_handle* h, const float* coeff, const
   if (!h || !coeff || !rho_hat) return RSO_ERR_INVALID_ARG;
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
   k_f2d_n<<<cdiv(h->sp.n_coeff, 256), 256, 0, h->stream>>>(coeff, h->coef_a, h->sp.n_coeff); rso::note_launch();
+  RSO_TRY(apart(h, &shell, rho_hat, h->e_a));
   RSO_TRY(coeff2density(h, h->coef_a, shell, rho_hat, true));
   return finish(h);
 }

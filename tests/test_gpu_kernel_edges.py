@@ -774,3 +774,45 @@ def test_mesh_memory_is_given_back(cuda):
         got = [j.result() for j in jobs]
     for g in got:
         assert g is None or all(np.array_equal(a, b) for a, b in zip(g, want))
+
+
+@pytest.mark.parametrize("shift", [-700, -1, 0, 1, 700])
+def test_maps_on_overlapping_arrays(cuda, shift):
+    """Outputs that overlap an input by all, most or a part of it, and the shell mask inside the output: the
+    bits of the calls on separate arrays."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.voids_box(21, 13, 11, nvoids=1)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"], Config(n_levels=2, first_factor=2))
+    n = g.set_spline_partition(3, 2, 4, 4)
+    rng = np.random.default_rng(89)
+    x, y = rng.uniform(0, 1, g.ne).astype(np.float32), rng.standard_normal(g.ne).astype(np.float32)
+    c = rng.normal(0.5, 0.15, n).astype(np.float32)
+    sh = (rng.random(g.ne) < 0.2).astype(np.uint8)
+    buf = cuda.empty(g.ne + 2000, device="cuda")
+    at = lambda k, size=None: buf[1000 + k:1000 + k + (size or g.ne)]  # noqa: E731
+    L, H = g.lib, g.h
+
+    def overlapping(call):
+        at(0).copy_(t(x, cuda))
+        assert call(at(0).data_ptr(), at(shift).data_ptr()) == 0
+        return at(shift).clone()
+
+    other = t(y, cuda)
+    assert cuda.equal(overlapping(lambda i, o: L.rso_heaviside(H, i, 8.0, None, o)), g.projectDensities(x, 8.0))
+    assert cuda.equal(overlapping(lambda i, o: L.rso_heaviside_chain(H, i, 8.0, other.data_ptr(), o)),
+                      g.projectSensitivity(x, 8.0, y))
+    assert cuda.equal(overlapping(lambda i, o: L.rso_heaviside_chain(H, other.data_ptr(), 8.0, i, o)),
+                      g.projectSensitivity(y, 8.0, x))
+    for r in (0.7, 2.0, 5.5):
+        assert cuda.equal(overlapping(lambda i, o: L.rso_filter(H, r, i, o)), g.filterSensitivity(r, x))
+        assert cuda.equal(overlapping(lambda i, o: L.rso_density_filter_adjoint(H, r, i, o)),
+                          g.densityFilter(r, x, adjoint=True))
+    xin, cin, mask = t(x, cuda), t(c, cuda), t(sh, cuda)
+    for call, want in ((lambda m, o: L.rso_heaviside(H, xin.data_ptr(), 8.0, m, o), g.projectDensities(x, 8.0, sh)),
+                       (lambda m, o: L.rso_coeff2density(H, cin.data_ptr(), m, o), g.coeff2density(c, sh))):
+        at(shift // 4, g.ne).view(cuda.uint8)[:g.ne].copy_(mask)
+        assert call(at(shift // 4).data_ptr(), at(0).data_ptr()) == 0
+        assert cuda.equal(at(0), want)
+    at(0, n).copy_(cin)
+    assert L.rso_coeff2density(H, at(0).data_ptr(), None, at(shift // 4).data_ptr()) == 0
+    assert cuda.equal(at(shift // 4), g.coeff2density(c))
