@@ -816,3 +816,52 @@ def test_maps_on_overlapping_arrays(cuda, shift):
     at(0, n).copy_(cin)
     assert L.rso_coeff2density(H, at(0).data_ptr(), None, at(shift // 4).data_ptr()) == 0
     assert cuda.equal(at(shift // 4), g.coeff2density(c))
+
+
+@pytest.mark.parametrize("radius", [0.7, 1.0, 2.0, 3.7, 4.4, 5.3])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, -3.4028234e38, 3.4028234e38])
+def test_filter_and_sums_on_extreme_values(cuda, radius, value):
+    """One extreme value, on an active or on an inactive element, against FP64 sums over the taps: it reaches
+    the elements within the radius and no other, and none from where the mask is off; 1e-6 relative."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    ex, ey, ez = 37, 11, 13
+    prob = P.voids_box(ex, ey, ez, nvoids=2)
+    em = prob["emask"].astype(bool)
+    em[6, 5, 30] = True
+    em[6, 5, 7] = False
+    prob["emask"] = em.astype(np.uint8)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"], Config(n_levels=2, first_factor=2))
+    x = np.random.default_rng(97).standard_normal(em.shape).astype(np.float32)
+    x[6, 5, 30] = value   # active
+    x[6, 5, 7] = value    # inactive
+    R = int(radius + 0.5)
+    num, den = np.zeros(em.shape), np.zeros(em.shape)
+    with np.errstate(invalid="ignore", over="ignore"):
+        xv = np.where(em, x.astype(np.float64), 0.0)
+        for dz in range(-R, R + 1):
+            for dy in range(-R, R + 1):
+                for dx in range(-R, R + 1):
+                    d2 = dx * dx + dy * dy + dz * dz
+                    if d2 > radius * radius:
+                        continue
+                    r = np.sqrt(d2) / radius
+                    w = 1 - 6 * r ** 2 + 8 * r ** 3 - 3 * r ** 4
+                    src = tuple(slice(max(d, 0), n + min(d, 0)) for d, n in zip((dz, dy, dx), em.shape))
+                    dst = tuple(slice(max(-d, 0), n + min(-d, 0)) for d, n in zip((dz, dy, dx), em.shape))
+                    num[dst] += np.where(em[src], w * xv[src], 0.0)
+                    den[dst] += np.where(em[src], w, 0.0)
+        want = np.where(em, num / np.where(em, den, 1.0), 0.0).astype(np.float32)
+    got = g.filterSensitivity(radius, x.ravel()).cpu().numpy().reshape(em.shape)
+    fin = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), fin) and np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(got[np.isinf(got)], want[np.isinf(want)])
+    assert np.all(np.abs(got[fin] - want[fin]) <= 1e-6 * np.maximum(np.abs(want[fin]), 1.0))
+    vol = g.volumeRatio(x.ravel())
+    ref = np.where(em, x.astype(np.float64), 0.0).sum()
+    one = g.volumeRatio(np.ones(em.size, np.float32)) / em.sum()  # the divisor counts padded elements
+    assert np.isnan(vol) if np.isnan(ref) else (vol == ref if np.isinf(ref) else abs(vol - ref * one) <= 1e-6 * abs(ref * one))
+    with np.errstate(invalid="ignore", over="ignore"):
+        s = 8.0 * (x.astype(np.float64) - 0.5)
+        step = np.clip(np.nan_to_num((np.tanh(4.0) + np.tanh(s)) / (2 * np.tanh(4.0)), nan=1e-3), 1e-3, 1.0)
+    heav = g.projectDensities(x.ravel(), 8.0).cpu().numpy().reshape(em.shape)
+    assert np.max(np.abs(heav - np.where(em, step, 0.0))) < 1e-7
