@@ -41,6 +41,16 @@ static dim3 elem_grid(const Level& l) {
   if (elem_block(l).y > 1) return dim3(cdiv(l.ex, 32), cdiv(l.ey, 8), std::min(l.ez, 65535));
   return dim3(cdiv((long long)l.ex * l.ey, 256), 1, std::min(l.ez, 65535));
 }
+// the thread's element of a plane; false outside the box
+__device__ __forceinline__ bool elem_of(const Level& L, int& x, int& y) {
+  unsigned i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (blockDim.y == 1) {  // in line
+    j = i / (unsigned)L.ex;
+    i -= j * (unsigned)L.ex;
+  }
+  x = (int)i, y = (int)j;
+  return i < (unsigned)L.ex && j < (unsigned)L.ey;
+}
 // one thread per column of zc elements: long where the tiles of a plane alone
 // give the GPU eight CTAs per SM, 4 at least (a plane is shared by two elements)
 static dim3 column_grid(const Level& l, int zc) { return dim3(cdiv(l.ex, 32), cdiv(l.ey, 8), cdiv(l.ez, zc)); }
@@ -63,56 +73,45 @@ __device__ __forceinline__ double power(double r, double p) {
 // In the sum/difference basis of the element's nodes, w = W u_e along each axis,
 // K0 = W^T B W with the block structure of fine_op.cu, so the quadratic form is
 // a sum over the eight blocks: about 120 operations where the 24 x 24 product
-// takes 600.  A thread marches along z, so that a node plane is loaded and
-// transformed once for the elements on both sides.  256^3: 1887 us with the
-// product (bound by the FP64 units), 303 with a thread per element.
+// takes 600.  256^3: 1887 us with the product (bound by the FP64 units), 382 with a
+// thread marching along z, which transforms a node plane once for the elements on
+// both sides but has too few loads in flight, 302 with a thread per element; 64^3
+// 10.7 and 8.5.
 // B.c in the order of cWp: A0 - B0, B0, A7 - B7, B7, P, Q, R, S.
 struct WalshB { double c[8]; };
 __global__ void __launch_bounds__(256) k_sensitivity(const Level L, const double* __restrict__ u,
                                                      const float* __restrict__ rho, const WalshB B, double p, int energy,
-                                                     float* __restrict__ out, const View V, int zc) {
-  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
-  if (x >= L.ex || y >= L.ey) return;
-  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.ez);
-  // xy modes of a face's four nodes; an element's upper face is the next one's lower
-  auto face = [&](int z, double (&f)[3][4]) {
+                                                     float* __restrict__ out, const View V) {
+  int x, y;
+  if (!elem_of(L, x, y)) return;
+  for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
+    const long long e = L.eidx(x, y, z), o = V.at(x, y, z);
+    if (!L.emask[e]) { out[o] = 0.f; continue; }
+    double w[8][3];  // modes (mx, my, mz) as bits, component
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      const double* q = u + L.nidx(x, y, z) + c * L.NP;
-      const double a00 = q[0], a10 = q[1], a01 = q[L.px], a11 = q[L.px + 1];
-      const double s0 = a00 + a10, d0 = a10 - a00, s1 = a01 + a11, d1 = a11 - a01;
-      f[c][0] = s0 + s1; f[c][1] = d0 + d1; f[c][2] = s1 - s0; f[c][3] = d1 - d0;
-    }
-  };
-  auto full = [&](double i, double j, double k, double ab, double bb) {
-    const double t = i + j + k;
-    return ab * (i * i + j * j + k * k) + bb * (t * t);
-  };
-  auto pair = [&](double i, double j) { return B.c[4] * (i * i + j * j) + 2.0 * B.c[5] * (i * j); };
-  auto both = [&](double i, double j, double k) { return B.c[6] * ((i + j) * (i + j)) + B.c[7] * (k * k); };
-  double f[3][4];
-  face(z0, f);
-  for (int z = z0; z < z1; z++) {
-    double up[3][4], w[8][3];  // modes (mx, my, mz) as bits, component
-    face(z + 1, up);
+      double f[2][4];  // xy modes of the lower and upper face
 #pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        w[m][c] = f[c][m] + up[c][m];
-        w[m + 4][c] = up[c][m] - f[c][m];
-        f[c][m] = up[c][m];
+      for (int b = 0; b < 2; b++) {
+        const double* q = u + L.nidx(x, y, z + b) + c * L.NP;
+        const double a00 = q[0], a10 = q[1], a01 = q[L.px], a11 = q[L.px + 1];
+        const double s0 = a00 + a10, d0 = a10 - a00, s1 = a01 + a11, d1 = a11 - a01;
+        f[b][0] = s0 + s1; f[b][1] = d0 + d1; f[b][2] = s1 - s0; f[b][3] = d1 - d0;
       }
+#pragma unroll
+      for (int m = 0; m < 4; m++) { w[m][c] = f[0][m] + f[1][m]; w[m + 4][c] = f[1][m] - f[0][m]; }
+    }
+    auto full = [&](double i, double j, double k, double ab, double bb) {
+      const double t = i + j + k;
+      return ab * (i * i + j * j + k * k) + bb * (t * t);
+    };
+    auto pair = [&](double i, double j) { return B.c[4] * (i * i + j * j) + 2.0 * B.c[5] * (i * j); };
+    auto both = [&](double i, double j, double k) { return B.c[6] * ((i + j) * (i + j)) + B.c[7] * (k * k); };
     double q = full(w[1][0], w[2][1], w[4][2], B.c[0], B.c[1]) + full(w[6][0], w[5][1], w[3][2], B.c[2], B.c[3]);
     q += pair(w[3][1], w[5][2]) + pair(w[3][0], w[6][2]) + pair(w[5][0], w[6][1]);
     q += both(w[2][0], w[1][1], w[7][2]) + both(w[4][0], w[1][2], w[7][1]) + both(w[4][1], w[2][2], w[7][0]);
-    const long long e = L.eidx(x, y, z);
-    float o = 0.f;
-    if (L.emask[e]) {
-      const double r = (double)rho[e];
-      o = energy ? (float)(power(r, p) * q) : (float)(-p * (p == 1.0 ? 1.0 : power(r, p - 1)) * q);
-    }
-    out[V.at(x, y, z)] = o;
+    const double r = (double)rho[e];
+    out[o] = energy ? (float)(power(r, p) * q) : (float)(-p * (p == 1.0 ? 1.0 : power(r, p - 1)) * q);
   }
 }
 
@@ -120,9 +119,8 @@ rso_status sensitivity(rso_handle* h, const double* u_pad, float* sens, int ener
   const Level& l = h->L[0];
   WalshB B;
   walsh_constants(h->K0, B.c);
-  const int zc = column_chunk(l);
-  k_sensitivity<<<column_grid(l, zc), dim3(32, 8), 0, h->stream>>>(l, u_pad, h->rho, B, h->cfg.penal, energy, sens,
-                                                                   view_of(l, dense), zc); rso::note_launch();
+  k_sensitivity<<<elem_grid(l), elem_block(l), 0, h->stream>>>(l, u_pad, h->rho, B, h->cfg.penal, energy, sens,
+                                                               view_of(l, dense)); rso::note_launch();
   return launch_check(h, "sensitivity");
 }
 
@@ -211,12 +209,8 @@ template <bool PADDED>
 __global__ void k_filter(const Level L, const FOff* __restrict__ off, int noff, const float* __restrict__ in,
                          float* __restrict__ out, int mode, const float* __restrict__ wsum, const View V) {
   // mode 0: out = sum w in / sum w;  1: out = sum w (weight sums, padded);  2: out = sum w in/W_n (adjoint)
-  unsigned x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (blockDim.y == 1) {  // the plane's elements in line
-    y = x / (unsigned)L.ex;
-    x -= y * (unsigned)L.ex;
-  }
-  if (x >= (unsigned)L.ex || y >= (unsigned)L.ey) return;
+  int x, y;
+  if (!elem_of(L, x, y)) return;
   for (int z = blockIdx.z; z < L.ez; z += gridDim.z) {
     const long long e = L.eidx(x, y, z), o = mode == 1 ? e : V.at(x, y, z);
     if (!L.emask[e]) { out[o] = 0.f; continue; }
