@@ -316,16 +316,16 @@ __global__ void __launch_bounds__(C4G * 3, 3) k_coarse4(const Level L, const flo
 // Jacobi update exchanges the three residual components through shared
 // memory.
 constexpr int CTY = 4;
-// thread (x, y, r) of a 32 x CTY x 3 tile at plane z of system bsys; ZERO:
-// u read as zero (a first step from a zero iterate).  sres is the tile's
-// shared exchange; every thread of the CTA calls this (MODE 2 synchronises it)
-// The vectors are plain pointers here: the persistent bottom kernel writes
-// them in earlier phases of the same launch, so their loads must be coherent
-// ones (the per-level kernel's own parameters carry __restrict__).
-template <typename T, int MODE, bool ZERO = false>
-__device__ __forceinline__ void coarse_r_node(const Level& L, const T* __restrict__ st, const T* u, const T* f,
-                                              T* out, T omega, const T* uprev, T c1, int x, int y, int z, int bsys,
-                                              T (*sres)[CTY][32]) {
+template <typename T, int MODE>
+__global__ void __launch_bounds__(32 * CTY * 3) k_coarse_r(const Level L, const T* __restrict__ st,
+                                                           const T* __restrict__ u, const T* __restrict__ f,
+                                                           T* __restrict__ out, T omega,
+                                                           const T* __restrict__ uprev, T c1) {
+  pdl_wait(u, f, out, uprev);
+  pdl_trigger();
+  __shared__ T sres[3][CTY][32];
+  const int bsys = blockIdx.z / L.nz;
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * CTY + threadIdx.y, z = blockIdx.z - bsys * L.nz;
   {
     const long long off = (long long)bsys * 3 * L.NP;
     u += off;
@@ -339,7 +339,7 @@ __device__ __forceinline__ void coarse_r_node(const Level& L, const T* __restric
   const long long n = in ? L.nidx(x, y, z) : 0;
   const bool act = in && (L.vclass[n] & NC_ACTIVE) != 0;
   T acc = 0;
-  if (act && !ZERO) {
+  if (act) {
 #pragma unroll
     for (int d = 0; d < 27; d++) {
       const long long nb = n + (d % 3 - 1) + (d / 3 % 3 - 1) * px + (d / 9 - 1) * pxy;
@@ -369,20 +369,8 @@ __device__ __forceinline__ void coarse_r_node(const Level& L, const T* __restric
   else { a0 = c02; a1 = -(S[0] * S[7] - S[1] * S[6]); a2 = S[0] * S[4] - S[1] * S[3]; }
   const T r0 = sres[0][threadIdx.y][threadIdx.x], r1 = sres[1][threadIdx.y][threadIdx.x],
           r2 = sres[2][threadIdx.y][threadIdx.x];
-  const T ur = ZERO ? T(0) : u[n + r * NP], pr = uprev ? uprev[n + r * NP] : T(0);
+  const T ur = u[n + r * NP], pr = uprev ? uprev[n + r * NP] : T(0);
   out[n + r * NP] = ur + c1 * (ur - pr) + (omega / det) * (a0 * r0 + a1 * r1 + a2 * r2);
-}
-template <typename T, int MODE>
-__global__ void __launch_bounds__(32 * CTY * 3) k_coarse_r(const Level L, const T* __restrict__ st,
-                                                           const T* __restrict__ u, const T* __restrict__ f,
-                                                           T* __restrict__ out, T omega,
-                                                           const T* __restrict__ uprev, T c1) {
-  pdl_wait(u, f, out, uprev);
-  pdl_trigger();
-  __shared__ T sres[3][CTY][32];
-  const int bsys = blockIdx.z / L.nz;
-  coarse_r_node<T, MODE>(L, st, u, f, out, omega, uprev, c1, blockIdx.x * 32 + threadIdx.x,
-                         blockIdx.y * CTY + threadIdx.y, blockIdx.z - bsys * L.nz, bsys, sres);
 }
 
 // Small levels (a few thousand to a few ten thousand nodes): the per-row
@@ -1472,15 +1460,6 @@ __global__ void __cluster_dims__(BOT_CTAS, 1, 1) __launch_bounds__(BOT_THREADS, 
   }
 }
 
-// The same bottom of the V-cycle as one persistent kernel over the whole GPU:
-// a cooperative launch (every CTA resident at once) whose phases are
-// separated by a grid-wide barrier.  FP32 sweeps run on four-node groups with
-// nine threads each and, on the levels that fit, on stencils held in shared
-// memory (below); FP64 sweeps with nine threads per node.  What bounds it is latency: a phase
-// is a barrier and one round of loads.  Per V-cycle, 2 + 2 Chebyshev steps: from
-// the 33^3 level of 256^3 down 174 -> 149 us (33^3 streamed, the rest held),
-// 93 x 71 x 85 110 -> 70 us, 64^3 96 -> 59 us, 49 x 38 x 56 68 -> 37 us (all
-// held), before: two-word barriers, every stencil streamed, two CTAs per SM.
 // FP64: a sweep (MODE 2) or residual (MODE 0) of the persistent kernel on tiles
 // of G9 consecutive nodes with nine threads each, one per neighbour row: 27
 // independent stencil loads a thread, the partial sums met in shared memory in
@@ -1569,13 +1548,9 @@ __device__ void gb_sweep9(const Level& L, const double* __restrict__ st, const d
 // latencies long.  The nine partial sums meet in shared memory in a fixed
 // order; four of the group's threads then finish one node each as k_coarse4
 // does (residual, or damped block Jacobi / Chebyshev step; halo rows
-// unwritten).  A team of 9 G9 threads takes a tile of G9 groups, the 128 nodes
+// unwritten).  A CTA of 9 G9 threads takes a tile of G9 groups, the 128 nodes
 // of one tile of the FP32 stencil.
-constexpr int kTeam = 9 * G9, kTeams = 1;
-static_assert(4 * G9 == ST_TILE, "a team's tile is a tile of the stencil");
-__device__ __forceinline__ void team_sync(int team) {
-  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeam) : "memory");
-}
+static_assert(4 * G9 == ST_TILE, "a CTA's tile is a tile of the stencil");
 struct GroupPos {
   long long p0 = 0;  // the group's first padded node
   int xp = 0;        // and its padded x
@@ -1607,7 +1582,7 @@ __device__ __forceinline__ GroupPos group_pos(const Level& L, long long g, bool 
 template <int MODE, bool ZERO, bool RES>
 __device__ __forceinline__ void group_step(const Level& L, const float* __restrict__ st, const GroupPos& P,
                                            const float* u, const float* f, float* out, float omega, const float* up,
-                                           float c1, int tg, int q, int team, float (*red)[12][G9]) {
+                                           float c1, int tg, int q, float (*red)[12][G9]) {
   const long long NP = L.NP, p0 = P.p0;
   const int pz = q / 3, py = q - 3 * pz;
   auto sat = [&](int k) { return RES ? (long long)(k * (int)ST_TILE + 4 * tg) : st_at<float>(NP, k, p0); };
@@ -1660,7 +1635,7 @@ __device__ __forceinline__ void group_step(const Level& L, const float* __restri
   for (int r = 0; r < 3; r++)
 #pragma unroll
     for (int k = 0; k < 4; k++) red[q][r * 4 + k][tg] = acc[r][k];
-  team_sync(team);
+  __syncthreads();
   if (fin) {
     // the node's nine partial sums in the order dz, dy = (-1, -1) .. (1, 1)
     float res[3];
@@ -1694,31 +1669,31 @@ __device__ __forceinline__ void group_step(const Level& L, const float* __restri
       out[n + 2 * NP] = uo[2] + c1 * (uo[2] - pv[2]) + id * (C * r0 + i21 * r1 + i22 * r2);
     }
   }
-  team_sync(team);  // red is reused by the next tile
+  __syncthreads();  // red is reused by the next tile
 }
-// A level's sweep, its tiles dealt to the teams of all CTAs, or, on a level
+// A level's sweep, its tiles dealt to all CTAs, or, on a level
 // whose tiles are held in shared memory (tile0 >= 0), every tile by its CTA.
 template <int MODE, bool ZERO>
 __device__ void gb_sweep4(const Level& L, const float* __restrict__ st, const float* u, const float* f, float* out,
                           float omega, const float* up, float c1, int tid, int tile0, const GroupPos& own,
-                          const float* sst, float (*red)[9][12][G9]) {
-  const int team = tid / kTeam, q = (tid - team * kTeam) / G9, tg = tid % G9;
+                          const float* sst, float (*red)[12][G9]) {
+  const int q = tid / G9, tg = tid % G9;
   const long long ng = L.NP / 4, VS = 3 * L.NP;
   if (tile0 >= 0) {
     const int t = (int)blockIdx.x - tile0;
-    if (team != 0 || t < 0 || (long long)t * G9 >= ng) return;
+    if (t < 0 || (long long)t * G9 >= ng) return;
     for (int b = 0; b < L.nb; b++)
       group_step<MODE, ZERO, true>(L, sst, own, u + b * VS, f + b * VS, out + b * VS, omega, up ? up + b * VS : nullptr,
-                                   c1, tg, q, team, red[team]);
+                                   c1, tg, q, red);
     return;
   }
   const long long ngt = ng * L.nb, ntile = (ngt + G9 - 1) / G9;
-  for (long long t = (long long)blockIdx.x * kTeams + team; t < ntile; t += (long long)gridDim.x * kTeams) {
+  for (long long t = blockIdx.x; t < ntile; t += gridDim.x) {
     const long long gg = t * G9 + tg;
     const long long b = gg < ngt ? (long long)((unsigned)gg / (unsigned)ng) : 0;
     const GroupPos P = group_pos(L, gg - b * ng, gg < ngt);
     group_step<MODE, ZERO, false>(L, st, P, u + b * VS, f + b * VS, out + b * VS, omega, up ? up + b * VS : nullptr, c1,
-                                  tg, q, team, red[team]);
+                                  tg, q, red);
   }
 }
 
@@ -1743,21 +1718,28 @@ __device__ __forceinline__ bool tile_landed(uint64_t* bar) {
   return false;
 }
 
-// threads of a CTA of the persistent kernel: the FP32 teams, or one thread per
-// neighbour row of G9 nodes (FP64)
+// threads of a CTA of the persistent kernel: one per neighbour row of G9 groups (FP32) or nodes (FP64)
+constexpr int kGbThreads = 9 * G9;
+// shared exchange of the sweeps: [9][12][G9] floats (FP32), [9][3][G9] doubles (FP64)
 template <typename T>
-constexpr int gb_threads() { return sizeof(T) == 4 ? kTeams * kTeam : 9 * G9; }
-// shared exchange of the sweeps: [teams][9][12][G9] floats (FP32), [9][3][G9] doubles (FP64)
-template <typename T>
-constexpr int gb_smem() { return sizeof(T) == 4 ? kTeams * 9 * 12 * G9 * 4 : 9 * 3 * G9 * (int)sizeof(T); }
+constexpr int gb_smem() { return sizeof(T) == 4 ? 9 * 12 * G9 * 4 : 9 * 3 * G9 * (int)sizeof(T); }
 
+// The same bottom of the V-cycle as one persistent kernel over the whole GPU:
+// a cooperative launch (every CTA resident at once) whose phases are
+// separated by a grid-wide barrier.  FP32 sweeps run on four-node groups with
+// nine threads each and, on the levels that fit, on stencils held in shared
+// memory (above); FP64 sweeps with nine threads per node.  What bounds it is
+// latency: a phase is a barrier and one round of loads.  Per V-cycle, 2 + 2 Chebyshev steps: from
+// the 33^3 level of 256^3 down 174 -> 149 us (33^3 streamed, the rest held),
+// 93 x 71 x 85 110 -> 70 us, 64^3 96 -> 59 us, 49 x 38 x 56 68 -> 37 us (all
+// held), before: two-word barriers, every stencil streamed, two CTAs per SM.
 template <typename T>
-__global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid_constant__ BottomArgs<T> A,
+__global__ void __launch_bounds__(kGbThreads, 1) k_bottom_grid(const __grid_constant__ BottomArgs<T> A,
                                                                     unsigned* bar) {
   __shared__ __align__(16) unsigned char sres[gb_smem<T>()];
   extern __shared__ __align__(128) unsigned char stile[];  // FP32: this CTA's stencil tile
   __shared__ __align__(8) uint64_t tbar;
-  constexpr int NT = gb_threads<T>();
+  constexpr int NT = kGbThreads;
   const int tid = threadIdx.x;
   const int g0 = blockIdx.x * NT + tid, gs = gridDim.x * NT;
   GroupPos own;
@@ -1809,7 +1791,7 @@ __global__ void __launch_bounds__(gb_threads<T>(), 1) k_bottom_grid(const __grid
     if constexpr (sizeof(T) == 4) {
       need_tile(li);
       gb_sweep4<MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, tid, A.tile0[li], own,
-                            reinterpret_cast<const float*>(stile), reinterpret_cast<float (*)[9][12][G9]>(sres));
+                            reinterpret_cast<const float*>(stile), reinterpret_cast<float (*)[12][G9]>(sres));
     } else {
       gb_sweep9<MODE, ZERO>(L, bv_st<T>(L), u, f, out, omega, up, c1, tid, reinterpret_cast<double (*)[3][G9]>(sres));
     }
@@ -2173,7 +2155,7 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
   int occ = occ_cache[ti][dev].load(std::memory_order_relaxed);
   if (occ <= 0) {
     RSO_CHECK_CUDA(h, cudaFuncSetAttribute(k_bottom_grid<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm));
-    RSO_CHECK_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bottom_grid<T>, gb_threads<T>(), dsm));
+    RSO_CHECK_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bottom_grid<T>, kGbThreads, dsm));
     occ_cache[ti][dev].store(occ, std::memory_order_relaxed);
   }
   int sms = 0;
@@ -2181,31 +2163,31 @@ rso_status bottom_vcycle(rso_handle* h, int lb, int pre, int post) {
   const long long most = (long long)occ * sms;
   // FP32: the levels whose stencil tiles are held in shared memory, the
   // smallest first, one tile per CTA; then as many CTAs as hold tiles, or as
-  // the streamed levels have pairs of tiles, or the transfers and the coarsest
+  // the streamed levels have tiles, or the transfers and the coarsest
   // solve have work for
   long long need = 1, held = 0;
   for (int li = 0; li < nl; li++) A.tile0[li] = -1;
   for (int li = nl - 1; li >= lb; li--) {
     const Level& l = h->L[li];
     if (sizeof(T) == 8) {
-      need = std::max<long long>(need, std::max(cdiv(l.nn * l.nb, G9), cdiv(3 * l.nn * l.nb, gb_threads<T>())));
+      need = std::max<long long>(need, std::max(cdiv(l.nn * l.nb, G9), cdiv(3 * l.nn * l.nb, kGbThreads)));
       continue;
     }
     const long long tiles = cdiv(l.NP, ST_TILE);
     if (li == nl - 1) {
-      need = std::max<long long>(need, cdiv(3LL * h->nc * l.nb, gb_threads<T>() / 32));
+      need = std::max<long long>(need, cdiv(3LL * h->nc * l.nb, kGbThreads / 32));
     } else if (held + tiles <= most) {
       A.tile0[li] = (int)held;
       held += tiles;
     } else {
-      need = std::max<long long>(need, cdiv(tiles * l.nb, kTeams));
+      need = std::max<long long>(need, tiles * l.nb);
     }
-    need = std::max<long long>(need, cdiv(3 * l.nn * l.nb, gb_threads<T>()));
+    need = std::max<long long>(need, cdiv(3 * l.nn * l.nb, kGbThreads));
   }
   const int grid = (int)std::max<long long>(1, std::min<long long>(std::max(need, held), most));
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(grid);
-  lc.blockDim = dim3(gb_threads<T>());
+  lc.blockDim = dim3(kGbThreads);
   lc.dynamicSmemBytes = dsm;
   lc.stream = h->stream;
   cudaLaunchAttribute at[1];
@@ -2233,8 +2215,8 @@ __global__ void k_gbar_selftest(unsigned* bar, int rounds, unsigned short_by, lo
 template rso_status bottom_vcycle<double>(rso_handle*, int, int, int);
 template rso_status bottom_vcycle<float>(rso_handle*, int, int, int);
 
-// once per handle: the support mask of every fine element, the list of
-// coarse elements that have support-touching children, and the cuBLAS handle
+// once per handle: the support mask of every fine element, and the list of
+// coarse elements that have support-touching children
 rso_status galerkin_setup(rso_handle* h) {
   if (h->L.size() < 2) return RSO_OK;
   const Level& f = h->L[0];
