@@ -457,7 +457,7 @@ rso_status filter(rso_handle* h, double R, const float* in, float* out, int adjo
 }
 
 // ---------------------------------------------------------------- volume
-// sum of the active elements: a warp per row of elements
+// sum of the active elements: a warp per 256 elements of a row
 constexpr int kSumBlocks = 592;
 __device__ __forceinline__ double warp_add(double v) {
 #pragma unroll
@@ -469,12 +469,14 @@ __global__ void __launch_bounds__(256) k_sum_elems(const Level L, const float* _
   __shared__ double ws[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double s = 0;
-  for (int r = blockIdx.x * 8 + warp; r < L.ey * L.ez; r += gridDim.x * 8) {
+  const int seg = (L.ex + 255) / 256;
+  for (long long i = blockIdx.x * 8 + warp; i < (long long)L.ey * L.ez * seg; i += gridDim.x * 8) {
+    const int r = (int)(i / seg), xa = 256 * (int)(i - (long long)r * seg), xb = min(xa + 256, L.ex);
     const int z = r / L.ey, y = r - z * L.ey;
     const uint8_t* m = L.emask + L.eidx(0, y, z);
     const float* q = a + V.at(0, y, z);
 #pragma unroll 8
-    for (int x = lane; x < L.ex; x += 32) {
+    for (int x = xa + lane; x < xb; x += 32) {
       const float v = q[x];
       s += m[x] ? (double)v : 0.0;
     }
@@ -490,7 +492,7 @@ __global__ void __launch_bounds__(256) k_sum_elems(const Level L, const float* _
 }
 rso_status sum_elems(rso_handle* h, const float* a, bool dense, double* dev_out) {
   const Level& l = h->L[0];
-  const int blocks = std::min(kSumBlocks, cdiv((long long)l.ey * l.ez, 8));
+  const int blocks = std::min(kSumBlocks, cdiv((long long)l.ey * l.ez * cdiv(l.ex, 256), 8));
   k_sum_elems<<<blocks, 256, 0, h->stream>>>(l, a, view_of(l, dense), h->red); rso::note_launch();
   RSO_TRY(launch_check(h, "sum_elems"));
   return reduce_partials(h, h->red, blocks, dev_out);

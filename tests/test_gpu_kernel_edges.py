@@ -865,3 +865,16 @@ def test_filter_and_sums_on_extreme_values(cuda, radius, value):
         step = np.clip(np.nan_to_num((np.tanh(4.0) + np.tanh(s)) / (2 * np.tanh(4.0)), nan=1e-3), 1e-3, 1.0)
     heav = g.projectDensities(x.ravel(), 8.0).cpu().numpy().reshape(em.shape)
     assert np.max(np.abs(heav - np.where(em, step, 0.0))) < 1e-7
+
+
+@pytest.mark.parametrize("dims", [(255, 5, 3), (256, 4, 4), (257, 3, 5), (1030, 3, 2), (16, 70, 70)])
+def test_volume_of_long_rows(cuda, dims):
+    """The volume on rows below, of and past a warp's 256 elements: FP64 sums, 1e-12 relative."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.voids_box(*dims, nvoids=1)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"], Config(n_levels=4, first_factor=2))
+    on = prob["emask"].ravel() > 0
+    x = np.random.default_rng(101).uniform(0.1, 1, g.ne).astype(np.float32)
+    per = g.volumeRatio(np.ones(g.ne, np.float32)) / on.sum()
+    want = x[on].astype(np.float64).sum() * per
+    assert abs(g.volumeRatio(x) - want) <= 1e-12 * want
