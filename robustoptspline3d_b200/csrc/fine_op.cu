@@ -1356,10 +1356,14 @@ static rso_status pair_tensor_maps(rso_handle* h, const Level& l, const float* u
 // fails if a staged-copy wait of the fine kernels gave up since the last call
 // (never in a healthy run); resets the device-wide count
 rso_status fine_stage_check(rso_handle* h) {
-  unsigned int n = 0, zero = 0, gb = 0;
-  RSO_CHECK_CUDA(h, cudaMemcpyFromSymbolAsync(&n, g_stage_timeouts, sizeof(n), 0, cudaMemcpyDeviceToHost, h->stream));
-  if (h->gbar) RSO_CHECK_CUDA(h, cudaMemcpyAsync(&gb, h->gbar + 2, sizeof(gb), cudaMemcpyDeviceToHost, h->stream));
+  // into pinned memory: copies into the stack would wait one by one (20 us of a V-cycle's 250 on a small box)
+  unsigned* flags = reinterpret_cast<unsigned*>(h->h_scal + 60);
+  const unsigned zero = 0;
+  flags[0] = flags[1] = 0;
+  RSO_CHECK_CUDA(h, cudaMemcpyFromSymbolAsync(flags, g_stage_timeouts, sizeof(unsigned), 0, cudaMemcpyDeviceToHost, h->stream));
+  if (h->gbar) RSO_CHECK_CUDA(h, cudaMemcpyAsync(flags + 1, h->gbar + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
   RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
+  const unsigned n = flags[0], gb = flags[1];
   if (gb != 0) {
     // nothing runs on the stream now: the barrier starts afresh
     RSO_CHECK_CUDA(h, cudaMemsetAsync(h->gbar, 0, sizeof(unsigned) * 4, h->stream));
