@@ -606,7 +606,8 @@ static SplineDev spline_dev(rso_handle* h, const float* knots_dev) {
 // coefficients (the rows are nb0 / ex of the elements: 1/8 for 32 coefficients
 // on 256).  D as well as N along z or y gives the rows of the derivatives.
 // Rows outside the knots are zero.
-__global__ void __launch_bounds__(256) k_rows_z(SplineDev S, int ez, const double* __restrict__ c,
+template <typename C>
+__global__ void __launch_bounds__(256) k_rows_z(SplineDev S, int ez, const C* __restrict__ c,
                                                 double* __restrict__ rn, double* __restrict__ rd) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long pl = (long long)S.nb0 * S.nb1;
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(256) k_rows_z(SplineDev S, int ez, const doubl
   double n = 0, d = 0;
   if (k0 >= 0)
     for (int q = 0; q < S.order; q++) {
-      const double v = c[ij + (k0 + q) * pl];
+      const double v = (double)c[ij + (k0 + q) * pl];
       n += v * S.N2[z * S.order + q];
       if (rd) d += v * S.D2[z * S.order + q];
     }
@@ -649,12 +650,14 @@ __global__ void __launch_bounds__(256) k_rows_y(SplineDev S, int ey, int ez, con
   if (rd) { out[t + comp] = dn; out[t + 2 * comp] = nd; }
 }
 
-static rso_status spline_rows(rso_handle* h, const SplineDev& S, const double* c, double* R, bool derivatives) {
+// coefficients in double or float (whose conversion is exact: no pass of its own)
+template <typename C>
+static rso_status spline_rows(rso_handle* h, const SplineDev& S, const C* c, double* R, bool derivatives) {
   const Level& l = h->L[0];
   const long long nz = (long long)S.nb0 * S.nb1 * l.ez, comp = (long long)S.nb0 * l.ey * l.ez;
   double* rn = h->sp.work[1];
   double* rd = derivatives ? rn + nz : nullptr;
-  k_rows_z<<<cdiv(nz, 256), 256, 0, h->stream>>>(S, l.ez, c, rn, rd); rso::note_launch();
+  k_rows_z<C><<<cdiv(nz, 256), 256, 0, h->stream>>>(S, l.ez, c, rn, rd); rso::note_launch();
   k_rows_y<<<cdiv(comp, 256), 256, 0, h->stream>>>(S, l.ey, l.ez, rn, rd, R, comp); rso::note_launch();
   return launch_check(h, "spline rows");
 }
@@ -691,7 +694,8 @@ __global__ void __launch_bounds__(256) k_coeff2density(const Level L, SplineDev 
   }
 }
 
-rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, float* out, bool dense) {
+template <typename C>
+rso_status coeff2density(rso_handle* h, const C* c, const uint8_t* shell, float* out, bool dense) {
   const Level& l = h->L[0];
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
   const SplineDev S = spline_dev(h, h->sp.knots_dev);
@@ -708,6 +712,8 @@ rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, f
   rso::note_launch();
   return launch_check(h, "coeff2density");
 }
+template rso_status coeff2density<double>(rso_handle*, const double*, const uint8_t*, float*, bool);
+template rso_status coeff2density<float>(rso_handle*, const float*, const uint8_t*, float*, bool);
 
 // ---------------------------------------------------------------- separable adjoint
 // Stage 1, x: a warp takes two rows of elements, kSeg elements at a time, their

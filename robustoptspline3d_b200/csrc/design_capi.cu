@@ -104,9 +104,8 @@ extern "C" rso_status rso_spline_axis(rso_handle* h, int axis, int* idx, double*
 extern "C" rso_status rso_coeff2density(rso_handle* h, const float* coeff, const uint8_t* shell, float* rho_hat) {
   if (!h || !coeff || !rho_hat) return RSO_ERR_INVALID_ARG;
   if (!h->sp.order) { h->err = "spline not set up"; return RSO_ERR_STATE; }
-  k_f2d_n<<<cdiv(h->sp.n_coeff, 256), 256, 0, h->stream>>>(coeff, h->coef_a, h->sp.n_coeff); rso::note_launch();
   RSO_TRY(apart(h, &shell, rho_hat, h->e_a));
-  RSO_TRY(coeff2density(h, h->coef_a, shell, rho_hat, true));
+  RSO_TRY(coeff2density(h, coeff, shell, rho_hat, true));
   return finish(h);
 }
 

@@ -219,8 +219,7 @@ extern "C" rso_status rso_oc_update_coeff(rso_handle* h, float* coeff_dev, const
   int itn = 0, trials = 0;
   auto volume_of = [&](const float* c, float* vr) -> rso_status {
     // coeff -> density (the reference's coeff2density), volume over the active elements
-    RSO_TRY(to_f64(h, c, h->coef_a, nc));
-    RSO_TRY(coeff2density(h, h->coef_a, nullptr, h->e_a));
+    RSO_TRY(coeff2density(h, c, nullptr, h->e_a));
     RSO_TRY(sum_elems(h, h->e_a, false, h->scal + 14));
     double s = 0;
     RSO_TRY(read_d(h, h->scal + 14, &s));

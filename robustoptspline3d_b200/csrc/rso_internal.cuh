@@ -497,7 +497,8 @@ rso_status heaviside(rso_handle* h, const float* in, double beta, const uint8_t*
 rso_status heaviside_chain(rso_handle* h, const float* rho, double beta, const float* gin, float* gout,
                            bool dense = false);
 rso_status filter(rso_handle* h, double radius, const float* in, float* out, int adjoint, bool dense = false);
-rso_status coeff2density(rso_handle* h, const double* c, const uint8_t* shell, float* out, bool dense = false);
+template <typename C>
+rso_status coeff2density(rso_handle* h, const C* c, const uint8_t* shell, float* out, bool dense = false);
 rso_status density2coeff(rso_handle* h, const float* g, const uint8_t* shell, double* dc, bool dense = false);
 rso_status selfsupport(rso_handle* h, const double* c, double beta, int mode, double opt_angle,
                        double default_angle, float* per_dense, double* dc, double* value, double* count,
