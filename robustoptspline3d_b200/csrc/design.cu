@@ -29,13 +29,14 @@ static View view_of(const Level& l, bool dense) {
   if (dense) return {0, (long long)l.ex * l.ey, l.ex};
   return {1 + (long long)l.qx * (1 + l.qy), (long long)l.qx * l.qy, l.qx};
 }
-// one thread per element: tiles of 32 x 8 of a plane, whose threads share their neighbours, or, where a fifth of
+// one thread per element: tiles of 32 x 8 of a plane, whose threads share their neighbours, or, where three sevenths of
 // such tiles' threads would lie outside the box, the plane's elements one after another (a block of 256 x 1).  General
-// filter, radius 6: 128^3 elements 3.0 ms in tiles, 3.3 in line; 8 x 8 x 512 elements 0.277 and 0.230, 4 x 16 x 512
-// 0.416 and 0.229.  A launch has at most 65535 planes: the kernels step on.
+// filter, radius 6: 128^3 elements 3.0 ms in tiles, 3.3 in line; 1500 x 6 x 6 0.155 and 0.203; 33 x 40 x 41 0.279 and
+// 0.261; 8 x 8 x 512 0.277 and 0.230; 4 x 16 x 512 0.416 and 0.229.  A launch has at most 65535 planes: the kernels
+// step on.
 static dim3 elem_block(const Level& l) {
   const long long tiles = (long long)cdiv(l.ex, 32) * cdiv(l.ey, 8) * 256;
-  return 4 * tiles <= 5LL * l.ex * l.ey ? dim3(32, 8) : dim3(256, 1);
+  return 4 * tiles <= 7LL * l.ex * l.ey ? dim3(32, 8) : dim3(256, 1);
 }
 static dim3 elem_grid(const Level& l) {
   if (elem_block(l).y > 1) return dim3(cdiv(l.ex, 32), cdiv(l.ey, 8), std::min(l.ez, 65535));
