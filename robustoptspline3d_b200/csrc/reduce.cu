@@ -328,9 +328,14 @@ rso_status zero_support(rso_handle* h, double* padded) {
 }
 
 // ---------------------------------------------------------------- elementwise
-__global__ void k_axpby(long long n, double a, const double* __restrict__ x, double b, double* __restrict__ y) {
+// y = a x + b y; a vector whose factor is zero is not read, so that what a new
+// buffer holds (zero times NaN is NaN) does not reach the result
+__global__ void k_axpby(long long n, double a, const double* x, double b, double* y) {
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < n) y[i] = a * x[i] + b * y[i];
+  if (i >= n) return;
+  if (a == 0) y[i] = b * y[i];
+  else if (b == 0) y[i] = a * x[i];
+  else y[i] = a * x[i] + b * y[i];
 }
 rso_status axpby(rso_handle* h, long long n, double a, const double* x, double b, double* y) {
   k_axpby<<<cdiv(n, 256), 256, 0, h->stream>>>(n, a, x, b, y); rso::note_launch();

@@ -878,3 +878,22 @@ def test_volume_of_long_rows(cuda, dims):
     per = g.volumeRatio(np.ones(g.ne, np.float32)) / on.sum()
     want = x[on].astype(np.float64).sum() * per
     assert abs(g.volumeRatio(x) - want) <= 1e-12 * want
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_worst_case_does_not_read_what_its_scratch_held(cuda, precision):
+    """The Lanczos vectors share their memory with the load projection: what a
+    projected vector left there (here NaN) has no part in the next search."""
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(16, 8, 8)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"],
+                      Config(poisson_ratio=0.4, n_levels=2, first_factor=2, precision=precision))
+    g.set_density(prob["rho"].astype(np.float32).ravel())
+    g.update_stencil()
+    want = g.worst_case(6, 0, 1e-10)
+    assert np.isfinite(want[0]) and bool(cuda.isfinite(want[2]).all())
+    g.forceProject(t(np.full(3 * g.nn, np.nan), cuda), 0)
+    got = g.worst_case(6, 0, 1e-10)
+    assert got[0] == want[0] and bool((got[1] == want[1]).all()) and bool((got[2] == want[2]).all())
+    assert np.array_equal(got[3], want[3])
+    g.close()
