@@ -238,7 +238,8 @@ rso_status rso_ref_numbering(rso_handle* h, int level, int* counts_host, int* gs
 rso_status rso_load_nodes(rso_handle* h, int* nodes_host, int* n_load);
 
 /* ---------------------------------------------------------------- operator and multigrid */
-/* element densities (ex*ey*ez floats, inactive entries ignored); Grid rho_e buffer */
+/* element densities (ex*ey*ez floats, inactive entries ignored); Grid rho_e buffer.
+ * rho_dev has been read when the call returns. */
 rso_status rso_set_density(rso_handle* h, const float* rho_dev);
 /* The current element densities (ex*ey*ez floats, device), the field
  * HierarchyGrid::writeDensity saves (grid/Grid.cpp:1267-1300, there as an

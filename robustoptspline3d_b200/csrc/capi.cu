@@ -374,9 +374,13 @@ extern "C" rso_status rso_level_dims(const rso_handle* h, int level, int* d) {
 // ---------------------------------------------------------------- operator
 extern "C" rso_status rso_set_density(rso_handle* h, const float* rho) {
   if (!h || !rho) return RSO_ERR_INVALID_ARG;
+  h->operators_ready = false;
   RSO_TRY(pad_elems_f(h, rho, h->rho));
   RSO_TRY(penalise(h));
-  h->operators_ready = false;
+  // the caller may free or overwrite rho once the call returns (a captured call runs later: its rho has to stay)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  RSO_CHECK_CUDA(h, cudaStreamIsCapturing(h->stream, &cap));
+  if (cap == cudaStreamCaptureStatusNone) RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
   return RSO_OK;
 }
 
@@ -408,9 +412,7 @@ extern "C" rso_status rso_set_density_points(rso_handle* h, int n, const int32_t
   // staged in a padded element buffer of the handle (at least ex*ey*ez floats)
   float* d = h->e_b;
   RSO_CHECK_CUDA(h, cudaMemcpyAsync(d, dense.data(), sizeof(float) * l0.ne, cudaMemcpyHostToDevice, h->stream));
-  RSO_TRY(rso_set_density(h, d));
-  RSO_CHECK_CUDA(h, cudaStreamSynchronize(h->stream));
-  return RSO_OK;
+  return rso_set_density(h, d);
 }
 
 extern "C" rso_status rso_update_operators(rso_handle* h) {

@@ -897,3 +897,25 @@ def test_worst_case_does_not_read_what_its_scratch_held(cuda, precision):
     assert got[0] == want[0] and bool((got[1] == want[1]).all()) and bool((got[2] == want[2]).all())
     assert np.array_equal(got[3], want[3])
     g.close()
+
+
+def test_set_density_has_read_its_argument(cuda):
+    """The densities are the caller's again once the call returns, also where the handle's stream is behind."""
+    import ctypes
+    from robustoptspline3d_b200 import Config, HierarchyGrid
+    prob = P.cantilever(24, 12, 12)
+    g = HierarchyGrid(prob["emask"], prob["fixed"], prob["load"], prob["normals"], Config(n_levels=2, first_factor=2))
+    stream = cuda.cuda.Stream()
+    assert g.lib.rso_set_stream(g.h, ctypes.c_void_p(stream.cuda_stream)) == 0
+    a = cuda.randn(4096, 4096, device="cuda")
+    rho = cuda.full((g.ne,), 0.25, device="cuda")
+    cuda.cuda.synchronize()
+    with cuda.cuda.stream(stream):
+        for _ in range(20):
+            a = (a @ a) * 1e-4
+    g.set_density(rho)
+    rho.fill_(0.75)
+    cuda.cuda.synchronize()
+    got = g.get_density().cpu().numpy()
+    assert (got[prob["emask"].ravel() > 0] == np.float32(0.25)).all()
+    g.close()
