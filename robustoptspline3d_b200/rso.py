@@ -539,7 +539,7 @@ class HierarchyGrid:
         self._chk(self.lib.rso_set_krylov_fp32_cycles(self.h, int(max_cycles)), "rso_set_krylov_fp32_cycles")
 
     def set_vcycle_graphs(self, on):
-        """Replay captured FP32 V-cycles from CUDA graphs (default) or launch every kernel."""
+        """Replay captured V-cycles from CUDA graphs (default) or launch every kernel."""
         self._chk(self.lib.rso_set_vcycle_graphs(self.h, 1 if on else 0), "rso_set_vcycle_graphs")
 
     def set_fine_zchunk(self, planes=0):
@@ -550,7 +550,7 @@ class HierarchyGrid:
         return int(self.lib.rso_fine_zchunk(self.h))
 
     def set_bottom_kernel(self, kind):
-        """Bottom of the FP32 V-cycle: 1 persistent grid-wide kernel, 0 8-CTA cluster kernel."""
+        """Bottom of the V-cycle: 1 persistent grid-wide kernel, 0 8-CTA cluster kernel."""
         self._chk(self.lib.rso_set_bottom_kernel(self.h, int(kind)), "rso_set_bottom_kernel")
 
     def bottom_kernel(self):
