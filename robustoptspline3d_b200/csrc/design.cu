@@ -458,7 +458,9 @@ rso_status filter(rso_handle* h, double R, const float* in, float* out, int adjo
 }
 
 // ---------------------------------------------------------------- volume
-// sum of the active elements: a warp per 256 elements of a row
+// Sum of the active elements: a warp per row, or per len elements of it (blockIdx.y).
+// Bound by the loads in flight, so 256 elements' are written out: 23 us at 256^3, 29
+// with the loop left to the compiler.
 constexpr int kSumBlocks = 592;
 __device__ __forceinline__ double warp_add(double v) {
 #pragma unroll
@@ -466,18 +468,25 @@ __device__ __forceinline__ double warp_add(double v) {
   return v;
 }
 __global__ void __launch_bounds__(256) k_sum_elems(const Level L, const float* __restrict__ a, const View V,
-                                                   double* __restrict__ part) {
+                                                   int len, double* __restrict__ part) {
   __shared__ double ws[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double s = 0;
-  const int seg = (L.ex + 255) / 256;
-  for (long long i = blockIdx.x * 8 + warp; i < (long long)L.ey * L.ez * seg; i += gridDim.x * 8) {
-    const int r = (int)(i / seg), xa = 256 * (int)(i - (long long)r * seg), xb = min(xa + 256, L.ex);
+  const int xa = blockIdx.y * len, xb = min(xa + len, L.ex);
+  for (int r = blockIdx.x * 8 + warp; r < L.ey * L.ez; r += gridDim.x * 8) {
     const int z = r / L.ey, y = r - z * L.ey;
     const uint8_t* m = L.emask + L.eidx(0, y, z);
     const float* q = a + V.at(0, y, z);
-#pragma unroll 8
-    for (int x = xa + lane; x < xb; x += 32) {
+    int x = xa + lane;
+    for (; x + 224 < xb; x += 256) {
+      float v[8];
+      uint8_t k[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) { v[j] = q[x + 32 * j]; k[j] = m[x + 32 * j]; }
+#pragma unroll
+      for (int j = 0; j < 8; j++) s += k[j] ? (double)v[j] : 0.0;
+    }
+    for (; x < xb; x += 32) {
       const float v = q[x];
       s += m[x] ? (double)v : 0.0;
     }
@@ -488,15 +497,18 @@ __global__ void __launch_bounds__(256) k_sum_elems(const Level L, const float* _
   if (threadIdx.x == 0) {
     double t = 0;
     for (int k = 0; k < 8; k++) t += ws[k];
-    part[blockIdx.x] = t;
+    part[blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
 }
 rso_status sum_elems(rso_handle* h, const float* a, bool dense, double* dev_out) {
   const Level& l = h->L[0];
-  const int blocks = std::min(kSumBlocks, cdiv((long long)l.ey * l.ez * cdiv(l.ex, 256), 8));
-  k_sum_elems<<<blocks, 256, 0, h->stream>>>(l, a, view_of(l, dense), h->red); rso::note_launch();
+  // rows past 256 elements are cut, at most kSumBlocks times: one warp's chain a row
+  // took 6 % of an OC coefficient update on 1500 x 6 x 6
+  const int len = 256 * cdiv(l.ex, 256 * kSumBlocks), cuts = cdiv(l.ex, len);
+  const dim3 grid(std::min(std::max(1, kSumBlocks / cuts), cdiv((long long)l.ey * l.ez, 8)), cuts);
+  k_sum_elems<<<grid, 256, 0, h->stream>>>(l, a, view_of(l, dense), len, h->red); rso::note_launch();
   RSO_TRY(launch_check(h, "sum_elems"));
-  return reduce_partials(h, h->red, blocks, dev_out);
+  return reduce_partials(h, h->red, grid.x * grid.y, dev_out);
 }
 
 rso_status volume(rso_handle* h, const float* rho, double* vol, bool dense) {
